@@ -272,12 +272,13 @@ int ps_rsqrt_check(const double *a, int64_t n, uint64_t *max_ulp, void *stream);
 /* number of kernels the library has launched since it was loaded */
 uint64_t ps_kernel_launches(void);
 /* Autotuner (no counterpart in the reference): times the whole mobility apply
- * of this context (the monomer far-field kernel, whose column-chunk width is
- * tuned, plus the combine that reads one partial sum per chunk) for each width
- * in {128, 256, 512, 1024} (reps applies each, CUDA events) and keeps the
- * fastest for this context and
- * for every context created afterwards in the process.  The width is
- * process-wide so that a replica's arithmetic stays independent of its batch.
+ * of this context (the monomer far-field kernel, whose widest tile edge is
+ * tuned, plus the combine that reads one partial sum per tile) for each widest
+ * edge in {128, 256, 512, 1024} (reps applies each, CUDA events; tiles are at
+ * most 256 wide, so 512 and 1024 stand for no lower limit than 256) and keeps
+ * the fastest for this context and for every context created afterwards in the
+ * process.  The edge is process-wide so that a replica's arithmetic stays
+ * independent of its batch.
  * best_cols / ms (4 timings, candidate order) may be NULL. */
 int ps_autotune(ps_ctx *ctx, int32_t reps, int32_t *best_cols, double *ms, void *stream);
 

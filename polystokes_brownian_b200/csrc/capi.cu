@@ -97,7 +97,7 @@ static int build(Engine &E, const ps_desc *descs, int R, int precision)
     long bead = 0, coll = 0, vec = 0, top = 0, vel = 0, schur = 0, ba = 0, cells = 0, ssinv = 0;
     std::vector<int> bead_offs(R + 1), vec_offs(R + 1), top_offs(R + 1), vel_offs(R + 1);
     std::vector<long> cell_offs(R + 1);
-    std::vector<Tile> aa, ab, bb;
+    std::vector<Tile> ab, bb;
     std::vector<int> schur_reps, ss_reps, sl_reps;
     long slv = 0;
     int ss_polish = 0;
@@ -139,7 +139,6 @@ static int build(Engine &E, const ps_desc *descs, int R, int precision)
         s.lub_bonded = d.lub_bonded;
         s.nper = d.Nmono_per_chain > 0 ? d.Nmono_per_chain : 1;
         s.ss_off = -1;
-        s.nch_aa = std::max(1, (d.Nm + ps::g_aa_chunk_cols - 1) / ps::g_aa_chunk_cols);
         s.nch_bb = std::max(1, std::min(BB_MAX_CHUNKS, (d.Nc + BB_CHUNK_COLS - 1) / BB_CHUNK_COLS));
         if (d.aa_mode == PS_AA_RPY) {
             double b = d.beta, b2 = b * b;
@@ -172,7 +171,6 @@ static int build(Engine &E, const ps_desc *descs, int R, int precision)
         if (d.Nc > 0) ba += (long)s.n_mtiles * d.Nc;
         for (int t = 0; t < s.n_mtiles; t++) {
             Tile tl = {r, t * TR, std::min(TR, d.Nm - t * TR), t};
-            if (d.mm_HI && d.Nm >= 2) aa.push_back(tl);
             if (d.Nc > 0) ab.push_back(tl);
         }
         if (d.Nc >= 2)
@@ -204,12 +202,11 @@ static int build(Engine &E, const ps_desc *descs, int R, int precision)
     auto by_cost = [&](const Tile &a, const Tile &b) {
         return E.segs[a.rep].Np > E.segs[b.rep].Np || (E.segs[a.rep].Np == E.segs[b.rep].Np && a.rep < b.rep);
     };
-    std::stable_sort(aa.begin(), aa.end(), by_cost);
     std::stable_sort(bb.begin(), bb.end(), by_cost);
-    E.n_aa_tiles = (int)aa.size(); E.n_ab_tiles = (int)ab.size(); E.n_bb_tiles = (int)bb.size();
+    E.n_ab_tiles = (int)ab.size(); E.n_bb_tiles = (int)bb.size();
     // grid extent in chunks: the largest per-replica chunk count
-    E.nch_aa = 1; E.nch_bb = 1;
-    for (auto &s : E.segs) { E.nch_aa = std::max(E.nch_aa, s.nch_aa); E.nch_bb = std::max(E.nch_bb, s.nch_bb); }
+    E.nch_bb = 1;
+    for (auto &s : E.segs) E.nch_bb = std::max(E.nch_bb, s.nch_bb);
     E.part_stride = top;
     int rc;
     if ((rc = upload(E.d_segs, E.segs))) return rc;
@@ -218,7 +215,6 @@ static int build(Engine &E, const ps_desc *descs, int R, int precision)
     if ((rc = upload(E.d_vel_offs, vel_offs))) return rc;
     if ((rc = upload(E.d_bead_offs, bead_offs))) return rc;
     if ((rc = upload(E.d_cell_offs, cell_offs))) return rc;
-    if ((rc = upload(E.d_aa_tiles, aa))) return rc;
     if ((rc = upload(E.d_ab_tiles, ab))) return rc;
     if ((rc = upload(E.d_bb_tiles, bb))) return rc;
     if ((rc = upload(E.d_schur_reps, schur_reps))) return rc;
@@ -317,7 +313,7 @@ static int build(Engine &E, const ps_desc *descs, int R, int precision)
     TRY_ALLOC(E.d_pos32lo, sizeof(float4) * bead);
     TRY_ALLOC(E.d_aa_te2, sizeof(float) * std::max<long>(R, 1));
     // pair partials
-    TRY_ALLOC(E.d_partAA, sizeof(double) * top * E.nch_aa);
+    if ((rc = ps::set_aa_chunking(E, ps::g_aa_chunk_cols))) return rc;   // tiles and partials of the monomer far field
     TRY_ALLOC(E.d_partAB, sizeof(double) * top);
     TRY_ALLOC(E.d_partBB, sizeof(double) * top * E.nch_bb);
     TRY_ALLOC(E.d_partBA, sizeof(double) * 11 * std::max<long>(ba, 1));

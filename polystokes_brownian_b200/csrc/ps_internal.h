@@ -90,14 +90,27 @@ struct Seg {
     int lub_bonded;    // lubricate bonded chain neighbours too
     int nper;          // monomers per chain
     int ss_off;        // offset of the inverse stresslet block (nc5^2 doubles), -1 if none
-    int nch_aa, nch_bb; // column chunks of the far-field pair kernels (functions of Nm, Nc alone)
+    int nch_bb;        // column chunks of the colloid far field (a function of Nc alone)
+    int aa_nt;         // tiles of the monomer far field (0: no monomer pairs), and as many partial slots per row
+    long paa_off;      // this replica's monomer far-field partials: aa_nt slots of nm3 doubles
     // monomer-monomer scalars as x = c0/r + c1/r^3, y = c2/r + c3/r^3 (r > 2 beta)
     // and x = c4 + c5 r, y = c6 + c7 r (r <= 2 beta), for the selected aa_mode
     float aa_c[8];
 };
 
-// Column chunk widths of the far-field pair kernels.
-constexpr int AA_CHUNK_COLS = 256;        // default; ps_autotune may pick another, process-wide
+// Tile edge of the monomer far field, a function of the replica's size alone so that its sums
+// do not depend on its batch.  Small edges spread a lone replica over the chip (a tile pair is a
+// block), large ones read and write fewer partial slots and amortise a block's start.  Whole
+// apply of one replica on a B200, FP32 / FP64, us: 985 beads, edge 64 11.0 / 11.7, edge 128 16.6 /
+// 18.5; 2000 beads, 13.0 / 17.8 and 14.3 / 15.9; 4096 beads, 31.6 / 49.3 and 28.8 / 43.1; 8192
+// beads, edge 128 72.9 / 131.9, edge 256 76.1 / 135.3; 16384 beads, 209 / 438 and 206 / 427.
+// ps_autotune may lower the widest edge, process-wide.
+constexpr int AA_TILE_MIN = 64, AA_TILE_MAX = 256;
+constexpr int aa_tile_edge(int Nm) { return Nm <= 1536 ? 64 : (Nm <= 12288 ? 128 : 256); }
+// one tile pair (I <= J) of a replica's monomer far field, edge S
+struct AaTile { int rep, I, J, S; };
+
+// Column chunk widths of the colloid far field.
 constexpr int BB_CHUNK_COLS = 64;        // colloid columns per chunk, for up to BB_MAX_CHUNKS chunks
 constexpr int BB_MAX_CHUNKS = 64;
 

@@ -62,8 +62,9 @@ struct Engine {
     double *d_trapinfo = nullptr;   // per replica: tstop, weaken_trap, unused
 
     // far-field pair work lists
-    Tile *d_aa_tiles = nullptr, *d_ab_tiles = nullptr, *d_bb_tiles = nullptr;
-    int n_aa_tiles = 0, n_ab_tiles = 0, n_bb_tiles = 0, nch_aa = 1, nch_bb = 1;
+    Tile *d_ab_tiles = nullptr, *d_bb_tiles = nullptr;
+    AaTile *d_aa_tiles = nullptr;
+    int n_aa_tiles = 0, n_ab_tiles = 0, n_bb_tiles = 0, nch_bb = 1;
     long part_stride = 0;
     double *d_partAA = nullptr, *d_partAB = nullptr, *d_partBB = nullptr, *d_partBA = nullptr;
     long nba = 0;
@@ -172,9 +173,9 @@ struct Engine {
     void *h_spec = nullptr;                        // pinned copy of the checks' outcomes
 };
 
-// monomer column chunk width of the far-field AA kernels: process-wide (every
-// context of the process chunks a replica the same way, which keeps a replica's
-// arithmetic independent of its batch); set by ps_autotune
+// widest tile edge of the monomer far field: process-wide (every context of the
+// process cuts a replica the same way, which keeps a replica's arithmetic
+// independent of its batch); set by ps_autotune
 extern int g_aa_chunk_cols;
 int set_aa_chunking(Engine &E, int cols);
 

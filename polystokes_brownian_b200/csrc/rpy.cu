@@ -3,13 +3,12 @@
 // y = M u over every replica of the batch, with M the grand mobility that the
 // reference assembles densely into A's top-left block (mm_HI, mob.cpp:843-1160)
 // or applies as the arrowhead shell (matfree_A.cpp:38-80).  Pair tensors are
-// recomputed on the fly from the positions (O(N) memory); the O(N^2) loops are
-// thread-per-row with column tiles staged in shared memory, so every lane of a
-// warp reads the same column entry (a shared-memory broadcast).  Columns are
-// split into chunks across blockIdx.y (AA_CHUNK_COLS monomer or BB_CHUNK_COLS
-// colloid columns per chunk, so the chunking of a replica depends on its own
-// size only); chunk partials are summed in fixed order by k_combine, so results
-// are deterministic and bit-identical whatever else shares the batch.
+// recomputed on the fly from the positions (O(N) memory).  Monomer pairs are
+// taken once each, tile pair by tile pair, and applied to both beads (below);
+// colloid rows sweep column chunks staged in shared memory.  Tiles and chunks
+// of a replica depend on its own size only, and their partial sums are added in
+// fixed order by k_combine, so results are deterministic and bit-identical
+// whatever else shares the batch.
 #include <algorithm>
 #include "ps_internal.h"
 #include "ps_kernels.h"
@@ -19,49 +18,35 @@ namespace ps {
 
 constexpr int RPY_THREADS = 128;
 
-// Compensated accumulator: plain for FP64, Kahan across column tiles for FP32.
-template <class T> struct Acc {
-    T s, c;
-    __device__ __forceinline__ void zero() { s = T(0); c = T(0); }
-    __device__ __forceinline__ void add(T v) { s += v; }
-    __device__ __forceinline__ T get() const { return s; }
-};
-template <> struct Acc<float> {
-    float s, c;
-    __device__ __forceinline__ void zero() { s = 0.f; c = 0.f; }
-    __device__ __forceinline__ void add(float v) {
-        float y = v - c, t = s + y;
-        c = (t - s) - y;
-        s = t;
-    }
-    __device__ __forceinline__ float get() const { return s; }
-};
-
 // ---------------------------------------------------------------------------
-// AA in FP32 with packed FP32x2 arithmetic (sm_100 FFMA2/FADD2/FMUL2), column
-// pairs in the two lanes: a thread owns rows i and i + 64 of a 128-row tile,
-// each held as a broadcast pair (loop-invariant), and advances both against
-// columns (j, j + 1) per step, four pairs per step.  Shared columns are stored
-// pairwise, so the loads deliver every operand pair as it is consumed, with no
-// per-column broadcast: sXY (-x_j, -x_j+1, -y_j, -y_j+1), sZU (-z_j, -z_j+1,
-// u0_j, u0_j+1), sUU (u1_j, u1_j+1, u2_j, u2_j+1); sLA (lo x_j, x_j+1, lo y_j,
-// y_j+1) and sLB (lo z_j, z_j+1, chain_j, chain_j+1) are read inside the exact
-// radius or by CHECK tiles.  An odd tile is padded with a column at 1e18
-// carrying u = 0.  Each row's two lane sums are added once per column tile,
-// then Kahan-summed across tiles.
+// Monomer-monomer far field (AA), each unordered pair once.  The pair block is
+// symmetric, so one evaluation of the geometry serves U_i += M_ij u_j and
+// U_j += M_ij u_i: 32 FMA-pipe operations per unordered pair against 2 x 22 when
+// every row sweeps every column.  The monomers of a replica are cut into tiles of
+// S beads (aa_tile_edge, a function of Nm alone) and a block takes one tile pair
+// (I, J), I <= J; a diagonal tile (I = J) sweeps its ordered pairs row by row.
 //
-// Positions are hi + lo floats.  Separations start as d = hi_i - hi_j, whose
-// error is at most 2^-23 X for a replica whose coordinates stay below X in
-// magnitude; within the replica's exact radius (r <= max(2.1 beta, X / 16), so
-// the hi-only relative error stays below 2^-19 where it is used) the warp adds
-// the low parts, d = (hi_i - hi_j) + (lo_i - lo_j), the same rounding as a full
-// hi + lo difference.  Self pairs and skipped same-chain pairs get rinv = 0,
-// which zeroes their contribution without a branch; the near-overlap form
-// (r <= 2 beta) lies inside the exact radius.  Far form in factored scalars:
-// y = ri (c + d ri^2), (x - y)/r^2 = ri^3 (a + b ri^2), a = c0 - c2, b = c1 - c3,
-// c = c2, d = c3; the near form (r^2 <= (2 beta)^2) overwrites both.
-constexpr int AAF_THREADS = 64;
-constexpr float AAC_PAD = 1e18f;
+// A warp takes cells of 64 rows x 64 columns (FP32, two columns per packed lane
+// pair) or 64 rows x 32 columns (FP64).  Lane l owns rows l and l + 32 in
+// registers and walks the cell's columns on the rotation (l + s) mod 32, s the
+// step, so the 32 lanes always hold 32 different columns: a row's sums stay in
+// its lane, and a column's sums travel with the column, one lane per step, by
+// shuffle -- no atomics, and both sides are summed in a fixed order.  A block's
+// warps split the tile pair into row groups and column groups, and for the
+// smallest edge into bands of steps, so that a replica of a few hundred beads
+// still spreads over the chip; their sums join in shared memory in FP64 in warp
+// order.  The block writes rows I into partial slot J and rows J into slot I, so
+// slot c of a row holds its sum over the columns of tile c, and k_combine adds
+// the slots in order.
+//
+// Bound: the FMA pipe (64 % busy at 16384 beads in FP32, the FP64 pipe 68 % in
+// FP64); what is left is fixed-latency waits at 16 warps per SM (124 and 128
+// registers; 96 registers and 20 warps measured slower, 215 against 198 us).
+// Against a sweep of all ordered pairs (two rows per thread, 256-column chunks),
+// one launch, FP32 / FP64: 516 beads 21.8 -> 4.8 us / 47.0 -> 5.1 us, 4096 beads
+// 32.5 -> 19.4 / 70.6 -> 33.8, 16384 beads 229 -> 198 / 530 -> 420; error against
+// 64-bit sums 1.8e-7 -> 1.1e-7, 1.6e-7 -> 1.4e-7 and 2.2e-7 -> 1.9e-7 in FP32.
+constexpr float AAC_PAD = 1e18f;       // padding columns sit at +AAC_PAD, padding rows at -AAC_PAD, with u = 0
 
 __device__ __forceinline__ float2 f2(float a) { return make_float2(a, a); }
 
@@ -75,37 +60,63 @@ __device__ __forceinline__ void aa_near_lane(bool n, float r2, float ri, float r
     }
 }
 
-template <bool CHECK, bool REF>
-__device__ __forceinline__ void aa_f2_cols(const float4 *__restrict__ sXY, const float4 *__restrict__ sZU,
+// AA in FP32 with packed FP32x2 arithmetic (sm_100 FFMA2/FADD2/FMUL2): rows A
+// and B of a lane as broadcast pairs (loop-invariant), two columns per step in
+// the packed lanes, four unordered pairs per step.  Shared columns are stored
+// pairwise, so the loads deliver every operand pair as it is consumed: sXY
+// (-x_j, -x_j+1, -y_j, -y_j+1), sZU (-z_j, -z_j+1, u0_j, u0_j+1), sUU (u1_j,
+// u1_j+1, u2_j, u2_j+1); sLA (lo x_j, x_j+1, lo y_j, y_j+1) and sLB (lo z_j,
+// z_j+1, chain_j, chain_j+1) are read inside the exact radius or by CHECK tiles.
+//
+// Positions are hi + lo floats.  Separations start as d = hi_i - hi_j, whose
+// error is at most 2^-23 X for a replica whose coordinates stay below X in
+// magnitude; within the replica's exact radius (r <= max(2.1 beta, X / 16), so
+// the hi-only relative error stays below 2^-19 where it is used) the warp adds
+// the low parts, d = (hi_i - hi_j) + (lo_i - lo_j), the same rounding as a full
+// hi + lo difference.  Self pairs and skipped same-chain pairs get rinv = 0,
+// which zeroes their contribution without a branch; the near-overlap form
+// (r <= 2 beta) lies inside the exact radius.  Far form in factored scalars:
+// y = ri (c + d ri^2), (x - y)/r^2 = ri^3 (a + b ri^2), a = c0 - c2, b = c1 - c3,
+// c = c2, d = c3; the near form (r^2 <= (2 beta)^2) overwrites both.
+struct AaRowsF {
+    float2 ax, ay, az, bx, by, bz;     // positions of rows A and B, broadcast
+    float2 au[3], bu[3];               // inputs of rows A and B, broadcast
+    float wA, wB;                      // chain ids
+    int iA, iB, gA, gB;                // replica-local and global bead indices
+};
+
+template <bool SYM, bool CHECK, bool REF>
+__device__ __forceinline__ void aa_f2_cell(const float4 *__restrict__ sXY, const float4 *__restrict__ sZU,
                                            const float4 *__restrict__ sUU, const float4 *__restrict__ sLA,
-                                           const float4 *__restrict__ sLB, int jt, int np, int iA, int iB,
-                                           bool chain_hi, float wA, float wB, float2 ax, float2 ay, float2 az,
-                                           float2 bx, float2 by, float2 bz, const float4 *__restrict__ plo, int bA,
-                                           int bB, float2 fa, float2 fb, float2 fc, float2 fd, const Seg &sg,
-                                           float te2, const double4 *__restrict__ p64, float2 (&t)[6])
+                                           const float4 *__restrict__ sLB, int jc, int s0, int ns, bool chain_hi,
+                                           const AaRowsF &R, const float4 *__restrict__ plo, float2 fa, float2 fb,
+                                           float2 fc, float2 fd, const Seg &sg, float te2,
+                                           const double4 *__restrict__ p64, float2 (&t)[6], float2 (&c)[3])
 {
+    const int lane = threadIdx.x & 31;
+    int k = (lane + s0) & 31;
 #pragma unroll 1
-    for (int k = 0; k < np; k++) {
+    for (int s = 0; s < ns; s++) {
         const float4 XY = sXY[k], ZU = sZU[k], UU = sUU[k];
         float2 dA[3], dB[3];
-        dA[0] = __fadd2_rn(ax, make_float2(XY.x, XY.y)); dA[1] = __fadd2_rn(ay, make_float2(XY.z, XY.w));
-        dA[2] = __fadd2_rn(az, make_float2(ZU.x, ZU.y));
-        dB[0] = __fadd2_rn(bx, make_float2(XY.x, XY.y)); dB[1] = __fadd2_rn(by, make_float2(XY.z, XY.w));
-        dB[2] = __fadd2_rn(bz, make_float2(ZU.x, ZU.y));
+        dA[0] = __fadd2_rn(R.ax, make_float2(XY.x, XY.y)); dA[1] = __fadd2_rn(R.ay, make_float2(XY.z, XY.w));
+        dA[2] = __fadd2_rn(R.az, make_float2(ZU.x, ZU.y));
+        dB[0] = __fadd2_rn(R.bx, make_float2(XY.x, XY.y)); dB[1] = __fadd2_rn(R.by, make_float2(XY.z, XY.w));
+        dB[2] = __fadd2_rn(R.bz, make_float2(ZU.x, ZU.y));
         float2 r2A = __ffma2_rn(dA[2], dA[2], __ffma2_rn(dA[1], dA[1], __fmul2_rn(dA[0], dA[0])));
         float2 r2B = __ffma2_rn(dB[2], dB[2], __ffma2_rn(dB[1], dB[1], __fmul2_rn(dB[0], dB[0])));
         bool eA0 = false, eA1 = false, eB0 = false, eB1 = false;
         if constexpr (CHECK) {
-            const int j = jt + 2 * k;
+            const int j = jc + 2 * k;
             const float4 LB = sLB[k];
-            eA0 = (j == iA) || (chain_hi && wA == LB.z);
-            eA1 = (j + 1 == iA) || (chain_hi && wA == LB.w);
-            eB0 = (j == iB) || (chain_hi && wB == LB.z);
-            eB1 = (j + 1 == iB) || (chain_hi && wB == LB.w);
+            eA0 = (j == R.iA) || (chain_hi && R.wA == LB.z);
+            eA1 = (j + 1 == R.iA) || (chain_hi && R.wA == LB.w);
+            eB0 = (j == R.iB) || (chain_hi && R.wB == LB.z);
+            eB1 = (j + 1 == R.iB) || (chain_hi && R.wB == LB.w);
         }
         const bool inner = __any_sync(0xffffffffu, fminf(fminf(r2A.x, r2A.y), fminf(r2B.x, r2B.y)) <= te2);
         if (inner) {
-            const float4 LA = sLA[k], LB = sLB[k], RA = __ldg(plo + bA), RB = __ldg(plo + bB);
+            const float4 LA = sLA[k], LB = sLB[k], RA = __ldg(plo + R.gA), RB = __ldg(plo + R.gB);
             const float2 cx = make_float2(-LA.x, -LA.y), cy = make_float2(-LA.z, -LA.w), cz = make_float2(-LB.x, -LB.y);
             dA[0] = __fadd2_rn(dA[0], __fadd2_rn(f2(RA.x), cx)); dA[1] = __fadd2_rn(dA[1], __fadd2_rn(f2(RA.y), cy));
             dA[2] = __fadd2_rn(dA[2], __fadd2_rn(f2(RA.z), cz));
@@ -129,21 +140,21 @@ __device__ __forceinline__ void aa_f2_cols(const float4 *__restrict__ sXY, const
                 // the reference's scalars jump at 2 beta (chain bonds often sit there): within a
                 // band of the FP32 test its own FP64 distance decides (RPY is continuous there)
                 const double tb = 2.0 * sg.beta;
-                const int j = jt + 2 * k;
+                const int j = jc + 2 * k;
                 auto decide = [&](bool e, float r2, int bi, int jj, bool &n) {
                     if (e || fabsf(r2 - tb2) > 1e-5f * tb2) return;
                     const double4 P = p64[bi], Q = p64[sg.bead_off + jj];
                     n = !(ref_pair_dist(P.x - Q.x, P.y - Q.y, P.z - Q.z) > tb);
                 };
-                decide(eA0, r2A.x, bA, j, nA0); decide(eA1, r2A.y, bA, j + 1, nA1);
-                decide(eB0, r2B.x, bB, j, nB0); decide(eB1, r2B.y, bB, j + 1, nB1);
+                decide(eA0, r2A.x, R.gA, j, nA0); decide(eA1, r2A.y, R.gA, j + 1, nA1);
+                decide(eB0, r2B.x, R.gB, j, nB0); decide(eB1, r2B.y, R.gB, j + 1, nB1);
             }
             aa_near_lane(nA0, r2A.x, riA.x, ri2A.x, nx0, nx1, ny0, ny1, yA.x, gA.x);
             aa_near_lane(nA1, r2A.y, riA.y, ri2A.y, nx0, nx1, ny0, ny1, yA.y, gA.y);
             aa_near_lane(nB0, r2B.x, riB.x, ri2B.x, nx0, nx1, ny0, ny1, yB.x, gB.x);
             aa_near_lane(nB1, r2B.y, riB.y, ri2B.y, nx0, nx1, ny0, ny1, yB.y, gB.y);
         }
-        // mob_a u = y u + (x - y)(d.u) d / r^2
+        // rows: mob_a u_j = y u_j + (x - y)(d.u_j) d / r^2
         const float2 u0 = make_float2(ZU.z, ZU.w), u1 = make_float2(UU.x, UU.y), u2 = make_float2(UU.z, UU.w);
         const float2 hA = __fmul2_rn(gA, __ffma2_rn(dA[2], u2, __ffma2_rn(dA[1], u1, __fmul2_rn(dA[0], u0))));
         const float2 hB = __fmul2_rn(gB, __ffma2_rn(dB[2], u2, __ffma2_rn(dB[1], u1, __fmul2_rn(dB[0], u0))));
@@ -153,96 +164,136 @@ __device__ __forceinline__ void aa_f2_cols(const float4 *__restrict__ sXY, const
         t[3] = __ffma2_rn(hB, dB[0], __ffma2_rn(yB, u0, t[3]));
         t[4] = __ffma2_rn(hB, dB[1], __ffma2_rn(yB, u1, t[4]));
         t[5] = __ffma2_rn(hB, dB[2], __ffma2_rn(yB, u2, t[5]));
+        if constexpr (SYM) {
+            // columns: the same block applied to the rows' inputs
+            const float2 kA = __fmul2_rn(gA, __ffma2_rn(dA[2], R.au[2], __ffma2_rn(dA[1], R.au[1], __fmul2_rn(dA[0], R.au[0]))));
+            const float2 kB = __fmul2_rn(gB, __ffma2_rn(dB[2], R.bu[2], __ffma2_rn(dB[1], R.bu[1], __fmul2_rn(dB[0], R.bu[0]))));
+#pragma unroll
+            for (int a = 0; a < 3; a++) {
+                c[a] = __ffma2_rn(kB, dB[a], __ffma2_rn(yB, R.bu[a], __ffma2_rn(kA, dA[a], __ffma2_rn(yA, R.au[a], c[a]))));
+                // hand the column's sums to the lane that takes it next
+                c[a].x = __shfl_sync(0xffffffffu, c[a].x, lane + 1);
+                c[a].y = __shfl_sync(0xffffffffu, c[a].y, lane + 1);
+            }
+        }
+        k = (k + 1) & 31;
     }
 }
 
+constexpr int AAF_THREADS = 128;
+
 template <bool REF>
-__global__ void __launch_bounds__(AAF_THREADS, 12)
-k_rpy_aa_f2(const Seg *__restrict__ segs, const Tile *__restrict__ tiles, const float4 *__restrict__ pos,
+__global__ void __launch_bounds__(AAF_THREADS, 4)
+k_rpy_aa_f2(const Seg *__restrict__ segs, const AaTile *__restrict__ tiles, const float4 *__restrict__ pos,
             const float4 *__restrict__ plo, const float *__restrict__ aa_te2, const double4 *__restrict__ p64,
-            const double *__restrict__ u, int in_top, double *__restrict__ part, long part_stride, int nchunk,
-            const char *__restrict__ done, int done_stride)
+            const double *__restrict__ u, int in_top, double *__restrict__ part, const char *__restrict__ done,
+            int done_stride)
 {
     pdl_enter();
-    if (done && *(const int *)(done + (long)tiles[blockIdx.x].rep * done_stride)) return;
-    __shared__ float4 sXY[64], sZU[64], sUU[64], sLA[64], sLB[64];
-    __shared__ float sK[12][AAF_THREADS];     // Kahan sums [0, 6) and compensations [6, 12), thread-private
-    const Tile tl = tiles[blockIdx.x];
+    const AaTile tl = tiles[blockIdx.x];
+    if (done && *(const int *)(done + (long)tl.rep * done_stride)) return;
     const Seg &sg = segs[tl.rep];
-    const int c = blockIdx.y;
-    nchunk = sg.nch_aa;               // per-replica chunk count: a function of Nm alone
-    if (c >= nchunk) return;
     // one instance per pair-scalar family: the reference's scalars take the FP64 branch decision
     if ((sg.aa_mode == PS_AA_REFERENCE) != REF) return;
-    const int Nm = sg.Nm, tid = threadIdx.x;
-    const int j0 = (int)((long)Nm * c / nchunk), j1 = (int)((long)Nm * (c + 1) / nchunk);
-    const int iA = tl.row0 + tid, iB = iA + AAF_THREADS;
-    const bool actA = tid < tl.nrow, actB = tid + AAF_THREADS < tl.nrow;
+    __shared__ float4 sCols[5][AA_TILE_MAX / 2];           // sXY, sZU, sUU, sLA, sLB
+    __shared__ float sCol[3 * 4 * AA_TILE_MAX];            // column sums per row group or band
+    __shared__ double sRow[3 * AA_TILE_MAX];               // row sums per column group or band (3 S slots in all)
+    const int Nm = sg.Nm, S = tl.S, tid = threadIdx.x, lane = tid & 31, w = tid >> 5;
+    const int i0 = tl.I * S, j0 = tl.J * S;
     const int uoff = in_top ? sg.top_off : sg.vec_off;
-    const int bA = sg.bead_off + (actA ? iA : tl.row0), bB = sg.bead_off + (actB ? iB : tl.row0);
-    const float4 PA = pos[bA], PB = pos[bB];
-    const float2 ax = f2(PA.x), ay = f2(PA.y), az = f2(PA.z), bx = f2(PB.x), by = f2(PB.y), bz = f2(PB.z);
-    const bool chain_hi = sg.chain_HI != 0;
+    for (int p = tid; p < S / 2; p += AAF_THREADS) {
+        float4 A[2], B[2];
+        float v[2][3];
+#pragma unroll
+        for (int h = 0; h < 2; h++) {
+            const int j = j0 + 2 * p + h;
+            if (j < Nm) {
+                A[h] = pos[sg.bead_off + j]; B[h] = plo[sg.bead_off + j];
+                for (int a = 0; a < 3; a++) v[h][a] = (float)u[uoff + 3 * j + a];
+            } else {
+                A[h] = make_float4(AAC_PAD, AAC_PAD, AAC_PAD, __int_as_float(0x7fc00000));
+                B[h] = make_float4(0.f, 0.f, 0.f, 0.f);
+                v[h][0] = v[h][1] = v[h][2] = 0.f;
+            }
+        }
+        sCols[0][p] = make_float4(-A[0].x, -A[1].x, -A[0].y, -A[1].y);
+        sCols[1][p] = make_float4(-A[0].z, -A[1].z, v[0][0], v[1][0]);
+        sCols[2][p] = make_float4(v[0][1], v[1][1], v[0][2], v[1][2]);
+        sCols[3][p] = make_float4(B[0].x, B[1].x, B[0].y, B[1].y);
+        sCols[4][p] = make_float4(B[0].z, B[1].z, A[0].w, A[1].w);
+    }
+    // the warp's share: edge 64, one cell in four bands of 8 steps; 128, 2 x 2 cells; 256, one
+    // row group of four cells each
+    const int rg = S == 64 ? 0 : (S == 128 ? w >> 1 : w);
+    const int cg0 = S == 128 ? w & 1 : 0, ncg = S == 256 ? 4 : 1;
+    const int s0 = S == 64 ? 8 * w : 0, ns = S == 64 ? 8 : 32;
+    const int rslot = S == 64 ? w : (S == 128 ? w & 1 : 0), nrslot = S == 64 ? 4 : (S == 128 ? 2 : 1);
+    const int cslot = S == 64 ? w : rg, ncslot = S == 128 ? 2 : 4;
+    AaRowsF R;
+    R.iA = i0 + 64 * rg + lane; R.iB = R.iA + 32;
+    const bool actA = R.iA < Nm, actB = R.iB < Nm;
+    R.gA = sg.bead_off + (actA ? R.iA : i0); R.gB = sg.bead_off + (actB ? R.iB : i0);
+    {
+        const float nan = __int_as_float(0x7fc00000);
+        const float4 pad = make_float4(-AAC_PAD, -AAC_PAD, -AAC_PAD, nan);
+        const float4 PA = actA ? pos[R.gA] : pad, PB = actB ? pos[R.gB] : pad;
+        R.ax = f2(PA.x); R.ay = f2(PA.y); R.az = f2(PA.z); R.bx = f2(PB.x); R.by = f2(PB.y); R.bz = f2(PB.z);
+        R.wA = PA.w; R.wB = PB.w;
+        for (int a = 0; a < 3; a++) {
+            R.au[a] = f2(actA ? (float)u[uoff + 3 * R.iA + a] : 0.f);
+            R.bu[a] = f2(actB ? (float)u[uoff + 3 * R.iB + a] : 0.f);
+        }
+    }
+    const bool chain_hi = sg.chain_HI != 0, diag = tl.I == tl.J;
     const float2 fa = f2(sg.aa_c[0] - sg.aa_c[2]), fb = f2(sg.aa_c[1] - sg.aa_c[3]);
     const float2 fc = f2(sg.aa_c[2]), fd = f2(sg.aa_c[3]);
     const float te2 = aa_te2[tl.rep];
+    double *rs = sRow + 3 * (rslot * S + 64 * rg + lane);  // this thread's own row sums (rows A, then B)
 #pragma unroll
-    for (int q = 0; q < 12; q++) sK[q][tid] = 0.f;
-    for (int jt = j0; jt < j1; jt += 128) {
-        const int nj = min(128, j1 - jt), np = (nj + 1) >> 1;
-        __syncthreads();
-        // one column pair per thread (64 pairs = 128 columns)
-        if (tid < np) {
-            float4 A[2], B[2];
-            float v[2][3];
-            for (int h = 0; h < 2; h++) {
-                const int jl = 2 * tid + h, j = jt + jl;
-                if (jl < nj) {
-                    A[h] = pos[sg.bead_off + j]; B[h] = plo[sg.bead_off + j];
-                    for (int a = 0; a < 3; a++) v[h][a] = (float)u[uoff + 3 * j + a];
-                } else {
-                    A[h] = make_float4(AAC_PAD, AAC_PAD, AAC_PAD, __int_as_float(0x7fc00000));
-                    B[h] = make_float4(0.f, 0.f, 0.f, 0.f);
-                    v[h][0] = v[h][1] = v[h][2] = 0.f;
-                }
-            }
-            sXY[tid] = make_float4(-A[0].x, -A[1].x, -A[0].y, -A[1].y);
-            sZU[tid] = make_float4(-A[0].z, -A[1].z, v[0][0], v[1][0]);
-            sUU[tid] = make_float4(v[0][1], v[1][1], v[0][2], v[1][2]);
-            sLA[tid] = make_float4(B[0].x, B[1].x, B[0].y, B[1].y);
-            sLB[tid] = make_float4(B[0].z, B[1].z, A[0].w, A[1].w);
-        }
-        __syncthreads();
-        float2 t[6] = {f2(0.f), f2(0.f), f2(0.f), f2(0.f), f2(0.f), f2(0.f)};
-        // rows of this tile are [row0, row0 + 128): only overlapping column tiles hold self pairs
-        const bool check = chain_hi || (jt < tl.row0 + 2 * AAF_THREADS && jt + nj > tl.row0);
-        if (check)
-            aa_f2_cols<true, REF>(sXY, sZU, sUU, sLA, sLB, jt, np, iA, iB, chain_hi, PA.w, PB.w, ax, ay, az, bx, by,
-                                  bz, plo, bA, bB, fa, fb, fc, fd, sg, te2, p64, t);
+    for (int a = 0; a < 3; a++) { rs[a] = 0.0; rs[96 + a] = 0.0; }
+    __syncthreads();
+    for (int cg = cg0; cg < cg0 + ncg; cg++) {
+        float2 t[6] = {f2(0.f), f2(0.f), f2(0.f), f2(0.f), f2(0.f), f2(0.f)}, c[3] = {f2(0.f), f2(0.f), f2(0.f)};
+        const int o = 32 * cg, jc = j0 + 64 * cg;
+        if (diag)
+            aa_f2_cell<false, true, REF>(sCols[0] + o, sCols[1] + o, sCols[2] + o, sCols[3] + o, sCols[4] + o, jc, s0,
+                                         ns, chain_hi, R, plo, fa, fb, fc, fd, sg, te2, p64, t, c);
+        else if (chain_hi)
+            aa_f2_cell<true, true, REF>(sCols[0] + o, sCols[1] + o, sCols[2] + o, sCols[3] + o, sCols[4] + o, jc, s0, ns,
+                                        true, R, plo, fa, fb, fc, fd, sg, te2, p64, t, c);
         else
-            aa_f2_cols<false, REF>(sXY, sZU, sUU, sLA, sLB, jt, np, iA, iB, chain_hi, PA.w, PB.w, ax, ay, az, bx, by,
-                                   bz, plo, bA, bB, fa, fb, fc, fd, sg, te2, p64, t);
-        // fold the two column lanes, then Kahan across column tiles
+            aa_f2_cell<true, false, REF>(sCols[0] + o, sCols[1] + o, sCols[2] + o, sCols[3] + o, sCols[4] + o, jc, s0,
+                                         ns, false, R, plo, fa, fb, fc, fd, sg, te2, p64, t, c);
 #pragma unroll
-        for (int q = 0; q < 6; q++) {
-            const float x = t[q].x + t[q].y;
-            const float sq = sK[q][tid], kq = sK[6 + q][tid];
-            const float yy = x - kq, tt = sq + yy;
-            sK[6 + q][tid] = (tt - sq) - yy;
-            sK[q][tid] = tt;
+        for (int a = 0; a < 3; a++) {
+            rs[a] += (double)(t[a].x + t[a].y);
+            rs[96 + a] += (double)(t[3 + a].x + t[3 + a].y);
+        }
+        if (!diag) {
+            float *o3 = sCol + 3 * (cslot * S + 64 * cg + 2 * ((lane + s0 + ns) & 31));
+#pragma unroll
+            for (int a = 0; a < 3; a++) { o3[a] = c[a].x; o3[3 + a] = c[a].y; }
         }
     }
-    double *o = part + (long)c * part_stride + sg.top_off;
-    if (actA) { o[3 * iA] = sK[0][tid]; o[3 * iA + 1] = sK[1][tid]; o[3 * iA + 2] = sK[2][tid]; }
-    if (actB) { o[3 * iB] = sK[3][tid]; o[3 * iB + 1] = sK[4][tid]; o[3 * iB + 2] = sK[5][tid]; }
+    __syncthreads();
+    double *oI = part + sg.paa_off + (long)tl.J * sg.nm3 + 3 * i0, *oJ = part + sg.paa_off + (long)tl.I * sg.nm3 + 3 * j0;
+    for (int e = tid; e < 3 * S; e += AAF_THREADS) {
+        if (3 * i0 + e < sg.nm3) {
+            double v = 0.0;
+            for (int q = 0; q < nrslot; q++) v += sRow[3 * S * q + e];
+            oI[e] = v;
+        }
+        if (!diag && 3 * j0 + e < sg.nm3) {
+            double v = 0.0;
+            for (int q = 0; q < ncslot; q++) v += (double)sCol[3 * S * q + e];
+            oJ[e] = v;
+        }
+    }
 }
 
-// ---------------------------------------------------------------------------
-// AA in FP64, two rows per thread.  A thread owns rows i and i + 64 of a 128-row
-// tile and sweeps 128-column tiles staged in shared memory as (x, y, z, chain)
-// and (u0, u1, u2, 0) double4 pairs, so each column's loads serve both rows.
-// Reciprocal square root: a single-precision seed (the float image taken with integer
-// operations) refined by the second-order
+// AA in FP64: rows l and l + 32 of a 64-row cell in a lane's registers, one
+// column per lane and step.  Reciprocal square root: a single-precision seed (the
+// float image taken with integer operations) refined by the second-order
 // term of the binomial series (1 - e)^(-1/2) = 1 + e/2 + 3 e^2 / 8 + O(e^3),
 // e = 1 - a y0^2 (Householder's iteration of order 2 for f(y) = y^-2 - a): from
 // a seed accurate to 2^-22 the truncation is below 2^-64, so the result is
@@ -251,7 +302,6 @@ k_rpy_aa_f2(const Seg *__restrict__ segs, const Tile *__restrict__ tiles, const 
 // ri = 0, which zeroes their contribution; the near form (r <= 2 beta) is taken
 // under a warp vote.  Far form in factored scalars: y = ri (c + d ri^2),
 // (x - y) / r^2 = ri^3 (a + b ri^2), a = c0 - c2, b = c1 - c3, c = c2, d = c3.
-constexpr int AAD_THREADS = 64;
 
 // Single-precision image of a positive double in [2^-126, 2^128) by exponent re-bias and
 // mantissa truncation (relative error below 2^-23), with integer operations only, so the
@@ -275,111 +325,175 @@ __device__ __forceinline__ double rsqrt_seeded(double a, float af)
 }
 __device__ __forceinline__ double rsqrt_seeded(double a) { return rsqrt_seeded(a, trunc_to_float(a)); }
 
-template <bool CHECK>
-__device__ __forceinline__ void aa_d2_cols(const double4 *__restrict__ sP, const double4 *__restrict__ sU, int jt,
-                                           int nj, int iA, int iB, bool chain_hi, double4 PA, double4 PB, double ca,
-                                           double cb, double cc, double cd, double tb, float tb2f, double n0,
-                                           double n1, double n2, double n3, double (&t)[6])
+struct AaScalD { double ca, cb, cc, cd, tb, n0, n1, n2, n3; float tb2f; };
+
+template <bool SYM, bool CHECK>
+__device__ __forceinline__ void aa_d2_cell(const double2 *__restrict__ sXY, const double2 *__restrict__ sZU,
+                                           const double2 *__restrict__ sUU, const double *__restrict__ sW, int jc, int s0,
+                                           int ns, int iA, int iB, bool chain_hi, const double4 &PA, const double4 &PB,
+                                           const double (&uA)[3], const double (&uB)[3], const AaScalD &K,
+                                           double (&t)[6], double (&c)[3])
 {
+    const int lane = threadIdx.x & 31;
+    int k = (lane + s0) & 31;
 #pragma unroll 1
-    for (int k = 0; k < nj; k++) {
-        const double4 P = sP[k], U = sU[k];
-        const double ax = PA.x - P.x, ay = PA.y - P.y, az = PA.z - P.z;
-        const double bx = PB.x - P.x, by = PB.y - P.y, bz = PB.z - P.z;
+    for (int s = 0; s < ns; s++) {
+        const double2 XY = sXY[k], ZU = sZU[k], UU = sUU[k];
+        const double ax = PA.x - XY.x, ay = PA.y - XY.y, az = PA.z - ZU.x;
+        const double bx = PB.x - XY.x, by = PB.y - XY.y, bz = PB.z - ZU.x;
         const double r2A = fma(az, az, fma(ay, ay, ax * ax));
         const double r2B = fma(bz, bz, fma(by, by, bx * bx));
         bool sA = false, sB = false;
         if constexpr (CHECK) {
-            const int j = jt + k;
-            sA = (j == iA) || (chain_hi && PA.w == P.w);
-            sB = (j == iB) || (chain_hi && PB.w == P.w);
+            const int j = jc + k;
+            sA = (j == iA) || (chain_hi && PA.w == sW[k]);
+            sB = (j == iB) || (chain_hi && PB.w == sW[k]);
         }
         const float fA = trunc_to_float(r2A), fB = trunc_to_float(r2B);
         const double riA = sA ? 0.0 : rsqrt_seeded(r2A, fA), riB = sB ? 0.0 : rsqrt_seeded(r2B, fB);
         const double qA = riA * riA, qB = riB * riB;
-        double yA = riA * fma(cd, qA, cc), yB = riB * fma(cd, qB, cc);
-        double gA = (qA * riA) * fma(cb, qA, ca), gB = (qB * riB) * fma(cb, qB, ca);
+        double yA = riA * fma(K.cd, qA, K.cc), yB = riB * fma(K.cd, qB, K.cc);
+        double gA = (qA * riA) * fma(K.cb, qA, K.ca), gB = (qB * riB) * fma(K.cb, qB, K.ca);
         // candidates for the near form (a single-precision test with a 1e-6 margin, off the FP64
         // pipe); the reference's own distance decides within the band
-        const bool nA = !sA && fA <= tb2f, nB = !sB && fB <= tb2f;
+        const bool nA = !sA && fA <= K.tb2f, nB = !sB && fB <= K.tb2f;
         if (__any_sync(0xffffffffu, nA || nB)) {
             if (nA) {
                 const double r = ref_pair_dist(ax, ay, az);
-                if (!(r > tb)) { const double ri = 1.0 / r, x = fma(n1, r, n0); yA = fma(n3, r, n2); gA = (x - yA) * ri * ri; }
+                if (!(r > K.tb)) { const double ri = 1.0 / r, x = fma(K.n1, r, K.n0); yA = fma(K.n3, r, K.n2); gA = (x - yA) * ri * ri; }
             }
             if (nB) {
                 const double r = ref_pair_dist(bx, by, bz);
-                if (!(r > tb)) { const double ri = 1.0 / r, x = fma(n1, r, n0); yB = fma(n3, r, n2); gB = (x - yB) * ri * ri; }
+                if (!(r > K.tb)) { const double ri = 1.0 / r, x = fma(K.n1, r, K.n0); yB = fma(K.n3, r, K.n2); gB = (x - yB) * ri * ri; }
             }
         }
-        const double hA = gA * fma(az, U.z, fma(ay, U.y, ax * U.x));
-        const double hB = gB * fma(bz, U.z, fma(by, U.y, bx * U.x));
-        t[0] = fma(hA, ax, fma(yA, U.x, t[0]));
-        t[1] = fma(hA, ay, fma(yA, U.y, t[1]));
-        t[2] = fma(hA, az, fma(yA, U.z, t[2]));
-        t[3] = fma(hB, bx, fma(yB, U.x, t[3]));
-        t[4] = fma(hB, by, fma(yB, U.y, t[4]));
-        t[5] = fma(hB, bz, fma(yB, U.z, t[5]));
+        const double hA = gA * fma(az, UU.y, fma(ay, UU.x, ax * ZU.y));
+        const double hB = gB * fma(bz, UU.y, fma(by, UU.x, bx * ZU.y));
+        t[0] = fma(hA, ax, fma(yA, ZU.y, t[0]));
+        t[1] = fma(hA, ay, fma(yA, UU.x, t[1]));
+        t[2] = fma(hA, az, fma(yA, UU.y, t[2]));
+        t[3] = fma(hB, bx, fma(yB, ZU.y, t[3]));
+        t[4] = fma(hB, by, fma(yB, UU.x, t[4]));
+        t[5] = fma(hB, bz, fma(yB, UU.y, t[5]));
+        if constexpr (SYM) {
+            const double kA = gA * fma(az, uA[2], fma(ay, uA[1], ax * uA[0]));
+            const double kB = gB * fma(bz, uB[2], fma(by, uB[1], bx * uB[0]));
+            c[0] = fma(kB, bx, fma(yB, uB[0], fma(kA, ax, fma(yA, uA[0], c[0]))));
+            c[1] = fma(kB, by, fma(yB, uB[1], fma(kA, ay, fma(yA, uA[1], c[1]))));
+            c[2] = fma(kB, bz, fma(yB, uB[2], fma(kA, az, fma(yA, uA[2], c[2]))));
+#pragma unroll
+            for (int a = 0; a < 3; a++) c[a] = __shfl_sync(0xffffffffu, c[a], lane + 1);
+        }
+        k = (k + 1) & 31;
     }
 }
 
-__global__ void __launch_bounds__(AAD_THREADS, 8)
-k_rpy_aa_d2(const Seg *__restrict__ segs, const Tile *__restrict__ tiles, const double4 *__restrict__ pos,
-            const double *__restrict__ u, int in_top, double *__restrict__ part, long part_stride, int nchunk,
-            const char *__restrict__ done, int done_stride)
+constexpr int AAD_THREADS = 256;
+
+__global__ void __launch_bounds__(AAD_THREADS, 2)
+k_rpy_aa_d2(const Seg *__restrict__ segs, const AaTile *__restrict__ tiles, const double4 *__restrict__ pos,
+            const double *__restrict__ u, int in_top, double *__restrict__ part, const char *__restrict__ done,
+            int done_stride)
 {
     pdl_enter();
-    if (done && *(const int *)(done + (long)tiles[blockIdx.x].rep * done_stride)) return;
-    __shared__ double4 sP[128], sU[128];
-    const Tile tl = tiles[blockIdx.x];
+    const AaTile tl = tiles[blockIdx.x];
+    if (done && *(const int *)(done + (long)tl.rep * done_stride)) return;
+    // columns (x, y | z, u0 | u1, u2 | chain), then the row sums in the same space
+    __shared__ double2 sCols[3][AA_TILE_MAX];
+    __shared__ double sW[AA_TILE_MAX], sCol[3 * 4 * AA_TILE_MAX];
+    double *sRow = reinterpret_cast<double *>(sCols);      // row sums per column group or band: 1536 doubles
+    static_assert(sizeof(sCols) >= 1536 * sizeof(double), "row sums alias the columns");
     const Seg &sg = segs[tl.rep];
-    const int c = blockIdx.y;
-    nchunk = sg.nch_aa;               // per-replica chunk count: a function of Nm alone
-    if (c >= nchunk) return;
-    const int Nm = sg.Nm, tid = threadIdx.x;
-    const int j0 = (int)((long)Nm * c / nchunk), j1 = (int)((long)Nm * (c + 1) / nchunk);
-    const int iA = tl.row0 + tid, iB = iA + AAD_THREADS;
-    const bool actA = tid < tl.nrow, actB = tid + AAD_THREADS < tl.nrow;
+    const int Nm = sg.Nm, S = tl.S, tid = threadIdx.x, lane = tid & 31, w = tid >> 5;
+    const int i0 = tl.I * S, j0 = tl.J * S;
     const int uoff = in_top ? sg.top_off : sg.vec_off;
-    const double4 PA = pos[sg.bead_off + (actA ? iA : tl.row0)], PB = pos[sg.bead_off + (actB ? iB : tl.row0)];
-    const bool chain_hi = sg.chain_HI != 0;
-    double c0, c1, c2, c3, n0, n1, n2, n3;
-    if (sg.aa_mode == PS_AA_RPY) {
-        const double b = sg.beta, b2 = b * b;
-        c0 = 1.5; c1 = -b2; c2 = 0.75; c3 = 0.5 * b2;
-        n0 = 1.0 / b; n1 = -0.1875 / b2; n2 = 1.0 / b; n3 = -0.28125 / b2;
-    } else {
-        c0 = 0.375; c1 = -2.0; c2 = 0.75; c3 = -0.5;
-        n0 = -1.0; n1 = 0.375; n2 = 1.0; n3 = -0.28125;
-    }
-    const double tb = 2.0 * sg.beta, ca = c0 - c2, cb = c1 - c3;
-    const float tb2f = (float)(tb * tb * (1.0 + 1e-6));
-    double a[6] = {0, 0, 0, 0, 0, 0};
-    for (int jt = j0; jt < j1; jt += 128) {
-        const int nj = min(128, j1 - jt);
-        __syncthreads();
-        for (int h = 0; h < 2; h++) {
-            const int jl = tid + h * AAD_THREADS;
-            if (jl < nj) {
-                const int j = jt + jl;
-                sP[jl] = pos[sg.bead_off + j];
-                sU[jl] = make_double4(u[uoff + 3 * j], u[uoff + 3 * j + 1], u[uoff + 3 * j + 2], 0.0);
-            }
+    for (int p = tid; p < S; p += AAD_THREADS) {
+        const int j = j0 + p;
+        if (j < Nm) {
+            const double4 P = pos[sg.bead_off + j];
+            const double *v = u + uoff + 3 * j;
+            sCols[0][p] = make_double2(P.x, P.y);
+            sCols[1][p] = make_double2(P.z, v[0]);
+            sCols[2][p] = make_double2(v[1], v[2]);
+            sW[p] = P.w;
+        } else {
+            sCols[0][p] = make_double2(AAC_PAD, AAC_PAD);
+            sCols[1][p] = make_double2(AAC_PAD, 0.0);
+            sCols[2][p] = make_double2(0.0, 0.0);
+            sW[p] = __longlong_as_double(0x7ff8000000000000ll);
         }
-        __syncthreads();
-        double t[6] = {0, 0, 0, 0, 0, 0};
-        // rows of this tile are [row0, row0 + 128): only overlapping column tiles hold self pairs
-        const bool check = chain_hi || (jt < tl.row0 + 2 * AAD_THREADS && jt + nj > tl.row0);
-        if (check)
-            aa_d2_cols<true>(sP, sU, jt, nj, iA, iB, chain_hi, PA, PB, ca, cb, c2, c3, tb, tb2f, n0, n1, n2, n3, t);
-        else
-            aa_d2_cols<false>(sP, sU, jt, nj, iA, iB, chain_hi, PA, PB, ca, cb, c2, c3, tb, tb2f, n0, n1, n2, n3, t);
-#pragma unroll
-        for (int q = 0; q < 6; q++) a[q] += t[q];
     }
-    double *o = part + (long)c * part_stride + sg.top_off;
-    if (actA) { o[3 * iA] = a[0]; o[3 * iA + 1] = a[1]; o[3 * iA + 2] = a[2]; }
-    if (actB) { o[3 * iB] = a[3]; o[3 * iB + 1] = a[4]; o[3 * iB + 2] = a[5]; }
+    // the warp's share: edge 64, one 64 x 32 cell per column group in four bands of 8 steps;
+    // 128, 2 x 4 cells; 256, a row group's four cells of one half of the columns
+    const int rg = S == 64 ? 0 : (S == 128 ? w >> 2 : w >> 1);
+    const int cg0 = S == 64 ? w & 1 : (S == 128 ? w & 3 : 4 * (w & 1)), ncg = S == 256 ? 4 : 1;
+    const int s0 = S == 64 ? 8 * (w >> 1) : 0, ns = S == 64 ? 8 : 32;
+    const int rslot = S == 64 ? w : (S == 128 ? w & 3 : w & 1), nrslot = S == 64 ? 8 : (S == 128 ? 4 : 2);
+    const int cslot = S == 64 ? w >> 1 : rg, ncslot = S == 128 ? 2 : 4;
+    const int iA = i0 + 64 * rg + lane, iB = iA + 32;
+    const bool actA = iA < Nm, actB = iB < Nm;
+    const double4 pad = make_double4(-AAC_PAD, -AAC_PAD, -AAC_PAD, __longlong_as_double(0x7ff8000000000000ll));
+    const double4 PA = actA ? pos[sg.bead_off + iA] : pad, PB = actB ? pos[sg.bead_off + iB] : pad;
+    double uA[3], uB[3];
+    for (int a = 0; a < 3; a++) {
+        uA[a] = actA ? u[uoff + 3 * iA + a] : 0.0;
+        uB[a] = actB ? u[uoff + 3 * iB + a] : 0.0;
+    }
+    const bool chain_hi = sg.chain_HI != 0, diag = tl.I == tl.J;
+    AaScalD K;
+    {
+        double c0, c1, c2, c3;
+        if (sg.aa_mode == PS_AA_RPY) {
+            const double b = sg.beta, b2 = b * b;
+            c0 = 1.5; c1 = -b2; c2 = 0.75; c3 = 0.5 * b2;
+            K.n0 = 1.0 / b; K.n1 = -0.1875 / b2; K.n2 = 1.0 / b; K.n3 = -0.28125 / b2;
+        } else {
+            c0 = 0.375; c1 = -2.0; c2 = 0.75; c3 = -0.5;
+            K.n0 = -1.0; K.n1 = 0.375; K.n2 = 1.0; K.n3 = -0.28125;
+        }
+        K.tb = 2.0 * sg.beta; K.ca = c0 - c2; K.cb = c1 - c3; K.cc = c2; K.cd = c3;
+        K.tb2f = (float)(K.tb * K.tb * (1.0 + 1e-6));
+    }
+    __syncthreads();
+    double racc[6] = {0, 0, 0, 0, 0, 0};
+    for (int cg = cg0; cg < cg0 + ncg; cg++) {
+        double c[3] = {0, 0, 0};
+        const int o = 32 * cg, jc = j0 + o;
+        if (diag)
+            aa_d2_cell<false, true>(sCols[0] + o, sCols[1] + o, sCols[2] + o, sW + o, jc, s0, ns, iA, iB, chain_hi, PA,
+                                    PB, uA, uB, K, racc, c);
+        else if (chain_hi)
+            aa_d2_cell<true, true>(sCols[0] + o, sCols[1] + o, sCols[2] + o, sW + o, jc, s0, ns, iA, iB, true, PA, PB,
+                                   uA, uB, K, racc, c);
+        else
+            aa_d2_cell<true, false>(sCols[0] + o, sCols[1] + o, sCols[2] + o, sW + o, jc, s0, ns, iA, iB, false, PA, PB,
+                                    uA, uB, K, racc, c);
+        if (!diag) {
+            double *o3 = sCol + 3 * (cslot * S + o + ((lane + s0 + ns) & 31));
+#pragma unroll
+            for (int a = 0; a < 3; a++) o3[a] = c[a];
+        }
+    }
+    __syncthreads();                                       // the columns have been read
+    {
+        double *o3 = sRow + 3 * (rslot * S + 64 * rg + lane);
+#pragma unroll
+        for (int a = 0; a < 3; a++) { o3[a] = racc[a]; o3[96 + a] = racc[3 + a]; }
+    }
+    __syncthreads();
+    double *oI = part + sg.paa_off + (long)tl.J * sg.nm3 + 3 * i0, *oJ = part + sg.paa_off + (long)tl.I * sg.nm3 + 3 * j0;
+    for (int e = tid; e < 3 * S; e += AAD_THREADS) {
+        if (3 * i0 + e < sg.nm3) {
+            double v = 0.0;
+            for (int q = 0; q < nrslot; q++) v += sRow[3 * S * q + e];
+            oI[e] = v;
+        }
+        if (!diag && 3 * j0 + e < sg.nm3) {
+            double v = 0.0;
+            for (int q = 0; q < ncslot; q++) v += sCol[3 * S * q + e];
+            oJ[e] = v;
+        }
+    }
 }
 
 // max |own - CUDA| / ulp(CUDA) of the reciprocal square root over a[0..n)
@@ -603,7 +717,7 @@ __device__ __forceinline__ int find_rep(const int *__restrict__ offs, int R, lon
 // (a single large replica otherwise leaves most SMs idle while every thread
 // walks its chunk partials four times over).
 __global__ void k_combine(const Seg *__restrict__ segs, RedTable T, int mode, const double *__restrict__ x,
-                          const double *__restrict__ scale, const double *__restrict__ partAA, int nchAA,
+                          const double *__restrict__ scale, const double *__restrict__ partAA, int with_aa,
                           const double *__restrict__ partAB, const double *__restrict__ partBB, int nchBB,
                           const double *__restrict__ partBA, const double *__restrict__ delta,
                           const double *__restrict__ lub_y, long part_stride, double *__restrict__ y,
@@ -623,10 +737,10 @@ __global__ void k_combine(const Seg *__restrict__ segs, RedTable T, int mode, co
         if (i < sg.nm3nc11) {
             if (i < sg.nm3) {
                 v = sg.beta_inv * x[xo + i];
-                if (sg.mm_HI) {
-                    const int nc = nchAA ? sg.nch_aa : 0;
+                if (with_aa) {
+                    const double *pa = partAA + sg.paa_off + i;      // one slot per column tile
 #pragma unroll 8
-                    for (int c = 0; c < nc; c++) v += partAA[(long)c * part_stride + sg.top_off + i];
+                    for (int c = 0; c < sg.aa_nt; c++) v += pa[(long)c * sg.nm3];
                 }
                 if (sg.Nc > 0) v += partAB[sg.top_off + i];
             } else {
@@ -686,17 +800,15 @@ void launch_pairs(Engine &E, const double *u, int in_top, cudaStream_t st, const
         if constexpr (sizeof(T) == 4)
         {
             if (E.any_aa_rpy)
-                ps_launch(k_rpy_aa_f2<false>, dim3(E.n_aa_tiles, E.nch_aa), AAF_THREADS, 0, st,
-                        E.d_segs, E.d_aa_tiles, E.d_pos32, E.d_pos32lo, E.d_aa_te2, E.d_pos64, u, in_top, E.d_partAA,
-                        E.part_stride, E.nch_aa, done, dstride);
+                ps_launch(k_rpy_aa_f2<false>, E.n_aa_tiles, AAF_THREADS, 0, st, E.d_segs, E.d_aa_tiles, E.d_pos32,
+                        E.d_pos32lo, E.d_aa_te2, E.d_pos64, u, in_top, E.d_partAA, done, dstride);
             if (E.any_aa_ref)
-                ps_launch(k_rpy_aa_f2<true>, dim3(E.n_aa_tiles, E.nch_aa), AAF_THREADS, 0, st,
-                        E.d_segs, E.d_aa_tiles, E.d_pos32, E.d_pos32lo, E.d_aa_te2, E.d_pos64, u, in_top, E.d_partAA,
-                        E.part_stride, E.nch_aa, done, dstride);
+                ps_launch(k_rpy_aa_f2<true>, E.n_aa_tiles, AAF_THREADS, 0, st, E.d_segs, E.d_aa_tiles, E.d_pos32,
+                        E.d_pos32lo, E.d_aa_te2, E.d_pos64, u, in_top, E.d_partAA, done, dstride);
         }
         else
-            ps_launch(k_rpy_aa_d2, dim3(E.n_aa_tiles, E.nch_aa), AAD_THREADS, 0, st,
-                    E.d_segs, E.d_aa_tiles, E.d_pos64, u, in_top, E.d_partAA, E.part_stride, E.nch_aa, done, dstride);
+            ps_launch(k_rpy_aa_d2, E.n_aa_tiles, AAD_THREADS, 0, st,
+                    E.d_segs, E.d_aa_tiles, E.d_pos64, u, in_top, E.d_partAA, done, dstride);
     }
     if (E.n_ab_tiles)
         ps_launch(k_rpy_ab<T>, E.n_ab_tiles, RPY_THREADS, 0, ss, E.d_segs, E.d_ab_tiles, pos, E.d_pos32lo, u, in_top, E.d_tab, E.d_partAB,
@@ -728,26 +840,43 @@ void apply_operator(Engine &E, int mode, const double *x, double *y, const doubl
     }
     const RedTable &T = mode == 0 ? E.red : E.red_top;
     ps_launch(k_combine, dim3((unsigned)T.nblk, RB_EPT), RB_THREADS, 0, st,
-            E.d_segs, T, mode, x, scale, E.d_partAA, skip_aa ? 0 : E.nch_aa, E.d_partAB, E.d_partBB, E.nch_bb,
+            E.d_segs, T, mode, x, scale, E.d_partAA, skip_aa ? 0 : 1, E.d_partAB, E.d_partBB, E.nch_bb,
             E.d_partBA, E.d_delta, lub_y, E.part_stride, y, dn, done_stride);
 }
 
 
-int g_aa_chunk_cols = AA_CHUNK_COLS;
+int g_aa_chunk_cols = AA_TILE_MAX;
 
-// re-chunk the monomer far field of a context: per-replica chunk counts, the
-// grid extent and the partial buffer
+// tiles of the monomer far field for a widest edge of `cols`: per-replica edges and
+// partial slots, the list of tile pairs (large tiles first) and the partial buffer
 int set_aa_chunking(Engine &E, int cols)
 {
-    E.nch_aa = 1;
-    for (auto &s : E.segs) {
-        s.nch_aa = std::max(1, (s.Nm + cols - 1) / cols);
-        E.nch_aa = std::max(E.nch_aa, s.nch_aa);
+    std::vector<AaTile> tiles;
+    long off = 0;
+    for (int r = 0; r < E.R; r++) {
+        Seg &s = E.segs[r];
+        const bool on = s.mm_HI && s.Nm >= 2;
+        const int S = std::min(aa_tile_edge(s.Nm), std::max(cols, AA_TILE_MIN));
+        s.aa_nt = on ? (s.Nm + S - 1) / S : 0;
+        s.paa_off = off;
+        off += (long)s.aa_nt * s.nm3;
+        for (int i = 0; i < s.aa_nt; i++)
+            for (int j = i; j < s.aa_nt; j++) tiles.push_back({r, i, j, S});
     }
+    std::stable_sort(tiles.begin(), tiles.end(), [](const AaTile &a, const AaTile &b) { return a.S > b.S; });
+    E.n_aa_tiles = (int)tiles.size();
     PS_CK(cudaDeviceSynchronize());
     cudaFree(E.d_partAA);
+    cudaFree(E.d_aa_tiles);
     E.d_partAA = nullptr;
-    PS_CK(cudaMalloc(&E.d_partAA, sizeof(double) * std::max<long>(E.ntop, 1) * E.nch_aa));
+    E.d_aa_tiles = nullptr;
+    if (cudaMalloc(&E.d_partAA, sizeof(double) * std::max<long>(off, 1)) != cudaSuccess ||
+        cudaMalloc(&E.d_aa_tiles, sizeof(AaTile) * std::max<size_t>(tiles.size(), 1)) != cudaSuccess) {
+        set_error(std::string("monomer far-field partial sums: ") + cudaGetErrorString(cudaGetLastError()));
+        return PS_ERR_NOMEM;
+    }
+    if (!tiles.empty())
+        PS_CK(cudaMemcpy(E.d_aa_tiles, tiles.data(), sizeof(AaTile) * tiles.size(), cudaMemcpyHostToDevice));
     PS_CK(cudaMemcpy(E.d_segs, E.segs.data(), sizeof(Seg) * E.segs.size(), cudaMemcpyHostToDevice));
     return PS_OK;
 }
@@ -765,10 +894,10 @@ int time_pairs(Engine &E, int which, int reps, const double *u, double *ms, cuda
     auto launch = [&]() {
         if (which == 0 && E.n_aa_tiles) {
             if (fp32) {
-                if (E.any_aa_rpy) ps_launch(k_rpy_aa_f2<false>, dim3(E.n_aa_tiles, E.nch_aa), AAF_THREADS, 0, st, E.d_segs, E.d_aa_tiles, (const float4 *)pos, E.d_pos32lo, E.d_aa_te2, E.d_pos64, u, 1, E.d_partAA, E.part_stride, E.nch_aa, nullptr, 0);
-                if (E.any_aa_ref) ps_launch(k_rpy_aa_f2<true>, dim3(E.n_aa_tiles, E.nch_aa), AAF_THREADS, 0, st, E.d_segs, E.d_aa_tiles, (const float4 *)pos, E.d_pos32lo, E.d_aa_te2, E.d_pos64, u, 1, E.d_partAA, E.part_stride, E.nch_aa, nullptr, 0);
+                if (E.any_aa_rpy) ps_launch(k_rpy_aa_f2<false>, E.n_aa_tiles, AAF_THREADS, 0, st, E.d_segs, E.d_aa_tiles, (const float4 *)pos, E.d_pos32lo, E.d_aa_te2, E.d_pos64, u, 1, E.d_partAA, nullptr, 0);
+                if (E.any_aa_ref) ps_launch(k_rpy_aa_f2<true>, E.n_aa_tiles, AAF_THREADS, 0, st, E.d_segs, E.d_aa_tiles, (const float4 *)pos, E.d_pos32lo, E.d_aa_te2, E.d_pos64, u, 1, E.d_partAA, nullptr, 0);
             }
-            else ps_launch(k_rpy_aa_d2, dim3(E.n_aa_tiles, E.nch_aa), AAD_THREADS, 0, st, E.d_segs, E.d_aa_tiles, E.d_pos64, u, 1, E.d_partAA, E.part_stride, E.nch_aa, nullptr, 0);
+            else ps_launch(k_rpy_aa_d2, E.n_aa_tiles, AAD_THREADS, 0, st, E.d_segs, E.d_aa_tiles, E.d_pos64, u, 1, E.d_partAA, nullptr, 0);
         } else if (which == 1 && E.n_ab_tiles) {
             if (fp32) ps_launch(k_rpy_ab<float>, E.n_ab_tiles, RPY_THREADS, 0, st, E.d_segs, E.d_ab_tiles, (const float4 *)pos, E.d_pos32lo, u, 1, E.d_tab, E.d_partAB, E.d_partBA, nullptr, 0);
             else ps_launch(k_rpy_ab<double>, E.n_ab_tiles, RPY_THREADS, 0, st, E.d_segs, E.d_ab_tiles, (const double4 *)pos, E.d_pos32lo, u, 1, E.d_tab, E.d_partAB, E.d_partBA, nullptr, 0);

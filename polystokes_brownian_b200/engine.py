@@ -117,7 +117,7 @@ class Batch:
         return t, k, xp[: 3 * self.ncoll]
 
     def autotune(self, reps: int = 5):
-        """Pick the monomer far-field column-chunk width for this process (ps_autotune);
+        """Pick the widest tile edge of the monomer far field for this process (ps_autotune);
         returns (width, {width: ms per mobility apply, combine included})."""
         best = C.c_int32(0)
         ms = (C.c_double * 4)()

@@ -14,7 +14,7 @@ arrivals are admitted, and finished trajectories retired, between steps:
   * when the active set changes the context is rebuilt over the new set and the
     continuing trajectories carry their state across: positions, quaternions,
     time, trap constant and centres, and their own noise stream (seed and step
-    counter) -- the kernels are per-replica deterministic (column chunking,
+    counter) -- the kernels are per-replica deterministic (far-field tiles,
     reductions and Philox streams depend on the replica alone), so a trajectory
     ends bit-identical whether it ran alone or in any mix;
   * to amortise rebuilds a finished trajectory's result is taken at its last
@@ -76,14 +76,19 @@ class _Slot:
     result: Result | None = None
 
 
+# (largest monomer count, tile edge) of the monomer far field
+AA_TILE_EDGES = ((1536, 64), (12288, 128), (math.inf, 256))
+
+
 def footprint_bytes(sysm: System, precision: int = _capi.PS_PREC_MIXED, lanczos_kmax: int = 64) -> int:
     """Device bytes one replica holds in a context: saddle vectors (13), mobility
-    vectors incl. the Lanczos basis (kmax + 6) and far-field chunk partials,
+    vectors incl. the Lanczos basis (kmax + 6), far-field partials (one slot per
+    monomer tile, AA_TILE_EDGES as aa_tile_edge in csrc/ps_internal.h),
     velocity vectors (27), positions, lists."""
     p = sysm.params
     Nm, Nc = p["Nm"], p["Nc"]
     n, top, vel, Np = 6 * Nm + 17 * Nc, 3 * Nm + 11 * Nc, 3 * Nm + 6 * Nc, Nm + Nc
-    nch = max(1, math.ceil(Nm / 256))
+    nch = max(1, math.ceil(Nm / next(e for n_max, e in AA_TILE_EDGES if Nm <= n_max)))
     b = 8 * (13 * n + (lanczos_kmax + 6 + nch) * top + 27 * vel) + 160 * Np + 4 * 16 * Np
     if Nc and 5 * Nc <= 64:
         b += 8 * (5 * Nc) ** 2
