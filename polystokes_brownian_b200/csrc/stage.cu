@@ -639,66 +639,148 @@ __global__ void k_assemble(int R, const Seg *__restrict__ segs, const double *__
 // S = Mcc_base - beta Mcm Mcm^T, eig, delta_j = max(0.1 - lambda_j, 0),
 // Delta = Q diag(delta) Q^T; Mcc_base holds the colloid self blocks plus the
 // colloid-colloid pair blocks (those the reference's shell cannot store).
-// Symmetric eigendecomposition by cyclic Jacobi in shared memory.
+// Symmetric eigendecomposition by parallel-ordered Jacobi in shared memory.
+//
+// Bound: latency (one block per replica, n <= 64).  The pair blocks of Mcm are
+// evaluated once per (monomer, colloid), a chunk of monomers at a time in shared
+// memory, and every thread then adds the chunk to its Gram entries; a Jacobi
+// sweep is n - 1 rounds of n / 2 disjoint rotations.  220 monomers and 2
+// colloids (n = 22): 2090 us with the blocks re-evaluated for every Gram entry and
+// one rotation at a time, 147 us now.
+constexpr int SCHUR_THREADS = 512;
+constexpr int SCHUR_BUF = 12288;      // doubles of the monomer chunk: 3 n per monomer
+
+// One sweep runs the round-robin schedule: with m = n rounded up to even, round t pairs
+// (m - 1, t) and ((t + k) mod (m - 1), (t - k) mod (m - 1)), k = 1 .. m/2 - 1; a pair that
+// holds the padding index rests.  The rotations of a round are disjoint, so each 2 x 2 block
+// (pair, pair) of A is rotated from both sides by one thread, and each row of Q by pairs.
+__device__ __forceinline__ void jacobi_pair(int m, int t, int k, int &p, int &q)
+{
+    int a, b;
+    if (k == 0) { a = m - 1; b = t; }
+    else {
+        a = t + k; if (a >= m - 1) a -= m - 1;
+        b = t - k; if (b < 0) b += m - 1;
+    }
+    p = a < b ? a : b;
+    q = a < b ? b : a;
+}
+
 __device__ void block_jacobi_eig(double *A, double *Q, int n, double *lam)
 {
     // A, Q: n x n row-major in shared memory; all threads of the block participate
-    for (int k = threadIdx.x; k < n * n; k += blockDim.x) Q[k] = (k / n == k % n) ? 1.0 : 0.0;
-    __shared__ double cs_sh[2];
-    __shared__ int conv;
+    __shared__ double rc[PS_MAX_NC11_SCHUR / 2], rs[PS_MAX_NC11_SCHUR / 2];
+    __shared__ double wsum[2][SCHUR_THREADS / 32];
+    const int tid = threadIdx.x, lane = tid & 31, wid = tid >> 5;
+    const int m = (n + 1) & ~1, np = m / 2;
+    for (int k = tid; k < n * n; k += blockDim.x) Q[k] = (k / n == k % n) ? 1.0 : 0.0;
     __syncthreads();
     for (int sweep = 0; sweep < 60; sweep++) {
-        if (threadIdx.x == 0) {
-            double off = 0, tot = 0;
-            for (int i = 0; i < n; i++) for (int j = 0; j < n; j++) { double v = A[i * n + j] * A[i * n + j]; tot += v; if (i != j) off += v; }
-            conv = (off <= 1e-30 * tot || off == 0.0);
+        double off = 0.0, tot = 0.0;
+        for (int k = tid; k < n * n; k += blockDim.x) {
+            const double v = A[k] * A[k];
+            tot += v;
+            if (k / n != k % n) off += v;
         }
+        for (int o = 16; o > 0; o >>= 1) {
+            off += __shfl_xor_sync(0xffffffffu, off, o);
+            tot += __shfl_xor_sync(0xffffffffu, tot, o);
+        }
+        if (lane == 0) { wsum[0][wid] = off; wsum[1][wid] = tot; }
         __syncthreads();
-        if (conv) break;
-        for (int p = 0; p < n - 1; p++)
-            for (int q = p + 1; q < n; q++) {
-                if (threadIdx.x == 0) {
-                    double apq = A[p * n + q];
-                    if (fabs(apq) < 1e-300) { cs_sh[0] = 1.0; cs_sh[1] = 0.0; }
-                    else {
-                        double theta = (A[q * n + q] - A[p * n + p]) / (2 * apq);
-                        double t = (theta >= 0 ? 1.0 : -1.0) / (fabs(theta) + sqrt(theta * theta + 1));
-                        double c = 1 / sqrt(t * t + 1);
-                        cs_sh[0] = c; cs_sh[1] = t * c;
+        off = 0.0; tot = 0.0;
+        for (int w = 0; w < (int)(blockDim.x >> 5); w++) { off += wsum[0][w]; tot += wsum[1][w]; }
+        if (off <= 1e-30 * tot || off == 0.0) break;      // the same sums in every thread
+        for (int t = 0; t < m - 1; t++) {
+            if (tid < np) {
+                int p, q;
+                jacobi_pair(m, t, tid, p, q);
+                double c = 1.0, sn = 0.0;
+                if (q < n) {
+                    const double apq = A[p * n + q];
+                    if (fabs(apq) >= 1e-300) {
+                        // tan of the rotation: 2 apq / (h +- sqrt(h^2 + 4 apq^2)), h = aqq - app
+                        const double h = A[q * n + q] - A[p * n + p], g = 2 * apq;
+                        const double tn = (h >= 0 ? g : -g) / (fabs(h) + sqrt(h * h + g * g));
+                        c = rsqrt(tn * tn + 1);
+                        sn = tn * c;
                     }
                 }
-                __syncthreads();
-                double c = cs_sh[0], sn = cs_sh[1];
-                if (sn != 0.0) {
-                    for (int k = threadIdx.x; k < n; k += blockDim.x) {
-                        double akp = A[k * n + p], akq = A[k * n + q];
-                        A[k * n + p] = c * akp - sn * akq; A[k * n + q] = sn * akp + c * akq;
-                    }
-                    __syncthreads();
-                    for (int k = threadIdx.x; k < n; k += blockDim.x) {
-                        double apk = A[p * n + k], aqk = A[q * n + k];
-                        A[p * n + k] = c * apk - sn * aqk; A[q * n + k] = sn * apk + c * aqk;
-                        double qkp = Q[k * n + p], qkq = Q[k * n + q];
-                        Q[k * n + p] = c * qkp - sn * qkq; Q[k * n + q] = sn * qkp + c * qkq;
-                    }
-                }
-                __syncthreads();
+                rc[tid] = c; rs[tid] = sn;
             }
+            __syncthreads();
+            for (int w = tid; w < np * np + np * n; w += blockDim.x) {
+                if (w < np * np) {
+                    // block of row pair k1 and column pair k2: B <- J1^T B J2
+                    const int k1 = w / np, k2 = w % np;
+                    int p1, q1, p2, q2;
+                    jacobi_pair(m, t, k1, p1, q1);
+                    jacobi_pair(m, t, k2, p2, q2);
+                    const double c1 = rc[k1], s1 = rs[k1], c2 = rc[k2], s2 = rs[k2];
+                    const bool h1 = q1 < n, h2 = q2 < n;
+                    double app = A[p1 * n + p2], apq = h2 ? A[p1 * n + q2] : 0.0;
+                    double aqp = h1 ? A[q1 * n + p2] : 0.0, aqq = h1 && h2 ? A[q1 * n + q2] : 0.0;
+                    const double bpp = c2 * app - s2 * apq, bpq = s2 * app + c2 * apq;
+                    const double bqp = c2 * aqp - s2 * aqq, bqq = s2 * aqp + c2 * aqq;
+                    A[p1 * n + p2] = c1 * bpp - s1 * bqp;
+                    if (h2) A[p1 * n + q2] = c1 * bpq - s1 * bqq;
+                    if (h1) A[q1 * n + p2] = s1 * bpp + c1 * bqp;
+                    if (h1 && h2) A[q1 * n + q2] = s1 * bpq + c1 * bqq;
+                } else {
+                    const int v = w - np * np, k = v / n, row = v % n;
+                    int p, q;
+                    jacobi_pair(m, t, k, p, q);
+                    if (q < n) {
+                        const double c = rc[k], sn = rs[k], qp = Q[row * n + p], qq = Q[row * n + q];
+                        Q[row * n + p] = c * qp - sn * qq;
+                        Q[row * n + q] = sn * qp + c * qq;
+                    }
+                }
+            }
+            __syncthreads();
+        }
     }
-    for (int i = threadIdx.x; i < n; i += blockDim.x) lam[i] = A[i * n + i];
+    for (int i = tid; i < n; i += blockDim.x) lam[i] = A[i * n + i];
     __syncthreads();
 }
 
-__global__ void k_schur(const Seg *__restrict__ segs, const int *__restrict__ reps, const double *__restrict__ x,
-                        double *__restrict__ delta, double *__restrict__ schurQ, double *__restrict__ schurL,
-                        const double *__restrict__ tab)
+// the 3 x 11 block of Mcm between monomer m and colloid c, columns by colloid component:
+// trans T^T[d] (reference: 0), rot B[:, d], stress G[d, :]; out[q] for axis d at out[d * ld + index]
+__device__ __forceinline__ void mcm_block(const Seg &s, const double *__restrict__ x, int m, int c, double *__restrict__ out,
+                                          int ld)
+{
+    double e[3];
+    const double dr = pair_geom(s, x, (long)s.bead_off + m, (long)s.bead_off + s.Nm + c, e);
+    const double ri = 1.0 / dr;
+    double yb, xg, yg, G[15];
+    ab_scalars<double>(ri, s.beta * s.beta, yb, xg, yg);
+    double xa = 0.0, ya = 0.0;
+    const bool rpy = s.ab_mode == PS_AB_RPY || s.ab_mode == PS_AB_RPY_REG;
+    if (rpy) ab_trans_scalars<double>(dr, ri, s.beta, s.ab_mode == PS_AB_RPY_REG, xa, ya, yb);
+    gt_flat<double>(e, xg, yg, G);
+    for (int d = 0; d < 3; d++) {
+        for (int q = 0; q < 3; q++) {
+            out[d * ld + 3 * c + q] = rpy ? xa * e[d] * e[q] + ya * ((d == q) - e[d] * e[q]) : 0.0;
+            // B[q][d] = yb eps_{q d k} e_k
+            const int kk = 3 - q - d;
+            const double eps = ((q - d + 3) % 3 == 2) ? 1.0 : -1.0;
+            out[d * ld + s.nc3 + 3 * c + q] = (q != d) ? yb * eps * e[kk] : 0.0;
+        }
+        for (int q = 0; q < 5; q++) out[d * ld + s.nc6 + 5 * c + q] = G[d * 5 + q];
+    }
+}
+
+__global__ void __launch_bounds__(SCHUR_THREADS)
+k_schur(const Seg *__restrict__ segs, const int *__restrict__ reps, const double *__restrict__ x,
+        double *__restrict__ delta, double *__restrict__ schurQ, double *__restrict__ schurL,
+        const double *__restrict__ tab)
 {
     pdl_enter();
     extern __shared__ double sm[];
     const int r = reps[blockIdx.x];
     const Seg &s = segs[r];
     const int n = s.nc11, Nm = s.Nm, Nc = s.Nc;
-    double *S = sm, *Q = sm + n * n, *lam = sm + 2 * n * n;
+    double *S = sm, *Q = sm + n * n, *lam = sm + 2 * n * n, *buf = sm + 2 * 64 * 64 + 64;
     // Mcc_base: self + BB pairs, built by applying the pair operator to unit vectors
     for (int k = threadIdx.x; k < n * n; k += blockDim.x) S[k] = 0.0;
     __syncthreads();
@@ -726,57 +808,32 @@ __global__ void k_schur(const Seg *__restrict__ segs, const int *__restrict__ re
             S[rowi * n + colj] += out[k];
         }
     }
-    __syncthreads();
-    // Gram of Mcm: column (m,d) entries per colloid c: trans T^T[d] (reference: 0),
-    // rot B[:,d], stress G[d,:]
-    for (int w = threadIdx.x; w < n * n; w += blockDim.x) {
-        int a = w / n, bcol = w % n;
-        if (bcol < a) continue;
-        int ca, qa, cb, qb;
-        auto decode = [&](int j, int &c, int &q) {
-            if (j < s.nc3) { c = j / 3; q = j % 3; }
-            else if (j < s.nc6) { c = (j - s.nc3) / 3; q = 3 + (j - s.nc3) % 3; }
-            else { c = (j - s.nc6) / 5; q = 6 + (j - s.nc6) % 5; }
-        };
-        decode(a, ca, qa); decode(bcol, cb, qb);
-        double acc = 0.0;
-        for (int m = 0; m < Nm; m++) {
-            double col_a[3], col_b[3];
-            for (int side = 0; side < 2; side++) {
-                int c = side ? cb : ca, q = side ? qb : qa;
-                double *col = side ? col_b : col_a;
-                double e[3];
-                double dr = pair_geom(s, x, (long)s.bead_off + m, (long)s.bead_off + Nm + c, e);
-                double ri = 1.0 / dr;
-                double yb, xg, yg;
-                ab_scalars<double>(ri, s.beta * s.beta, yb, xg, yg);
-                double xa = 0.0, ya = 0.0;
-                if (s.ab_mode == PS_AB_RPY || s.ab_mode == PS_AB_RPY_REG)
-                    ab_trans_scalars<double>(dr, ri, s.beta, s.ab_mode == PS_AB_RPY_REG, xa, ya, yb);
-                for (int d = 0; d < 3; d++) {
-                    double v;
-                    if (q < 3) {
-                        if (s.ab_mode == PS_AB_RPY || s.ab_mode == PS_AB_RPY_REG) {
-                            v = xa * e[d] * e[q] + ya * ((d == q) - e[d] * e[q]);
-                        } else v = 0.0;
-                    } else if (q < 6) {
-                        int aa = q - 3;   // B[aa][d] = yb eps_{aa d k} e_k
-                        int kk = 3 - aa - d;
-                        double eps = 0.0;
-                        if (aa != d && kk >= 0 && kk < 3) eps = ((aa - d + 3) % 3 == 2) ? 1.0 : -1.0;
-                        v = (aa != d) ? yb * eps * e[kk] : 0.0;
-                    } else {
-                        double G[15];
-                        gt_flat<double>(e, xg, yg, G);
-                        v = G[d * 5 + (q - 6)];
-                    }
-                    col[d] = v;
-                }
+    // Gram of Mcm over chunks of monomers; Q holds the upper triangle's sums meanwhile, each
+    // entry added to by one thread in monomer order
+    for (int w = threadIdx.x; w < n * n; w += blockDim.x) Q[w] = 0.0;
+    const int mch = SCHUR_BUF / (3 * n);
+    for (int m0 = 0; m0 < Nm; m0 += mch) {
+        const int nm = min(mch, Nm - m0);
+        __syncthreads();
+        for (int w = threadIdx.x; w < nm * Nc; w += blockDim.x) mcm_block(s, x, m0 + w / Nc, w % Nc, buf + 3 * n * (w / Nc), n);
+        __syncthreads();
+        for (int w = threadIdx.x; w < n * n; w += blockDim.x) {
+            const int a = w / n, c = w % n;
+            if (c < a) continue;
+            double acc = Q[w];
+            for (int m = 0; m < nm; m++) {
+                const double *b = buf + 3 * n * m;
+                acc += b[a] * b[c] + b[n + a] * b[n + c] + b[2 * n + a] * b[2 * n + c];
             }
-            acc += col_a[0] * col_b[0] + col_a[1] * col_b[1] + col_a[2] * col_b[2];
+            Q[w] = acc;
         }
-        S[a * n + bcol] -= s.beta * acc;
-        if (bcol != a) S[bcol * n + a] -= s.beta * acc;
+    }
+    __syncthreads();
+    for (int w = threadIdx.x; w < n * n; w += blockDim.x) {
+        const int a = w / n, c = w % n;
+        if (c < a) continue;
+        S[w] -= s.beta * Q[w];
+        if (c != a) S[c * n + a] -= s.beta * Q[w];
     }
     __syncthreads();
     block_jacobi_eig(S, Q, n, lam);
@@ -806,9 +863,9 @@ int stage_assemble(Engine &E, cudaStream_t st)
 int stage_schur(Engine &E, cudaStream_t st)
 {
     if (!E.n_schur_reps) return PS_OK;
-    size_t smem = sizeof(double) * (2 * 64 * 64 + 64);
+    size_t smem = sizeof(double) * (2 * 64 * 64 + 64 + SCHUR_BUF);
     PS_CK(cudaFuncSetAttribute(k_schur, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-    ps_launch(k_schur, E.n_schur_reps, 256, smem, st, E.d_segs, E.d_schur_reps, E.d_x, E.d_delta, E.d_schurQ, E.d_schurL,
+    ps_launch(k_schur, E.n_schur_reps, SCHUR_THREADS, smem, st, E.d_segs, E.d_schur_reps, E.d_x, E.d_delta, E.d_schurQ, E.d_schurL,
             E.d_tab);
     PS_CK(cudaGetLastError());
     return PS_OK;
