@@ -625,6 +625,166 @@ __device__ void warp_tql(double *d, double *e, double *Z, double *rot, int n)
     }
 }
 
+// The eigenpairs of T_m (diagonal d, off-diagonal e, n <= LZ_KMAX) by one block:
+// eigenvalues by Sturm counts, all at once, eigenvectors from twisted
+// factorisations, one per pair of threads (Dhillon & Parlett, Linear Algebra
+// Appl. 387 (2004) 1).  d gets the eigenvalues, column j of Z the unit vector of
+// eigenvalue j.  Vectors of close eigenvalues come out orthogonal to rounding
+// over their gap only; the caller makes up for that to first order, and where
+// U U^T e1 misses e1 by more than 1e-10 (nearly equal eigenvalues) or the input
+// is not finite, false is returned and the caller falls back on the QL iteration.
+//
+// Bound: latency.  The QL recurrence is one chain of about 0.8 n^2 rotations of
+// some 100 ns; here a chain is n multiply-adds per bisection step and n divisions
+// per factorisation.  m = 40: 230 us by QL, 36 us by this.
+constexpr int LZE_THREADS = 512;
+constexpr int LZE_TEAM = LZE_THREADS / LZ_KMAX;    // threads per eigenvalue
+// doubles of shared memory: d, e, scaled copies, multipliers and vectors
+constexpr int LZE_SMEM = 6 * LZ_KMAX + 3 * LZ_KMAX * (LZ_KMAX + 1);
+
+// eigenvalues below x of the tridiagonal matrix with diagonal a and squared
+// off-diagonal b2: sign changes of the characteristic polynomials of its leading
+// blocks (Givens), rescaled every eight steps.  |a - x| <= 2 by the caller's scaling.
+__device__ __forceinline__ int sturm_below(const double *__restrict__ a, const double *__restrict__ b2, int n, double x)
+{
+    double p0 = 1.0, p1 = a[0] - x;
+    bool neg = p1 < 0.0 || p1 == 0.0;          // a zero counts with the sign opposite to its predecessor
+    int cnt = neg;
+    for (int i = 1; i < n; i++) {
+        const double p2 = fma(a[i] - x, p1, -(b2[i - 1] * p0));
+        const bool ng = p2 < 0.0 || (p2 == 0.0 && !neg);
+        cnt += ng != neg;
+        neg = ng;
+        p0 = p1;
+        p1 = p2;
+        if ((i & 7) == 0) {
+            const double m = fmax(fabs(p0), fabs(p1));
+            if (m < 1e-100) { p0 *= 1e100; p1 *= 1e100; }
+        }
+    }
+    return cnt;
+}
+
+__device__ bool block_tridiag_eig(double *d, const double *e, double *a, double *b, double *b2, double *Z, double *Lf,
+                                  double *Lb, int n)
+{
+    constexpr int LD = LZ_KMAX + 1;
+    __shared__ double sc[2];
+    const int tid = threadIdx.x, lane = tid & 31;
+    // shift and scale so that Gershgorin's discs fill [-1, 1]
+    if (tid < 32) {
+        double lo = 1e300, hi = -1e300;
+        bool fin = true;
+        for (int i = lane; i < n; i += 32) {
+            const double r = (i > 0 ? fabs(e[i - 1]) : 0.0) + (i < n - 1 ? fabs(e[i]) : 0.0);
+            lo = fmin(lo, d[i] - r);
+            hi = fmax(hi, d[i] + r);
+            fin = fin && isfinite(d[i]) && isfinite(r);
+        }
+        for (int o = 16; o > 0; o >>= 1) {
+            lo = fmin(lo, __shfl_xor_sync(0xffffffffu, lo, o));
+            hi = fmax(hi, __shfl_xor_sync(0xffffffffu, hi, o));
+        }
+        fin = __all_sync(0xffffffffu, fin);
+        if (lane == 0) {
+            const double h = 0.5 * (hi - lo);
+            sc[0] = 0.5 * (hi + lo);
+            sc[1] = fin && h > 0.0 && isfinite(h) ? h : 0.0;
+        }
+    }
+    __syncthreads();
+    const double mid = sc[0], half = sc[1];
+    if (half == 0.0) return false;
+    for (int i = tid; i < n; i += LZE_THREADS) {
+        a[i] = (d[i] - mid) / half;
+        const double bi = i < n - 1 ? e[i] / half : 0.0;
+        b[i] = bi;
+        b2[i] = bi * bi;
+    }
+    __syncthreads();
+    // eigenvalue k of team k: the bracket shrinks by LZE_TEAM + 1 per round
+    const int k = tid / LZE_TEAM, t = tid % LZE_TEAM;
+    const int kk = k < n ? k : n - 1;                      // idle teams mirror the last (whole warps stay together)
+    double lo = -1.0 - 1e-12, hi = 1.0 + 1e-12;
+    const unsigned sh = lane & ~(LZE_TEAM - 1);
+    for (int round = 0; round < 17; round++) {             // 9^17 > 2^53
+        const double w = (hi - lo) * (1.0 / (LZE_TEAM + 1));
+        const double x = lo + (t + 1) * w;
+        const bool above = sturm_below(a, b2, n, x) > kk;  // eigenvalue kk lies below x
+        const unsigned m = (__ballot_sync(0xffffffffu, above) >> sh) & ((1u << LZE_TEAM) - 1);
+        const int f = m ? __ffs(m) - 1 : LZE_TEAM;         // the first point above it
+        const double l2 = lo + f * w;
+        hi = f < LZE_TEAM ? lo + (f + 1) * w : hi;
+        lo = f > 0 ? l2 : lo;
+    }
+    const double th = 0.5 * (lo + hi);
+    // twisted factorisation of T - theta: thread 0 of the team from the top, thread 1 from the bottom
+    const double tiny = 1e-18;
+    if (k < n && t == 0) {
+        double p = a[0] - th;
+        for (int i = 0; i < n; i++) {
+            if (fabs(p) < tiny) p = p < 0.0 ? -tiny : tiny;
+            Lf[i * LD + k] = p;
+            if (i + 1 < n) p = (a[i + 1] - th) - b2[i] / p;
+        }
+    } else if (k < n && t == 1) {
+        double p = a[n - 1] - th;
+        for (int i = n - 1; i >= 0; i--) {
+            if (fabs(p) < tiny) p = p < 0.0 ? -tiny : tiny;
+            Lb[i * LD + k] = p;
+            if (i > 0) p = (a[i - 1] - th) - b2[i - 1] / p;
+        }
+    }
+    __syncwarp();
+    if (k < n && t < 2) {
+        // the twist where the pivot is smallest; each thread takes its side of it
+        int kt = 0;
+        double g = 1e300;
+        for (int i = 0; i < n; i++) {
+            const double v = fabs(Lf[i * LD + k] + Lb[i * LD + k] - (a[i] - th));
+            if (v < g) { g = v; kt = i; }
+        }
+        double z = 1.0, nz = t == 0 ? 1.0 : 0.0;
+        if (t == 0) {
+            Z[kt * LD + k] = 1.0;
+            for (int i = kt - 1; i >= 0; i--) {
+                z *= -b[i] / Lf[i * LD + k];
+                Z[i * LD + k] = z;
+                nz += z * z;
+            }
+        } else {
+            for (int i = kt + 1; i < n; i++) {
+                z *= -b[i - 1] / Lb[i * LD + k];
+                Z[i * LD + k] = z;
+                nz += z * z;
+            }
+        }
+        const unsigned two = 3u << sh;
+        nz += __shfl_xor_sync(two, nz, 1);
+        __syncwarp(two);
+        const double rn = rsqrt(nz);
+        for (int i = t == 0 ? 0 : kt + 1; i < (t == 0 ? kt + 1 : n); i++) Z[i * LD + k] *= rn;
+        if (t == 0) d[k] = fma(th, half, mid);
+    }
+    __syncthreads();
+    return true;
+}
+
+// y = Z x or Z^T x, a team per entry (n <= LZ_KMAX entries, leading dimension ld), scaled
+// and added: y_k = ca c_k + cb sum; every thread of the block takes part
+__device__ __forceinline__ void team_matvec(const double *__restrict__ Z, int ld, bool trans, const double *__restrict__ x,
+                                            int n, double ca, const double *__restrict__ c, double cb,
+                                            double *__restrict__ y)
+{
+    const int k = threadIdx.x / LZE_TEAM, t = threadIdx.x % LZE_TEAM;
+    double v = 0.0;
+    if (k < n)
+        for (int j = t; j < n; j += LZE_TEAM) v += (trans ? Z[j * ld + k] : Z[k * ld + j]) * x[j];
+    for (int o = LZE_TEAM / 2; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
+    if (k < n && t == 0) y[k] = ca * c[k] + cb * v;
+    __syncthreads();
+}
+
 // A check's outcome for one replica, written by the speculative checks.
 struct LzSpec {
     int conv;      // converged at m
@@ -633,67 +793,92 @@ struct LzSpec {
     int pad;
 };
 
-// one warp per replica: eig of T_m, g = b0 U sqrt(max(theta,0)) U^T e1,
+// one block per replica: eig of T_m, g = b0 U sqrt(max(theta,0)) U^T e1,
 // convergence ||g - g_prev|| <= tol ||g|| (the Lanczos basis is orthonormal).
 // final_ = 1: the final estimate, on the replica's own m when it is done, into lz.
 // final_ = 0: a speculative check beside the next basis vectors: it reads the
 // snapshot `snap` of lz taken when it was launched (the vectors that follow
 // move lz on) and writes its outcome into spec; the host applies it later
 // (k_lz_spec_apply).  g_prev is the previous check's g in both cases.
-__global__ void k_lz_check(int R, LzScal *__restrict__ lz, const LzScal *__restrict__ snap, LzSpec *__restrict__ spec,
-                           const double *__restrict__ alpha, const double *__restrict__ betad, double *__restrict__ gbuf,
-                           int m, double tol, int final_)
+__global__ void __launch_bounds__(LZE_THREADS)
+k_lz_check(int R, LzScal *__restrict__ lz, const LzScal *__restrict__ snap, LzSpec *__restrict__ spec,
+           const double *__restrict__ alpha, const double *__restrict__ betad, double *__restrict__ gbuf,
+           int m, double tol, int final_)
 {
     pdl_enter();
     extern __shared__ double sm[];
+    __shared__ double red[2][2];
+    __shared__ int rneg[2];
     const int r = blockIdx.x;
     const LzScal L = final_ ? lz[r] : snap[r];
-    const int lane = threadIdx.x;
+    const int tid = threadIdx.x, lane = tid & 31, wid = tid >> 5;
     if (!final_ && L.done) {
-        if (lane == 0) spec[r] = LzSpec{0, L.m, 1, 0};
+        if (tid == 0) spec[r] = LzSpec{0, L.m, 1, 0};
         return;
     }
-    int mr = L.done ? L.m : m;
+    const int mr = L.done ? L.m : m;
     if (mr <= 0) {
-        if (!final_ && lane == 0) spec[r] = LzSpec{0, 0, 0, 0};
+        if (!final_ && tid == 0) spec[r] = LzSpec{0, 0, 0, 0};
         return;
     }
-    double *d = sm, *e = sm + LZ_KMAX, *Z = sm + 2 * LZ_KMAX, *rot = Z + LZ_KMAX * LZ_KMAX;
-    for (int i = lane; i < mr; i += 32) {
-        d[i] = alpha[(long)LZ_KMAX * r + i];
-        e[i] = (i < mr - 1) ? betad[(long)LZ_KMAX * r + i] : 0.0;
-    }
-    __syncwarp();
-    warp_tql(d, e, Z, rot, mr);
-    __syncwarp();
-    double *g = gbuf + (long)(LZ_KMAX + 1) * r;   // g[0..m-1], g[LZ_KMAX] = |g|^2 of previous
-    double diff2 = 0, nrm2 = 0;
-    int nneg = 0;
-    for (int i = lane; i < LZ_KMAX; i += 32) {
-        double gi = 0;
-        if (i < mr) {
-            for (int j = 0; j < mr; j++) {
-                double th = d[j];
-                double sq = th > 0 ? sqrt(th) : 0.0;
-                gi += Z[i * mr + j] * sq * Z[0 * mr + j];
-            }
-            gi *= L.b0;
+    double *d = sm, *e = d + LZ_KMAX, *a = e + LZ_KMAX, *b = a + LZ_KMAX, *b2 = b + LZ_KMAX, *v = b2 + LZ_KMAX;
+    double *Z = v + LZ_KMAX, *Lf = Z + LZ_KMAX * (LZ_KMAX + 1), *Lb = Lf + LZ_KMAX * (LZ_KMAX + 1);
+    auto load = [&]() {
+        for (int i = tid; i < mr; i += LZE_THREADS) {
+            d[i] = alpha[(long)LZ_KMAX * r + i];
+            e[i] = (i < mr - 1) ? betad[(long)LZ_KMAX * r + i] : 0.0;
         }
-        double old = g[i];
-        diff2 += (gi - old) * (gi - old);
-        nrm2 += gi * gi;
+        __syncthreads();
+    };
+    load();
+    int ld = LZ_KMAX + 1;
+    // v = U^T e1 and a = U v, which is e1 when the vectors are orthonormal
+    bool ok = block_tridiag_eig(d, e, a, b, b2, Z, Lf, Lb, mr);
+    if (ok) {
+        for (int j = tid; j < mr; j += LZE_THREADS) v[j] = Z[j];
+        __syncthreads();
+        team_matvec(Z, ld, false, v, mr, 0.0, v, 1.0, a);
+        bool miss = false;
+        for (int i = tid; i < mr; i += LZE_THREADS) miss = miss || !(fabs(a[i] - (i == 0)) <= 1e-10);
+        ok = !__syncthreads_or(miss);
+    }
+    if (!ok) {
+        load();
+        ld = mr;
+        if (wid == 0) {
+            warp_tql(d, e, Z, Lf, mr);
+            __syncwarp();
+            for (int j = lane; j < mr; j += 32) { v[j] = Z[j]; a[j] = j == 0; }
+        }
+        __syncthreads();
+    }
+    // f(T) e1 with U (U^T U)^(-1/2) in place of U, to first order in U^T U - I:
+    // w = f (3 v - U^T U v) / 2, then U (3 w - U^T U w) / 2
+    team_matvec(Z, ld, true, a, mr, 1.5, v, -0.5, b);
+    for (int j = tid; j < mr; j += LZE_THREADS) b[j] *= d[j] > 0 ? sqrt(d[j]) : 0.0;
+    __syncthreads();
+    team_matvec(Z, ld, false, b, mr, 0.0, b, 1.0, a);
+    team_matvec(Z, ld, true, a, mr, 1.5, b, -0.5, b2);
+    team_matvec(Z, ld, false, b2, mr, 0.0, b2, L.b0, a);
+    double *g = gbuf + (long)(LZ_KMAX + 1) * r;   // g[0..m-1] of the previous check
+    if (tid < LZ_KMAX) {
+        const int i = tid;
+        const double gi = i < mr ? a[i] : 0.0, old = g[i];
+        double diff2 = (gi - old) * (gi - old), nrm2 = gi * gi;
+        int nneg = i < mr && d[i] < 0.0;
         if (i < mr) g[i] = gi;
+        for (int o = 16; o > 0; o >>= 1) {
+            diff2 += __shfl_down_sync(0xffffffffu, diff2, o);
+            nrm2 += __shfl_down_sync(0xffffffffu, nrm2, o);
+            nneg += __shfl_down_sync(0xffffffffu, nneg, o);
+        }
+        if (lane == 0) { red[wid][0] = diff2; red[wid][1] = nrm2; rneg[wid] = nneg; }
     }
-    for (int j = lane; j < mr; j += 32) nneg += d[j] < 0.0;
-    for (int o = 16; o > 0; o >>= 1) {
-        diff2 += __shfl_down_sync(0xffffffffu, diff2, o);
-        nrm2 += __shfl_down_sync(0xffffffffu, nrm2, o);
-        nneg += __shfl_down_sync(0xffffffffu, nneg, o);
-    }
-    if (lane == 0) {
-        const int conv = sqrt(diff2) <= tol * sqrt(nrm2);
+    __syncthreads();
+    if (tid == 0) {
+        const int conv = sqrt(red[0][0] + red[1][0]) <= tol * sqrt(red[0][1] + red[1][1]);
         if (final_) {
-            lz[r].nneg = nneg;
+            lz[r].nneg = rneg[0] + rneg[1];
             if (!lz[r].done) {
                 lz[r].m = mr;
                 lz[r].done = 1;
@@ -902,7 +1087,8 @@ int lanczos_sqrt(Engine &E, const double *z, double *w, const ps_sqrt_opts *o, p
     bool small = (long)E.R * LZC_CTAS <= 128;
     for (const Seg &sg : E.segs)
         small = small && (sg.nm3nc11 + RB_SPAN - 1) / RB_SPAN <= LZC_VB * LZC_SLOTS;
-    size_t smem = sizeof(double) * (4 * LZ_KMAX + LZ_KMAX * LZ_KMAX);
+    const size_t smem = sizeof(double) * LZE_SMEM;
+    PS_CK(cudaFuncSetAttribute(k_lz_check, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
     std::vector<LzScal> hl(E.R);
     LzScal *snap = lz + E.R;                                 // the scalars when a check was launched
     LzSpec *spec = (LzSpec *)(snap + E.R);                   // the checks' outcomes
@@ -937,7 +1123,7 @@ int lanczos_sqrt(Engine &E, const double *z, double *w, const ps_sqrt_opts *o, p
             PS_CK(cudaMemcpyAsync(snap, lz, sizeof(LzScal) * E.R, cudaMemcpyDeviceToDevice, st));
             PS_CK(cudaEventRecord(E.ev_fork2, st));
             PS_CK(cudaStreamWaitEvent(E.side2, E.ev_fork2, 0));
-            ps_launch(k_lz_check, E.R, 32, smem, E.side2, E.R, lz, snap, spec, alpha, betad, gbuf, j + 1,
+            ps_launch(k_lz_check, E.R, LZE_THREADS, smem, E.side2, E.R, lz, snap, spec, alpha, betad, gbuf, j + 1,
                     tol, 0);
             PS_CK(cudaMemcpyAsync(hspec, spec, sizeof(LzSpec) * E.R, cudaMemcpyDeviceToHost, E.side2));
             PS_CK(cudaEventRecord(E.ev_chk, E.side2));
@@ -950,7 +1136,7 @@ int lanczos_sqrt(Engine &E, const double *z, double *w, const ps_sqrt_opts *o, p
         ps_launch(k_lz_spec_apply, (E.R + 127) / 128, 128, 0, st, E.R, lz, spec);
     }
     // final estimate: replicas at the cap, replicas stopped by breakdown, and the converged ones on their own m
-    ps_launch(k_lz_check, E.R, 32, smem, st, E.R, lz, snap, spec, alpha, betad, gbuf,
+    ps_launch(k_lz_check, E.R, LZE_THREADS, smem, st, E.R, lz, snap, spec, alpha, betad, gbuf,
             std::min(j + 1, kmax), tol, 1);
     ps_launch(k_lz_combine, T.nblk, RB_THREADS, 0, st, T, V, ldv, lz, gbuf, w);
     PS_CK(cudaMemcpyAsync(hl.data(), lz, sizeof(LzScal) * E.R, cudaMemcpyDeviceToHost, st));
