@@ -15,7 +15,6 @@
 #include <cmath>
 #include <cstdio>
 #include <vector>
-#include <cooperative_groups.h>
 #include "ps_internal.h"
 #include "ps_kernels.h"
 #include "ps_reduce.cuh"
@@ -46,7 +45,7 @@ int build_red_table(Engine &E, RedTable &T, int layout)
     PS_CK(cudaMalloc(&T.d_first, sizeof(int) * E.R));
     PS_CK(cudaMalloc(&T.d_count, sizeof(int) * E.R));
     PS_CK(cudaMalloc(&T.d_counter, sizeof(int) * E.R));
-    PS_CK(cudaMalloc(&T.d_part, sizeof(double) * 65 * T.nblk));   // 4 for scalar sums, 65 for Lanczos dots
+    PS_CK(cudaMalloc(&T.d_part, sizeof(double) * 4 * T.nblk));
     PS_CK(cudaMemcpy(T.d_blk, blk.data(), sizeof(RBlk) * T.nblk, cudaMemcpyHostToDevice));
     PS_CK(cudaMemcpy(T.d_first, first.data(), sizeof(int) * E.R, cudaMemcpyHostToDevice));
     PS_CK(cudaMemcpy(T.d_count, cnt.data(), sizeof(int) * E.R, cudaMemcpyHostToDevice));
@@ -329,198 +328,135 @@ struct LzScal {
     double b0;
     int m, done, nneg;
 };
-constexpr int LZ_KMAX = 64;
 
-// Partial dots of q (held by the block's threads in qv) against V_0..V_j, one
-// block of the table; the last block of the replica sums the partials in block
-// order into h[].  An inactive block contributes zeros.
-__device__ __forceinline__ void lz_dots_block(const RedTable &T, const RBlk &B, const double *__restrict__ V, long ldv,
-                                              const double (&qv)[RB_EPT], bool act, int j, double *__restrict__ h)
-{
-    __shared__ double sh[RB_THREADS / 32][LZ_KMAX + 1];
-    __shared__ bool last;
-    const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
-    // eight basis vectors per pass keep 8 x RB_EPT loads in flight.  Each dot is
-    // summed in element order and reduced by the same shuffle tree as one at a time.
-    for (int i0 = 0; i0 <= j; i0 += 8) {
-        double v[8];
-#pragma unroll
-        for (int c = 0; c < 8; c++) {
-            v[c] = 0.0;
-            if (act && i0 + c <= j) {
-                const double *Vi = V + (long)(i0 + c) * ldv + B.start;
-#pragma unroll
-                for (int k = 0; k < RB_EPT; k++) {
-                    const int e = threadIdx.x + k * RB_THREADS;
-                    if (e < B.len) v[c] += Vi[e] * qv[k];
-                }
-            }
-        }
-#pragma unroll
-        for (int c = 0; c < 8; c++) {
-            double t = v[c];
-            for (int o = 16; o > 0; o >>= 1) t += __shfl_down_sync(0xffffffffu, t, o);
-            if (lane == 0 && i0 + c <= j) sh[wid][i0 + c] = t;
-        }
-    }
-    __syncthreads();
-    // block partial for i stored at d_part[(LZ_KMAX+1) * blk + i]
-    if (threadIdx.x <= j) {
-        double t = 0;
-        for (int w = 0; w < RB_THREADS / 32; w++) t += sh[w][threadIdx.x];
-        T.d_part[(long)(LZ_KMAX + 1) * blockIdx.x + threadIdx.x] = t;
-    }
-    __threadfence();
-    __syncthreads();
-    if (threadIdx.x == 0) {
-        int t = atomicAdd(&T.d_counter[B.rep], 1);
-        last = (t == T.d_count[B.rep] - 1);
-    }
-    __syncthreads();
-    if (!last) return;
-    __threadfence();
-    int f = T.d_first[B.rep], c = T.d_count[B.rep];
-    if (threadIdx.x <= j) {
-        double t = 0;
-        for (int k = 0; k < c; k++) t += ((volatile double *)T.d_part)[(long)(LZ_KMAX + 1) * (f + k) + threadIdx.x];
-        h[(long)(LZ_KMAX + 1) * B.rep + threadIdx.x] = t;
-    }
-    __syncthreads();
-    if (threadIdx.x == 0) T.d_counter[B.rep] = 0;
-}
+// Reorthogonalisation of one Lanczos vector, q = M V_j against V_0..V_j: two
+// passes of classical Gram-Schmidt.  One thread owns one entry of the replica's
+// vector, in sub-blocks of 256 entries (a quarter of a reduction-table block).
+// The combine that forms q also forms the first pass's dots (k_combine), then
+// k_lz_sub_dots subtracts and forms the second pass's dots, k_lz_sub_norm
+// subtracts and forms the norm, k_lz_next tests for breakdown and scales.  Each
+// kernel leaves its sub-blocks' sums in memory, and every block of the next one
+// adds its replica's sums itself, in a fixed order that depends on the vector's
+// length alone -- no counters and no fences, and a replica's noise does not depend
+// on its batch.
+//
+// Bound: latency and L2 (the basis is read twice from L2 and once from L1 per
+// vector, k_lz_sub_dots reading its slices twice).  With 1024 entries per block of
+// 256 threads, or one cluster of eight blocks per replica, too few loads were in
+// flight: a vector with its apply took 42 us at 1024 beads (27 now), 72 us at the
+// 4097-bead brush (52 now), and the four sweeps of 64 replicas, 62000 beads, 100 us
+// (50 now).
+constexpr int LZ_SUB = RB_THREADS;                    // entries of a sub-block
+static_assert(RB_SPAN == RB_EPT * LZ_SUB, "RB_EPT sub-blocks per table block");
 
-// h = V_0..V_j dotted with q (first pass of the Gram-Schmidt step)
-__global__ void k_lz_dots(RedTable T, const double *__restrict__ V, long ldv, const double *__restrict__ q, int j,
-                          const LzScal *__restrict__ lz, double *__restrict__ h)
+// the replica's total of the sub-block sums part[][i], i <= j, into h[] (shared)
+__device__ __forceinline__ void lz_total(const RedTable &T, const RBlk &B, const Seg &s, const double *__restrict__ part,
+                                         int j, double *__restrict__ h)
 {
-    pdl_enter();
-    const RBlk B = T.d_blk[blockIdx.x];
-    const bool act = !lz[B.rep].done;
-    // q held in registers (a block spans at most RB_EPT elements per thread)
-    double qv[RB_EPT];
-#pragma unroll
-    for (int k = 0; k < RB_EPT; k++) {
-        const int e = threadIdx.x + k * RB_THREADS;
-        qv[k] = (act && e < B.len) ? q[B.start + e] : 0.0;
-    }
-    lz_dots_block(T, B, V, ldv, qv, act, j, h);
-}
-
-// The first pass's subtraction and the second pass's dots in one sweep:
-// q -= sum_i h_i V_i (per element in the order i = 0..j), alpha_j = h_j, then
-// h2 = V_0..V_j dotted with the new q, which the block still holds in registers.
-// The block's slices of V are read twice, the second time from cache.  Same
-// arithmetic, in the same order, as the subtraction and dots kernels one after
-// the other.
-__global__ void k_lz_sub_dots(RedTable T, const double *__restrict__ V, long ldv, double *__restrict__ q, int j,
-                              const LzScal *__restrict__ lz, const double *__restrict__ h, double *__restrict__ alpha,
-                              double *__restrict__ h2)
-{
-    pdl_enter();
-    const RBlk B = T.d_blk[blockIdx.x];
-    const bool act = !lz[B.rep].done;
-    double acc[RB_EPT];
-    if (act) {
-        const double *hr = h + (long)(LZ_KMAX + 1) * B.rep;
-#pragma unroll
-        for (int k = 0; k < RB_EPT; k++) {
-            const int e = threadIdx.x + k * RB_THREADS;
-            acc[k] = e < B.len ? q[B.start + e] : 0.0;
-        }
+    __shared__ double sh4[RB_THREADS / LZ_KMAX][LZ_KMAX];
+    constexpr int G = RB_THREADS / LZ_KMAX;
+    const int i = threadIdx.x % LZ_KMAX, g = threadIdx.x / LZ_KMAX;
+    const int nb = (s.nm3nc11 + LZ_SUB - 1) / LZ_SUB;
+    const double *p = part + (long)RB_EPT * T.d_first[B.rep] * LZ_KMAX + i;
+    double t = 0.0;
+    if (i <= j) {
 #pragma unroll 4
-        for (int i = 0; i <= j; i++) {
-            const double hi = hr[i];
-            const double *Vi = V + (long)i * ldv + B.start;
-#pragma unroll
-            for (int k = 0; k < RB_EPT; k++) {
-                const int e = threadIdx.x + k * RB_THREADS;
-                if (e < B.len) acc[k] -= hi * Vi[e];
-            }
-        }
-#pragma unroll
-        for (int k = 0; k < RB_EPT; k++) {
-            const int e = threadIdx.x + k * RB_THREADS;
-            if (e < B.len) q[B.start + e] = acc[k];
-            else acc[k] = 0.0;
-        }
-        if (threadIdx.x == 0 && (B.start == T.d_blk[T.d_first[B.rep]].start))
-            alpha[(long)LZ_KMAX * B.rep + j] = 0.0 + hr[j];
-    } else {
-#pragma unroll
-        for (int k = 0; k < RB_EPT; k++) acc[k] = 0.0;
+        for (int b = g; b < nb; b += G) t += p[(long)b * LZ_KMAX];
     }
-    lz_dots_block(T, B, V, ldv, acc, act, j, h2);
+    sh4[g][i] = t;
+    __syncthreads();
+    if (threadIdx.x <= j) {
+        double v = 0.0;
+        for (int c = 0; c < G; c++) v += sh4[c][threadIdx.x];
+        h[threadIdx.x] = v;
+    }
+    __syncthreads();
 }
 
-// The second pass's subtraction, the norm and the breakdown test in one sweep:
-// q -= sum_i h2_i V_i, alpha_j += h2_j, nrm2 = q.q summed as the segmented dot
-// sums it (the same elements per thread, shuffle tree and block order), and the
-// replica's last block records m = j + 1 and stops the replica on an invariant
-// subspace.  A done replica's blocks only take part in the norm, of its
-// unchanged q, as the segmented dot would.
-__global__ void k_lz_sub_norm(RedTable T, const double *__restrict__ V, long ldv, double *__restrict__ q, int j,
-                              LzScal *__restrict__ lz, const double *__restrict__ h2, double *__restrict__ alpha,
-                              double *__restrict__ nrm2)
+// q -= sum_i h_i V_i for this thread's entry, i = 0..j in order
+__device__ __forceinline__ double lz_subtract(const double *__restrict__ V, long ldv, long k, double q, int j,
+                                              const double *__restrict__ h)
+{
+#pragma unroll 8
+    for (int i = 0; i <= j; i++) q -= h[i] * V[(long)i * ldv + k];
+    return q;
+}
+
+__global__ void k_lz_sub_dots(RedTable T, const Seg *__restrict__ segs, const double *__restrict__ V, long ldv,
+                              double *__restrict__ q, int j, const LzScal *__restrict__ lz,
+                              const double *__restrict__ part1, double *__restrict__ alpha, double *__restrict__ part2)
 {
     pdl_enter();
-    __shared__ double sh[RB_THREADS / 32][1];
     const RBlk B = T.d_blk[blockIdx.x];
-    const bool act = !lz[B.rep].done;
-    double acc[RB_EPT];
-#pragma unroll
-    for (int k = 0; k < RB_EPT; k++) {
-        const int e = threadIdx.x + k * RB_THREADS;
-        acc[k] = e < B.len ? q[B.start + e] : 0.0;
-    }
+    const int e = blockIdx.y * LZ_SUB + threadIdx.x;
+    if (blockIdx.y * LZ_SUB >= B.len || lz[B.rep].done) return;
+    __shared__ double h[LZ_KMAX];
+    lz_total(T, B, segs[B.rep], part1, j, h);
+    const bool act = e < B.len;
+    const long k = (long)B.start + e;
+    double v = 0.0;
     if (act) {
-        const double *hr = h2 + (long)(LZ_KMAX + 1) * B.rep;
-#pragma unroll 4
-        for (int i = 0; i <= j; i++) {
-            const double hi = hr[i];
-            const double *Vi = V + (long)i * ldv + B.start;
-#pragma unroll
-            for (int k = 0; k < RB_EPT; k++) {
-                const int e = threadIdx.x + k * RB_THREADS;
-                if (e < B.len) acc[k] -= hi * Vi[e];
-            }
-        }
-#pragma unroll
-        for (int k = 0; k < RB_EPT; k++) {
-            const int e = threadIdx.x + k * RB_THREADS;
-            if (e < B.len) q[B.start + e] = acc[k];
-        }
-        if (threadIdx.x == 0 && (B.start == T.d_blk[T.d_first[B.rep]].start))
-            alpha[(long)LZ_KMAX * B.rep + j] = alpha[(long)LZ_KMAX * B.rep + j] + hr[j];
+        v = lz_subtract(V, ldv, k, q[k], j, h);
+        q[k] = v;
     }
+    if (threadIdx.x == 0 && blockIdx.y == 0 && (int)blockIdx.x == T.d_first[B.rep]) alpha[(long)LZ_KMAX * B.rep + j] = h[j];
+    lz_block_dots(V, ldv, k, act, v, j, part2 + (long)LZ_KMAX * (RB_EPT * blockIdx.x + blockIdx.y));
+}
+
+__global__ void k_lz_sub_norm(RedTable T, const Seg *__restrict__ segs, const double *__restrict__ V, long ldv,
+                              double *__restrict__ q, int j, const LzScal *__restrict__ lz,
+                              const double *__restrict__ part2, double *__restrict__ alpha, double *__restrict__ npart)
+{
+    pdl_enter();
+    const RBlk B = T.d_blk[blockIdx.x];
+    const int e = blockIdx.y * LZ_SUB + threadIdx.x;
+    if (blockIdx.y * LZ_SUB >= B.len || lz[B.rep].done) return;
+    __shared__ double h[LZ_KMAX], sh[RB_THREADS / 32][1];
+    lz_total(T, B, segs[B.rep], part2, j, h);
     double v[1] = {0.0};
-#pragma unroll
-    for (int k = 0; k < RB_EPT; k++) {
-        const int e = threadIdx.x + k * RB_THREADS;
-        if (e < B.len) v[0] += acc[k] * acc[k];
+    if (e < B.len) {
+        const long k = (long)B.start + e;
+        const double t = lz_subtract(V, ldv, k, q[k], j, h);
+        q[k] = t;
+        v[0] = t * t;
     }
+    if (threadIdx.x == 0 && blockIdx.y == 0 && (int)blockIdx.x == T.d_first[B.rep]) alpha[(long)LZ_KMAX * B.rep + j] += h[j];
     block_sum<1>(v, sh);
-    double tot[1];
-    if (finish_block<1>(T, B, blockIdx.x, v, tot)) {
-        nrm2[B.rep] = tot[0];
-        LzScal &l = lz[B.rep];
-        if (!l.done) {
-            l.m = j + 1;
-            if (sqrt(tot[0]) <= 1e-12 * l.b0) l.done = 2;   // 2: finalise with m = j+1
-        }
-    }
+    if (threadIdx.x == 0) npart[RB_EPT * blockIdx.x + blockIdx.y] = v[0];
 }
 
-// V_{j+1} = q / ||q||; beta_j = ||q||  (norm from nrm[rep])
-__global__ void k_lz_next(RedTable T, double *__restrict__ V, long ldv, const double *__restrict__ q, int j,
-                          LzScal *__restrict__ lz, const double *__restrict__ nrm2, double *__restrict__ betad)
+// beta_j = ||q||, V_{j+1} = q / beta_j, m = j + 1; an invariant subspace stops the replica.
+// (done may be set by the replica's first block while others still read it: they find the
+// same breakdown themselves and write nothing either way.)
+__global__ void k_lz_next(RedTable T, const Seg *__restrict__ segs, double *__restrict__ V, long ldv,
+                          const double *__restrict__ q, int j, int kmax, LzScal *__restrict__ lz,
+                          const double *__restrict__ npart, double *__restrict__ betad)
 {
     pdl_enter();
     const RBlk B = T.d_blk[blockIdx.x];
-    if (lz[B.rep].done) return;
-    double bj = sqrt(nrm2[B.rep]);
-    double inv = bj > 0 ? 1.0 / bj : 0.0;
-    for (int e = threadIdx.x; e < B.len; e += RB_THREADS) V[(long)(j + 1) * ldv + B.start + e] = q[B.start + e] * inv;
-    if (threadIdx.x == 0 && (B.start == T.d_blk[T.d_first[B.rep]].start)) betad[(long)LZ_KMAX * B.rep + j] = bj;
+    const int e = blockIdx.y * LZ_SUB + threadIdx.x;
+    if (blockIdx.y * LZ_SUB >= B.len || lz[B.rep].done) return;
+    __shared__ double tot;
+    const int first = T.d_first[B.rep];
+    if (threadIdx.x < 32) {
+        const int nb = (segs[B.rep].nm3nc11 + LZ_SUB - 1) / LZ_SUB;
+        double t = 0.0;
+        for (int b = threadIdx.x; b < nb; b += 32) t += npart[RB_EPT * first + b];
+        for (int o = 16; o > 0; o >>= 1) t += __shfl_xor_sync(0xffffffffu, t, o);
+        if (threadIdx.x == 0) tot = t;
+    }
+    __syncthreads();
+    const double bj = sqrt(tot);
+    const bool broken = bj <= 1e-12 * lz[B.rep].b0;
+    if (!broken && j + 1 < kmax && e < B.len) {
+        const long k = (long)B.start + e;
+        V[(long)(j + 1) * ldv + k] = q[k] * (bj > 0 ? 1.0 / bj : 0.0);
+    }
+    if (threadIdx.x == 0 && blockIdx.y == 0 && (int)blockIdx.x == first) {
+        lz[B.rep].m = j + 1;
+        if (broken) lz[B.rep].done = 2;             // finalise with m = j + 1
+        else if (j + 1 < kmax) betad[(long)LZ_KMAX * B.rep + j] = bj;
+    }
 }
 
 __global__ void k_lz_init(RedTable T, const Seg *__restrict__ segs, double *__restrict__ V,
@@ -915,155 +851,6 @@ __global__ void k_lz_combine(RedTable T, const double *__restrict__ V, long ldv,
     }
 }
 
-// One Lanczos iteration's orthogonalisation for small batches, in one launch:
-// one cluster of LZC_CTAS blocks per replica.  Both passes of the
-// reorthogonalisation (dots against V_0..V_j, then q -= V h), the norm, the
-// breakdown test and the next basis vector, with cluster barriers between the
-// phases and the cross-block sums read through distributed shared memory.
-// The arithmetic is bit for bit that of the launch sequence it replaces
-// (k_lz_dots, k_lz_sub_dots, k_lz_sub_norm, k_lz_next): the replica's
-// vector is cut into the reduction table's RB_SPAN blocks, each half of a
-// block (RB_THREADS threads) forms an RB block's partials with the same
-// thread-to-element map, shuffle tree and warp order, and every sum over RB
-// blocks runs in block order.  So a replica's noise does not depend on which
-// path its batch takes.  Used when the batch fits one wave of clusters and each
-// replica at most LZC_SLOTS RB blocks per half-block; a replica that is done
-// leaves with its whole cluster (the flag is read before any block writes it).
-namespace cgr = cooperative_groups;
-constexpr int LZC_CTAS = 8, LZC_HALVES = 2, LZC_THREADS = RB_THREADS * LZC_HALVES, LZC_SLOTS = 4;
-constexpr int LZC_VB = LZC_CTAS * LZC_HALVES;         // virtual RB-table blocks per cluster
-
-__global__ void __cluster_dims__(LZC_CTAS, 1, 1) __launch_bounds__(LZC_THREADS)
-k_lz_orth_cluster(const Seg *__restrict__ segs, double *__restrict__ V, long ldv, double *__restrict__ q, int j,
-                  int kmax, LzScal *__restrict__ lz, double *__restrict__ alpha, double *__restrict__ betad)
-{
-    pdl_enter();
-    cgr::cluster_group cl = cgr::this_cluster();
-    const int rank = (int)cl.block_rank();
-    const int r = blockIdx.x / LZC_CTAS;
-    const int half = threadIdx.x / RB_THREADS, t = threadIdx.x % RB_THREADS;
-    const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
-    constexpr int HW = RB_THREADS / 32;                   // warps per half
-    __shared__ double part[2][LZC_HALVES][LZC_SLOTS][LZ_KMAX + 1];   // per pass: RB-block partial dots
-    __shared__ double npart[LZC_HALVES][LZC_SLOTS];       // RB-block partial norms
-    __shared__ double sh[LZC_THREADS / 32][8];
-    __shared__ double hsh[LZ_KMAX + 1];
-    if (lz[r].done) return;                     // the whole cluster: no block has written lz yet
-    const Seg &s = segs[r];
-    const int n = s.nm3nc11;
-    const long base = s.top_off;
-    const int nb = (n + RB_SPAN - 1) / RB_SPAN, nslot = (nb + LZC_VB - 1) / LZC_VB;
-    const int vb = rank * LZC_HALVES + half;
-    double alpha_j = 0.0;
-    for (int pass = 0; pass < 2; pass++) {
-        for (int sl = 0; sl < nslot; sl++) {
-            const int rb = vb + LZC_VB * sl;
-            const long st = (long)rb * RB_SPAN;
-            const int len = rb < nb ? min(RB_SPAN, n - rb * RB_SPAN) : 0;
-            double qv[RB_EPT];
-#pragma unroll
-            for (int k = 0; k < RB_EPT; k++) {
-                const int e = t + k * RB_THREADS;
-                qv[k] = e < len ? q[base + st + e] : 0.0;
-            }
-            for (int i0 = 0; i0 <= j; i0 += 8) {
-                double v[8];
-#pragma unroll
-                for (int c = 0; c < 8; c++) {
-                    v[c] = 0.0;
-                    if (i0 + c <= j) {
-                        const double *Vi = V + (long)(i0 + c) * ldv + base + st;
-#pragma unroll
-                        for (int k = 0; k < RB_EPT; k++) {
-                            const int e = t + k * RB_THREADS;
-                            if (e < len) v[c] += Vi[e] * qv[k];
-                        }
-                    }
-                }
-#pragma unroll
-                for (int c = 0; c < 8; c++) {
-                    double x = v[c];
-                    for (int o = 16; o > 0; o >>= 1) x += __shfl_down_sync(0xffffffffu, x, o);
-                    if (lane == 0) sh[wid][c] = x;
-                }
-                __syncthreads();
-                if (t < 8 && i0 + t <= j) {
-                    double x = 0.0;
-                    for (int w = 0; w < HW; w++) x += sh[half * HW + w][t];
-                    part[pass][half][sl][i0 + t] = x;
-                }
-                __syncthreads();
-            }
-        }
-        cl.sync();
-        for (int i = threadIdx.x; i <= j; i += LZC_THREADS) {   // h_i over the RB blocks in block order
-            double h = 0.0;
-            for (int rb = 0; rb < nb; rb++) {
-                const int v2 = rb % LZC_VB;
-                h += cl.map_shared_rank(&part[pass][v2 % LZC_HALVES][rb / LZC_VB][0], v2 / LZC_HALVES)[i];
-            }
-            hsh[i] = h;
-        }
-        __syncthreads();
-        for (int sl = 0; sl < nslot; sl++) {                   // q -= sum_i h_i V_i, i = 0..j per element
-            const int rb = vb + LZC_VB * sl;
-            if (rb >= nb) break;
-            const long st = (long)rb * RB_SPAN;
-            const int len = min(RB_SPAN, n - rb * RB_SPAN);
-            for (int k = 0; k < RB_EPT; k++) {
-                const int e = t + k * RB_THREADS;
-                if (e >= len) break;
-                double acc = q[base + st + e];
-                for (int i = 0; i <= j; i++) acc -= hsh[i] * V[(long)i * ldv + base + st + e];
-                q[base + st + e] = acc;
-            }
-        }
-        alpha_j += hsh[j];
-        __syncthreads();
-    }
-    for (int sl = 0; sl < nslot; sl++) {                       // RB-block norms, as seg_dot
-        const int rb = vb + LZC_VB * sl;
-        const long st = (long)rb * RB_SPAN;
-        const int len = rb < nb ? min(RB_SPAN, n - rb * RB_SPAN) : 0;
-        double x = 0.0;
-        for (int e = t; e < len; e += RB_THREADS) x += q[base + st + e] * q[base + st + e];
-        for (int o = 16; o > 0; o >>= 1) x += __shfl_down_sync(0xffffffffu, x, o);
-        if (lane == 0) sh[wid][0] = x;
-        __syncthreads();
-        if (t == 0) {
-            double y = 0.0;
-            for (int w = 0; w < HW; w++) y += sh[half * HW + w][0];
-            npart[half][sl] = y;
-        }
-        __syncthreads();
-    }
-    cl.sync();
-    double nrm2 = 0.0;
-    for (int rb = 0; rb < nb; rb++) {
-        const int v2 = rb % LZC_VB;
-        nrm2 += cl.map_shared_rank(&npart[v2 % LZC_HALVES][rb / LZC_VB], v2 / LZC_HALVES)[0];
-    }
-    cl.sync();                                  // no block leaves while others read its shared memory
-    const double bj = sqrt(nrm2);
-    const bool broken = bj <= 1e-12 * lz[r].b0;
-    if (rank == 0 && threadIdx.x == 0) {
-        alpha[(long)LZ_KMAX * r + j] = alpha_j;
-        lz[r].m = j + 1;
-        if (broken) lz[r].done = 2;             // invariant subspace: finalise with m = j + 1
-        else if (j + 1 < kmax) betad[(long)LZ_KMAX * r + j] = bj;
-    }
-    if (!broken && j + 1 < kmax) {
-        const double inv = bj > 0 ? 1.0 / bj : 0.0;
-        for (int sl = 0; sl < nslot; sl++) {
-            const int rb = vb + LZC_VB * sl;
-            if (rb >= nb) break;
-            const long st = (long)rb * RB_SPAN;
-            const int len = min(RB_SPAN, n - rb * RB_SPAN);
-            for (int e = t; e < len; e += RB_THREADS) V[(long)(j + 1) * ldv + base + st + e] = q[base + st + e] * inv;
-        }
-    }
-}
-
 int lanczos_sqrt(Engine &E, const double *z, double *w, const ps_sqrt_opts *o, ps_sqrt_result *res, cudaStream_t st)
 {
     int kmax = o && o->kmax > 0 ? o->kmax : 40;
@@ -1073,20 +860,17 @@ int lanczos_sqrt(Engine &E, const double *z, double *w, const ps_sqrt_opts *o, p
     long ldv = E.ntop;
     double *V = E.d_lzV, *q = E.d_lzq;
     LzScal *lz = (LzScal *)E.d_lzs;
-    double *h = E.d_lzT;                                    // [R][LZ_KMAX+1]
-    double *alpha = h + (long)(LZ_KMAX + 1) * E.R;          // [R][LZ_KMAX]
+    double *alpha = E.d_lzT;                                // [R][LZ_KMAX]
     double *betad = alpha + (long)LZ_KMAX * E.R;            // [R][LZ_KMAX]
     double *gbuf = betad + (long)LZ_KMAX * E.R;             // [R][LZ_KMAX+1]
     double *nrm2 = gbuf + (long)(LZ_KMAX + 1) * E.R;        // [R]
-    double *h2 = nrm2 + E.R;                                // [R][LZ_KMAX+1]: the second pass's dots
+    // sub-block sums of the reorthogonalisation: both passes' dots, the norm
+    double *part1 = E.d_lzp, *part2 = part1 + (long)LZ_KMAX * RB_EPT * T.nblk;
+    double *npart = part2 + (long)LZ_KMAX * RB_EPT * T.nblk;
     seg_dot(E, T, z, z, nrm2, st);
     ps_launch(k_lz_init, T.nblk, RB_THREADS, 0, st, T, E.d_segs, V, z, lz, nrm2);
     PS_CK(cudaMemsetAsync(gbuf, 0, sizeof(double) * (LZ_KMAX + 1) * E.R, st));
     const int check = 8;   // convergence test every 8 vectors; the cap is handled after the loop
-    // batches that fit one wave of clusters orthogonalise in one cluster launch per vector
-    bool small = (long)E.R * LZC_CTAS <= 128;
-    for (const Seg &sg : E.segs)
-        small = small && (sg.nm3nc11 + RB_SPAN - 1) / RB_SPAN <= LZC_VB * LZC_SLOTS;
     const size_t smem = sizeof(double) * LZE_SMEM;
     PS_CK(cudaFuncSetAttribute(k_lz_check, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
     std::vector<LzScal> hl(E.R);
@@ -1096,19 +880,13 @@ int lanczos_sqrt(Engine &E, const double *z, double *w, const ps_sqrt_opts *o, p
     bool pending = false;
     int j = 0;
     for (j = 0; j < kmax; j++) {
+        const LzDots dots = {V, ldv, j, part1};
         apply_operator(E, 1, V + (long)j * ldv, q, nullptr, E.precision == PS_PREC_MIXED, st, &lz[0].done,
-                       (int)sizeof(LzScal));
-        if (small) {
-            ::ps_launch_count++, k_lz_orth_cluster<<<E.R * LZC_CTAS, LZC_THREADS, 0, st>>>(E.d_segs, V, ldv, q, j, kmax, lz,
-                                                                                       alpha, betad);
-        } else {
-            // two-pass classical Gram-Schmidt in three sweeps over the basis, then the next vector
-            ps_launch(k_lz_dots, T.nblk, RB_THREADS, 0, st, T, V, ldv, q, j, lz, h);
-            ps_launch(k_lz_sub_dots, T.nblk, RB_THREADS, 0, st, T, V, ldv, q, j, lz, h, alpha, h2);
-            ps_launch(k_lz_sub_norm, T.nblk, RB_THREADS, 0, st, T, V, ldv, q, j, lz, h2, alpha, nrm2);
-            if (j + 1 < kmax)
-                ps_launch(k_lz_next, T.nblk, RB_THREADS, 0, st, T, V, ldv, q, j, lz, nrm2, betad);
-        }
+                       (int)sizeof(LzScal), false, &dots);
+        const dim3 sub((unsigned)T.nblk, RB_EPT);
+        ps_launch(k_lz_sub_dots, sub, RB_THREADS, 0, st, T, E.d_segs, V, ldv, q, j, lz, part1, alpha, part2);
+        ps_launch(k_lz_sub_norm, sub, RB_THREADS, 0, st, T, E.d_segs, V, ldv, q, j, lz, part2, alpha, npart);
+        ps_launch(k_lz_next, sub, RB_THREADS, 0, st, T, E.d_segs, V, ldv, q, j, kmax, lz, npart, betad);
         if ((j + 1) % check == 0 && j + 1 < kmax) {
             if (pending) {
                 // the previous check (normally finished long before): apply its outcomes

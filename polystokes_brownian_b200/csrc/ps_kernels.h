@@ -29,6 +29,12 @@ struct RedTable {
     double *d_part = nullptr;    // nblk x 4 partial sums
 };
 
+constexpr int LZ_KMAX = 64;      // cap of the Lanczos basis
+
+// the Lanczos dots that the combine of an apply forms on the way (rows V_0..V_j of leading
+// dimension ldv): sub-block sums, LZ_KMAX per sub-block of the output table
+struct LzDots { const double *V; long ldv; int j; double *part; };
+
 // Per-replica scalars of the lubricated resistance-form PCG.
 struct PcgScal {
     double rz, alpha, beta, tol, err;
@@ -163,7 +169,7 @@ struct Engine {
 
     // Lanczos workspace
     int lz_kmax = 0;
-    double *d_lzV = nullptr, *d_lzT = nullptr, *d_lzw = nullptr, *d_lzq = nullptr;
+    double *d_lzV = nullptr, *d_lzT = nullptr, *d_lzp = nullptr, *d_lzw = nullptr, *d_lzq = nullptr;
     double *d_lzs = nullptr;
 
     cudaStream_t side = nullptr;                   // far field: small pair kernels beside the monomer kernel
@@ -195,8 +201,10 @@ int obs_read(Engine &E, ps_obs_out *out, cudaStream_t st);
 // whose flag is nonzero are skipped by every kernel of the apply.
 // skip_aa: leave out the monomer-monomer pairs -- exact for every colloid row,
 // and for the monomer rows when the monomer inputs are zero.
+// dots (mode 1): the combine also forms the result's dots with the Lanczos basis.
 void apply_operator(Engine &E, int mode, const double *x, double *y, const double *scale, bool fp32, cudaStream_t st,
-                    const void *done = nullptr, int done_stride = 0, bool skip_aa = false);
+                    const void *done = nullptr, int done_stride = 0, bool skip_aa = false,
+                    const LzDots *dots = nullptr);
 int time_pairs(Engine &E, int which, int reps, const double *u, double *ms, cudaStream_t st);
 int fma_peak(int fp64, double *tflops, cudaStream_t st);
 int rsqrt_check(const double *a, long n, unsigned long long *max_ulp, cudaStream_t st);

@@ -716,12 +716,13 @@ __device__ __forceinline__ int find_rep(const int *__restrict__ offs, int R, lon
 // once; blockIdx.y splits an entry's span so that each thread sums one output
 // (a single large replica otherwise leaves most SMs idle while every thread
 // walks its chunk partials four times over).
+template <bool DOTS>
 __global__ void k_combine(const Seg *__restrict__ segs, RedTable T, int mode, const double *__restrict__ x,
                           const double *__restrict__ scale, const double *__restrict__ partAA, int with_aa,
                           const double *__restrict__ partAB, const double *__restrict__ partBB, int nchBB,
                           const double *__restrict__ partBA, const double *__restrict__ delta,
                           const double *__restrict__ lub_y, long part_stride, double *__restrict__ y,
-                          const char *__restrict__ done, int done_stride)
+                          const char *__restrict__ done, int done_stride, LzDots ld)
 {
     pdl_enter();
     const RBlk B = T.d_blk[blockIdx.x];
@@ -730,8 +731,11 @@ __global__ void k_combine(const Seg *__restrict__ segs, RedTable T, int mode, co
     const Seg &sg = segs[r];
     const int xo = mode == 0 ? sg.vec_off : sg.top_off;
     const double s = scale ? scale[r] : 1.0;
-    for (int e = blockIdx.y * blockDim.x + threadIdx.x; e < B.len; e += blockDim.x * gridDim.y) {
-        const long k = (long)B.start + e;
+    // grid.y = RB_EPT: one entry per thread
+    const int e = blockIdx.y * RB_THREADS + threadIdx.x;
+    const long k = (long)B.start + e;
+    double out = 0.0;
+    if (e < B.len) {
         const int i = (int)(k - xo);
         double v = 0.0;
         if (i < sg.nm3nc11) {
@@ -776,7 +780,12 @@ __global__ void k_combine(const Seg *__restrict__ segs, RedTable T, int mode, co
             v = -x[xo + j];
             if (sg.lub_on && lub_y) v -= lub_y[sg.vel_off + j];
         }
-        y[k] = s * v;
+        out = s * v;
+        y[k] = out;
+    }
+    if constexpr (DOTS) {
+        if (blockIdx.y * RB_THREADS < B.len)
+            lz_block_dots(ld.V, ld.ldv, k, e < B.len, out, ld.j, ld.part + (long)LZ_KMAX * (RB_EPT * blockIdx.x + blockIdx.y));
     }
 }
 
@@ -827,7 +836,7 @@ void launch_pairs(Engine &E, const double *u, int in_top, cudaStream_t st, const
 }
 
 void apply_operator(Engine &E, int mode, const double *x, double *y, const double *scale, bool fp32, cudaStream_t st,
-                    const void *done, int done_stride, bool skip_aa)
+                    const void *done, int done_stride, bool skip_aa, const LzDots *dots)
 {
     int in_top = mode == 1;
     const char *dn = (const char *)done;
@@ -839,9 +848,14 @@ void apply_operator(Engine &E, int mode, const double *x, double *y, const doubl
         lub_y = E.d_luby;
     }
     const RedTable &T = mode == 0 ? E.red : E.red_top;
-    ps_launch(k_combine, dim3((unsigned)T.nblk, RB_EPT), RB_THREADS, 0, st,
-            E.d_segs, T, mode, x, scale, E.d_partAA, skip_aa ? 0 : 1, E.d_partAB, E.d_partBB, E.nch_bb,
-            E.d_partBA, E.d_delta, lub_y, E.part_stride, y, dn, done_stride);
+    const dim3 grid((unsigned)T.nblk, RB_EPT);
+    const int with_aa = skip_aa ? 0 : 1;
+    if (dots)
+        ps_launch(k_combine<true>, grid, RB_THREADS, 0, st, E.d_segs, T, mode, x, scale, E.d_partAA, with_aa, E.d_partAB,
+                E.d_partBB, E.nch_bb, E.d_partBA, E.d_delta, lub_y, E.part_stride, y, dn, done_stride, *dots);
+    else
+        ps_launch(k_combine<false>, grid, RB_THREADS, 0, st, E.d_segs, T, mode, x, scale, E.d_partAA, with_aa, E.d_partAB,
+                E.d_partBB, E.nch_bb, E.d_partBA, E.d_delta, lub_y, E.part_stride, y, dn, done_stride, LzDots{});
 }
 
 

@@ -45,3 +45,24 @@ def test_exhausted_krylov_root(x):
     ref = po.sqrtm_eig(M, z)
     assert np.linalg.norm(w.cpu().numpy() - ref) <= 1e-10 * np.linalg.norm(ref)
     b.close()
+
+
+@pytest.mark.parametrize("n", [85, 86, 171, 341, 342, 683])
+def test_root_at_sub_block_edges(n):
+    """Vector lengths around the sub-blocks of 256 and table blocks of 1024 entries.  A dilute
+    cloud is well conditioned (eigenvalues within a factor of a few), so 64 vectors reach
+    rounding: 1e-11 allows for the growth of the basis's rounding errors."""
+    import torch
+    from polystokes_brownian_b200.engine import Batch
+    s = _system(np.random.default_rng(n).uniform(-1.0, 1.0, size=(n, 3)) * 40.0 * n ** (1.0 / 3.0))
+    o = po.OracleSim(po.default_params(**s.params), s.x.ravel())
+    o.stage()
+    M = o.dense_mobility()
+    z = np.random.default_rng(1).normal(size=M.shape[0])
+    lam, Q = np.linalg.eigh(M)
+    ref = (Q * np.sqrt(lam)) @ (Q.T @ z)
+    b = Batch([s])
+    b.stage()
+    w, _ = b.sqrtm(torch.from_numpy(z).cuda(), kmax=64, tol=1e-15)
+    assert np.linalg.norm(w.cpu().numpy() - ref) <= 1e-11 * np.linalg.norm(ref)
+    b.close()
