@@ -54,7 +54,7 @@ static void free_engine(Engine &E)
 {
     void *ptrs[] = {E.d_segs, E.d_vec_offs, E.d_top_offs, E.d_vel_offs, E.d_bead_offs, E.d_x, E.d_q, E.d_xpos0,
                     E.d_xn, E.d_pos64, E.d_pos32, E.d_pos32lo, E.d_aa_te2, E.d_chain, E.d_coll_rep, E.d_chs, E.d_time, E.d_ktrap, E.d_trapinfo,
-                    E.d_aa_tiles, E.d_ab_tiles, E.d_bb_tiles, E.d_partAA, E.d_partAB, E.d_partBB, E.d_partBA,
+                    E.d_aa_tiles, E.d_bb_tiles, E.d_partAA, E.d_partAB, E.d_partBB, E.d_partBA,
                     E.d_tab, E.d_stale, E.d_aa_last, E.d_delta, E.d_schurQ, E.d_schurL, E.d_schur_reps, E.d_ss_reps,
                     E.d_bond_ptr, E.d_bond_nbr, E.d_bond_sgn, E.d_cell, E.d_cell_start, E.d_cell_sorted,
                     E.d_cell_count, E.d_cellgeo, E.d_cell_offs, E.d_nbr_ptr, E.d_nbr, E.d_nbr_count, E.d_lubtab,
@@ -76,9 +76,6 @@ static void free_engine(Engine &E)
     for (void *p : ptrs)
         if (p) cudaFree(p);
     if (E.h_nactive) cudaFreeHost(E.h_nactive);
-    if (E.ev_fork) cudaEventDestroy(E.ev_fork);
-    if (E.ev_join) cudaEventDestroy(E.ev_join);
-    if (E.side) cudaStreamDestroy(E.side);
     if (E.ev_fork2) cudaEventDestroy(E.ev_fork2);
     if (E.ev_chk) cudaEventDestroy(E.ev_chk);
     if (E.side2) cudaStreamDestroy(E.side2);
@@ -98,7 +95,7 @@ static int build(Engine &E, const ps_desc *descs, int R, int precision)
     long bead = 0, coll = 0, vec = 0, top = 0, vel = 0, schur = 0, ba = 0, cells = 0, ssinv = 0;
     std::vector<int> bead_offs(R + 1), vec_offs(R + 1), top_offs(R + 1), vel_offs(R + 1);
     std::vector<long> cell_offs(R + 1);
-    std::vector<Tile> ab, bb;
+    std::vector<Tile> bb;
     std::vector<int> schur_reps, ss_reps, sl_reps;
     long slv = 0;
     int ss_polish = 0;
@@ -166,15 +163,10 @@ static int build(Engine &E, const ps_desc *descs, int R, int precision)
         if (d.mm_HI && ((d.Nm >= 2 && d.aa_mode == PS_AA_REFERENCE) || (d.Nm >= 1 && d.Nc >= 1 && d.ab_mode == PS_AB_REFERENCE))) {
             E.any_indef = true;
         }
-        // tiles
-        s.n_mtiles = (d.Nm + TR - 1) / TR;
+            s.n_mtiles = (d.Nm + TR - 1) / TR;
         s.ba_off = (int)ba;
         if (d.Nc > 0) ba += (long)s.n_mtiles * d.Nc;
-        for (int t = 0; t < s.n_mtiles; t++) {
-            Tile tl = {r, t * TR, std::min(TR, d.Nm - t * TR), t};
-            if (d.Nc > 0) ab.push_back(tl);
-        }
-        if (d.Nc >= 2)
+        if (d.Nm == 0 && d.Nc >= 2)
             for (int t = 0; t * TR < d.Nc; t++) bb.push_back({r, t * TR, std::min(TR, d.Nc - t * TR), t});
         bead_offs[r] = (int)bead; vec_offs[r] = (int)vec; top_offs[r] = (int)top; vel_offs[r] = (int)vel;
         cell_offs[r] = cells;
@@ -183,7 +175,7 @@ static int build(Engine &E, const ps_desc *descs, int R, int precision)
         E.maxNp = std::max(E.maxNp, s.Np);
         if (d.kT > 0) kTpos++; else kTzero++;
         if (d.mm_HI) E.any_mmhi = true;
-        if (d.mm_HI && d.Nm >= 2) (d.aa_mode == PS_AA_RPY ? E.any_aa_rpy : E.any_aa_ref) = true;
+        if (d.Nm > 0) (d.aa_mode == PS_AA_RPY ? E.any_aa_rpy : E.any_aa_ref) = true;
         E.segs[r] = s;
     }
     if (kTpos && kTzero) {
@@ -204,7 +196,7 @@ static int build(Engine &E, const ps_desc *descs, int R, int precision)
         return E.segs[a.rep].Np > E.segs[b.rep].Np || (E.segs[a.rep].Np == E.segs[b.rep].Np && a.rep < b.rep);
     };
     std::stable_sort(bb.begin(), bb.end(), by_cost);
-    E.n_ab_tiles = (int)ab.size(); E.n_bb_tiles = (int)bb.size();
+    E.n_bb_tiles = (int)bb.size();
     // grid extent in chunks: the largest per-replica chunk count
     E.nch_bb = 1;
     for (auto &s : E.segs) E.nch_bb = std::max(E.nch_bb, s.nch_bb);
@@ -216,7 +208,6 @@ static int build(Engine &E, const ps_desc *descs, int R, int precision)
     if ((rc = upload(E.d_vel_offs, vel_offs))) return rc;
     if ((rc = upload(E.d_bead_offs, bead_offs))) return rc;
     if ((rc = upload(E.d_cell_offs, cell_offs))) return rc;
-    if ((rc = upload(E.d_ab_tiles, ab))) return rc;
     if ((rc = upload(E.d_bb_tiles, bb))) return rc;
     if ((rc = upload(E.d_schur_reps, schur_reps))) return rc;
     if ((rc = upload(E.d_ss_reps, ss_reps))) return rc;
@@ -347,12 +338,6 @@ static int build(Engine &E, const ps_desc *descs, int R, int precision)
     TRY_ALLOC(E.d_sinv, sizeof(double) * R);
     TRY_ALLOC(E.d_nactive, sizeof(int));
     PS_CK(cudaMallocHost(&E.h_nactive, sizeof(int)));
-    // side stream for the far field's small pair kernels (monomer-colloid, colloid-colloid),
-    // which run beside the monomer pair kernel; non-blocking so that the legacy default
-    // stream does not serialise it, ordered by the fork and join events only
-    PS_CK(cudaStreamCreateWithFlags(&E.side, cudaStreamNonBlocking));
-    PS_CK(cudaEventCreateWithFlags(&E.ev_fork, cudaEventDisableTiming));
-    PS_CK(cudaEventCreateWithFlags(&E.ev_join, cudaEventDisableTiming));
     // the Lanczos convergence checks run on their own stream beside the next basis vectors
     PS_CK(cudaStreamCreateWithFlags(&E.side2, cudaStreamNonBlocking));
     PS_CK(cudaEventCreateWithFlags(&E.ev_fork2, cudaEventDisableTiming));

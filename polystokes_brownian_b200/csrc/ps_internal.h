@@ -107,8 +107,11 @@ struct Seg {
 // ps_autotune may lower the widest edge, process-wide.
 constexpr int AA_TILE_MIN = 64, AA_TILE_MAX = 256;
 constexpr int aa_tile_edge(int Nm) { return Nm <= 1536 ? 64 : (Nm <= 12288 ? 128 : 256); }
-// one tile pair (I <= J) of a replica's monomer far field, edge S
+// one block of the far field of a replica with monomers: a tile pair (I <= J) of edge S of the
+// monomer far field; S = FAR_AB, monomer tile I against the colloids; S = FAR_BB, colloid row
+// tile I against column chunk J
 struct AaTile { int rep, I, J, S; };
+constexpr int FAR_AB = 0, FAR_BB = -1;
 
 // Column chunk widths of the colloid far field.
 constexpr int BB_CHUNK_COLS = 64;        // colloid columns per chunk, for up to BB_MAX_CHUNKS chunks

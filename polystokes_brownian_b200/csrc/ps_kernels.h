@@ -49,7 +49,7 @@ struct Engine {
     long ntot = 0, ncoll = 0, nvec = 0, ntop = 0, nvel = 0;
     int maxNp = 0;
     bool any_lub = false, any_shell_schur = false, any_kT = false, any_mmhi = false;
-    bool any_aa_ref = false, any_aa_rpy = false;   // monomer HI replicas in the reference's / RPY pair scalars
+    bool any_aa_ref = false, any_aa_rpy = false;   // replicas with monomers in the reference's / RPY pair scalars
 
     Seg *d_segs = nullptr;
     int *d_vec_offs = nullptr, *d_top_offs = nullptr, *d_vel_offs = nullptr, *d_bead_offs = nullptr;
@@ -68,9 +68,9 @@ struct Engine {
     double *d_trapinfo = nullptr;   // per replica: tstop, weaken_trap, unused
 
     // far-field pair work lists
-    Tile *d_ab_tiles = nullptr, *d_bb_tiles = nullptr;
-    AaTile *d_aa_tiles = nullptr;
-    int n_aa_tiles = 0, n_ab_tiles = 0, n_bb_tiles = 0, nch_bb = 1;
+    AaTile *d_aa_tiles = nullptr;    // n_far_pre monomer-colloid and colloid blocks, then n_aa_tiles monomer tile pairs
+    Tile *d_bb_tiles = nullptr;      // colloid row tiles of the replicas without monomers
+    int n_far_pre = 0, n_aa_tiles = 0, n_bb_tiles = 0, nch_bb = 1;
     long part_stride = 0;
     double *d_partAA = nullptr, *d_partAB = nullptr, *d_partBB = nullptr, *d_partBA = nullptr;
     long nba = 0;
@@ -172,8 +172,6 @@ struct Engine {
     double *d_lzV = nullptr, *d_lzT = nullptr, *d_lzp = nullptr, *d_lzw = nullptr, *d_lzq = nullptr;
     double *d_lzs = nullptr;
 
-    cudaStream_t side = nullptr;                   // far field: small pair kernels beside the monomer kernel
-    cudaEvent_t ev_fork = nullptr, ev_join = nullptr;
     cudaStream_t side2 = nullptr;                  // Lanczos convergence checks beside the next basis vectors
     cudaEvent_t ev_fork2 = nullptr, ev_chk = nullptr;
     void *h_spec = nullptr;                        // pinned copy of the checks' outcomes

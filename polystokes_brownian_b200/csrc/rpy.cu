@@ -19,6 +19,214 @@ namespace ps {
 constexpr int RPY_THREADS = 128;
 
 // ---------------------------------------------------------------------------
+// AB/BA: a tile of 128 monomers x the colloids of the replica.  Monomer outputs
+// go to part_m (no chunking: Nc is small whenever Nm > 0); each colloid's output
+// from this tile's monomers is block-reduced into part_ba (one 11-vector per
+// (monomer tile, colloid)).  The blocks are applied in contracted form as for
+// colloid pairs (bb_apply): with S^ the stresslet as a symmetric traceless
+// matrix, v = S^ e and kg = xg + 2 yg,
+//   monomer: T F_c + yb e x T_c + 2 yg v - kg (e.v) e
+//   colloid: T^T F_m, yb F_m x e, flat(yg (e F_m^T + F_m e^T) - kg (e.F_m) e e^T),
+// T = x e e^T + y (1 - e e^T) in RPY mode; in reference mode the replica's stale
+// 3x3 block tab (row-major mob_a[a][b]), nothing on the shell path.
+constexpr int AB_TILE = 128, AB_WARPS = AB_TILE / 32;
+
+// sums of eleven values over the warp by halving exchanges; the lane ends with value idx
+template <class T>
+__device__ __forceinline__ T warp_sum11(const T (&c)[11], int lane, int &idx)
+{
+    T v[8];
+    const bool up = lane & 16;
+#pragma unroll
+    for (int k = 0; k < 8; k++) {
+        const T hi = k < 3 ? c[8 + k] : T(0);
+        v[k] = (up ? hi : c[k]) + __shfl_xor_sync(0xffffffffu, up ? c[k] : hi, 16);
+    }
+#pragma unroll
+    for (int h = 4, o = 8; h >= 1; h >>= 1, o >>= 1) {
+        const bool u = lane & o;
+#pragma unroll
+        for (int k = 0; k < h; k++) v[k] = (u ? v[k + h] : v[k]) + __shfl_xor_sync(0xffffffffu, u ? v[k] : v[k + h], o);
+    }
+    idx = ((lane >> 4) & 1) * 8 + ((lane >> 3) & 1) * 4 + ((lane >> 2) & 1) * 2 + ((lane >> 1) & 1);
+    return v[0] + __shfl_xor_sync(0xffffffffu, v[0], 1);
+}
+
+template <class T>
+__device__ __forceinline__ void ab_block(const Seg &sg, int rep, int mt, const typename V4<T>::t *__restrict__ pos,
+                                         const float4 *__restrict__ plo, const double *__restrict__ u, int uoff,
+                                         const double *__restrict__ tab, double *__restrict__ part_m,
+                                         double *__restrict__ part_ba, T (*red)[AB_WARPS][12])
+{
+    typedef typename V4<T>::t P4;
+    constexpr bool F32 = sizeof(T) == 4;
+    const int Nm = sg.Nm, Nc = sg.Nc, lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
+    const int i = AB_TILE * mt + threadIdx.x;
+    const bool active = threadIdx.x < AB_TILE && i < Nm;
+    const long bi = (long)sg.bead_off + (active ? i : AB_TILE * mt);
+    const P4 pm = pos[bi];
+    T f[3], om[3] = {0, 0, 0};
+    for (int a = 0; a < 3; a++) f[a] = active ? (T)u[uoff + 3 * i + a] : T(0);
+    const int mode = sg.ab_mode;
+    const bool rpy = mode == PS_AB_RPY || mode == PS_AB_RPY_REG, stale = !rpy && sg.mm_HI;
+    const T beta2 = T(sg.beta * sg.beta);
+    for (int cc = 0; cc < Nc; cc++) {
+        if (wid < AB_WARPS) {
+            const P4 pc = pos[sg.bead_off + Nm + cc];
+            T F[3], Q[3], S[5];
+            for (int a = 0; a < 3; a++) {
+                F[a] = (T)u[uoff + sg.nm3 + 3 * cc + a];
+                Q[a] = (T)u[uoff + sg.nm3 + sg.nc3 + 3 * cc + a];
+            }
+            for (int q = 0; q < 5; q++) S[q] = (T)u[uoff + sg.nm3nc6 + 5 * cc + q];
+            T dx = pm.x - pc.x, dy = pm.y - pc.y, dz = pm.z - pc.z;
+            if constexpr (F32) {
+                const float4 lm = plo[bi], lc = plo[sg.bead_off + Nm + cc];
+                dx += lm.x - lc.x; dy += lm.y - lc.y; dz += lm.z - lc.z;
+            }
+            const T r2 = dx * dx + dy * dy + dz * dz, rinv = rsqrt_t<T>(r2);
+            const T e0 = dx * rinv, e1 = dy * rinv, e2 = dz * rinv;
+            T yb, xg, yg;
+            ab_scalars<T>(rinv, beta2, yb, xg, yg);
+            T c[11];
+            if (rpy) {
+                T xa, ya;
+                ab_trans_scalars<T>(r2 * rinv, rinv, T(sg.beta), mode == PS_AB_RPY_REG, xa, ya, yb);
+                const T tF = (xa - ya) * (e0 * F[0] + e1 * F[1] + e2 * F[2]);
+                const T tf = (xa - ya) * (e0 * f[0] + e1 * f[1] + e2 * f[2]);
+                om[0] += ya * F[0] + tF * e0; om[1] += ya * F[1] + tF * e1; om[2] += ya * F[2] + tF * e2;
+                c[0] = ya * f[0] + tf * e0; c[1] = ya * f[1] + tf * e1; c[2] = ya * f[2] + tf * e2;
+            } else {
+                for (int a = 0; a < 3; a++) c[a] = T(0);
+                if (stale)
+                    for (int a = 0; a < 3; a++)
+                        for (int b = 0; b < 3; b++) {
+                            const T t = (T)tab[9 * rep + 3 * a + b];
+                            om[a] += t * F[b];
+                            c[b] += t * f[a];
+                        }
+            }
+            const T kg = xg + T(2) * yg;
+            const T v0 = S[0] * e0 + S[1] * e1 + S[2] * e2, v1 = S[1] * e0 + S[4] * e1 + S[3] * e2;
+            const T v2 = S[2] * e0 + S[3] * e1 - (S[0] + S[4]) * e2;
+            const T ks = kg * (e0 * v0 + e1 * v1 + e2 * v2);
+            om[0] += yb * (e1 * Q[2] - e2 * Q[1]) + T(2) * yg * v0 - ks * e0;
+            om[1] += yb * (e2 * Q[0] - e0 * Q[2]) + T(2) * yg * v1 - ks * e1;
+            om[2] += yb * (e0 * Q[1] - e1 * Q[0]) + T(2) * yg * v2 - ks * e2;
+            c[3] = yb * (f[1] * e2 - f[2] * e1);
+            c[4] = yb * (f[2] * e0 - f[0] * e2);
+            c[5] = yb * (f[0] * e1 - f[1] * e0);
+            const T kf = kg * (e0 * f[0] + e1 * f[1] + e2 * f[2]);
+            const T w0 = T(2) * yg * f[0] - kf * e0, w1 = T(2) * yg * f[1] - kf * e1, w2 = T(2) * yg * f[2] - kf * e2;
+            const T z22 = e2 * w2;                 // Z = (e w^T + w e^T) / 2
+            c[6] = e0 * w0 - z22;
+            c[7] = e0 * w1 + e1 * w0;
+            c[8] = e0 * w2 + e2 * w0;
+            c[9] = e1 * w2 + e2 * w1;
+            c[10] = e1 * w1 - z22;
+            if (!active)
+                for (int q = 0; q < 11; q++) c[q] = T(0);
+            int idx;
+            const T t = warp_sum11<T>(c, lane, idx);
+            if (!(lane & 1) && idx < 11) red[cc & 1][wid][idx] = t;
+        }
+        __syncthreads();                           // two buffers: the next colloid's sums do not overtake these
+        if (threadIdx.x < 11) {
+            T v = 0;
+            for (int w = 0; w < AB_WARPS; w++) v += red[cc & 1][w][threadIdx.x];
+            part_ba[((long)sg.ba_off + (long)mt * Nc + cc) * 11 + threadIdx.x] = (double)v;
+        }
+    }
+    if (active) {
+        double *o = part_m + sg.top_off + 3 * i;
+        for (int a = 0; a < 3; a++) o[a] = (double)om[a];
+    }
+}
+
+// ---------------------------------------------------------------------------
+// BB: colloid rows x colloid columns (FTS, 11 -> 11), FP64.  SPLIT threads per row
+// (a block is SPLIT x RPY_THREADS threads): thread group h takes the tile
+// columns h, h + SPLIT, ...; the groups' sums are joined in group order in
+// shared memory, so a replica of a thousand colloids fills the SMs without
+// more chunk partials.
+struct BbSmem { double4 sp[64]; double su[64 * 11]; };
+
+template <int SPLIT>
+__device__ __forceinline__ void bb_block(const Seg &sg, int rt, int c, const double4 *__restrict__ pos,
+                                         const double *__restrict__ u, int uoff, double *__restrict__ part,
+                                         long part_stride, BbSmem &sm, double (*sred)[11][RPY_THREADS])
+{
+    constexpr int CT = 64;
+    const int row = threadIdx.x % RPY_THREADS, grp = threadIdx.x / RPY_THREADS;
+    const int Nc = sg.Nc, Nm = sg.Nm;
+    const int j0 = (int)((long)Nc * c / sg.nch_bb), j1 = (int)((long)Nc * (c + 1) / sg.nch_bb);
+    const int i = RPY_THREADS * rt + row;
+    const bool active = i < Nc;
+    const double4 pi = pos[sg.bead_off + Nm + (active ? i : RPY_THREADS * rt)];
+    double out[11];   // accumulated over the chunk's column tiles in column order
+    for (int q = 0; q < 11; q++) out[q] = 0.0;
+    for (int jt = j0; jt < j1; jt += CT) {
+        const int nj = min(CT, j1 - jt);
+        __syncthreads();
+        for (int t = threadIdx.x; t < nj * 11; t += blockDim.x) {
+            int k = t / 11, q = t - 11 * k, j = jt + k;
+            int idx = q < 3 ? sg.nm3 + 3 * j + q : (q < 6 ? sg.nm3 + sg.nc3 + 3 * j + (q - 3) : sg.nm3nc6 + 5 * j + (q - 6));
+            sm.su[t] = u[uoff + idx];
+        }
+        if (threadIdx.x < nj) sm.sp[threadIdx.x] = pos[sg.bead_off + Nm + jt + threadIdx.x];
+        __syncthreads();
+        for (int k = grp; k < nj; k += SPLIT) {
+            const int j = jt + k;
+            if (j == i) continue;
+            const double4 pj = sm.sp[k];
+            const bool lo = i < j;
+            double dx = pi.x - pj.x, dy = pi.y - pj.y, dz = pi.z - pj.z;
+            if (!lo) { dx = -dx; dy = -dy; dz = -dz; }
+            const double r2 = dx * dx + dy * dy + dz * dz;
+            const double rinv = rsqrt(r2);
+            const double e[3] = {dx * rinv, dy * rinv, dz * rinv};
+            bb_apply<double>(e, r2 * rinv, rinv, lo, sm.su + 11 * k, out);
+        }
+    }
+    if constexpr (SPLIT > 1) {
+        if (grp > 0)
+            for (int q = 0; q < 11; q++) sred[grp - 1][q][row] = out[q];
+        __syncthreads();
+    }
+    if (grp == 0 && active) {
+        for (int g = 0; g < SPLIT - 1; g++)
+            for (int q = 0; q < 11; q++) out[q] += sred[g][q][row];
+        double *o = part + (long)c * part_stride + sg.top_off;
+        for (int a = 0; a < 3; a++) {
+            o[sg.nm3 + 3 * i + a] = out[a];
+            o[sg.nm3 + sg.nc3 + 3 * i + a] = out[3 + a];
+        }
+        for (int q = 0; q < 5; q++) o[sg.nm3nc6 + 5 * i + q] = out[6 + q];
+    }
+}
+
+// Colloid pairs of the replicas without monomers (suspensions); those beside
+// monomers ride in the monomer kernels' launches.
+constexpr int BB_SPLIT = 4;
+__global__ void __launch_bounds__(RPY_THREADS * BB_SPLIT)
+k_rpy_bb(const Seg *__restrict__ segs, const Tile *__restrict__ tiles, const double4 *__restrict__ pos,
+         const double *__restrict__ u, int in_top, double *__restrict__ part, long part_stride,
+         const char *__restrict__ done, int done_stride)
+{
+    pdl_enter();
+    const Tile tl = tiles[blockIdx.x];
+    if (done && *(const int *)(done + (long)tl.rep * done_stride)) return;
+    __shared__ BbSmem sm;
+    __shared__ double sred[BB_SPLIT - 1][11][RPY_THREADS];
+    const Seg &sg = segs[tl.rep];
+    if ((int)blockIdx.y >= sg.nch_bb) return;
+    bb_block<BB_SPLIT>(sg, tl.mtile, blockIdx.y, pos, u, in_top ? sg.top_off : sg.vec_off, part, part_stride, sm, sred);
+}
+
+// The partial sums of one apply, as the far-field kernels write them.
+struct FarOut { double *aa, *ab, *ba, *bb; const double *tab; long bb_stride; };
+
+// ---------------------------------------------------------------------------
 // Monomer-monomer far field (AA), each unordered pair once.  The pair block is
 // symmetric, so one evaluation of the geometry serves U_i += M_ij u_j and
 // U_j += M_ij u_i: 32 FMA-pipe operations per unordered pair against 2 x 22 when
@@ -186,8 +394,7 @@ template <bool REF>
 __global__ void __launch_bounds__(AAF_THREADS, 4)
 k_rpy_aa_f2(const Seg *__restrict__ segs, const AaTile *__restrict__ tiles, const float4 *__restrict__ pos,
             const float4 *__restrict__ plo, const float *__restrict__ aa_te2, const double4 *__restrict__ p64,
-            const double *__restrict__ u, int in_top, double *__restrict__ part, const char *__restrict__ done,
-            int done_stride)
+            const double *__restrict__ u, int in_top, FarOut O, const char *__restrict__ done, int done_stride)
 {
     pdl_enter();
     const AaTile tl = tiles[blockIdx.x];
@@ -195,9 +402,26 @@ k_rpy_aa_f2(const Seg *__restrict__ segs, const AaTile *__restrict__ tiles, cons
     const Seg &sg = segs[tl.rep];
     // one instance per pair-scalar family: the reference's scalars take the FP64 branch decision
     if ((sg.aa_mode == PS_AA_REFERENCE) != REF) return;
-    __shared__ float4 sCols[5][AA_TILE_MAX / 2];           // sXY, sZU, sUU, sLA, sLB
-    __shared__ float sCol[3 * 4 * AA_TILE_MAX];            // column sums per row group or band
-    __shared__ double sRow[3 * AA_TILE_MAX];               // row sums per column group or band (3 S slots in all)
+    __shared__ union {
+        struct {
+            float4 cols[5][AA_TILE_MAX / 2];               // sXY, sZU, sUU, sLA, sLB
+            float col[3 * 4 * AA_TILE_MAX];                // column sums per row group or band
+            double row[3 * AA_TILE_MAX];                   // row sums per column group or band (3 S slots in all)
+        } aa;
+        float red[2][AB_WARPS][12];
+        BbSmem bb;
+    } sm;
+    if (tl.S == FAR_AB) {
+        ab_block<float>(sg, tl.rep, tl.I, pos, plo, u, in_top ? sg.top_off : sg.vec_off, O.tab, O.ab, O.ba, sm.red);
+        return;
+    }
+    if (tl.S == FAR_BB) {
+        bb_block<1>(sg, tl.I, tl.J, p64, u, in_top ? sg.top_off : sg.vec_off, O.bb, O.bb_stride, sm.bb, nullptr);
+        return;
+    }
+    float4 (&sCols)[5][AA_TILE_MAX / 2] = sm.aa.cols;
+    float *sCol = sm.aa.col;
+    double *sRow = sm.aa.row;
     const int Nm = sg.Nm, S = tl.S, tid = threadIdx.x, lane = tid & 31, w = tid >> 5;
     const int i0 = tl.I * S, j0 = tl.J * S;
     const int uoff = in_top ? sg.top_off : sg.vec_off;
@@ -276,7 +500,7 @@ k_rpy_aa_f2(const Seg *__restrict__ segs, const AaTile *__restrict__ tiles, cons
         }
     }
     __syncthreads();
-    double *oI = part + sg.paa_off + (long)tl.J * sg.nm3 + 3 * i0, *oJ = part + sg.paa_off + (long)tl.I * sg.nm3 + 3 * j0;
+    double *oI = O.aa + sg.paa_off + (long)tl.J * sg.nm3 + 3 * i0, *oJ = O.aa + sg.paa_off + (long)tl.I * sg.nm3 + 3 * j0;
     for (int e = tid; e < 3 * S; e += AAF_THREADS) {
         if (3 * i0 + e < sg.nm3) {
             double v = 0.0;
@@ -392,18 +616,33 @@ constexpr int AAD_THREADS = 256;
 
 __global__ void __launch_bounds__(AAD_THREADS, 2)
 k_rpy_aa_d2(const Seg *__restrict__ segs, const AaTile *__restrict__ tiles, const double4 *__restrict__ pos,
-            const double *__restrict__ u, int in_top, double *__restrict__ part, const char *__restrict__ done,
-            int done_stride)
+            const double *__restrict__ u, int in_top, FarOut O, const char *__restrict__ done, int done_stride)
 {
     pdl_enter();
     const AaTile tl = tiles[blockIdx.x];
     if (done && *(const int *)(done + (long)tl.rep * done_stride)) return;
-    // columns (x, y | z, u0 | u1, u2 | chain), then the row sums in the same space
-    __shared__ double2 sCols[3][AA_TILE_MAX];
-    __shared__ double sW[AA_TILE_MAX], sCol[3 * 4 * AA_TILE_MAX];
-    double *sRow = reinterpret_cast<double *>(sCols);      // row sums per column group or band: 1536 doubles
-    static_assert(sizeof(sCols) >= 1536 * sizeof(double), "row sums alias the columns");
+    __shared__ union {
+        struct {
+            double2 cols[3][AA_TILE_MAX];                  // x, y | z, u0 | u1, u2; then the row sums in the same space
+            double w[AA_TILE_MAX], col[3 * 4 * AA_TILE_MAX];   // chain ids; column sums per row group or band
+        } aa;
+        double red[2][AB_WARPS][12];
+        struct { BbSmem t; double sred[AAD_THREADS / RPY_THREADS - 1][11][RPY_THREADS]; } bb;
+    } sm;
     const Seg &sg = segs[tl.rep];
+    if (tl.S == FAR_AB) {
+        ab_block<double>(sg, tl.rep, tl.I, pos, nullptr, u, in_top ? sg.top_off : sg.vec_off, O.tab, O.ab, O.ba, sm.red);
+        return;
+    }
+    if (tl.S == FAR_BB) {
+        bb_block<AAD_THREADS / RPY_THREADS>(sg, tl.I, tl.J, pos, u, in_top ? sg.top_off : sg.vec_off, O.bb, O.bb_stride,
+                                            sm.bb.t, sm.bb.sred);
+        return;
+    }
+    double2 (&sCols)[3][AA_TILE_MAX] = sm.aa.cols;
+    double *sW = sm.aa.w, *sCol = sm.aa.col;
+    double *sRow = reinterpret_cast<double *>(sCols);      // row sums per column group or band: 1536 doubles
+    static_assert(sizeof(sm.aa.cols) >= 1536 * sizeof(double), "row sums alias the columns");
     const int Nm = sg.Nm, S = tl.S, tid = threadIdx.x, lane = tid & 31, w = tid >> 5;
     const int i0 = tl.I * S, j0 = tl.J * S;
     const int uoff = in_top ? sg.top_off : sg.vec_off;
@@ -481,7 +720,7 @@ k_rpy_aa_d2(const Seg *__restrict__ segs, const AaTile *__restrict__ tiles, cons
         for (int a = 0; a < 3; a++) { o3[a] = racc[a]; o3[96 + a] = racc[3 + a]; }
     }
     __syncthreads();
-    double *oI = part + sg.paa_off + (long)tl.J * sg.nm3 + 3 * i0, *oJ = part + sg.paa_off + (long)tl.I * sg.nm3 + 3 * j0;
+    double *oI = O.aa + sg.paa_off + (long)tl.J * sg.nm3 + 3 * i0, *oJ = O.aa + sg.paa_off + (long)tl.I * sg.nm3 + 3 * j0;
     for (int e = tid; e < 3 * S; e += AAD_THREADS) {
         if (3 * i0 + e < sg.nm3) {
             double v = 0.0;
@@ -505,195 +744,6 @@ __global__ void k_rsqrt_check(long n, const double *__restrict__ a, unsigned lon
     const double ref = rsqrt(a[i]), own = rsqrt_seeded(a[i]);
     long long d = __double_as_longlong(own) - __double_as_longlong(ref);
     atomicMax(worst, (unsigned long long)(d < 0 ? -d : d));
-}
-
-// ---------------------------------------------------------------------------
-// AB/BA: monomer rows x colloids of the same replica.  Monomer outputs go to
-// part_m (no chunking: Nc is small whenever Nm > 0); each colloid's output from
-// this tile's monomers is block-reduced into part_ba (one 11-vector per
-// (monomer tile, colloid)).  tab: per-replica 3x3 translational block
-// (reference mode, row-major mob_a[a][b]); ignored in RPY mode.
-template <class T>
-__global__ void __launch_bounds__(RPY_THREADS)
-k_rpy_ab(const Seg *__restrict__ segs, const Tile *__restrict__ tiles, const typename V4<T>::t *__restrict__ pos,
-         const float4 *__restrict__ plo, const double *__restrict__ u, int in_top, const double *__restrict__ tab,
-         double *__restrict__ part_m, double *__restrict__ part_ba, const char *__restrict__ done, int done_stride)
-{
-    pdl_enter();
-    if (done && *(const int *)(done + (long)tiles[blockIdx.x].rep * done_stride)) return;
-    typedef typename V4<T>::t P4;
-    constexpr bool F32 = sizeof(T) == 4;
-    __shared__ T red[RPY_THREADS / 32][12];
-    const Tile tl = tiles[blockIdx.x];
-    const Seg &sg = segs[tl.rep];
-    const int i = tl.row0 + threadIdx.x;
-    const bool active = threadIdx.x < tl.nrow;
-    const int uoff = in_top ? sg.top_off : sg.vec_off;
-    const int Nm = sg.Nm, Nc = sg.Nc;
-    P4 pm = pos[sg.bead_off + (active ? i : tl.row0)];
-    T fm[3];
-    for (int a = 0; a < 3; a++) fm[a] = active ? (T)u[uoff + 3 * i + a] : T(0);
-    T Tm[9];
-    const int mode = sg.ab_mode;
-    const bool shell = !sg.mm_HI;
-    for (int a = 0; a < 9; a++) Tm[a] = (T)tab[9 * tl.rep + a];
-    const T beta2 = T(sg.beta * sg.beta);
-    T om0 = 0, om1 = 0, om2 = 0;
-    const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
-    for (int cc = 0; cc < Nc; cc++) {
-        P4 pc = pos[sg.bead_off + Nm + cc];
-        T Fc[3], Tc[3], Sc[5];
-        for (int a = 0; a < 3; a++) {
-            Fc[a] = (T)u[uoff + sg.nm3 + 3 * cc + a];
-            Tc[a] = (T)u[uoff + sg.nm3 + sg.nc3 + 3 * cc + a];
-        }
-        for (int q = 0; q < 5; q++) Sc[q] = (T)u[uoff + sg.nm3nc6 + 5 * cc + q];
-        T dx = pm.x - pc.x, dy = pm.y - pc.y, dz = pm.z - pc.z;
-        if constexpr (F32) {
-            float4 lm = plo[sg.bead_off + (active ? i : tl.row0)], lc = plo[sg.bead_off + Nm + cc];
-            dx += lm.x - lc.x; dy += lm.y - lc.y; dz += lm.z - lc.z;
-        }
-        T r2 = dx * dx + dy * dy + dz * dz;
-        T rinv = rsqrt_t<T>(r2);
-        T e[3] = {dx * rinv, dy * rinv, dz * rinv};
-        T yb, xg, yg;
-        ab_scalars<T>(rinv, beta2, yb, xg, yg);
-        T G[15];
-        gt_flat<T>(e, xg, yg, G);
-        T TT[9];
-        if (mode == PS_AB_RPY || mode == PS_AB_RPY_REG) {
-            T xa, ya;
-            ab_trans_scalars<T>(r2 * rinv, rinv, T(sg.beta), mode == PS_AB_RPY_REG, xa, ya, yb);
-            for (int a = 0; a < 3; a++)
-                for (int b = 0; b < 3; b++) TT[a * 3 + b] = xa * e[a] * e[b] + ya * ((a == b ? T(1) : T(0)) - e[a] * e[b]);
-        } else if (shell) {
-            for (int a = 0; a < 9; a++) TT[a] = T(0);
-        } else {
-            for (int a = 0; a < 9; a++) TT[a] = Tm[a];
-        }
-        // monomer row: T F_c + B^T T_c + G S_c, B^T v = yb (e x v)
-        T btx = yb * (e[1] * Tc[2] - e[2] * Tc[1]);
-        T bty = yb * (e[2] * Tc[0] - e[0] * Tc[2]);
-        T btz = yb * (e[0] * Tc[1] - e[1] * Tc[0]);
-        T gs[3];
-        for (int a = 0; a < 3; a++) {
-            T acc = 0;
-            for (int q = 0; q < 5; q++) acc += G[a * 5 + q] * Sc[q];
-            gs[a] = acc;
-        }
-        om0 += TT[0] * Fc[0] + TT[1] * Fc[1] + TT[2] * Fc[2] + btx + gs[0];
-        om1 += TT[3] * Fc[0] + TT[4] * Fc[1] + TT[5] * Fc[2] + bty + gs[1];
-        om2 += TT[6] * Fc[0] + TT[7] * Fc[1] + TT[8] * Fc[2] + btz + gs[2];
-        // colloid row from this monomer: [T^T F_m ; B F_m ; G^T F_m], B v = yb (v x e)
-        T cv[11];
-        for (int a = 0; a < 3; a++) cv[a] = TT[0 * 3 + a] * fm[0] + TT[1 * 3 + a] * fm[1] + TT[2 * 3 + a] * fm[2];
-        cv[3] = yb * (fm[1] * e[2] - fm[2] * e[1]);
-        cv[4] = yb * (fm[2] * e[0] - fm[0] * e[2]);
-        cv[5] = yb * (fm[0] * e[1] - fm[1] * e[0]);
-        for (int q = 0; q < 5; q++) cv[6 + q] = G[0 * 5 + q] * fm[0] + G[1 * 5 + q] * fm[1] + G[2 * 5 + q] * fm[2];
-        if (!active)
-            for (int q = 0; q < 11; q++) cv[q] = T(0);
-        // deterministic block reduction
-        for (int q = 0; q < 11; q++) {
-            T v = cv[q];
-            for (int o = 16; o > 0; o >>= 1) v += __shfl_down_sync(0xffffffffu, v, o);
-            if (lane == 0) red[wid][q] = v;
-        }
-        __syncthreads();
-        if (threadIdx.x < 11) {
-            T v = 0;
-            for (int w = 0; w < RPY_THREADS / 32; w++) v += red[w][threadIdx.x];
-            part_ba[((long)sg.ba_off + (long)tl.mtile * Nc + cc) * 11 + threadIdx.x] = (double)v;
-        }
-        __syncthreads();
-    }
-    if (active) {
-        double *o = part_m + sg.top_off + 3 * i;
-        o[0] = (double)om0; o[1] = (double)om1; o[2] = (double)om2;
-    }
-}
-
-// ---------------------------------------------------------------------------
-// BB: colloid rows x colloid columns (FTS, 11 -> 11).  BB_SPLIT threads per row
-// (a block is BB_SPLIT x RPY_THREADS threads): thread group h takes the tile
-// columns h, h + BB_SPLIT, ...; the groups' sums are joined in group order in
-// shared memory, so a replica of a thousand colloids fills the SMs without
-// more chunk partials.
-constexpr int BB_SPLIT = 4;
-template <class T>
-__global__ void __launch_bounds__(RPY_THREADS * BB_SPLIT)
-k_rpy_bb(const Seg *__restrict__ segs, const Tile *__restrict__ tiles, const typename V4<T>::t *__restrict__ pos,
-         const float4 *__restrict__ plo, const double *__restrict__ u, int in_top, double *__restrict__ part,
-         long part_stride, int nchunk, const char *__restrict__ done, int done_stride)
-{
-    pdl_enter();
-    if (done && *(const int *)(done + (long)tiles[blockIdx.x].rep * done_stride)) return;
-    typedef typename V4<T>::t P4;
-    constexpr bool F32 = sizeof(T) == 4;
-    constexpr int CT = 64;
-    __shared__ P4 sp[CT];
-    __shared__ float4 sl[F32 ? CT : 1];
-    __shared__ T su[CT * 11];
-    __shared__ T sred[BB_SPLIT - 1][11][RPY_THREADS];
-    const Tile tl = tiles[blockIdx.x];
-    const Seg &sg = segs[tl.rep];
-    const int c = blockIdx.y;
-    nchunk = sg.nch_bb;
-    if (c >= nchunk) return;
-    const int row = threadIdx.x % RPY_THREADS, grp = threadIdx.x / RPY_THREADS;
-    const int Nc = sg.Nc, Nm = sg.Nm;
-    const int j0 = (int)((long)Nc * c / nchunk), j1 = (int)((long)Nc * (c + 1) / nchunk);
-    const int i = tl.row0 + row;
-    const bool active = row < tl.nrow;
-    const int uoff = in_top ? sg.top_off : sg.vec_off;
-    P4 pi = pos[sg.bead_off + Nm + (active ? i : tl.row0)];
-    float4 li = make_float4(0.f, 0.f, 0.f, 0.f);
-    if constexpr (F32) li = plo[sg.bead_off + Nm + (active ? i : tl.row0)];
-    T out[11];   // accumulated over the chunk's column tiles in column order
-    for (int q = 0; q < 11; q++) out[q] = T(0);
-    for (int jt = j0; jt < j1; jt += CT) {
-        int nj = min(CT, j1 - jt);
-        __syncthreads();
-        for (int t = threadIdx.x; t < nj * 11; t += blockDim.x) {
-            int k = t / 11, q = t - 11 * k, j = jt + k;
-            int idx = q < 3 ? sg.nm3 + 3 * j + q : (q < 6 ? sg.nm3 + sg.nc3 + 3 * j + (q - 3) : sg.nm3nc6 + 5 * j + (q - 6));
-            su[t] = (T)u[uoff + idx];
-        }
-        if (threadIdx.x < nj) {
-            sp[threadIdx.x] = pos[sg.bead_off + Nm + jt + threadIdx.x];
-            if constexpr (F32) sl[threadIdx.x] = plo[sg.bead_off + Nm + jt + threadIdx.x];
-        }
-        __syncthreads();
-        for (int k = grp; k < nj; k += BB_SPLIT) {
-            int j = jt + k;
-            if (j == i) continue;
-            P4 pj = sp[k];
-            bool lo = i < j;
-            T dx = pi.x - pj.x, dy = pi.y - pj.y, dz = pi.z - pj.z;
-            if constexpr (F32) {
-                float4 lj = sl[k];
-                dx += li.x - lj.x; dy += li.y - lj.y; dz += li.z - lj.z;
-            }
-            if (!lo) { dx = -dx; dy = -dy; dz = -dz; }
-            T r2 = dx * dx + dy * dy + dz * dz;
-            T rinv = rsqrt_t<T>(r2);
-            T e[3] = {dx * rinv, dy * rinv, dz * rinv};
-            bb_apply<T>(e, r2 * rinv, rinv, lo, su + 11 * k, out);
-        }
-    }
-    if (grp > 0)
-        for (int q = 0; q < 11; q++) sred[grp - 1][q][row] = out[q];
-    __syncthreads();
-    if (grp == 0 && active) {
-        for (int g = 0; g < BB_SPLIT - 1; g++)
-            for (int q = 0; q < 11; q++) out[q] += sred[g][q][row];
-        double *o = part + (long)c * part_stride + sg.top_off;
-        for (int a = 0; a < 3; a++) {
-            o[sg.nm3 + 3 * i + a] = (double)out[a];
-            o[sg.nm3 + sg.nc3 + 3 * i + a] = (double)out[3 + a];
-        }
-        for (int q = 0; q < 5; q++) o[sg.nm3nc6 + 5 * i + q] = (double)out[6 + q];
-    }
 }
 
 // ---------------------------------------------------------------------------
@@ -791,48 +841,36 @@ __global__ void k_combine(const Seg *__restrict__ segs, RedTable T, int mode, co
 
 // ---------------------------------------------------------------------------
 // host launchers
-template <class T>
-void launch_pairs(Engine &E, const double *u, int in_top, cudaStream_t st, const char *done, int dstride, bool skip_aa)
+// Far-field blocks of the replicas with monomers: monomer-colloid and colloid-colloid
+// blocks first (E.n_far_pre of them), then the monomer tile pairs, in one launch per
+// pair-scalar family (they were three launches, two of them on a side stream: 6 us of
+// fork and join on an apply of 12 us).  Colloid-colloid FTS blocks stay FP64 in the mixed
+// form: near contact the far-field FTS mobility is ill-conditioned and FP32 blocks leave a
+// 1.2e-6 velocity error on a suspension at gap 0.01 (FP64: tracks rtol); they are cheap
+// wherever monomers carry the O(N^2) work.
+static void launch_far(Engine &E, const double *u, int in_top, bool fp32, int first, int n, cudaStream_t st,
+                       const char *done, int dstride)
 {
-    const typename V4<T>::t *pos = (const typename V4<T>::t *)(sizeof(T) == 8 ? (const void *)E.d_pos64 : (const void *)E.d_pos32);
-    // the monomer-colloid and colloid-colloid kernels (a few microseconds each, few blocks)
-    // run on the side stream beside the monomer kernel; they write their own partials,
-    // and the join orders them before the combine
-    const bool fork = E.side && E.n_aa_tiles && !skip_aa && (E.n_ab_tiles || E.n_bb_tiles);
-    cudaStream_t ss = st;
-    if (fork) {
-        cudaEventRecord(E.ev_fork, st);
-        cudaStreamWaitEvent(E.side, E.ev_fork, 0);
-        ss = E.side;
+    if (n <= 0) return;
+    const FarOut O = {E.d_partAA, E.d_partAB, E.d_partBA, E.d_partBB, E.d_tab, E.part_stride};
+    const AaTile *tiles = E.d_aa_tiles + first;
+    if (!fp32) {
+        ps_launch(k_rpy_aa_d2, n, AAD_THREADS, 0, st, E.d_segs, tiles, E.d_pos64, u, in_top, O, done, dstride);
+        return;
     }
-    if (E.n_aa_tiles && !skip_aa) {
-        if constexpr (sizeof(T) == 4)
-        {
-            if (E.any_aa_rpy)
-                ps_launch(k_rpy_aa_f2<false>, E.n_aa_tiles, AAF_THREADS, 0, st, E.d_segs, E.d_aa_tiles, E.d_pos32,
-                        E.d_pos32lo, E.d_aa_te2, E.d_pos64, u, in_top, E.d_partAA, done, dstride);
-            if (E.any_aa_ref)
-                ps_launch(k_rpy_aa_f2<true>, E.n_aa_tiles, AAF_THREADS, 0, st, E.d_segs, E.d_aa_tiles, E.d_pos32,
-                        E.d_pos32lo, E.d_aa_te2, E.d_pos64, u, in_top, E.d_partAA, done, dstride);
-        }
-        else
-            ps_launch(k_rpy_aa_d2, E.n_aa_tiles, AAD_THREADS, 0, st,
-                    E.d_segs, E.d_aa_tiles, E.d_pos64, u, in_top, E.d_partAA, done, dstride);
-    }
-    if (E.n_ab_tiles)
-        ps_launch(k_rpy_ab<T>, E.n_ab_tiles, RPY_THREADS, 0, ss, E.d_segs, E.d_ab_tiles, pos, E.d_pos32lo, u, in_top, E.d_tab, E.d_partAB,
-                E.d_partBA, done, dstride);
-    // colloid-colloid FTS blocks stay FP64 in the mixed form: near contact the
-    // far-field FTS mobility is ill-conditioned and FP32 blocks leave a 1.2e-6
-    // velocity error on a suspension at gap 0.01 (FP64: tracks rtol); they are
-    // cheap wherever monomers carry the O(N^2) work
+    if (E.any_aa_rpy)
+        ps_launch(k_rpy_aa_f2<false>, n, AAF_THREADS, 0, st, E.d_segs, tiles, E.d_pos32, E.d_pos32lo, E.d_aa_te2, E.d_pos64,
+                u, in_top, O, done, dstride);
+    if (E.any_aa_ref)
+        ps_launch(k_rpy_aa_f2<true>, n, AAF_THREADS, 0, st, E.d_segs, tiles, E.d_pos32, E.d_pos32lo, E.d_aa_te2, E.d_pos64,
+                u, in_top, O, done, dstride);
+}
+
+static void launch_bb(Engine &E, const double *u, int in_top, cudaStream_t st, const char *done, int dstride)
+{
     if (E.n_bb_tiles)
-        ps_launch(k_rpy_bb<double>, dim3(E.n_bb_tiles, E.nch_bb), RPY_THREADS * BB_SPLIT, 0, ss,
-                E.d_segs, E.d_bb_tiles, E.d_pos64, E.d_pos32lo, u, in_top, E.d_partBB, E.part_stride, E.nch_bb, done, dstride);
-    if (fork) {
-        cudaEventRecord(E.ev_join, E.side);
-        cudaStreamWaitEvent(st, E.ev_join, 0);
-    }
+        ps_launch(k_rpy_bb, dim3(E.n_bb_tiles, E.nch_bb), RPY_THREADS * BB_SPLIT, 0, st, E.d_segs, E.d_bb_tiles, E.d_pos64,
+                u, in_top, E.d_partBB, E.part_stride, done, dstride);
 }
 
 void apply_operator(Engine &E, int mode, const double *x, double *y, const double *scale, bool fp32, cudaStream_t st,
@@ -840,8 +878,8 @@ void apply_operator(Engine &E, int mode, const double *x, double *y, const doubl
 {
     int in_top = mode == 1;
     const char *dn = (const char *)done;
-    if (fp32) launch_pairs<float>(E, x, in_top, st, dn, done_stride, skip_aa);
-    else launch_pairs<double>(E, x, in_top, st, dn, done_stride, skip_aa);
+    launch_far(E, x, in_top, fp32, 0, E.n_far_pre + (skip_aa ? 0 : E.n_aa_tiles), st, dn, done_stride);
+    launch_bb(E, x, in_top, st, dn, done_stride);
     const double *lub_y = nullptr;
     if (mode == 0 && E.any_lub) {
         lub_apply(E, x, E.d_luby, st);
@@ -865,7 +903,7 @@ int g_aa_chunk_cols = AA_TILE_MAX;
 // partial slots, the list of tile pairs (large tiles first) and the partial buffer
 int set_aa_chunking(Engine &E, int cols)
 {
-    std::vector<AaTile> tiles;
+    std::vector<AaTile> pre, tiles;
     long off = 0;
     for (int r = 0; r < E.R; r++) {
         Seg &s = E.segs[r];
@@ -876,9 +914,18 @@ int set_aa_chunking(Engine &E, int cols)
         off += (long)s.aa_nt * s.nm3;
         for (int i = 0; i < s.aa_nt; i++)
             for (int j = i; j < s.aa_nt; j++) tiles.push_back({r, i, j, S});
+        if (s.Nm > 0) {
+            if (s.Nc > 0)
+                for (int t = 0; t < s.n_mtiles; t++) pre.push_back({r, t, 0, FAR_AB});
+            if (s.Nc >= 2)
+                for (int t = 0; t * RPY_THREADS < s.Nc; t++)
+                    for (int c = 0; c < s.nch_bb; c++) pre.push_back({r, t, c, FAR_BB});
+        }
     }
     std::stable_sort(tiles.begin(), tiles.end(), [](const AaTile &a, const AaTile &b) { return a.S > b.S; });
     E.n_aa_tiles = (int)tiles.size();
+    E.n_far_pre = (int)pre.size();
+    tiles.insert(tiles.begin(), pre.begin(), pre.end());
     PS_CK(cudaDeviceSynchronize());
     cudaFree(E.d_partAA);
     cudaFree(E.d_aa_tiles);
@@ -897,26 +944,21 @@ int set_aa_chunking(Engine &E, int cols)
 
 // ---------------------------------------------------------------------------
 // diagnostics: average duration (CUDA events on `st`) of one far-field kernel
-// which: 0 AA pair kernel, 1 AB/BA kernel, 2 BB kernel, 3 whole mobility apply
+// which: 0 monomer pairs, 1 monomer-colloid pairs and the colloid pairs beside monomers, 2 colloid pairs of
+// replicas without monomers, 3 whole mobility apply
 int time_pairs(Engine &E, int which, int reps, const double *u, double *ms, cudaStream_t st)
 {
     bool fp32 = E.precision == PS_PREC_MIXED;
-    const void *pos = fp32 ? (const void *)E.d_pos32 : (const void *)E.d_pos64;
     cudaEvent_t a, b;
     cudaEventCreate(&a);
     cudaEventCreate(&b);
     auto launch = [&]() {
-        if (which == 0 && E.n_aa_tiles) {
-            if (fp32) {
-                if (E.any_aa_rpy) ps_launch(k_rpy_aa_f2<false>, E.n_aa_tiles, AAF_THREADS, 0, st, E.d_segs, E.d_aa_tiles, (const float4 *)pos, E.d_pos32lo, E.d_aa_te2, E.d_pos64, u, 1, E.d_partAA, nullptr, 0);
-                if (E.any_aa_ref) ps_launch(k_rpy_aa_f2<true>, E.n_aa_tiles, AAF_THREADS, 0, st, E.d_segs, E.d_aa_tiles, (const float4 *)pos, E.d_pos32lo, E.d_aa_te2, E.d_pos64, u, 1, E.d_partAA, nullptr, 0);
-            }
-            else ps_launch(k_rpy_aa_d2, E.n_aa_tiles, AAD_THREADS, 0, st, E.d_segs, E.d_aa_tiles, E.d_pos64, u, 1, E.d_partAA, nullptr, 0);
-        } else if (which == 1 && E.n_ab_tiles) {
-            if (fp32) ps_launch(k_rpy_ab<float>, E.n_ab_tiles, RPY_THREADS, 0, st, E.d_segs, E.d_ab_tiles, (const float4 *)pos, E.d_pos32lo, u, 1, E.d_tab, E.d_partAB, E.d_partBA, nullptr, 0);
-            else ps_launch(k_rpy_ab<double>, E.n_ab_tiles, RPY_THREADS, 0, st, E.d_segs, E.d_ab_tiles, (const double4 *)pos, E.d_pos32lo, u, 1, E.d_tab, E.d_partAB, E.d_partBA, nullptr, 0);
-        } else if (which == 2 && E.n_bb_tiles) {
-            ps_launch(k_rpy_bb<double>, dim3(E.n_bb_tiles, E.nch_bb), RPY_THREADS * BB_SPLIT, 0, st, E.d_segs, E.d_bb_tiles, E.d_pos64, E.d_pos32lo, u, 1, E.d_partBB, E.part_stride, E.nch_bb, nullptr, 0);
+        if (which == 0) {
+            launch_far(E, u, 1, fp32, E.n_far_pre, E.n_aa_tiles, st, nullptr, 0);
+        } else if (which == 1) {
+            launch_far(E, u, 1, fp32, 0, E.n_far_pre, st, nullptr, 0);
+        } else if (which == 2) {
+            launch_bb(E, u, 1, st, nullptr, 0);
         } else if (which == 3) {
             apply_operator(E, 1, u, E.d_tmp_top2, nullptr, fp32, st);
         }
