@@ -59,7 +59,7 @@ static void free_engine(Engine &E)
                     E.d_bond_ptr, E.d_bond_nbr, E.d_bond_sgn, E.d_cell, E.d_cell_start, E.d_cell_sorted,
                     E.d_cell_count, E.d_cellgeo, E.d_cell_offs, E.d_nbr_ptr, E.d_nbr, E.d_nbr_count, E.d_lubtab,
                     E.d_luby, E.d_lub_diag, E.d_lub_ptr, E.d_lub_nbr, E.d_lub_cidx, E.d_tmp_vel, E.d_tmp_vel2, E.d_zlub, E.d_D, E.d_z, E.d_v, E.d_xw, E.d_Rr[0],
-                    E.d_Rr[1], E.d_Rr[2], E.d_W[0], E.d_W[1], E.d_W[2], E.d_mr, E.d_sinv, E.d_nactive,
+                    E.d_Rr[1], E.d_Rr[2], E.d_W[0], E.d_W[1], E.d_W[2], E.d_mr, E.d_mrp, E.d_nactive,
                     E.d_rhs, E.d_X, E.d_Xd, E.d_Xdet, E.d_Wn, E.d_vdn, E.d_vdc, E.d_vb, E.d_up, E.d_ud,
                     E.d_drift, E.d_sb, E.d_fext, E.d_fb, E.d_wr, E.d_tmp_top, E.d_tmp_top2, E.d_lzV, E.d_lzT,
                     E.d_lzw, E.d_lzq, E.d_lzp, E.d_lzs, E.d_ssinv, E.d_pcg, E.d_pV, E.d_pr, E.d_pz, E.d_pp, E.d_ps,
@@ -334,8 +334,7 @@ static int build(Engine &E, const ps_desc *descs, int R, int precision)
     TRY_ALLOC(E.d_z, sizeof(double) * vec);
     TRY_ALLOC(E.d_v, sizeof(double) * vec);
     for (int k = 0; k < 3; k++) { TRY_ALLOC(E.d_Rr[k], sizeof(double) * vec); TRY_ALLOC(E.d_W[k], sizeof(double) * vec); }
-    TRY_ALLOC(E.d_mr, sizeof(ps::MinresScal) * R);
-    TRY_ALLOC(E.d_sinv, sizeof(double) * R);
+    TRY_ALLOC(E.d_mr, sizeof(ps::MinresScal) * 2 * R);
     TRY_ALLOC(E.d_nactive, sizeof(int));
     PS_CK(cudaMallocHost(&E.h_nactive, sizeof(int)));
     // the Lanczos convergence checks run on their own stream beside the next basis vectors
@@ -344,6 +343,7 @@ static int build(Engine &E, const ps_desc *descs, int R, int precision)
     PS_CK(cudaEventCreateWithFlags(&E.ev_chk, cudaEventDisableTiming));
     PS_CK(cudaMallocHost(&E.h_spec, 16 * (size_t)std::max(E.R, 1)));
     if ((rc = ps::build_red_table(E, E.red, 0))) return rc;
+    TRY_ALLOC(E.d_mrp, sizeof(double) * 2 * ps::RB_EPT * E.red.nblk);
     if ((rc = ps::build_red_table(E, E.red_top, 1))) return rc;
     // step workspace
     TRY_ALLOC(E.d_rhs, sizeof(double) * vec);
@@ -650,7 +650,7 @@ int ps_assemble(ps_ctx *ctx, void *stream)
 int ps_matmult(ps_ctx *ctx, const double *x, double *y, void *stream)
 {
     if (!ctx || !x || !y) return PS_ERR_ARG;
-    ps::apply_operator(ctx->E, 0, x, y, nullptr, ctx->E.precision == PS_PREC_MIXED, S(stream));
+    ps::apply_operator(ctx->E, 0, x, y, ctx->E.precision == PS_PREC_MIXED, S(stream));
     PS_CK(cudaGetLastError());
     return PS_OK;
 }
@@ -658,7 +658,7 @@ int ps_matmult(ps_ctx *ctx, const double *x, double *y, void *stream)
 int ps_mobility_apply(ps_ctx *ctx, const double *u, double *y, void *stream)
 {
     if (!ctx || !u || !y) return PS_ERR_ARG;
-    ps::apply_operator(ctx->E, 1, u, y, nullptr, ctx->E.precision == PS_PREC_MIXED, S(stream));
+    ps::apply_operator(ctx->E, 1, u, y, ctx->E.precision == PS_PREC_MIXED, S(stream));
     PS_CK(cudaGetLastError());
     return PS_OK;
 }

@@ -84,7 +84,7 @@ __global__ void k_mr_init(RedTable T, const Seg *segs, const double *__restrict_
                           const double *__restrict__ D, double *__restrict__ r, double *__restrict__ z,
                           double *__restrict__ x, MinresScal *mr, int warm, double rtol, int maxit,
                           double *__restrict__ v, double *__restrict__ w0, double *__restrict__ w1,
-                          double *__restrict__ w2, double *__restrict__ sinv)
+                          double *__restrict__ w2)
 {
     pdl_enter();
     __shared__ double sh[RB_THREADS / 32][3];
@@ -121,127 +121,45 @@ __global__ void k_mr_init(RedTable T, const Seg *segs, const double *__restrict_
             m.cs = -1; m.sn = 0; m.sinv = 1.0 / m.beta;
         }
         mr[B.rep] = m;
-        sinv[B.rep] = m.sinv;
     }
 }
 
-// (b) of iteration k: pending w/x update of iteration k-1, v = z/beta,
-// Av -= (beta/oldb) r_{k-1}, alfa = v.Av
-__global__ void k_mr_alpha(RedTable T, const double *__restrict__ z, double *__restrict__ v,
-                           double *__restrict__ Av, const double *__restrict__ rkm1, double *__restrict__ wnew,
-                           const double *__restrict__ w1, const double *__restrict__ w2, double *__restrict__ x,
-                           MinresScal *mr, int k)
+// An iteration's vector work, one entry per thread (sub-blocks of RB_THREADS entries): the
+// combine of the apply goes on with mr_alpha (ps_reduce.cuh), k_mr_beta follows.  The
+// scalars between them are recomputed by every block from the sub-block sums of the kernel
+// before (rep_total), so no kernel ends in a last block that sums and runs the recurrence
+// while the chip waits.  mr_alpha closes iteration k - 1 (its scalars, the w and x update) and
+// opens iteration k: v = z / beta, Av = A z / beta - (beta / oldb) r_{k-1}, sums of
+// alfa = v.Av.  k_mr_beta: r_{k+1} = Av - (alfa / beta) r_k, z = r_{k+1} / D, sums of r.z.  The
+// scalars of iteration k live in st[k & 1]: a kernel reads one and its replica's first block
+// writes the other.
+//
+// Bound: latency (a dependent launch with an L2 round trip takes some 4 us).  516 beads, one
+// iteration: 21.5 us with a launch for each half and last-block sums, 16.5 us without
+// them, 14.2 us with the first half in the combine.
+__global__ void k_mr_beta(RedTable T, const Seg *__restrict__ segs, double *__restrict__ Av, const double *__restrict__ rk,
+                          const double *__restrict__ D, double *__restrict__ z, MinresScal *__restrict__ st,
+                          const double *__restrict__ pa, double *__restrict__ pb)
 {
     pdl_enter();
-    __shared__ double sh[RB_THREADS / 32][1];
     const RBlk B = T.d_blk[blockIdx.x];
-    const MinresScal m = mr[B.rep];
+    const int e = blockIdx.y * RB_THREADS + threadIdx.x;
+    if (blockIdx.y * RB_THREADS >= B.len || st[B.rep].done) return;
+    __shared__ double sh[RB_THREADS / 32][1];
+    const int first = T.d_first[B.rep];
+    const double alfa = rep_total(pa + RB_EPT * first, (segs[B.rep].n + RB_THREADS - 1) / RB_THREADS);
+    if (blockIdx.y == 0 && (int)blockIdx.x == first && threadIdx.x == 0) st[B.rep].alfa = alfa;
     double s[1] = {0.0};
-    const bool upd = m.pending != 0;
-    const bool act = !m.done;
-    const double c1 = (k >= 2) ? m.beta / m.oldb : 0.0;
-    for (int e = threadIdx.x; e < B.len; e += RB_THREADS) {
-        long q = B.start + e;
-        if (upd) {
-            double wn = (v[q] - m.up_oldeps * w1[q] - m.up_delta * w2[q]) * m.up_ginv;
-            wnew[q] = wn;
-            x[q] += m.up_phi * wn;
-        }
-        if (act) {
-            double vq = z[q] * m.sinv;
-            double a = Av[q];
-            if (k >= 2) a -= c1 * rkm1[q];
-            v[q] = vq;
-            Av[q] = a;
-            s[0] += vq * a;
-        }
+    if (e < B.len) {
+        const long q = (long)B.start + e;
+        const double a = Av[q] - (alfa / st[B.rep].beta) * rk[q];
+        const double zq = a / D[q];
+        Av[q] = a;
+        z[q] = zq;
+        s[0] = a * zq;
     }
     block_sum<1>(s, sh);
-    double tot[1];
-    if (finish_block<1>(T, B, blockIdx.x, s, tot)) {
-        if (upd) mr[B.rep].pending = 0;
-        if (act) mr[B.rep].alfa = tot[0];
-    }
-}
-
-// (c) of iteration k: r_{k+1} = Av - (alfa/beta) r_k, z = r_{k+1}/D,
-// beta_{k+1} = sqrt(r_{k+1}.z), Givens rotation, convergence test.
-__global__ void k_mr_beta(RedTable T, double *__restrict__ Av, const double *__restrict__ rk,
-                          const double *__restrict__ D, double *__restrict__ z, MinresScal *mr, int maxit,
-                          int *nactive, double *__restrict__ sinv)
-{
-    pdl_enter();
-    __shared__ double sh[RB_THREADS / 32][1];
-    const RBlk B = T.d_blk[blockIdx.x];
-    const MinresScal m0 = mr[B.rep];
-    double s[1] = {0.0};
-    const bool act = !m0.done;
-    if (act) {
-        const double c2 = m0.alfa / m0.beta;
-        for (int e = threadIdx.x; e < B.len; e += RB_THREADS) {
-            long q = B.start + e;
-            double a = Av[q] - c2 * rk[q];
-            double zq = a / D[q];
-            Av[q] = a;
-            z[q] = zq;
-            s[0] += a * zq;
-        }
-    }
-    block_sum<1>(s, sh);
-    double tot[1];
-    if (finish_block<1>(T, B, blockIdx.x, s, tot)) {
-        if (!act) return;
-        MinresScal m = m0;
-        m.it += 1;
-        double bb = tot[0];
-        m.oldb = m.beta;
-        if (bb < 0) { m.done = 1; m.reason = -8; mr[B.rep] = m; atomicSub(nactive, 1); return; }
-        m.beta = sqrt(bb);
-        double oldeps = m.epsln;
-        double delta = m.cs * m.dbar + m.sn * m.alfa;
-        double gbar = m.sn * m.dbar - m.cs * m.alfa;
-        m.epsln = m.sn * m.beta;
-        m.dbar = -m.cs * m.beta;
-        double gamma = sqrt(gbar * gbar + m.beta * m.beta);
-        if (gamma < 2.2250738585072014e-308) gamma = 2.2250738585072014e-308;
-        m.cs = gbar / gamma;
-        m.sn = m.beta / gamma;
-        double phi = m.cs * m.phibar;
-        m.phibar = m.sn * m.phibar;
-        m.up_oldeps = oldeps; m.up_delta = delta; m.up_ginv = 1.0 / gamma; m.up_phi = phi;
-        m.pending = 1;
-        m.np = m.np * fabs(m.sn);
-        if (m.np <= m.ttol) { m.done = 1; m.reason = 2; }
-        else if (m.beta == 0.0) { m.done = 1; m.reason = 3; }
-        else if (m.it >= maxit) { m.done = 1; m.reason = -3; }
-        m.sinv = m.beta != 0.0 ? 1.0 / m.beta : 0.0;
-        mr[B.rep] = m;
-        sinv[B.rep] = m.sinv;
-        if (m.done) atomicSub(nactive, 1);
-    }
-}
-
-// final pending update (after the last iteration)
-__global__ void k_mr_flush(RedTable T, const double *__restrict__ v, double *__restrict__ wnew,
-                           const double *__restrict__ w1, const double *__restrict__ w2, double *__restrict__ x,
-                           MinresScal *mr)
-{
-    pdl_enter();
-    __shared__ double sh[RB_THREADS / 32][1];
-    const RBlk B = T.d_blk[blockIdx.x];
-    const MinresScal m = mr[B.rep];
-    if (m.pending) {
-        for (int e = threadIdx.x; e < B.len; e += RB_THREADS) {
-            long q = B.start + e;
-            double wn = (v[q] - m.up_oldeps * w1[q] - m.up_delta * w2[q]) * m.up_ginv;
-            wnew[q] = wn;
-            x[q] += m.up_phi * wn;
-        }
-    }
-    double s[1] = {0.0};
-    block_sum<1>(s, sh);
-    double tot[1];
-    if (finish_block<1>(T, B, blockIdx.x, s, tot)) mr[B.rep].pending = 0;
+    if (threadIdx.x == 0) pb[RB_EPT * blockIdx.x + blockIdx.y] = s[0];
 }
 
 int minres_solve(Engine &E, const double *b, double *x, const ps_ksp_opts *o, ps_ksp_result *res, cudaStream_t st)
@@ -255,13 +173,12 @@ int minres_solve(Engine &E, const double *b, double *x, const ps_ksp_opts *o, ps
     if (rc) return rc;
     const double *Ax = nullptr;
     if (opt.warm) {
-        apply_operator(E, 0, x, E.d_Rr[2], nullptr, false, st);
+        apply_operator(E, 0, x, E.d_Rr[2], false, st);
         Ax = E.d_Rr[2];
     }
-    // r_1 in slot 1 (slot k % 3 holds r_k)
+    // r_1 in slot 1 (slot k % 3 holds r_k); scalars in d_mr[(k & 1) R ..]
     ps_launch(k_mr_init, T.nblk, RB_THREADS, 0, st, T, E.d_segs, b, Ax, E.d_D, E.d_Rr[1], E.d_z, x, E.d_mr, opt.warm,
-            opt.rtol, opt.maxit, E.d_v, E.d_W[0], E.d_W[1], E.d_W[2],
-            E.d_sinv);
+            opt.rtol, opt.maxit, E.d_v, E.d_W[0], E.d_W[1], E.d_W[2]);
     PS_CK(cudaGetLastError());
     // count active replicas
     std::vector<MinresScal> hm(E.R);
@@ -271,37 +188,36 @@ int minres_solve(Engine &E, const double *b, double *x, const ps_ksp_opts *o, ps
     for (auto &m : hm) nact += !m.done;
     *E.h_nactive = nact;
     PS_CK(cudaMemcpyAsync(E.d_nactive, E.h_nactive, sizeof(int), cudaMemcpyHostToDevice, st));
-    int k = 0;
-    while (nact > 0 && k < opt.maxit) {
-        for (int j = 0; j < opt.check_every && k < opt.maxit; j++) {
-            k++;
-            double *Av = E.d_Rr[(k + 1) % 3];
-            const double *rk = E.d_Rr[k % 3];
-            const double *rkm1 = E.d_Rr[(k + 2) % 3];
-            // iteration k-1's update writes w_{k-1} into slot (k-1)%3; w_{k-2}, w_{k-3}... in the others
-            double *wnew = E.d_W[(k + 2) % 3];
-            const double *w1 = E.d_W[(k + 0) % 3];   // w_{k-3}
-            const double *w2 = E.d_W[(k + 1) % 3];   // w_{k-2}
-            // A v_k = (1/beta_k) A z_k: the operator applies the per-replica scale
-            apply_operator(E, 0, E.d_z, Av, E.d_sinv, E.precision == PS_PREC_MIXED, st, &E.d_mr[0].done,
-                           (int)sizeof(MinresScal));
-            ps_launch(k_mr_alpha, T.nblk, RB_THREADS, 0, st, T, E.d_z, E.d_v, Av, rkm1, wnew, w1, w2, x, E.d_mr, k);
-            ps_launch(k_mr_beta, T.nblk, RB_THREADS, 0, st, T, Av, rk, E.d_D, E.d_z, E.d_mr, opt.maxit, E.d_nactive,
-                    E.d_sinv);
+    double *pa = E.d_mrp, *pb = pa + (long)RB_EPT * T.nblk;
+    const dim3 sub((unsigned)T.nblk, RB_EPT);
+    MinresScal *last = E.d_mr;
+    // the apply of iteration k closes iteration k - 1, so the check stands between the apply and
+    // k_mr_beta, and a solve that converged at k - 1 has spent one apply of iteration k
+    for (int k = 1, next = opt.check_every + 1; nact > 0; k++) {
+        double *Av = E.d_Rr[(k + 1) % 3];
+        const double *rk = E.d_Rr[k % 3];
+        const double *rkm1 = E.d_Rr[(k + 2) % 3];
+        // iteration k - 1's update writes w_{k-1} into slot (k-1)%3; w_{k-3} and w_{k-2} are in the others
+        double *wnew = E.d_W[(k + 2) % 3];
+        const double *w1 = E.d_W[(k + 0) % 3], *w2 = E.d_W[(k + 1) % 3];
+        MinresScal *s0 = E.d_mr + (long)E.R * ((k - 1) & 1), *s1 = E.d_mr + (long)E.R * (k & 1);
+        const MrAlpha al = {E.d_z, rkm1, w1, w2, pb, E.d_v, wnew, x, pa, s0, s1, E.d_nactive, k, opt.maxit};
+        apply_operator(E, 0, E.d_z, Av, E.precision == PS_PREC_MIXED, st, &s0[0].done, (int)sizeof(MinresScal), false,
+                       nullptr, &al);
+        last = s1;
+        if (k == next || k > opt.maxit) {
+            PS_CK(cudaMemcpyAsync(E.h_nactive, E.d_nactive, sizeof(int), cudaMemcpyDeviceToHost, st));
+            PS_CK(cudaStreamSynchronize(st));
+            nact = *E.h_nactive;
+            if (k > opt.maxit) break;
+            // long solves are looked at less often: a missed stop costs launches of blocks that leave at
+            // once (about 8 us an iteration), a look some 15 us
+            next += std::max(opt.check_every, std::min(k / 4, 4 * opt.check_every));
         }
-        PS_CK(cudaMemcpyAsync(E.h_nactive, E.d_nactive, sizeof(int), cudaMemcpyDeviceToHost, st));
-        PS_CK(cudaStreamSynchronize(st));
-        nact = *E.h_nactive;
+        if (nact > 0)
+            ps_launch(k_mr_beta, sub, RB_THREADS, 0, st, T, E.d_segs, Av, rk, E.d_D, E.d_z, s1, pa, pb);
     }
-    // the last iteration's pending update: w_k into slot (k+3)%3 == k%3 ... uses w_{k-1}, w_{k-2}
-    {
-        int kk = k + 1;
-        double *wnew = E.d_W[(kk + 2) % 3];
-        const double *w1 = E.d_W[(kk + 0) % 3];
-        const double *w2 = E.d_W[(kk + 1) % 3];
-        ps_launch(k_mr_flush, T.nblk, RB_THREADS, 0, st, T, E.d_v, wnew, w1, w2, x, E.d_mr);
-    }
-    PS_CK(cudaMemcpyAsync(hm.data(), E.d_mr, sizeof(MinresScal) * E.R, cudaMemcpyDeviceToHost, st));
+    PS_CK(cudaMemcpyAsync(hm.data(), last, sizeof(MinresScal) * E.R, cudaMemcpyDeviceToHost, st));
     PS_CK(cudaStreamSynchronize(st));
     PS_CK(cudaGetLastError());
     int worst = 1000, itmax = 0;
@@ -881,7 +797,7 @@ int lanczos_sqrt(Engine &E, const double *z, double *w, const ps_sqrt_opts *o, p
     int j = 0;
     for (j = 0; j < kmax; j++) {
         const LzDots dots = {V, ldv, j, part1};
-        apply_operator(E, 1, V + (long)j * ldv, q, nullptr, E.precision == PS_PREC_MIXED, st, &lz[0].done,
+        apply_operator(E, 1, V + (long)j * ldv, q, E.precision == PS_PREC_MIXED, st, &lz[0].done,
                        (int)sizeof(LzScal), false, &dots);
         const dim3 sub((unsigned)T.nblk, RB_EPT);
         ps_launch(k_lz_sub_dots, sub, RB_THREADS, 0, st, T, E.d_segs, V, ldv, q, j, lz, part1, alpha, part2);
@@ -1106,10 +1022,10 @@ int schur_lanczos_noise(Engine &E, const double *fb, const double *ymcm, double 
     for (int j = 0; j < kmax; j++) {
         ps_launch(k_sl_load, gb, thr, 0, st, E.ntop, E.d_top_offs, E.R, E.d_segs, E.d_slV, sc, j, 0,
                 nullptr, E.d_sl_u);
-        apply_operator(E, 1, E.d_sl_u, E.d_sl_y, nullptr, false, st, E.d_sl_skip, (int)sizeof(int));
+        apply_operator(E, 1, E.d_sl_u, E.d_sl_y, false, st, E.d_sl_skip, (int)sizeof(int));
         ps_launch(k_sl_load, gb, thr, 0, st, E.ntop, E.d_top_offs, E.R, E.d_segs, E.d_slV, sc, j, 1,
                 E.d_sl_y, E.d_sl_u);
-        apply_operator(E, 1, E.d_sl_u, E.d_sl_y2, nullptr, false, st, E.d_sl_skip, (int)sizeof(int));
+        apply_operator(E, 1, E.d_sl_u, E.d_sl_y2, false, st, E.d_sl_skip, (int)sizeof(int));
         ps_launch(k_sl_iter, ns, SL_THREADS, 0, st, E.d_segs, E.d_sl_reps, E.d_slV, E.d_slT, sc,
                 E.d_sl_skip, E.d_sl_y, E.d_sl_y2, j);
     }

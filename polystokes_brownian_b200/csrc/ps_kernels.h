@@ -35,6 +35,15 @@ constexpr int LZ_KMAX = 64;      // cap of the Lanczos basis
 // dimension ldv): sub-block sums, LZ_KMAX per sub-block of the output table
 struct LzDots { const double *V; long ldv; int j; double *part; };
 
+// the first half of a MINRES iteration, which the combine of its apply goes on with (krylov.cu)
+struct MrAlpha {
+    const double *z, *rkm1, *w1, *w2, *pb;   // z_k, r_{k-1}, w_{k-3}, w_{k-2}, sub-block sums of r_k.z_k
+    double *v, *wnew, *x, *pa;               // v_k, w_{k-1}, the solution, sub-block sums of v.Av
+    const MinresScal *st0;                   // scalars after iteration k - 2's end
+    MinresScal *st1;                         // ... and after iteration k - 1's
+    int *nactive, k, maxit;
+};
+
 // Per-replica scalars of the lubricated resistance-form PCG.
 struct PcgScal {
     double rz, alpha, beta, tol, err;
@@ -153,7 +162,7 @@ struct Engine {
     double *d_D = nullptr, *d_z = nullptr, *d_v = nullptr, *d_xw = nullptr;
     double *d_Rr[3] = {nullptr, nullptr, nullptr}, *d_W[3] = {nullptr, nullptr, nullptr};
     MinresScal *d_mr = nullptr;
-    double *d_sinv = nullptr;
+    double *d_mrp = nullptr;         // MINRES sub-block sums of both dots
     int *d_nactive = nullptr;
     int *h_nactive = nullptr;        // pinned
 
@@ -200,9 +209,10 @@ int obs_read(Engine &E, ps_obs_out *out, cudaStream_t st);
 // skip_aa: leave out the monomer-monomer pairs -- exact for every colloid row,
 // and for the monomer rows when the monomer inputs are zero.
 // dots (mode 1): the combine also forms the result's dots with the Lanczos basis.
-void apply_operator(Engine &E, int mode, const double *x, double *y, const double *scale, bool fp32, cudaStream_t st,
+// mr (mode 0): the combine goes on with the first half of a MINRES iteration.
+void apply_operator(Engine &E, int mode, const double *x, double *y, bool fp32, cudaStream_t st,
                     const void *done = nullptr, int done_stride = 0, bool skip_aa = false,
-                    const LzDots *dots = nullptr);
+                    const LzDots *dots = nullptr, const MrAlpha *mr = nullptr);
 int time_pairs(Engine &E, int which, int reps, const double *u, double *ms, cudaStream_t st);
 int fma_peak(int fp64, double *tflops, cudaStream_t st);
 int rsqrt_check(const double *a, long n, unsigned long long *max_ulp, cudaStream_t st);

@@ -59,6 +59,99 @@ __device__ __forceinline__ bool finish_block(const RedTable &T, const RBlk &b, i
     return false;
 }
 
+// Total of a replica's sub-block sums (sub-blocks of RB_THREADS entries, nb of them, from
+// part[RB_EPT * first] on), the same in every thread of the block and in a fixed order.  Every
+// block of a kernel adds its replica's sums itself: no counters, no fences, no last block.
+__device__ __forceinline__ double rep_total(const double *__restrict__ part, int nb)
+{
+    __shared__ double ws[RB_THREADS / 32], tot;
+    double t = 0.0;
+    for (int b = threadIdx.x; b < nb; b += RB_THREADS) t += part[b];
+    for (int o = 16; o > 0; o >>= 1) t += __shfl_down_sync(0xffffffffu, t, o);
+    if ((threadIdx.x & 31) == 0) ws[threadIdx.x >> 5] = t;
+    __syncthreads();
+    if (threadIdx.x == 0) {
+        double v = 0.0;
+#pragma unroll
+        for (int w = 0; w < RB_THREADS / 32; w++) v += ws[w];
+        tot = v;
+    }
+    __syncthreads();
+    return tot;
+}
+
+// MINRES scalars after an iteration, from its r.z total bb (Paige & Saunders; PETSc's test):
+// the pending w/x update, the next beta, convergence
+__device__ __forceinline__ void minres_advance(MinresScal &m, double bb, int maxit)
+{
+    m.it += 1;
+    m.oldb = m.beta;
+    m.pending = 0;
+    if (bb < 0) { m.done = 1; m.reason = -8; return; }
+    m.beta = sqrt(bb);
+    const double oldeps = m.epsln;
+    const double delta = m.cs * m.dbar + m.sn * m.alfa;
+    const double gbar = m.sn * m.dbar - m.cs * m.alfa;
+    m.epsln = m.sn * m.beta;
+    m.dbar = -m.cs * m.beta;
+    double gamma = sqrt(gbar * gbar + m.beta * m.beta);
+    if (gamma < 2.2250738585072014e-308) gamma = 2.2250738585072014e-308;
+    m.cs = gbar / gamma;
+    m.sn = m.beta / gamma;
+    const double phi = m.cs * m.phibar;
+    m.phibar = m.sn * m.phibar;
+    m.up_oldeps = oldeps; m.up_delta = delta; m.up_ginv = 1.0 / gamma; m.up_phi = phi;
+    m.pending = 1;
+    m.np = m.np * fabs(m.sn);
+    if (m.np <= m.ttol) { m.done = 1; m.reason = 2; }
+    else if (m.beta == 0.0) { m.done = 1; m.reason = 3; }
+    else if (m.it >= maxit) { m.done = 1; m.reason = -3; }
+    m.sinv = m.beta != 0.0 ? 1.0 / m.beta : 0.0;
+}
+
+// First half of a MINRES iteration for one entry per thread: index q of the saddle vectors (act:
+// the entry exists), Az its product; B, the block of the saddle table.  Writes Av over it.
+// Returns at once for a replica that was done, carrying its scalars on.
+__device__ __forceinline__ void mr_alpha(const RedTable &T, const RBlk &B, int n, long q, bool act, double Az,
+                                         const MrAlpha &A, double *__restrict__ Av)
+{
+    __shared__ MinresScal sm;
+    __shared__ double sh[RB_THREADS / 32][1];
+    const int first = T.d_first[B.rep];
+    const bool lead = blockIdx.y == 0 && (int)blockIdx.x == first && threadIdx.x == 0;
+    const double bb = A.k > 1 ? rep_total(A.pb + RB_EPT * first, (n + RB_THREADS - 1) / RB_THREADS) : 0.0;
+    if (threadIdx.x == 0) {
+        MinresScal m = A.st0[B.rep];
+        if (A.k > 1) minres_advance(m, bb, A.maxit);
+        sm = m;
+        if (lead) {
+            if (m.done) atomicSub(A.nactive, 1);
+            m.pending = 0;                                 // applied below
+            A.st1[B.rep] = m;
+        }
+    }
+    __syncthreads();
+    double s[1] = {0.0};
+    if (act) {
+        if (sm.pending) {
+            const double wn = (A.v[q] - sm.up_oldeps * A.w1[q] - sm.up_delta * A.w2[q]) * sm.up_ginv;
+            A.wnew[q] = wn;
+            A.x[q] += sm.up_phi * wn;
+        }
+        if (!sm.done) {
+            const double vq = A.z[q] * sm.sinv;
+            double a = Az * sm.sinv;
+            if (A.k >= 2) a -= (sm.beta / sm.oldb) * A.rkm1[q];
+            A.v[q] = vq;
+            Av[q] = a;
+            s[0] = vq * a;
+        }
+    }
+    if (sm.done) return;
+    block_sum<1>(s, sh);
+    if (threadIdx.x == 0) A.pa[RB_EPT * blockIdx.x + blockIdx.y] = s[0];
+}
+
 // sums of sixteen values over the warp by halving exchanges (16 double shuffles): the lane
 // ends with the total of value idx (each total in two lanes)
 __device__ __forceinline__ double warp_sum16(double (&v)[16], int lane, int &idx)

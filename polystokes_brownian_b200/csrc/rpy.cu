@@ -766,21 +766,28 @@ __device__ __forceinline__ int find_rep(const int *__restrict__ offs, int R, lon
 // once; blockIdx.y splits an entry's span so that each thread sums one output
 // (a single large replica otherwise leaves most SMs idle while every thread
 // walks its chunk partials four times over).
-template <bool DOTS>
+// what a combine goes on with
+enum { CB_PLAIN, CB_DOTS, CB_MINRES };
+struct NoTail {};
+
+template <int TAIL, class X>
 __global__ void k_combine(const Seg *__restrict__ segs, RedTable T, int mode, const double *__restrict__ x,
-                          const double *__restrict__ scale, const double *__restrict__ partAA, int with_aa,
+                          const double *__restrict__ partAA, int with_aa,
                           const double *__restrict__ partAB, const double *__restrict__ partBB, int nchBB,
                           const double *__restrict__ partBA, const double *__restrict__ delta,
                           const double *__restrict__ lub_y, long part_stride, double *__restrict__ y,
-                          const char *__restrict__ done, int done_stride, LzDots ld)
+                          const char *__restrict__ done, int done_stride, X tail)
 {
     pdl_enter();
     const RBlk B = T.d_blk[blockIdx.x];
     const int r = B.rep;
-    if (done && *(const int *)(done + (long)r * done_stride)) return;   // converged replica: skip
+    if (done && *(const int *)(done + (long)r * done_stride)) {         // converged replica: skip
+        if constexpr (TAIL == CB_MINRES)
+            if (blockIdx.y == 0 && (int)blockIdx.x == T.d_first[r] && threadIdx.x == 0) tail.st1[r] = tail.st0[r];
+        return;
+    }
     const Seg &sg = segs[r];
     const int xo = mode == 0 ? sg.vec_off : sg.top_off;
-    const double s = scale ? scale[r] : 1.0;
     // grid.y = RB_EPT: one entry per thread
     const int e = blockIdx.y * RB_THREADS + threadIdx.x;
     const long k = (long)B.start + e;
@@ -830,13 +837,13 @@ __global__ void k_combine(const Seg *__restrict__ segs, RedTable T, int mode, co
             v = -x[xo + j];
             if (sg.lub_on && lub_y) v -= lub_y[sg.vel_off + j];
         }
-        out = s * v;
-        y[k] = out;
+        out = v;
+        if constexpr (TAIL != CB_MINRES) y[k] = v;
     }
-    if constexpr (DOTS) {
-        if (blockIdx.y * RB_THREADS < B.len)
-            lz_block_dots(ld.V, ld.ldv, k, e < B.len, out, ld.j, ld.part + (long)LZ_KMAX * (RB_EPT * blockIdx.x + blockIdx.y));
-    }
+    if (blockIdx.y * RB_THREADS >= B.len) return;
+    if constexpr (TAIL == CB_DOTS)
+        lz_block_dots(tail.V, tail.ldv, k, e < B.len, out, tail.j, tail.part + (long)LZ_KMAX * (RB_EPT * blockIdx.x + blockIdx.y));
+    if constexpr (TAIL == CB_MINRES) mr_alpha(T, B, sg.n, k, e < B.len, out, tail, y);
 }
 
 // ---------------------------------------------------------------------------
@@ -873,8 +880,8 @@ static void launch_bb(Engine &E, const double *u, int in_top, cudaStream_t st, c
                 u, in_top, E.d_partBB, E.part_stride, done, dstride);
 }
 
-void apply_operator(Engine &E, int mode, const double *x, double *y, const double *scale, bool fp32, cudaStream_t st,
-                    const void *done, int done_stride, bool skip_aa, const LzDots *dots)
+void apply_operator(Engine &E, int mode, const double *x, double *y, bool fp32, cudaStream_t st,
+                    const void *done, int done_stride, bool skip_aa, const LzDots *dots, const MrAlpha *mr)
 {
     int in_top = mode == 1;
     const char *dn = (const char *)done;
@@ -889,13 +896,15 @@ void apply_operator(Engine &E, int mode, const double *x, double *y, const doubl
     const dim3 grid((unsigned)T.nblk, RB_EPT);
     const int with_aa = skip_aa ? 0 : 1;
     if (dots)
-        ps_launch(k_combine<true>, grid, RB_THREADS, 0, st, E.d_segs, T, mode, x, scale, E.d_partAA, with_aa, E.d_partAB,
-                E.d_partBB, E.nch_bb, E.d_partBA, E.d_delta, lub_y, E.part_stride, y, dn, done_stride, *dots);
+        ps_launch(k_combine<CB_DOTS, LzDots>, grid, RB_THREADS, 0, st, E.d_segs, T, mode, x, E.d_partAA, with_aa, E.d_partAB, E.d_partBB,
+                E.nch_bb, E.d_partBA, E.d_delta, lub_y, E.part_stride, y, dn, done_stride, *dots);
+    else if (mr)
+        ps_launch(k_combine<CB_MINRES, MrAlpha>, grid, RB_THREADS, 0, st, E.d_segs, T, mode, x, E.d_partAA, with_aa, E.d_partAB, E.d_partBB,
+                E.nch_bb, E.d_partBA, E.d_delta, lub_y, E.part_stride, y, dn, done_stride, *mr);
     else
-        ps_launch(k_combine<false>, grid, RB_THREADS, 0, st, E.d_segs, T, mode, x, scale, E.d_partAA, with_aa, E.d_partAB,
-                E.d_partBB, E.nch_bb, E.d_partBA, E.d_delta, lub_y, E.part_stride, y, dn, done_stride, LzDots{});
+        ps_launch(k_combine<CB_PLAIN, NoTail>, grid, RB_THREADS, 0, st, E.d_segs, T, mode, x, E.d_partAA, with_aa, E.d_partAB, E.d_partBB,
+                E.nch_bb, E.d_partBA, E.d_delta, lub_y, E.part_stride, y, dn, done_stride, NoTail{});
 }
-
 
 int g_aa_chunk_cols = AA_TILE_MAX;
 
@@ -960,7 +969,7 @@ int time_pairs(Engine &E, int which, int reps, const double *u, double *ms, cuda
         } else if (which == 2) {
             launch_bb(E, u, 1, st, nullptr, 0);
         } else if (which == 3) {
-            apply_operator(E, 1, u, E.d_tmp_top2, nullptr, fp32, st);
+            apply_operator(E, 1, u, E.d_tmp_top2, fp32, st);
         }
     };
     launch();   // warm

@@ -922,11 +922,11 @@ __global__ void k_ps_S(long ntot, const int *__restrict__ bead_offs, int R, cons
 // d_py = M [u ; 0], d_pu2 = [0 ; -M_SS^{-1} (d_py)_S], d_py2 = M d_pu2
 static void mr_apply(Engine &E, bool fp32, const void *dn, int ds, cudaStream_t st)
 {
-    apply_operator(E, 1, E.d_pu, E.d_py, nullptr, fp32, st, dn, ds);
+    apply_operator(E, 1, E.d_pu, E.d_py, fp32, st, dn, ds);
     if (E.n_ss_reps) {
         ps_launch(k_ss_apply, E.n_ss_reps, 64, 0, st, E.d_segs, E.d_ss_reps, E.d_ssinv, E.d_py, 1, -1.0,
                 nullptr, 1, 0.0, E.d_pu2, 1, (const char *)dn, ds);
-        apply_operator(E, 1, E.d_pu2, E.d_py2, nullptr, fp32, st, dn, ds, true);
+        apply_operator(E, 1, E.d_pu2, E.d_py2, fp32, st, dn, ds, true);
     }
 }
 
@@ -1402,7 +1402,7 @@ static int pair_solve(Engine &E, const double *b, double *x, const ps_ksp_opts *
         // g: u2 = [0 ; M_SS^{-1} b_S]
         ps_launch(k_ss_apply, E.n_ss_reps, 64, 0, st, E.d_segs, E.d_ss_reps, E.d_ssinv, b, 0, 1.0, nullptr,
                 0, 0.0, E.d_pu2, 1, nullptr, 0);
-        apply_operator(E, 1, E.d_pu2, E.d_py2, nullptr, fp32, st, nullptr, 0, true);
+        apply_operator(E, 1, E.d_pu2, E.d_py2, fp32, st, nullptr, 0, true);
     }
     ps_launch(k_pcg_g, TV.nblk, RB_THREADS, 0, st, TV, E.d_segs, b, E.d_py2, g);
     ps_launch(k_ps_c, TV.nblk, RB_THREADS, 0, st, TV, E.d_segs, b, cvel, E.d_pu);
@@ -1556,10 +1556,10 @@ int structured_solve(Engine &E, const double *b, double *x, const ps_ksp_opts *o
     bool fp32 = E.precision == PS_PREC_MIXED;
     ps_launch(k_struct_init, nb, thr, 0, st, E.nvec, E.d_vec_offs, E.R, E.d_segs, b, x);
     if (E.n_ss_reps) {
-        apply_operator(E, 0, x, y, nullptr, fp32, st);   // y_top = M [F_t ; 0]
+        apply_operator(E, 0, x, y, fp32, st);   // y_top = M [F_t ; 0]
         ps_launch(k_struct_ss, E.n_ss_reps, 256, 0, st, E.d_segs, E.d_ss_reps, E.d_x, E.d_delta, b, y, x);
     }
-    apply_operator(E, 0, x, y, nullptr, fp32, st);       // y_top = M F
+    apply_operator(E, 0, x, y, fp32, st);       // y_top = M F
     ps_launch(k_struct_u, nb, thr, 0, st, E.nvec, E.d_vec_offs, E.R, E.d_segs, b, y, x);
     PS_CK(cudaGetLastError());
     ps_ksp_result r0 = {2, 0, 0, 0.0};

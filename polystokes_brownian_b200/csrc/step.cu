@@ -74,7 +74,7 @@ int slip_noise(Engine &E, const double *fb, double *W, const ps_sqrt_opts *o, ps
         int thr = 256;
         ps_launch(k_zero_colloid_dofs, (unsigned)((E.ntop + thr - 1) / thr), thr, 0, st, E.ntop, E.d_top_offs, E.R, E.d_segs,
                 fb, E.d_tmp_top);
-        apply_operator(E, 1, E.d_tmp_top, E.d_tmp_top2, nullptr, false, st);
+        apply_operator(E, 1, E.d_tmp_top, E.d_tmp_top2, false, st);
         if (E.n_schur_reps)
             ps_launch(k_shell_noise, E.n_schur_reps, 128, 0, st, E.d_segs, E.d_schur_reps, fb, E.d_tmp_top2,
                     E.d_schurQ, E.d_schurL, W);
@@ -327,7 +327,7 @@ static int solve(Engine &E, const double *b, double *x, int warm, const ps_step_
         const int thr = 256;
         const unsigned g = (unsigned)((E.nvec + thr - 1) / thr);
         for (int k = 0; k < sweeps; k++) {
-            apply_operator(E, 0, x, E.d_ref_d, nullptr, false, st);
+            apply_operator(E, 0, x, E.d_ref_d, false, st);
             ps_launch(k_resid, g, thr, 0, st, E.nvec, b, E.d_ref_d, E.d_ref_r);
             ps_ksp_opts oc = o;
             oc.warm = 0;
