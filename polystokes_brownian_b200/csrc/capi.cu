@@ -95,7 +95,7 @@ static int build(Engine &E, const ps_desc *descs, int R, int precision)
     long bead = 0, coll = 0, vec = 0, top = 0, vel = 0, schur = 0, ba = 0, cells = 0, ssinv = 0;
     std::vector<int> bead_offs(R + 1), vec_offs(R + 1), top_offs(R + 1), vel_offs(R + 1);
     std::vector<long> cell_offs(R + 1);
-    std::vector<Tile> bb;
+    std::vector<Tile> bb, bbw;
     std::vector<int> schur_reps, ss_reps, sl_reps;
     long slv = 0;
     int ss_polish = 0;
@@ -157,17 +157,22 @@ static int build(Engine &E, const ps_desc *descs, int R, int precision)
         if (s.shell_schur) { s.schur_off = (int)schur; schur += (long)s.nc11 * s.nc11; schur_reps.push_back(r); }
         if (d.Nc > 0) {
             if (s.nc5 <= 64) { ss_reps.push_back(r); s.ss_off = (int)ssinv; ssinv += (long)s.nc5 * s.nc5; }
-            else { ss_polish++; E.any_indef = true; }   // colloid suspensions: far-field FTS indefinite near contact
+            else { ss_polish++; s.indef = 1; E.any_indef = true; }   // colloid suspensions: far-field FTS indefinite near contact
         }
         // the reference's own monomer pair scalars make the far-field mobility indefinite
         if (d.mm_HI && ((d.Nm >= 2 && d.aa_mode == PS_AA_REFERENCE) || (d.Nm >= 1 && d.Nc >= 1 && d.ab_mode == PS_AB_REFERENCE))) {
+            s.indef = 1;
             E.any_indef = true;
         }
             s.n_mtiles = (d.Nm + TR - 1) / TR;
         s.ba_off = (int)ba;
         if (d.Nc > 0) ba += (long)s.n_mtiles * d.Nc;
         if (d.Nm == 0 && d.Nc >= 2)
-            for (int t = 0; t * TR < d.Nc; t++) bb.push_back({r, t * TR, std::min(TR, d.Nc - t * TR), t});
+        {
+            const bool wide = bb_wide(d.Nc, s.nch_bb);
+            const int tr = wide ? BB_WIDE : BB_TILE;
+            for (int t = 0; t * tr < d.Nc; t++) (wide ? bbw : bb).push_back({r, t * tr, std::min(tr, d.Nc - t * tr), t});
+        }
         bead_offs[r] = (int)bead; vec_offs[r] = (int)vec; top_offs[r] = (int)top; vel_offs[r] = (int)vel;
         cell_offs[r] = cells;
         cells += CELL_CAP_PER_MONO * d.Nm + CELL_CAP_BASE;
@@ -196,6 +201,8 @@ static int build(Engine &E, const ps_desc *descs, int R, int precision)
         return E.segs[a.rep].Np > E.segs[b.rep].Np || (E.segs[a.rep].Np == E.segs[b.rep].Np && a.rep < b.rep);
     };
     std::stable_sort(bb.begin(), bb.end(), by_cost);
+    E.n_bb_wide = (int)bbw.size();
+    bb.insert(bb.begin(), bbw.begin(), bbw.end());
     E.n_bb_tiles = (int)bb.size();
     // grid extent in chunks: the largest per-replica chunk count
     E.nch_bb = 1;

@@ -15,6 +15,7 @@
 #include <cmath>
 #include <cstdio>
 #include <vector>
+#include <cooperative_groups.h>
 #include "ps_internal.h"
 #include "ps_kernels.h"
 #include "ps_reduce.cuh"
@@ -254,7 +255,8 @@ struct LzScal {
 // kernel leaves its sub-blocks' sums in memory, and every block of the next one
 // adds its replica's sums itself, in a fixed order that depends on the vector's
 // length alone -- no counters and no fences, and a replica's noise does not depend
-// on its batch.
+// on its batch.  Replicas whose far field may be indefinite take k_lz_orth_cluster and
+// the QL check instead (lz_fixed).
 //
 // Bound: latency and L2 (the basis is read twice from L2 and once from L1 per
 // vector, k_lz_sub_dots reading its slices twice).  With 1024 entries per block of
@@ -263,6 +265,17 @@ struct LzScal {
 // 4097-bead brush (52 now), and the four sweeps of 64 replicas, 62000 beads, 100 us
 // (50 now).
 constexpr int LZ_SUB = RB_THREADS;                    // entries of a sub-block
+constexpr int LZC_CTAS = 8, LZC_HALVES = 2, LZC_THREADS = RB_THREADS * LZC_HALVES, LZC_SLOTS = 4;
+constexpr int LZC_VB = LZC_CTAS * LZC_HALVES;         // virtual RB-table blocks per cluster
+// Replicas that keep the summation order of the reduction table's blocks, one cluster each, and the
+// QL iteration, up to LZC_VB * LZC_SLOTS blocks (5957 colloids).  Their far field may be
+// indefinite: about one in ten of the saddle solves that their noise drives is close to
+// singular, takes hundreds to thousands of iterations and returns, within rtol, whatever the
+// rounding before it selects, so another order of these sums moves positions by 1e-9 to 1e-6.
+__device__ __host__ __forceinline__ bool lz_fixed(const Seg &s)
+{
+    return s.indef && (s.nm3nc11 + RB_SPAN - 1) / RB_SPAN <= LZC_VB * LZC_SLOTS;
+}
 static_assert(RB_SPAN == RB_EPT * LZ_SUB, "RB_EPT sub-blocks per table block");
 
 // the replica's total of the sub-block sums part[][i], i <= j, into h[] (shared)
@@ -305,7 +318,7 @@ __global__ void k_lz_sub_dots(RedTable T, const Seg *__restrict__ segs, const do
     pdl_enter();
     const RBlk B = T.d_blk[blockIdx.x];
     const int e = blockIdx.y * LZ_SUB + threadIdx.x;
-    if (blockIdx.y * LZ_SUB >= B.len || lz[B.rep].done) return;
+    if (blockIdx.y * LZ_SUB >= B.len || lz[B.rep].done || lz_fixed(segs[B.rep])) return;
     __shared__ double h[LZ_KMAX];
     lz_total(T, B, segs[B.rep], part1, j, h);
     const bool act = e < B.len;
@@ -326,7 +339,7 @@ __global__ void k_lz_sub_norm(RedTable T, const Seg *__restrict__ segs, const do
     pdl_enter();
     const RBlk B = T.d_blk[blockIdx.x];
     const int e = blockIdx.y * LZ_SUB + threadIdx.x;
-    if (blockIdx.y * LZ_SUB >= B.len || lz[B.rep].done) return;
+    if (blockIdx.y * LZ_SUB >= B.len || lz[B.rep].done || lz_fixed(segs[B.rep])) return;
     __shared__ double h[LZ_KMAX], sh[RB_THREADS / 32][1];
     lz_total(T, B, segs[B.rep], part2, j, h);
     double v[1] = {0.0};
@@ -351,7 +364,7 @@ __global__ void k_lz_next(RedTable T, const Seg *__restrict__ segs, double *__re
     pdl_enter();
     const RBlk B = T.d_blk[blockIdx.x];
     const int e = blockIdx.y * LZ_SUB + threadIdx.x;
-    if (blockIdx.y * LZ_SUB >= B.len || lz[B.rep].done) return;
+    if (blockIdx.y * LZ_SUB >= B.len || lz[B.rep].done || lz_fixed(segs[B.rep])) return;
     __shared__ double tot;
     const int first = T.d_first[B.rep];
     if (threadIdx.x < 32) {
@@ -653,7 +666,7 @@ struct LzSpec {
 // move lz on) and writes its outcome into spec; the host applies it later
 // (k_lz_spec_apply).  g_prev is the previous check's g in both cases.
 __global__ void __launch_bounds__(LZE_THREADS)
-k_lz_check(int R, LzScal *__restrict__ lz, const LzScal *__restrict__ snap, LzSpec *__restrict__ spec,
+k_lz_check(int R, const Seg *__restrict__ segs, LzScal *__restrict__ lz, const LzScal *__restrict__ snap, LzSpec *__restrict__ spec,
            const double *__restrict__ alpha, const double *__restrict__ betad, double *__restrict__ gbuf,
            int m, double tol, int final_)
 {
@@ -662,6 +675,7 @@ k_lz_check(int R, LzScal *__restrict__ lz, const LzScal *__restrict__ snap, LzSp
     __shared__ double red[2][2];
     __shared__ int rneg[2];
     const int r = blockIdx.x;
+    if (lz_fixed(segs[r])) return;
     const LzScal L = final_ ? lz[r] : snap[r];
     const int tid = threadIdx.x, lane = tid & 31, wid = tid >> 5;
     if (!final_ && L.done) {
@@ -741,6 +755,79 @@ k_lz_check(int R, LzScal *__restrict__ lz, const LzScal *__restrict__ snap, LzSp
     }
 }
 
+// k_lz_check for the replicas that keep their order (lz_fixed), one warp per replica: QL, g summed
+// eigenvalue by eigenvalue.  eig of T_m, g = b0 U sqrt(max(theta,0)) U^T e1,
+// convergence ||g - g_prev|| <= tol ||g|| (the Lanczos basis is orthonormal).
+// final_ = 1: the final estimate, on the replica's own m when it is done, into lz.
+// final_ = 0: a speculative check beside the next basis vectors: it reads the
+// snapshot `snap` of lz taken when it was launched (the vectors that follow
+// move lz on) and writes its outcome into spec; the host applies it later
+// (k_lz_spec_apply).  g_prev is the previous check's g in both cases.
+__global__ void k_lz_check_ql(int R, const Seg *__restrict__ segs, LzScal *__restrict__ lz, const LzScal *__restrict__ snap, LzSpec *__restrict__ spec,
+                           const double *__restrict__ alpha, const double *__restrict__ betad, double *__restrict__ gbuf,
+                           int m, double tol, int final_)
+{
+    pdl_enter();
+    extern __shared__ double sm[];
+    const int r = blockIdx.x;
+    if (!lz_fixed(segs[r])) return;
+    const LzScal L = final_ ? lz[r] : snap[r];
+    const int lane = threadIdx.x;
+    if (!final_ && L.done) {
+        if (lane == 0) spec[r] = LzSpec{0, L.m, 1, 0};
+        return;
+    }
+    int mr = L.done ? L.m : m;
+    if (mr <= 0) {
+        if (!final_ && lane == 0) spec[r] = LzSpec{0, 0, 0, 0};
+        return;
+    }
+    double *d = sm, *e = sm + LZ_KMAX, *Z = sm + 2 * LZ_KMAX, *rot = Z + LZ_KMAX * LZ_KMAX;
+    for (int i = lane; i < mr; i += 32) {
+        d[i] = alpha[(long)LZ_KMAX * r + i];
+        e[i] = (i < mr - 1) ? betad[(long)LZ_KMAX * r + i] : 0.0;
+    }
+    __syncwarp();
+    warp_tql(d, e, Z, rot, mr);
+    __syncwarp();
+    double *g = gbuf + (long)(LZ_KMAX + 1) * r;   // g[0..m-1], g[LZ_KMAX] = |g|^2 of previous
+    double diff2 = 0, nrm2 = 0;
+    int nneg = 0;
+    for (int i = lane; i < LZ_KMAX; i += 32) {
+        double gi = 0;
+        if (i < mr) {
+            for (int j = 0; j < mr; j++) {
+                double th = d[j];
+                double sq = th > 0 ? sqrt(th) : 0.0;
+                gi += Z[i * mr + j] * sq * Z[0 * mr + j];
+            }
+            gi *= L.b0;
+        }
+        double old = g[i];
+        diff2 += (gi - old) * (gi - old);
+        nrm2 += gi * gi;
+        if (i < mr) g[i] = gi;
+    }
+    for (int j = lane; j < mr; j += 32) nneg += d[j] < 0.0;
+    for (int o = 16; o > 0; o >>= 1) {
+        diff2 += __shfl_down_sync(0xffffffffu, diff2, o);
+        nrm2 += __shfl_down_sync(0xffffffffu, nrm2, o);
+        nneg += __shfl_down_sync(0xffffffffu, nneg, o);
+    }
+    if (lane == 0) {
+        const int conv = sqrt(diff2) <= tol * sqrt(nrm2);
+        if (final_) {
+            lz[r].nneg = nneg;
+            if (!lz[r].done) {
+                lz[r].m = mr;
+                lz[r].done = 1;
+            }
+        } else {
+            spec[r] = LzSpec{conv, mr, conv, 0};
+        }
+    }
+}
+
 // a speculative check's outcome, applied in stream order after the vectors that
 // ran beside it: a replica that had converged at m stops there (done, m), as if
 // the check had held the vectors back; the vectors it took meanwhile are unused
@@ -767,6 +854,148 @@ __global__ void k_lz_combine(RedTable T, const double *__restrict__ V, long ldv,
     }
 }
 
+// One Lanczos iteration's orthogonalisation of the replicas that keep their order (lz_fixed), in one
+// launch: one cluster of LZC_CTAS blocks per replica.  Both passes of the
+// reorthogonalisation (dots against V_0..V_j, then q -= V h), the norm, the
+// breakdown test and the next basis vector, with cluster barriers between the
+// phases and the cross-block sums read through distributed shared memory.  The
+// replica's vector is cut into the reduction table's RB_SPAN blocks, each half of a
+// block (RB_THREADS threads) forms an RB block's partials, and every sum over RB
+// blocks runs in block order.  A replica that is done leaves with its whole cluster
+// (the flag is read before any block writes it).
+namespace cgr = cooperative_groups;
+
+__global__ void __cluster_dims__(LZC_CTAS, 1, 1) __launch_bounds__(LZC_THREADS)
+k_lz_orth_cluster(const Seg *__restrict__ segs, double *__restrict__ V, long ldv, double *__restrict__ q, int j,
+                  int kmax, LzScal *__restrict__ lz, double *__restrict__ alpha, double *__restrict__ betad)
+{
+    pdl_enter();
+    cgr::cluster_group cl = cgr::this_cluster();
+    const int rank = (int)cl.block_rank();
+    const int r = blockIdx.x / LZC_CTAS;
+    const int half = threadIdx.x / RB_THREADS, t = threadIdx.x % RB_THREADS;
+    const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
+    constexpr int HW = RB_THREADS / 32;                   // warps per half
+    __shared__ double part[2][LZC_HALVES][LZC_SLOTS][LZ_KMAX + 1];   // per pass: RB-block partial dots
+    __shared__ double npart[LZC_HALVES][LZC_SLOTS];       // RB-block partial norms
+    __shared__ double sh[LZC_THREADS / 32][8];
+    __shared__ double hsh[LZ_KMAX + 1];
+    const Seg &s = segs[r];
+    if (lz[r].done || !lz_fixed(s)) return;     // the whole cluster: no block has written lz yet
+    const int n = s.nm3nc11;
+    const long base = s.top_off;
+    const int nb = (n + RB_SPAN - 1) / RB_SPAN, nslot = (nb + LZC_VB - 1) / LZC_VB;
+    const int vb = rank * LZC_HALVES + half;
+    double alpha_j = 0.0;
+    for (int pass = 0; pass < 2; pass++) {
+        for (int sl = 0; sl < nslot; sl++) {
+            const int rb = vb + LZC_VB * sl;
+            const long st = (long)rb * RB_SPAN;
+            const int len = rb < nb ? min(RB_SPAN, n - rb * RB_SPAN) : 0;
+            double qv[RB_EPT];
+#pragma unroll
+            for (int k = 0; k < RB_EPT; k++) {
+                const int e = t + k * RB_THREADS;
+                qv[k] = e < len ? q[base + st + e] : 0.0;
+            }
+            for (int i0 = 0; i0 <= j; i0 += 8) {
+                double v[8];
+#pragma unroll
+                for (int c = 0; c < 8; c++) {
+                    v[c] = 0.0;
+                    if (i0 + c <= j) {
+                        const double *Vi = V + (long)(i0 + c) * ldv + base + st;
+#pragma unroll
+                        for (int k = 0; k < RB_EPT; k++) {
+                            const int e = t + k * RB_THREADS;
+                            if (e < len) v[c] += Vi[e] * qv[k];
+                        }
+                    }
+                }
+#pragma unroll
+                for (int c = 0; c < 8; c++) {
+                    double x = v[c];
+                    for (int o = 16; o > 0; o >>= 1) x += __shfl_down_sync(0xffffffffu, x, o);
+                    if (lane == 0) sh[wid][c] = x;
+                }
+                __syncthreads();
+                if (t < 8 && i0 + t <= j) {
+                    double x = 0.0;
+                    for (int w = 0; w < HW; w++) x += sh[half * HW + w][t];
+                    part[pass][half][sl][i0 + t] = x;
+                }
+                __syncthreads();
+            }
+        }
+        cl.sync();
+        for (int i = threadIdx.x; i <= j; i += LZC_THREADS) {   // h_i over the RB blocks in block order
+            double h = 0.0;
+            for (int rb = 0; rb < nb; rb++) {
+                const int v2 = rb % LZC_VB;
+                h += cl.map_shared_rank(&part[pass][v2 % LZC_HALVES][rb / LZC_VB][0], v2 / LZC_HALVES)[i];
+            }
+            hsh[i] = h;
+        }
+        __syncthreads();
+        for (int sl = 0; sl < nslot; sl++) {                   // q -= sum_i h_i V_i, i = 0..j per element
+            const int rb = vb + LZC_VB * sl;
+            if (rb >= nb) break;
+            const long st = (long)rb * RB_SPAN;
+            const int len = min(RB_SPAN, n - rb * RB_SPAN);
+            for (int k = 0; k < RB_EPT; k++) {
+                const int e = t + k * RB_THREADS;
+                if (e >= len) break;
+                double acc = q[base + st + e];
+                for (int i = 0; i <= j; i++) acc -= hsh[i] * V[(long)i * ldv + base + st + e];
+                q[base + st + e] = acc;
+            }
+        }
+        alpha_j += hsh[j];
+        __syncthreads();
+    }
+    for (int sl = 0; sl < nslot; sl++) {                       // RB-block norms, as seg_dot
+        const int rb = vb + LZC_VB * sl;
+        const long st = (long)rb * RB_SPAN;
+        const int len = rb < nb ? min(RB_SPAN, n - rb * RB_SPAN) : 0;
+        double x = 0.0;
+        for (int e = t; e < len; e += RB_THREADS) x += q[base + st + e] * q[base + st + e];
+        for (int o = 16; o > 0; o >>= 1) x += __shfl_down_sync(0xffffffffu, x, o);
+        if (lane == 0) sh[wid][0] = x;
+        __syncthreads();
+        if (t == 0) {
+            double y = 0.0;
+            for (int w = 0; w < HW; w++) y += sh[half * HW + w][0];
+            npart[half][sl] = y;
+        }
+        __syncthreads();
+    }
+    cl.sync();
+    double nrm2 = 0.0;
+    for (int rb = 0; rb < nb; rb++) {
+        const int v2 = rb % LZC_VB;
+        nrm2 += cl.map_shared_rank(&npart[v2 % LZC_HALVES][rb / LZC_VB], v2 / LZC_HALVES)[0];
+    }
+    cl.sync();                                  // no block leaves while others read its shared memory
+    const double bj = sqrt(nrm2);
+    const bool broken = bj <= 1e-12 * lz[r].b0;
+    if (rank == 0 && threadIdx.x == 0) {
+        alpha[(long)LZ_KMAX * r + j] = alpha_j;
+        lz[r].m = j + 1;
+        if (broken) lz[r].done = 2;             // invariant subspace: finalise with m = j + 1
+        else if (j + 1 < kmax) betad[(long)LZ_KMAX * r + j] = bj;
+    }
+    if (!broken && j + 1 < kmax) {
+        const double inv = bj > 0 ? 1.0 / bj : 0.0;
+        for (int sl = 0; sl < nslot; sl++) {
+            const int rb = vb + LZC_VB * sl;
+            if (rb >= nb) break;
+            const long st = (long)rb * RB_SPAN;
+            const int len = min(RB_SPAN, n - rb * RB_SPAN);
+            for (int e = t; e < len; e += RB_THREADS) V[(long)(j + 1) * ldv + base + st + e] = q[base + st + e] * inv;
+        }
+    }
+}
+
 int lanczos_sqrt(Engine &E, const double *z, double *w, const ps_sqrt_opts *o, ps_sqrt_result *res, cudaStream_t st)
 {
     int kmax = o && o->kmax > 0 ? o->kmax : 40;
@@ -787,7 +1016,9 @@ int lanczos_sqrt(Engine &E, const double *z, double *w, const ps_sqrt_opts *o, p
     ps_launch(k_lz_init, T.nblk, RB_THREADS, 0, st, T, E.d_segs, V, z, lz, nrm2);
     PS_CK(cudaMemsetAsync(gbuf, 0, sizeof(double) * (LZ_KMAX + 1) * E.R, st));
     const int check = 8;   // convergence test every 8 vectors; the cap is handled after the loop
-    const size_t smem = sizeof(double) * LZE_SMEM;
+    bool any_fixed = false, any_free = false;
+    for (const Seg &sg : E.segs) (lz_fixed(sg) ? any_fixed : any_free) = true;
+    const size_t smem = sizeof(double) * LZE_SMEM, smem_ql = sizeof(double) * (4 * LZ_KMAX + LZ_KMAX * LZ_KMAX);
     PS_CK(cudaFuncSetAttribute(k_lz_check, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
     std::vector<LzScal> hl(E.R);
     LzScal *snap = lz + E.R;                                 // the scalars when a check was launched
@@ -798,11 +1029,15 @@ int lanczos_sqrt(Engine &E, const double *z, double *w, const ps_sqrt_opts *o, p
     for (j = 0; j < kmax; j++) {
         const LzDots dots = {V, ldv, j, part1};
         apply_operator(E, 1, V + (long)j * ldv, q, E.precision == PS_PREC_MIXED, st, &lz[0].done,
-                       (int)sizeof(LzScal), false, &dots);
+                       (int)sizeof(LzScal), false, any_free ? &dots : nullptr);
         const dim3 sub((unsigned)T.nblk, RB_EPT);
-        ps_launch(k_lz_sub_dots, sub, RB_THREADS, 0, st, T, E.d_segs, V, ldv, q, j, lz, part1, alpha, part2);
-        ps_launch(k_lz_sub_norm, sub, RB_THREADS, 0, st, T, E.d_segs, V, ldv, q, j, lz, part2, alpha, npart);
-        ps_launch(k_lz_next, sub, RB_THREADS, 0, st, T, E.d_segs, V, ldv, q, j, kmax, lz, npart, betad);
+        if (any_fixed)
+            ps_launch(k_lz_orth_cluster, E.R * LZC_CTAS, LZC_THREADS, 0, st, E.d_segs, V, ldv, q, j, kmax, lz, alpha, betad);
+        if (any_free) {
+            ps_launch(k_lz_sub_dots, sub, RB_THREADS, 0, st, T, E.d_segs, V, ldv, q, j, lz, part1, alpha, part2);
+            ps_launch(k_lz_sub_norm, sub, RB_THREADS, 0, st, T, E.d_segs, V, ldv, q, j, lz, part2, alpha, npart);
+            ps_launch(k_lz_next, sub, RB_THREADS, 0, st, T, E.d_segs, V, ldv, q, j, kmax, lz, npart, betad);
+        }
         if ((j + 1) % check == 0 && j + 1 < kmax) {
             if (pending) {
                 // the previous check (normally finished long before): apply its outcomes
@@ -817,8 +1052,12 @@ int lanczos_sqrt(Engine &E, const double *z, double *w, const ps_sqrt_opts *o, p
             PS_CK(cudaMemcpyAsync(snap, lz, sizeof(LzScal) * E.R, cudaMemcpyDeviceToDevice, st));
             PS_CK(cudaEventRecord(E.ev_fork2, st));
             PS_CK(cudaStreamWaitEvent(E.side2, E.ev_fork2, 0));
-            ps_launch(k_lz_check, E.R, LZE_THREADS, smem, E.side2, E.R, lz, snap, spec, alpha, betad, gbuf, j + 1,
-                    tol, 0);
+            if (any_free)
+                ps_launch(k_lz_check, E.R, LZE_THREADS, smem, E.side2, E.R, E.d_segs, lz, snap, spec, alpha, betad, gbuf,
+                        j + 1, tol, 0);
+            if (any_fixed)
+                ps_launch(k_lz_check_ql, E.R, 32, smem_ql, E.side2, E.R, E.d_segs, lz, snap, spec, alpha, betad, gbuf, j + 1,
+                        tol, 0);
             PS_CK(cudaMemcpyAsync(hspec, spec, sizeof(LzSpec) * E.R, cudaMemcpyDeviceToHost, E.side2));
             PS_CK(cudaEventRecord(E.ev_chk, E.side2));
             pending = true;
@@ -830,8 +1069,12 @@ int lanczos_sqrt(Engine &E, const double *z, double *w, const ps_sqrt_opts *o, p
         ps_launch(k_lz_spec_apply, (E.R + 127) / 128, 128, 0, st, E.R, lz, spec);
     }
     // final estimate: replicas at the cap, replicas stopped by breakdown, and the converged ones on their own m
-    ps_launch(k_lz_check, E.R, LZE_THREADS, smem, st, E.R, lz, snap, spec, alpha, betad, gbuf,
-            std::min(j + 1, kmax), tol, 1);
+    if (any_free)
+        ps_launch(k_lz_check, E.R, LZE_THREADS, smem, st, E.R, E.d_segs, lz, snap, spec, alpha, betad, gbuf,
+                std::min(j + 1, kmax), tol, 1);
+    if (any_fixed)
+        ps_launch(k_lz_check_ql, E.R, 32, smem_ql, st, E.R, E.d_segs, lz, snap, spec, alpha, betad, gbuf,
+                std::min(j + 1, kmax), tol, 1);
     ps_launch(k_lz_combine, T.nblk, RB_THREADS, 0, st, T, V, ldv, lz, gbuf, w);
     PS_CK(cudaMemcpyAsync(hl.data(), lz, sizeof(LzScal) * E.R, cudaMemcpyDeviceToHost, st));
     PS_CK(cudaStreamSynchronize(st));

@@ -91,6 +91,7 @@ struct Seg {
     int nper;          // monomers per chain
     int ss_off;        // offset of the inverse stresslet block (nc5^2 doubles), -1 if none
     int nch_bb;        // column chunks of the colloid far field (a function of Nc alone)
+    int indef;         // the replica's far field may be indefinite (krylov.cu lz_fixed)
     int aa_nt;         // tiles of the monomer far field (0: no monomer pairs), and as many partial slots per row
     long paa_off;      // this replica's monomer far-field partials: aa_nt slots of nm3 doubles
     // monomer-monomer scalars as x = c0/r + c1/r^3, y = c2/r + c3/r^3 (r > 2 beta)
@@ -113,9 +114,12 @@ constexpr int aa_tile_edge(int Nm) { return Nm <= 1536 ? 64 : (Nm <= 12288 ? 128
 struct AaTile { int rep, I, J, S; };
 constexpr int FAR_AB = 0, FAR_BB = -1;
 
-// Column chunk widths of the colloid far field.
-constexpr int BB_CHUNK_COLS = 64;        // colloid columns per chunk, for up to BB_MAX_CHUNKS chunks
-constexpr int BB_MAX_CHUNKS = 64;
+// Column chunk width of the colloid far field, for up to BB_MAX_CHUNKS chunks, and its row tiles:
+// BB_TILE rows (four blocks per SM), BB_WIDE rows (one block per SM) where those are one wave that
+// nearly fills the chip.  Both add in the same order.  One launch with 32 and with 128 rows:
+// 512 colloids 9.6 and 17.8 us, 1024 colloids (128 wide blocks) 19.8 and 18.1, 1600 (325) 37.9 and 51.1.
+constexpr int BB_TILE = 32, BB_WIDE = 128, BB_CHUNK_COLS = 64, BB_MAX_CHUNKS = 64;
+constexpr bool bb_wide(int Nc, int nch) { return (Nc + BB_WIDE - 1) / BB_WIDE * nch <= 148 && Nc > 896; }
 
 // Row tile of the far-field pair kernels.
 struct Tile { int rep; int row0; int nrow; int mtile; };

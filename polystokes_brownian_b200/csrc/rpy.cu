@@ -16,7 +16,27 @@
 
 namespace ps {
 
-constexpr int RPY_THREADS = 128;
+// Single-precision image of a positive double in [2^-126, 2^128) by exponent re-bias and
+// mantissa truncation (relative error below 2^-23), with integer operations only, so the
+// FP64 pipe is left to the arithmetic; seed_as_double widens a positive normal float exactly.
+__device__ __forceinline__ float trunc_to_float(double a)
+{
+    const int hi = __double2hiint(a), lo = __double2loint(a);
+    return __int_as_float(((hi - (896 << 20)) << 3) | (int)((unsigned)lo >> 29));
+}
+__device__ __forceinline__ double seed_as_double(float f)
+{
+    const int b = __float_as_int(f);
+    return __hiloint2double((b >> 3) + (896 << 20), b << 29);
+}
+
+__device__ __forceinline__ double rsqrt_seeded(double a, float af)
+{
+    const double y = seed_as_double(rsqrtf(af));
+    const double e = fma(-(a * y), y, 1.0);
+    return fma(y * e, fma(0.375, e, 0.5), y);
+}
+__device__ __forceinline__ double rsqrt_seeded(double a) { return rsqrt_seeded(a, trunc_to_float(a)); }
 
 // ---------------------------------------------------------------------------
 // AB/BA: a tile of 128 monomers x the colloids of the replica.  Monomer outputs
@@ -144,36 +164,43 @@ __device__ __forceinline__ void ab_block(const Seg &sg, int rep, int mt, const t
 }
 
 // ---------------------------------------------------------------------------
-// BB: colloid rows x colloid columns (FTS, 11 -> 11), FP64.  SPLIT threads per row
-// (a block is SPLIT x RPY_THREADS threads): thread group h takes the tile
-// columns h, h + SPLIT, ...; the groups' sums are joined in group order in
-// shared memory, so a replica of a thousand colloids fills the SMs without
-// more chunk partials.
-struct BbSmem { double4 sp[64]; double su[64 * 11]; };
+// BB: colloid rows x colloid columns (FTS, 11 -> 11), FP64.  A block takes BB_ROWS
+// rows of one column chunk, one row per lane; warp h of SPLIT takes the chunk's
+// columns h, h + SPLIT, ... (every lane the same column: shared-memory broadcasts),
+// and the warps' sums are joined in warp order in shared memory.
+//
+// Bound: the chain of a pair's dependent FP64 operations; small blocks spread a suspension
+// over all SMs.  Against blocks of 128 rows, one launch: 300
+// colloids 17.0 -> 9.2 us, 512 17.8 -> 9.6, 1600 51.1 -> 37.9.
+// The order of the sums and the arithmetic of a pair are what they were: the solves of a
+// suspension whose far field is close to singular return, within rtol, whatever their rounding
+// selects.  (A pair action of 140 operations for 190 and chunks of 32 columns gave 14.9 us at
+// 1024 colloids, and positions off by 1e-6 in one step of ten.)
+constexpr int BB_ROWS = BB_TILE, BB_CT = 64;
+struct BbSmem { double4 sp[BB_CT]; double su[BB_CT * 11]; };
 
-template <int SPLIT>
+template <int ROWS, int SPLIT>
 __device__ __forceinline__ void bb_block(const Seg &sg, int rt, int c, const double4 *__restrict__ pos,
                                          const double *__restrict__ u, int uoff, double *__restrict__ part,
-                                         long part_stride, BbSmem &sm, double (*sred)[11][RPY_THREADS])
+                                         long part_stride, BbSmem &sm, double (*sred)[11][ROWS])
 {
-    constexpr int CT = 64;
-    const int row = threadIdx.x % RPY_THREADS, grp = threadIdx.x / RPY_THREADS;
+    const int row = threadIdx.x % ROWS, grp = threadIdx.x / ROWS;
     const int Nc = sg.Nc, Nm = sg.Nm;
     const int j0 = (int)((long)Nc * c / sg.nch_bb), j1 = (int)((long)Nc * (c + 1) / sg.nch_bb);
-    const int i = RPY_THREADS * rt + row;
+    const int i = ROWS * rt + row;
     const bool active = i < Nc;
-    const double4 pi = pos[sg.bead_off + Nm + (active ? i : RPY_THREADS * rt)];
+    const double4 pi = pos[sg.bead_off + Nm + (active ? i : ROWS * rt)];
     double out[11];   // accumulated over the chunk's column tiles in column order
     for (int q = 0; q < 11; q++) out[q] = 0.0;
-    for (int jt = j0; jt < j1; jt += CT) {
-        const int nj = min(CT, j1 - jt);
+    for (int jt = j0; jt < j1; jt += BB_CT) {
+        const int nj = min(BB_CT, j1 - jt);
         __syncthreads();
         for (int t = threadIdx.x; t < nj * 11; t += blockDim.x) {
             int k = t / 11, q = t - 11 * k, j = jt + k;
             int idx = q < 3 ? sg.nm3 + 3 * j + q : (q < 6 ? sg.nm3 + sg.nc3 + 3 * j + (q - 3) : sg.nm3nc6 + 5 * j + (q - 6));
             sm.su[t] = u[uoff + idx];
         }
-        if (threadIdx.x < nj) sm.sp[threadIdx.x] = pos[sg.bead_off + Nm + jt + threadIdx.x];
+        for (int t = threadIdx.x; t < nj; t += blockDim.x) sm.sp[t] = pos[sg.bead_off + Nm + jt + t];
         __syncthreads();
         for (int k = grp; k < nj; k += SPLIT) {
             const int j = jt + k;
@@ -208,7 +235,8 @@ __device__ __forceinline__ void bb_block(const Seg &sg, int rt, int c, const dou
 // Colloid pairs of the replicas without monomers (suspensions); those beside
 // monomers ride in the monomer kernels' launches.
 constexpr int BB_SPLIT = 4;
-__global__ void __launch_bounds__(RPY_THREADS * BB_SPLIT)
+template <int ROWS>
+__global__ void __launch_bounds__(ROWS * BB_SPLIT)
 k_rpy_bb(const Seg *__restrict__ segs, const Tile *__restrict__ tiles, const double4 *__restrict__ pos,
          const double *__restrict__ u, int in_top, double *__restrict__ part, long part_stride,
          const char *__restrict__ done, int done_stride)
@@ -217,10 +245,10 @@ k_rpy_bb(const Seg *__restrict__ segs, const Tile *__restrict__ tiles, const dou
     const Tile tl = tiles[blockIdx.x];
     if (done && *(const int *)(done + (long)tl.rep * done_stride)) return;
     __shared__ BbSmem sm;
-    __shared__ double sred[BB_SPLIT - 1][11][RPY_THREADS];
+    __shared__ double sred[BB_SPLIT - 1][11][ROWS];
     const Seg &sg = segs[tl.rep];
     if ((int)blockIdx.y >= sg.nch_bb) return;
-    bb_block<BB_SPLIT>(sg, tl.mtile, blockIdx.y, pos, u, in_top ? sg.top_off : sg.vec_off, part, part_stride, sm, sred);
+    bb_block<ROWS, BB_SPLIT>(sg, tl.mtile, blockIdx.y, pos, u, in_top ? sg.top_off : sg.vec_off, part, part_stride, sm, sred);
 }
 
 // The partial sums of one apply, as the far-field kernels write them.
@@ -409,14 +437,15 @@ k_rpy_aa_f2(const Seg *__restrict__ segs, const AaTile *__restrict__ tiles, cons
             double row[3 * AA_TILE_MAX];                   // row sums per column group or band (3 S slots in all)
         } aa;
         float red[2][AB_WARPS][12];
-        BbSmem bb;
+        struct { BbSmem t; double sred[AAF_THREADS / BB_ROWS - 1][11][BB_ROWS]; } bb;
     } sm;
     if (tl.S == FAR_AB) {
         ab_block<float>(sg, tl.rep, tl.I, pos, plo, u, in_top ? sg.top_off : sg.vec_off, O.tab, O.ab, O.ba, sm.red);
         return;
     }
     if (tl.S == FAR_BB) {
-        bb_block<1>(sg, tl.I, tl.J, p64, u, in_top ? sg.top_off : sg.vec_off, O.bb, O.bb_stride, sm.bb, nullptr);
+        bb_block<BB_ROWS, AAF_THREADS / BB_ROWS>(sg, tl.I, tl.J, p64, u, in_top ? sg.top_off : sg.vec_off, O.bb, O.bb_stride,
+                                        sm.bb.t, sm.bb.sred);
         return;
     }
     float4 (&sCols)[5][AA_TILE_MAX / 2] = sm.aa.cols;
@@ -527,28 +556,6 @@ k_rpy_aa_f2(const Seg *__restrict__ segs, const AaTile *__restrict__ tiles, cons
 // under a warp vote.  Far form in factored scalars: y = ri (c + d ri^2),
 // (x - y) / r^2 = ri^3 (a + b ri^2), a = c0 - c2, b = c1 - c3, c = c2, d = c3.
 
-// Single-precision image of a positive double in [2^-126, 2^128) by exponent re-bias and
-// mantissa truncation (relative error below 2^-23), with integer operations only, so the
-// FP64 pipe is left to the arithmetic; seed_as_double widens a positive normal float exactly.
-__device__ __forceinline__ float trunc_to_float(double a)
-{
-    const int hi = __double2hiint(a), lo = __double2loint(a);
-    return __int_as_float(((hi - (896 << 20)) << 3) | (int)((unsigned)lo >> 29));
-}
-__device__ __forceinline__ double seed_as_double(float f)
-{
-    const int b = __float_as_int(f);
-    return __hiloint2double((b >> 3) + (896 << 20), b << 29);
-}
-
-__device__ __forceinline__ double rsqrt_seeded(double a, float af)
-{
-    const double y = seed_as_double(rsqrtf(af));
-    const double e = fma(-(a * y), y, 1.0);
-    return fma(y * e, fma(0.375, e, 0.5), y);
-}
-__device__ __forceinline__ double rsqrt_seeded(double a) { return rsqrt_seeded(a, trunc_to_float(a)); }
-
 struct AaScalD { double ca, cb, cc, cd, tb, n0, n1, n2, n3; float tb2f; };
 
 template <bool SYM, bool CHECK>
@@ -627,7 +634,7 @@ k_rpy_aa_d2(const Seg *__restrict__ segs, const AaTile *__restrict__ tiles, cons
             double w[AA_TILE_MAX], col[3 * 4 * AA_TILE_MAX];   // chain ids; column sums per row group or band
         } aa;
         double red[2][AB_WARPS][12];
-        struct { BbSmem t; double sred[AAD_THREADS / RPY_THREADS - 1][11][RPY_THREADS]; } bb;
+        struct { BbSmem t; double sred[AAD_THREADS / BB_ROWS - 1][11][BB_ROWS]; } bb;
     } sm;
     const Seg &sg = segs[tl.rep];
     if (tl.S == FAR_AB) {
@@ -635,7 +642,7 @@ k_rpy_aa_d2(const Seg *__restrict__ segs, const AaTile *__restrict__ tiles, cons
         return;
     }
     if (tl.S == FAR_BB) {
-        bb_block<AAD_THREADS / RPY_THREADS>(sg, tl.I, tl.J, pos, u, in_top ? sg.top_off : sg.vec_off, O.bb, O.bb_stride,
+        bb_block<BB_ROWS, AAD_THREADS / BB_ROWS>(sg, tl.I, tl.J, pos, u, in_top ? sg.top_off : sg.vec_off, O.bb, O.bb_stride,
                                             sm.bb.t, sm.bb.sred);
         return;
     }
@@ -766,9 +773,72 @@ __device__ __forceinline__ int find_rep(const int *__restrict__ offs, int R, lon
 // once; blockIdx.y splits an entry's span so that each thread sums one output
 // (a single large replica otherwise leaves most SMs idle while every thread
 // walks its chunk partials four times over).
+// v + the n partial sums p[0], p[stride], ... in order, eight loads in flight
+__device__ __forceinline__ double add_slots(double v, const double *__restrict__ p, int n, long stride)
+{
+    for (int c = 0; c < n; c += 8) {
+        double t[8];
+#pragma unroll
+        for (int k = 0; k < 8; k++) t[k] = c + k < n ? p[(c + k) * stride] : 0.0;
+#pragma unroll
+        for (int k = 0; k < 8; k++) v += t[k];
+    }
+    return v;
+}
+
 // what a combine goes on with
 enum { CB_PLAIN, CB_DOTS, CB_MINRES };
 struct NoTail {};
+
+// entry k (index i within the replica) of the product
+__device__ __forceinline__ double combine_entry(const Seg &sg, int mode, int i, int xo, const double *__restrict__ x,
+                                                const double *__restrict__ partAA, int with_aa,
+                                                const double *__restrict__ partAB, const double *__restrict__ partBB,
+                                                const double *__restrict__ partBA, const double *__restrict__ delta,
+                                                const double *__restrict__ lub_y, long part_stride)
+{
+    double v = 0.0;
+    if (i < sg.nm3nc11) {
+        if (i < sg.nm3) {
+            v = sg.beta_inv * x[xo + i];
+            if (with_aa) {
+                v = add_slots(v, partAA + sg.paa_off + i, sg.aa_nt, sg.nm3);      // one slot per column tile
+            }
+            if (sg.Nc > 0) v += partAB[sg.top_off + i];
+        } else {
+            int j = i - sg.nm3;          // colloid-local DOF in [0, nc11)
+            int cidx, q;                 // colloid index, component
+            double self;
+            if (j < sg.nc3) { cidx = j / 3; q = j % 3; self = x[xo + i]; }
+            else if (j < sg.nc6) { cidx = (j - sg.nc3) / 3; q = 3 + (j - sg.nc3) % 3; self = 0.75 * x[xo + i]; }
+            else {
+                cidx = (j - sg.nc6) / 5; q = 6 + (j - sg.nc6) % 5;
+                int sb = xo + sg.nm3nc6 + 5 * cidx, p = q - 6;
+                self = 1.8 * x[sb + p];
+                if (p == 0) self += 0.9 * x[sb + 4];
+                if (p == 4) self += 0.9 * x[sb + 0];
+            }
+            v = self;
+            if (sg.Nc >= 2) {
+                v = add_slots(v, partBB + sg.top_off + i, sg.nch_bb, part_stride);
+            }
+            if (sg.Nm > 0)
+                for (int t = 0; t < sg.n_mtiles; t++) v += partBA[((long)sg.ba_off + (long)t * sg.Nc + cidx) * 11 + q];
+            if (sg.shell_schur) {
+                const double *D = delta + sg.schur_off + (long)j * sg.nc11;
+                double acc = 0.0;
+                for (int b = 0; b < sg.nc11; b++) acc += D[b] * x[xo + sg.nm3 + b];
+                v += acc;
+            }
+        }
+        if (mode == 0 && i < sg.nm3nc6) v -= x[xo + sg.nm3nc11 + i];
+    } else {
+        int j = i - sg.nm3nc11;
+        v = -x[xo + j];
+        if (sg.lub_on && lub_y) v -= lub_y[sg.vel_off + j];
+    }
+    return v;
+}
 
 template <int TAIL, class X>
 __global__ void k_combine(const Seg *__restrict__ segs, RedTable T, int mode, const double *__restrict__ x,
@@ -793,56 +863,13 @@ __global__ void k_combine(const Seg *__restrict__ segs, RedTable T, int mode, co
     const long k = (long)B.start + e;
     double out = 0.0;
     if (e < B.len) {
-        const int i = (int)(k - xo);
-        double v = 0.0;
-        if (i < sg.nm3nc11) {
-            if (i < sg.nm3) {
-                v = sg.beta_inv * x[xo + i];
-                if (with_aa) {
-                    const double *pa = partAA + sg.paa_off + i;      // one slot per column tile
-#pragma unroll 8
-                    for (int c = 0; c < sg.aa_nt; c++) v += pa[(long)c * sg.nm3];
-                }
-                if (sg.Nc > 0) v += partAB[sg.top_off + i];
-            } else {
-                int j = i - sg.nm3;          // colloid-local DOF in [0, nc11)
-                int cidx, q;                 // colloid index, component
-                double self;
-                if (j < sg.nc3) { cidx = j / 3; q = j % 3; self = x[xo + i]; }
-                else if (j < sg.nc6) { cidx = (j - sg.nc3) / 3; q = 3 + (j - sg.nc3) % 3; self = 0.75 * x[xo + i]; }
-                else {
-                    cidx = (j - sg.nc6) / 5; q = 6 + (j - sg.nc6) % 5;
-                    int sb = xo + sg.nm3nc6 + 5 * cidx, p = q - 6;
-                    self = 1.8 * x[sb + p];
-                    if (p == 0) self += 0.9 * x[sb + 4];
-                    if (p == 4) self += 0.9 * x[sb + 0];
-                }
-                v = self;
-                if (sg.Nc >= 2) {
-#pragma unroll 8
-                    for (int c = 0; c < sg.nch_bb; c++) v += partBB[(long)c * part_stride + sg.top_off + i];
-                }
-                if (sg.Nm > 0)
-                    for (int t = 0; t < sg.n_mtiles; t++) v += partBA[((long)sg.ba_off + (long)t * sg.Nc + cidx) * 11 + q];
-                if (sg.shell_schur) {
-                    const double *D = delta + sg.schur_off + (long)j * sg.nc11;
-                    double acc = 0.0;
-                    for (int b = 0; b < sg.nc11; b++) acc += D[b] * x[xo + sg.nm3 + b];
-                    v += acc;
-                }
-            }
-            if (mode == 0 && i < sg.nm3nc6) v -= x[xo + sg.nm3nc11 + i];
-        } else {
-            int j = i - sg.nm3nc11;
-            v = -x[xo + j];
-            if (sg.lub_on && lub_y) v -= lub_y[sg.vel_off + j];
-        }
-        out = v;
-        if constexpr (TAIL != CB_MINRES) y[k] = v;
+        out = combine_entry(sg, mode, (int)(k - xo), xo, x, partAA, with_aa, partAB, partBB, partBA, delta, lub_y, part_stride);
+        if constexpr (TAIL != CB_MINRES) y[k] = out;
     }
     if (blockIdx.y * RB_THREADS >= B.len) return;
     if constexpr (TAIL == CB_DOTS)
-        lz_block_dots(tail.V, tail.ldv, k, e < B.len, out, tail.j, tail.part + (long)LZ_KMAX * (RB_EPT * blockIdx.x + blockIdx.y));
+        lz_block_dots(tail.V, tail.ldv, k, e < B.len, out, tail.j,
+                      tail.part + (long)LZ_KMAX * (RB_EPT * blockIdx.x + blockIdx.y));
     if constexpr (TAIL == CB_MINRES) mr_alpha(T, B, sg.n, k, e < B.len, out, tail, y);
 }
 
@@ -875,9 +902,12 @@ static void launch_far(Engine &E, const double *u, int in_top, bool fp32, int fi
 
 static void launch_bb(Engine &E, const double *u, int in_top, cudaStream_t st, const char *done, int dstride)
 {
-    if (E.n_bb_tiles)
-        ps_launch(k_rpy_bb, dim3(E.n_bb_tiles, E.nch_bb), RPY_THREADS * BB_SPLIT, 0, st, E.d_segs, E.d_bb_tiles, E.d_pos64,
-                u, in_top, E.d_partBB, E.part_stride, done, dstride);
+    if (E.n_bb_wide)
+        ps_launch(k_rpy_bb<BB_WIDE>, dim3(E.n_bb_wide, E.nch_bb), BB_WIDE * BB_SPLIT, 0, st, E.d_segs, E.d_bb_tiles,
+                E.d_pos64, u, in_top, E.d_partBB, E.part_stride, done, dstride);
+    if (E.n_bb_tiles > E.n_bb_wide)
+        ps_launch(k_rpy_bb<BB_ROWS>, dim3(E.n_bb_tiles - E.n_bb_wide, E.nch_bb), BB_ROWS * BB_SPLIT, 0, st, E.d_segs,
+                E.d_bb_tiles + E.n_bb_wide, E.d_pos64, u, in_top, E.d_partBB, E.part_stride, done, dstride);
 }
 
 void apply_operator(Engine &E, int mode, const double *x, double *y, bool fp32, cudaStream_t st,
@@ -927,7 +957,7 @@ int set_aa_chunking(Engine &E, int cols)
             if (s.Nc > 0)
                 for (int t = 0; t < s.n_mtiles; t++) pre.push_back({r, t, 0, FAR_AB});
             if (s.Nc >= 2)
-                for (int t = 0; t * RPY_THREADS < s.Nc; t++)
+                for (int t = 0; t * BB_ROWS < s.Nc; t++)
                     for (int c = 0; c < s.nch_bb; c++) pre.push_back({r, t, c, FAR_BB});
         }
     }
