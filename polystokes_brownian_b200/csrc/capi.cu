@@ -62,17 +62,16 @@ static void free_engine(Engine &E)
                     E.d_Rr[1], E.d_Rr[2], E.d_W[0], E.d_W[1], E.d_W[2], E.d_mr, E.d_mrp, E.d_nactive,
                     E.d_rhs, E.d_X, E.d_Xd, E.d_Xdet, E.d_Wn, E.d_vdn, E.d_vdc, E.d_vb, E.d_up, E.d_ud,
                     E.d_drift, E.d_sb, E.d_fext, E.d_fb, E.d_wr, E.d_tmp_top, E.d_tmp_top2, E.d_lzV, E.d_lzT,
-                    E.d_lzw, E.d_lzq, E.d_lzp, E.d_lzs, E.d_ssinv, E.d_pcg, E.d_pV, E.d_pr, E.d_pz, E.d_pp, E.d_ps,
-                    E.d_pAp, E.d_pg, E.d_pu, E.d_py, E.d_pu2, E.d_py2, E.d_rseed, E.d_rstep,
+                    E.d_lzw, E.d_lzq, E.d_lzp, E.d_lzs, E.d_ssinv, E.d_pcg, E.d_pV, E.d_pz, E.d_pp,
+                    E.d_pblk, E.d_pbp, E.d_pg, E.d_pu, E.d_py, E.d_pu2, E.d_py2, E.d_rseed, E.d_rstep,
                     E.d_lubc_ptr, E.d_lubc_nbr, E.d_lub_pairs, E.d_pS, E.d_pP, E.d_py_[0], E.d_py_[1], E.d_py_[2],
-                    E.d_py_[3], E.d_py_[4], E.d_ppart, E.d_scan_sums, E.d_sv[0], E.d_sv[1], E.d_sv[2],
-                    E.d_sv[3], E.d_sv[4], E.d_sbead[0], E.d_sbead[1], E.d_ppart2, E.d_pmr,
+                    E.d_py_[3], E.d_py_[4], E.d_scan_sums, E.d_pmr,
                     E.d_pmp[0], E.d_pmp[1], E.d_pmp[2], E.d_pmp[3], E.d_pmp[4], E.d_pmp[5], E.d_pmp[6],
-                    E.d_pmp[7], E.d_pmp[8], E.d_pmp[9], E.d_pms[0], E.d_pms[1], E.d_pms[2], E.d_pms[3],
+                    E.d_pmp[7], E.d_pmp[8], E.d_pmd, E.d_pms[0], E.d_pms[1], E.d_pms[2], E.d_pms[3],
                     E.d_pms[4], E.d_pms[5], E.d_pms[6], E.d_pms[7], E.d_pms[8], E.d_obs_acc, E.d_obs_prev,
                     E.d_obs_ring, E.d_obs_msd, E.d_obs_hasprev, E.d_obs_hb, E.d_obs_ht, E.d_obs_msdn,
                     E.d_sl_reps, E.d_sl_skip, E.d_slV, E.d_slT, E.d_sl_sc, E.d_sl_u, E.d_sl_y, E.d_sl_y2,
-                    E.d_cell_big, E.d_cell_nbig, E.d_cell_tmp, E.d_ref_r, E.d_ref_d, E.d_pm_cnt, E.d_fresh};
+                    E.d_cell_big, E.d_cell_nbig, E.d_cell_tmp, E.d_ref_r, E.d_ref_d, E.d_fresh};
     for (void *p : ptrs)
         if (p) cudaFree(p);
     if (E.h_nactive) cudaFreeHost(E.h_nactive);
@@ -83,7 +82,6 @@ static void free_engine(Engine &E)
     ps::free_red_table(E.red);
     ps::free_red_table(E.red_top);
     ps::free_red_table(E.red_vel);
-    ps::free_red_table(E.red_bead);
 }
 
 static int build(Engine &E, const ps_desc *descs, int R, int precision)
@@ -368,17 +366,24 @@ static int build(Engine &E, const ps_desc *descs, int R, int precision)
     if (E.any_lub || ss_polish) {
         E.n_ssinv = ssinv;
         TRY_ALLOC(E.d_ssinv, sizeof(double) * std::max<long>(ssinv, 1));
-        TRY_ALLOC(E.d_pcg, sizeof(ps::PcgScal) * R);
-        double **pv[] = {&E.d_pV, &E.d_pr, &E.d_pz, &E.d_pp, &E.d_ps, &E.d_pAp, &E.d_pg};
+        TRY_ALLOC(E.d_pcg, sizeof(ps::PcgScal) * 2 * R);
+        double **pv[] = {&E.d_pV, &E.d_pz, &E.d_pp, &E.d_pg};
         for (double **p : pv) TRY_ALLOC(*p, sizeof(double) * vel);
         double **pt[] = {&E.d_pu, &E.d_py, &E.d_pu2, &E.d_py2};
         for (double **p : pt) TRY_ALLOC(*p, sizeof(double) * top);
         if ((rc = ps::build_red_table(E, E.red_vel, 2))) return rc;
-        if ((rc = ps::build_red_table(E, E.red_bead, 3))) return rc;
-        for (auto &p : E.d_sv) TRY_ALLOC(p, sizeof(double) * top);
-        for (auto &p : E.d_sbead) TRY_ALLOC(p, sizeof(double) * bead);
         for (auto &p : E.d_pms) TRY_ALLOC(p, sizeof(double) * top);
-        TRY_ALLOC(E.d_pmr, sizeof(ps::MinresScal) * R);
+        TRY_ALLOC(E.d_pmr, sizeof(ps::MinresScal) * 2 * R);
+        // work split of the pair space: by the replica's beads alone
+        std::vector<ps::PairBlk> pb;
+        for (int r = 0; r < R; r++) {
+            const Seg &s = E.segs[r];
+            const int per = std::max(s.Nm ? 32 : 2, (s.Np + 511) / 512), G = (s.Np + per - 1) / per, first = (int)pb.size();
+            for (int b = 0; b < G; b++) pb.push_back({r, b, G, first});
+        }
+        E.n_pblk = (int)pb.size();
+        if ((rc = upload(E.d_pblk, pb))) return rc;
+        TRY_ALLOC(E.d_pbp, sizeof(double) * 3 * E.n_pblk);
     }
     // Lanczos
     if (E.any_mmhi) {

@@ -20,6 +20,10 @@ struct MinresScal {
 // Reduction block table entry: a contiguous range of one replica's segment.
 struct RBlk { int rep; int start; int len; };
 
+// Block of the pair space: share b of G of a replica's near pairs, beads and colloids; first:
+// the replica's first block (solve.cu).
+struct PairBlk { int rep, b, G, first; };
+
 struct RedTable {
     int nblk = 0;
     RBlk *d_blk = nullptr;       // per block
@@ -44,9 +48,9 @@ struct MrAlpha {
     int *nactive, k, maxit;
 };
 
-// Per-replica scalars of the lubricated resistance-form PCG.
+// Per-replica scalars of the pair-space CG.
 struct PcgScal {
-    double rz, alpha, beta, tol, err;
+    double rz, beta, tol, err;
     int it, done, reason, pad;
 };
 
@@ -129,14 +133,15 @@ struct Engine {
     int *d_lubc_ptr = nullptr, *d_lubc_nbr = nullptr; int2 *d_lub_pairs = nullptr; long lubc_cap = 0;  // canonical
     // pair-space lubricated solve: per pair K^{1/2} and preconditioner blocks (12x12), CG vectors (12 per pair)
     double *d_pS = nullptr, *d_pP = nullptr, *d_py_[5] = {nullptr, nullptr, nullptr, nullptr, nullptr};
-    double *d_ppart = nullptr; long pair_cap = 0;
+    long pair_cap = 0, pm_cap = 0;   // pairs that the pair-space buffers and the MINRES vectors hold
+    PairBlk *d_pblk = nullptr; int n_pblk = 0;
+    double *d_pbp = nullptr;         // block sums of the pair-space dots (3 per block)
     // pair blocks d_pS / d_pP hold the setup of the current staged positions
     // (cleared by every packing, table change and reallocation)
     bool ps_setup_valid = false;
-    // stresslet unknowns of replicas without a dense stresslet inverse (mobility layout), per-bead partials
-    double *d_sv[5] = {nullptr, nullptr, nullptr, nullptr, nullptr}, *d_sbead[2] = {nullptr, nullptr};
-    // pair-space MINRES: 10 pair-storage vectors (3 r, 3 w, v, z, x, Az), 9 stresslet-storage vectors, scalars
-    double *d_pmp[10] = {}, *d_pms[9] = {}, *d_ppart2 = nullptr;
+    // pair-space MINRES: 9 pair-storage and 9 stresslet-storage vectors (3 r, 3 w, v, z, x), scalars
+    double *d_pmp[9] = {}, *d_pms[9] = {};
+    double *d_pmd = nullptr;         // its dots: three times a number per pair, then per bead
     MinresScal *d_pmr = nullptr;
     bool any_indef = false;          // some replica's far field may be indefinite: pair-space MINRES
 
@@ -147,7 +152,6 @@ struct Engine {
     int obs_nbins = 0, obs_lags = 0;
     double obs_bmax = 0.0, obs_tmax = 0.0;
     long obs_n = 0;
-    RedTable red_bead;               // over beads (pair-space sums by lower bead)
 
     // Krylov workspace
     RedTable red;                    // over saddle vectors
@@ -156,8 +160,7 @@ struct Engine {
     // lubricated structured solve: inverse stresslet blocks, PCG state (velocity layout)
     double *d_ssinv = nullptr; long n_ssinv = 0;
     PcgScal *d_pcg = nullptr;
-    double *d_pV = nullptr, *d_pr = nullptr, *d_pz = nullptr, *d_pp = nullptr, *d_ps = nullptr, *d_pAp = nullptr,
-           *d_pg = nullptr;
+    double *d_pV = nullptr, *d_pz = nullptr, *d_pp = nullptr, *d_pg = nullptr;   // -b_bot, L z, L p, g
     double *d_pu = nullptr, *d_py = nullptr, *d_pu2 = nullptr, *d_py2 = nullptr;   // mobility layout
     double *d_D = nullptr, *d_z = nullptr, *d_v = nullptr, *d_xw = nullptr;
     double *d_Rr[3] = {nullptr, nullptr, nullptr}, *d_W[3] = {nullptr, nullptr, nullptr};
@@ -172,7 +175,6 @@ struct Engine {
     double *d_drift = nullptr, *d_sb = nullptr, *d_fext = nullptr, *d_fb = nullptr, *d_wr = nullptr;
     double *d_tmp_top = nullptr, *d_tmp_top2 = nullptr;
     double *d_ref_r = nullptr, *d_ref_d = nullptr;   // iterative refinement: residual, correction (allocated on first use)
-    int *d_pm_cnt = nullptr;                         // pair-space MINRES: items finished per replica (first use)
     uint64_t seed = 12345, step_counter = 0;
     uint64_t *d_rseed = nullptr, *d_rstep = nullptr;   // per-replica Philox key and step counter
 

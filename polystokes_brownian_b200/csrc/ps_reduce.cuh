@@ -59,25 +59,21 @@ __device__ __forceinline__ bool finish_block(const RedTable &T, const RBlk &b, i
     return false;
 }
 
-// Total of a replica's sub-block sums (sub-blocks of RB_THREADS entries, nb of them, from
-// part[RB_EPT * first] on), the same in every thread of the block and in a fixed order.  Every
-// block of a kernel adds its replica's sums itself: no counters, no fences, no last block.
+// Total of a replica's nb block sums, the same in every thread of the block and in a fixed
+// order (of nb and the block's width, at most RB_THREADS).  Every block of a kernel adds its
+// replica's sums itself: no counters, no fences, no last block.
 __device__ __forceinline__ double rep_total(const double *__restrict__ part, int nb)
 {
-    __shared__ double ws[RB_THREADS / 32], tot;
+    __shared__ double ws[RB_THREADS / 32];
     double t = 0.0;
-    for (int b = threadIdx.x; b < nb; b += RB_THREADS) t += part[b];
+    for (int b = threadIdx.x; b < nb; b += blockDim.x) t += part[b];
     for (int o = 16; o > 0; o >>= 1) t += __shfl_down_sync(0xffffffffu, t, o);
+    __syncthreads();                       // an earlier total has been read
     if ((threadIdx.x & 31) == 0) ws[threadIdx.x >> 5] = t;
     __syncthreads();
-    if (threadIdx.x == 0) {
-        double v = 0.0;
-#pragma unroll
-        for (int w = 0; w < RB_THREADS / 32; w++) v += ws[w];
-        tot = v;
-    }
-    __syncthreads();
-    return tot;
+    t = 0.0;
+    for (int w = 0; w < (int)(blockDim.x >> 5); w++) t += ws[w];
+    return t;
 }
 
 // MINRES scalars after an iteration, from its r.z total bb (Paige & Saunders; PETSc's test):

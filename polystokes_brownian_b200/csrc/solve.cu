@@ -223,13 +223,14 @@ __global__ void k_ss_apply(const Seg *__restrict__ segs, const int *__restrict__
     }
 }
 
-// reference norm ||D^{-1} b|| over the saddle vector; initial scalars
-__global__ void k_pcg_start(RedTable T, const Seg *__restrict__ segs, const double *__restrict__ b,
-                            const double *__restrict__ D, PcgScal *pc, double rtol)
+// reference norm ||D^{-1} b|| over the saddle vector; initial scalars; all R replicas active
+__global__ void k_pcg_start(RedTable T, const double *__restrict__ b, const double *__restrict__ D, PcgScal *pc,
+                            double rtol, int R, int *__restrict__ nactive)
 {
     pdl_enter();
     __shared__ double sh[RB_THREADS / 32][1];
     const RBlk B = T.d_blk[blockIdx.x];
+    if (blockIdx.x == 0 && threadIdx.x == 0) *nactive = R;
     double v[1] = {0.0};
     for (int e = threadIdx.x; e < B.len; e += RB_THREADS) {
         double t = b[B.start + e] / D[B.start + e];
@@ -238,27 +239,9 @@ __global__ void k_pcg_start(RedTable T, const Seg *__restrict__ segs, const doub
     block_sum<1>(v, sh);
     double tot[1];
     if (finish_block<1>(T, B, blockIdx.x, v, tot)) {
-        const Seg &s = segs[B.rep];
         PcgScal p = {};
         p.tol = rtol * sqrt(tot[0]);
-        (void)s;
-        p.done = 0;
-        p.reason = 0;
         pc[B.rep] = p;
-    }
-}
-
-// g = b_tt - (M [0 ; M_SS^{-1} b_S])_t ; velocity-layout loops over the velocity table
-__global__ void k_pcg_g(RedTable T, const Seg *__restrict__ segs, const double *__restrict__ b,
-                        const double *__restrict__ y2, double *__restrict__ g)
-{
-    pdl_enter();
-    const RBlk B = T.d_blk[blockIdx.x];
-    const Seg &s = segs[B.rep];
-    for (int e = threadIdx.x; e < B.len; e += RB_THREADS) {
-        long k = B.start + e;
-        int j = (int)(k - s.vel_off);
-        g[k] = b[s.vec_off + j] - (s.ss_off >= 0 ? y2[s.top_off + j] : 0.0);
     }
 }
 
@@ -287,8 +270,7 @@ __global__ void k_pcg_g(RedTable T, const Seg *__restrict__ segs, const double *
 // size, with or without lubrication.
 //
 // Pair vectors hold 12 entries per canonical pair q (monomer pairs use the
-// first 6); pair-space sums run over the bead reduction table, each pair
-// attributed to its lower bead, and stresslet sums per colloid bead.
+// first 6).
 
 constexpr int PS_THREADS = 64;
 
@@ -471,22 +453,25 @@ __device__ void ps_setup_colloid_pair(const Seg &s, long lo, long hi, const doub
 // thread each, closed form, compact 6 x 6 blocks (row stride 6).  Colloid pairs:
 // one warp per colloid in the blocks past the pair blocks, taking the canonical
 // pairs for which it is the lower bead (ps_setup_colloid_pair), 12 x 12 blocks.
+// Where every bead is a colloid (warp_pairs), one warp per pair instead (1024
+// colloids: 105 -> 22 us).
 __global__ void __launch_bounds__(PS_THREADS)
 k_ps_setup(long npair, const int2 *__restrict__ pairs, const int *__restrict__ bead_offs, int R,
            const Seg *__restrict__ segs, const double *__restrict__ x, const double *__restrict__ chain,
            const double *__restrict__ tab, int nrow, long ncoll, const int *__restrict__ coll_rep,
-           const int *__restrict__ cptr, double *__restrict__ Sout, double *__restrict__ Pout)
+           const int *__restrict__ cptr, double *__restrict__ Sout, double *__restrict__ Pout, int warp_pairs)
 {
     pdl_enter();
     __shared__ PsWarpSmem wsm[PS_THREADS / 32];
-    const long nbp = (npair + blockDim.x - 1) / blockDim.x;
+    const long nbp = warp_pairs ? 0 : (npair + blockDim.x - 1) / blockDim.x;
     if (blockIdx.x >= nbp) {
         const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
-        const long c = (long)(blockIdx.x - nbp) * (blockDim.x >> 5) + wid;
-        if (c >= ncoll) return;
-        const Seg &s = segs[coll_rep[c]];
-        const long b = s.bead_off + s.Nm + (c - s.coll_off);
-        for (int q = cptr[b]; q < cptr[b + 1]; q++)
+        const long c = (long)(blockIdx.x - nbp) * (blockDim.x >> 5) + wid;   // pair or colloid of this warp
+        if (c >= (warp_pairs ? npair : ncoll)) return;
+        const Seg &s = segs[warp_pairs ? rep_of_b(bead_offs, R, pairs[c].x) : coll_rep[c]];
+        const long b = warp_pairs ? (long)pairs[c].x : s.bead_off + s.Nm + (c - s.coll_off);
+        const long q0 = warp_pairs ? c : cptr[b], q1 = warp_pairs ? c + 1 : cptr[b + 1];
+        for (long q = q0; q < q1; q++)
             ps_setup_colloid_pair(s, b, pairs[q].y, x, tab, nrow, Sout + 144L * q, Pout + 144L * q, wsm[wid], lane);
         return;
     }
@@ -522,116 +507,59 @@ static void launch_ps_setup(Engine &E, cudaStream_t st)
 {
     const long npair = E.lub_npairs;
     const long nbp = (npair + PS_THREADS - 1) / PS_THREADS, nbc = (E.ncoll + PS_THREADS / 32 - 1) / (PS_THREADS / 32);
-    ps_launch(k_ps_setup, (unsigned)(nbp + nbc), PS_THREADS, 0, st,
+    const bool warp_pairs = E.ntot == E.ncoll;
+    ps_launch(k_ps_setup, (unsigned)(warp_pairs ? (npair + PS_THREADS / 32 - 1) / (PS_THREADS / 32) : nbp + nbc), PS_THREADS, 0, st,
             npair, E.d_lub_pairs, E.d_bead_offs, E.R, E.d_segs, E.d_x, E.d_chain, E.d_lubtab, E.lub_nrow, E.ncoll,
-            E.d_coll_rep, E.d_lubc_ptr, E.d_pS, E.d_pP);
+            E.d_coll_rep, E.d_lubc_ptr, E.d_pS, E.d_pP, warp_pairs ? 1 : 0);
 }
 
-// v = L y (+ add): per bead, the rows of S_q y_q that belong to it, summed over
-// its near pairs; optionally written into the first nm3nc6 entries of a
-// mobility-layout vector and reduced into ||D^{-1} L y||^2 per bead
-// (constraint-row entries of D).  Monomer beads take one thread each and sum
-// their pairs in ascending partner order.  Colloid beads, which gather the
-// long lists (every near monomer and colloid), take one warp each from the
-// blocks past the bead blocks: lane l sums the pairs l, l + 32, ... of the
-// colloid's list and a fixed butterfly joins the lanes, so the order is fixed.
-__device__ __forceinline__ void ps_L_pair(const double *__restrict__ Sq, const double *__restrict__ yq, bool low,
-                                          int ng, int nd, double acc[6])
+// ---------------------------------------------------------------------------
+// Work split of the pair space.  A replica of Np beads has a fixed number of blocks
+// (PairBlk, built with the context: 32 beads each, 2 where it has only colloids, whose
+// near pairs are many and 12 x 12, and never more than 512); block b takes the b-th share of the replica's
+// canonical pairs, of its beads and of its colloids, whatever the lists of the staging
+// hold.  Blocks never mix replicas, each leaves one sum per dot, and the blocks of the
+// next kernel add their replica's sums themselves (rep_total) and run the scalar
+// recurrence on them: no counters, no fences, no separate reductions, and an order that
+// depends on the replica alone.
+//
+// Bound: latency (a dependent launch with an L2 round trip, 3 to 4 us each).  A CG
+// iteration of a lubricated replica took 7 launches beside the applies, now 4: the
+// direction, L^T, the update, and one gather for L z and for the residual test's L r
+// (u = L p is kept by its own recurrence L p = L z + beta L p).  Lubricated steps: 980
+// beads 5.50 -> 5.25 ms, 64 replicas of 62000 beads 22.8 -> 19.8 ms.
+constexpr int PB_THREADS = 128;
+constexpr int LT_LANES = 16;                 // lanes per pair: lane a owns entry a of the pair vectors
+
+struct PairTab {
+    const PairBlk *blk;
+    const int2 *pairs;
+    const int *cptr;                         // canonical pairs by lower bead
+    const Seg *segs;
+};
+
+// share b of n items
+__device__ __forceinline__ int share(int n, int b, int G) { return (int)((long)n * b / G); }
+
+// canonical pairs [lo, hi) of a block
+__device__ __forceinline__ void pair_share(const PairTab &T, const PairBlk &B, const Seg &s, long &lo, long &hi)
 {
-    double yv[12];
-#pragma unroll
-    for (int c = 0; c < 12; c++) yv[c] = c < nd ? yq[c] : 0.0;
-    for (int g = 0; g < ng; g++)
-#pragma unroll
-        for (int k = 0; k < 3; k++) {
-            const double *row = Sq + (6 * g + (low ? 0 : 3) + k) * nd;
-            double v = 0.0;
-#pragma unroll
-            for (int c = 0; c < 12; c++)
-                if (c < nd) v += row[c] * yv[c];
-            acc[3 * g + k] += v;
-        }
+    const int q0 = T.cptr[s.bead_off], n = T.cptr[s.bead_off + s.Np] - q0;
+    lo = q0 + share(n, B.b, B.G);
+    hi = q0 + share(n, B.b + 1, B.G);
 }
 
-__device__ __forceinline__ void ps_L_out(const Seg &s, int i, long b, const double acc[6], const double *__restrict__ add,
-                                         double *__restrict__ vel, double *__restrict__ top,
-                                         const double *__restrict__ D, double *__restrict__ bead_part)
+__device__ __forceinline__ double pb_sum(double v)
 {
-    const bool mono = i < s.Nm;
-    int tb, wb;
-    vel_dofs(s, i, tb, wb);
-    double nrm = 0.0;
-    for (int g = 0; g < (mono ? 1 : 2); g++)
-        for (int k = 0; k < 3; k++) {
-            const int d = (g == 0 ? tb : wb) + k;
-            double v = acc[3 * g + k] + (add ? add[s.vel_off + d] : 0.0);
-            if (vel) vel[s.vel_off + d] = v;
-            if (top) top[s.top_off + d] = v;
-            if (D) { double t = acc[3 * g + k] / D[s.vec_off + s.nm3nc11 + d]; nrm += t * t; }
-        }
-    if (bead_part) bead_part[b] = nrm;
+    __shared__ double ws[PB_THREADS / 32];
+    for (int o = 16; o > 0; o >>= 1) v += __shfl_down_sync(0xffffffffu, v, o);
+    __syncthreads();
+    if ((threadIdx.x & 31) == 0) ws[threadIdx.x >> 5] = v;
+    __syncthreads();
+    double t = 0.0;
+    for (int w = 0; w < PB_THREADS / 32; w++) t += ws[w];
+    return t;
 }
-
-__global__ void k_ps_L(long ntot, long ncoll, const int *__restrict__ coll_rep, const int *__restrict__ bead_offs,
-                       int R, const Seg *__restrict__ segs, const int *__restrict__ sptr, const int *__restrict__ snbr,
-                       const int *__restrict__ cidx, const double *__restrict__ S, const double *__restrict__ y,
-                       const double *__restrict__ add, double *__restrict__ vel, double *__restrict__ top,
-                       const double *__restrict__ D, double *__restrict__ bead_part, const char *__restrict__ done,
-                       int dstride)
-{
-    pdl_enter();
-    const long nbb = (ntot + blockDim.x - 1) / blockDim.x;
-    double acc[6] = {0, 0, 0, 0, 0, 0};
-    if (blockIdx.x >= nbb) {
-        const long c = (long)(blockIdx.x - nbb) * (blockDim.x >> 5) + (threadIdx.x >> 5);
-        if (c >= ncoll) return;
-        const int lane = threadIdx.x & 31, r = coll_rep[c];
-        if (rep_done(done, dstride, r)) return;
-        const Seg &s = segs[r];
-        const int i = s.Nm + (int)(c - s.coll_off);
-        const long b = s.bead_off + i;
-        for (int t = sptr[b] + lane; t < sptr[b + 1]; t += 32) {
-            const int qa = cidx[t];
-            if (qa < 0) continue;                       // not in the canonical list (lists disagree)
-            ps_L_pair(S + 144L * qa, y + 12L * qa, b < (long)snbr[t], 2, 12, acc);
-        }
-#pragma unroll
-        for (int q = 0; q < 6; q++)
-            for (int o = 16; o > 0; o >>= 1) acc[q] += __shfl_xor_sync(0xffffffffu, acc[q], o);
-        if (lane == 0) ps_L_out(s, i, b, acc, add, vel, top, D, bead_part);
-        return;
-    }
-    const long b = (long)blockIdx.x * blockDim.x + threadIdx.x;
-    if (b >= ntot) return;
-    const int r = rep_of_b(bead_offs, R, b);
-    if (rep_done(done, dstride, r)) return;
-    const Seg &s = segs[r];
-    const int i = (int)(b - s.bead_off);
-    if (i >= s.Nm) return;                              // colloid: one warp in the blocks past nbb
-    for (int t = sptr[b]; t < sptr[b + 1]; t++) {
-        const int qa = cidx[t];
-        if (qa < 0) continue;
-        ps_L_pair(S + 144L * qa, y + 12L * qa, b < (long)snbr[t], 1, 6, acc);   // monomer pairs: 6 x 6 blocks
-    }
-    ps_L_out(s, i, b, acc, add, vel, top, D, bead_part);
-}
-
-static void launch_ps_L(Engine &E, const double *y, const double *add, double *vel, double *top, const double *D,
-                        double *bead_part, const char *done, int dstride, cudaStream_t st)
-{
-    const int thr = 128;
-    const long nbb = (E.ntot + thr - 1) / thr, nbc = (E.ncoll + thr / 32 - 1) / (thr / 32);
-    ps_launch(k_ps_L, (unsigned)(nbb + nbc), thr, 0, st,
-            E.ntot, E.ncoll, E.d_coll_rep, E.d_bead_offs, E.R, E.d_segs, E.d_lub_ptr, E.d_lub_nbr, E.d_lub_cidx, E.d_pS,
-            y, add, vel, top, D, bead_part, done, dstride);
-}
-
-// w_q = sign * S_q z_q (+ p_q), z gathered from the velocity rows of the Mr apply
-// (y + y2 for replicas with a dense stresslet block) plus an optional velocity
-// vector; part[q] = p_q . w_q.  Sixteen lanes per pair: lane a gathers z_a and
-// forms row a (rows and columns past nd, 6 for monomer pairs, add nothing), and
-// a fixed butterfly over the sixteen lanes forms the dot.
-constexpr int LT_LANES = 16;
 
 // z_a = (P_q r)_a for lane a of a pair's team (r_c held by lane c); rows and
 // columns past nd (6 for monomer pairs) add nothing, columns in ascending order
@@ -646,23 +574,12 @@ __device__ __forceinline__ double pm_matvec(const double *__restrict__ Pq, int a
     return z;
 }
 
-__global__ void k_ps_LT(long npair, const int2 *__restrict__ pairs, const int *__restrict__ bead_offs, int R,
-                        const Seg *__restrict__ segs, const double *__restrict__ S, const double *__restrict__ y,
-                        const double *__restrict__ y2, const double *__restrict__ addv, double sign,
-                        const double *__restrict__ p, double *__restrict__ w, double *__restrict__ part,
-                        const char *__restrict__ done, int dstride)
+// entry a of S_q (y + y2 (+ addv)) gathered at the pair's DOFs: lane a gathers entry a and
+// forms row a (the L^T of an apply's output)
+__device__ __forceinline__ double lt_row(const Seg &s, long lo, long hi, int a, int nd, unsigned team,
+                                         const double *__restrict__ Sq, const double *__restrict__ y,
+                                         const double *__restrict__ y2, const double *__restrict__ addv)
 {
-    pdl_enter();
-    const long q = ((long)blockIdx.x * blockDim.x + threadIdx.x) / LT_LANES;
-    const int a = threadIdx.x % LT_LANES;
-    const unsigned team = 0xffffu << (threadIdx.x & 16);
-    if (q >= npair) return;                       // whole teams leave together
-    const long lo = pairs[q].x, hi = pairs[q].y;
-    const int r = rep_of_b(bead_offs, R, lo);
-    if (rep_done(done, dstride, r)) return;
-    const Seg &s = segs[r];
-    const bool mono = (lo - s.bead_off) < s.Nm;
-    const int nd = mono ? 6 : 12;
     double za = 0.0;
     if (a < nd) {
         const long bd = (a % 6) < 3 ? lo : hi;
@@ -671,158 +588,337 @@ __global__ void k_ps_LT(long npair, const int2 *__restrict__ pairs, const int *_
         const int d = (a < 6 ? tb : wb) + a % 3;
         za = y[s.top_off + d] + (s.ss_off >= 0 ? y2[s.top_off + d] : 0.0) + (addv ? addv[s.vel_off + d] : 0.0);
     }
-    const double *Sq = S + 144L * q + a * nd;
-    double v = 0.0;
-#pragma unroll
-    for (int c = 0; c < 12; c++) {
-        const double zc = __shfl_sync(team, za, c, LT_LANES);
-        if (a < nd && c < nd) v += Sq[c] * zc;
-    }
-    v *= sign;
-    double dot = 0.0;
-    if (a < 12) {
-        if (p) { v += p[12 * q + a]; dot = p[12 * q + a] * v; }
-        w[12 * q + a] = v;
-    }
-    if (part) {
-#pragma unroll
-        for (int o = LT_LANES / 2; o > 0; o >>= 1) dot += __shfl_xor_sync(team, dot, o, LT_LANES);
-        if (a == 0) part[q] = dot;
-    }
+    return pm_matvec(Sq, a, nd, za, team);
 }
 
-// first iterate: y = 0, r = rhs (in rv), z = P r, p = z, part = r . z;
-// a team of LT_LANES lanes per pair, lane a owning entry a
-__global__ void k_ps_init(long npair, const int2 *__restrict__ pairs, const int *__restrict__ bead_offs, int R,
-                          const Seg *__restrict__ segs, const double *__restrict__ P, double *__restrict__ yv,
-                          const double *__restrict__ rv, double *__restrict__ zv, double *__restrict__ pv,
-                          double *__restrict__ part)
+// The loop over a block's pairs, a team of LT_LANES lanes per pair: for every lane of the team,
+// w = load(q, lo, hi, nd, a, team), what a kernel can fetch and form before it knows the
+// replica's scalars, then work(w, q, nd, a, team).  The first pair's load runs ahead of mid(),
+// which adds the sums and runs the recurrence, so that their round trips overlap.
+template <class L, class M, class W>
+__device__ __forceinline__ void for_pairs(const PairTab &T, const PairBlk &B, const Seg &s, L load, M mid, W work)
 {
-    pdl_enter();
-    const long q = ((long)blockIdx.x * blockDim.x + threadIdx.x) / LT_LANES;
+    long q0, q1;
+    pair_share(T, B, s, q0, q1);
     const int a = threadIdx.x % LT_LANES;
     const unsigned team = 0xffffu << (threadIdx.x & 16);
-    if (q >= npair) return;
-    const long lo = pairs[q].x;
-    const Seg &s = segs[rep_of_b(bead_offs, R, lo)];
-    const int nd = (lo - s.bead_off) < s.Nm ? 6 : 12;     // monomer pairs: 6 x 6 block, zero elsewhere
-    const long e = 12 * q + a;
-    const double ra = a < 12 ? rv[e] : 0.0;
-    const double v = pm_matvec(P + 144L * q, a, nd, ra, team);
-    double dot = 0.0;
-    if (a < 12) {
-        zv[e] = v;
-        pv[e] = v;
-        yv[e] = 0.0;
-        dot = ra * v;
+    long q = q0 + threadIdx.x / LT_LANES;
+    int nd = 12;
+    auto get = [&]() {
+        const int2 p = T.pairs[q];
+        nd = (p.x - s.bead_off) < s.Nm ? 6 : 12;                     // monomer pairs: 6 x 6 blocks
+        return load(q, (long)p.x, (long)p.y, nd, a, team);
+    };
+    decltype(load(0L, 0L, 0L, 0, 0, 0u)) w{};
+    if (q < q1) w = get();
+    if (!mid()) return;
+    while (q < q1) {
+        work(w, q, nd, a, team);
+        q += PB_THREADS / LT_LANES;
+        if (q < q1) w = get();
     }
+}
+
+template <class F>
+__device__ __forceinline__ void for_pairs(const PairTab &T, const PairBlk &B, const Seg &s, F f)
+{
+    for_pairs(T, B, s, [](long, long lo, long hi, int, int, unsigned) { return longlong2{lo, hi}; }, []() { return true; },
+              [&](longlong2 p, long q, int nd, int a, unsigned team) { f(q, p.x, p.y, nd, a, team); });
+}
+
+// row a of a pair's block
+struct Row12 { double v[12]; };
+__device__ __forceinline__ Row12 block_row(const double *__restrict__ P, int a, int nd)
+{
+    Row12 r;
 #pragma unroll
-    for (int o = LT_LANES / 2; o > 0; o >>= 1) dot += __shfl_xor_sync(team, dot, o, LT_LANES);
-    if (a == 0) part[q] = dot;
+    for (int c = 0; c < 12; c++) r.v[c] = a < nd && c < nd ? P[a * nd + c] : 0.0;
+    return r;
 }
-
-// y += alpha p ; r -= alpha Ap ; z = P r ; part = r . z; a team per pair as k_ps_init
-__global__ void k_ps_update(long npair, const int2 *__restrict__ pairs, const int *__restrict__ bead_offs, int R,
-                            const Seg *__restrict__ segs, const PcgScal *__restrict__ pc, const double *__restrict__ P,
-                            const double *__restrict__ pv, const double *__restrict__ Ap, double *__restrict__ yv,
-                            double *__restrict__ rv, double *__restrict__ zv, double *__restrict__ part)
+__device__ __forceinline__ double row_dot(const Row12 &r, double x, unsigned team)
 {
-    pdl_enter();
-    const long q = ((long)blockIdx.x * blockDim.x + threadIdx.x) / LT_LANES;
-    const int a = threadIdx.x % LT_LANES;
-    const unsigned team = 0xffffu << (threadIdx.x & 16);
-    if (q >= npair) return;
-    const long lo = pairs[q].x;
-    const int r = rep_of_b(bead_offs, R, lo);
-    const PcgScal sc = pc[r];
-    if (sc.done) return;
-    // monomer pairs: 6 x 6 blocks, and entries 6..11 of every pair vector stay zero
-    const int nd = (lo - segs[r].bead_off) < segs[r].Nm ? 6 : 12;
-    const long e = 12 * q + a;
-    double ra = 0.0;
-    if (a < nd) {
-        yv[e] += sc.alpha * pv[e];
-        ra = rv[e] - sc.alpha * Ap[e];
-        rv[e] = ra;
-    }
-    const double v = pm_matvec(P + 144L * q, a, nd, ra, team);
-    double dot = 0.0;
-    if (a < nd) {
-        zv[e] = v;
-        dot = ra * v;
-    }
+    double z = 0.0;
 #pragma unroll
-    for (int o = LT_LANES / 2; o > 0; o >>= 1) dot += __shfl_xor_sync(team, dot, o, LT_LANES);
-    if (a == 0) part[q] = dot;
+    for (int c = 0; c < 12; c++) z += r.v[c] * __shfl_sync(team, x, c, LT_LANES);
+    return z;
 }
 
-// p = z + beta p, one thread per pair-vector entry
-__global__ void k_ps_dir(long npair, const int2 *__restrict__ pairs, const int *__restrict__ bead_offs, int R,
-                         const PcgScal *__restrict__ pc, const double *__restrict__ zv, double *__restrict__ pv)
+// (L y)_d = sum over the bead's near pairs of the rows of S_q y_q that belong to it, for two
+// vectors at once (y1 may be null): a monomer's three rows by three lanes of a quad, pairs
+// in ascending partner order; a colloid's six rows by two groups of six lanes of sixteen,
+// the pairs of its list added in the order of a warp with a lane per pair and a butterfly over
+// the lanes (16, 8, 4, 2, 1).  f(dof, (L y0)_d, (L y1)_d) once per row.
+template <class F>
+__device__ __forceinline__ void for_gather(const PairBlk &B, const Seg &s, const int *__restrict__ sptr,
+                                           const int *__restrict__ snbr, const int *__restrict__ cidx,
+                                           const double *__restrict__ S, const double *__restrict__ y0,
+                                           const double *__restrict__ y1, F f)
 {
-    pdl_enter();
-    const long e = (long)blockIdx.x * blockDim.x + threadIdx.x;
-    if (e >= 12 * npair) return;
-    const PcgScal &sc = pc[rep_of_b(bead_offs, R, pairs[e / 12].x)];
-    if (sc.done) return;
-    pv[e] = zv[e] + sc.beta * pv[e];
-}
-
-// per-replica sums over the bead table: pair partials by lower bead plus the
-// per-bead stresslet partials (add0), and the per-bead residual partials
-// (bead_part + add1).
-// mode 0: alpha = rz / sum(part);  mode 1: first check (rz, err);  mode 2: iteration check
-__global__ void k_ps_reduce(RedTable T, const int *__restrict__ cptr, const double *__restrict__ part,
-                            const double *__restrict__ bead_part, const double *__restrict__ add0,
-                            const double *__restrict__ add1, PcgScal *pc, int mode, int maxit, int *nactive)
-{
-    pdl_enter();
-    __shared__ double sh[RB_THREADS / 32][2];
-    const RBlk B = T.d_blk[blockIdx.x];
-    if (pc[B.rep].done) return;
-    double v[2] = {0.0, 0.0};
-    // pairs are stored by lower bead, so the block's beads own one contiguous pair range
-    for (long q = cptr[B.start] + threadIdx.x; q < cptr[B.start + B.len]; q += RB_THREADS) v[0] += part[q];
-    for (int e = threadIdx.x; e < B.len; e += RB_THREADS) {
-        long b = B.start + e;
-        if (add0) v[0] += add0[b];
-        if (bead_part) v[1] += bead_part[b];
-        if (add1) v[1] += add1[b];
-    }
-    block_sum<2>(v, sh);
-    double tot[2];
-    if (finish_block<2>(T, B, blockIdx.x, v, tot)) {
-        PcgScal p = pc[B.rep];
-        if (mode == 0) {
-            if (tot[0] <= 0.0) { p.done = 1; p.reason = -8; atomicSub(nactive, 1); }
-            else p.alpha = p.rz / tot[0];
-        } else {
-            p.err = sqrt(tot[1]);
-            if (mode == 2) p.it++;
-            if (p.err <= p.tol) { p.done = 1; p.reason = 2; }
-            else if (tot[0] <= 0.0) { p.done = 1; p.reason = -8; }
-            else if (p.it >= maxit) { p.done = 1; p.reason = -3; }
-            else {
-                p.beta = mode == 1 ? 0.0 : tot[0] / p.rz;
-                p.rz = tot[0];
-            }
-            if (p.done) atomicSub(nactive, 1);
+    const int i0 = share(s.Np, B.b, B.G), i1 = share(s.Np, B.b + 1, B.G);
+    // the rows of pairs t0, t0 + step, ... of bead b's list, added up in order
+    auto rows = [&](long b, int row, int nd, int t0, int step, double &v0, double &v1) {
+        for (int t = sptr[b] + t0; t < sptr[b + 1]; t += step) {
+            const int q = cidx[t];
+            if (q < 0) continue;                            // not in the canonical list (lists disagree)
+            const double *r = S + 144L * q + (6 * (row / 3) + (b < (long)snbr[t] ? 0 : 3) + row % 3) * nd;
+            double a = 0.0, c = 0.0;
+#pragma unroll
+            for (int k = 0; k < 12; k++)
+                if (k < nd) {
+                    const double sk = r[k];
+                    a += sk * y0[12L * q + k];
+                    if (y1) c += sk * y1[12L * q + k];
+                }
+            v0 += a;
+            v1 += c;
         }
-        pc[B.rep] = p;
+    };
+    const int row4 = threadIdx.x & 3;
+    for (int i = i0 + (threadIdx.x >> 2); i < min(i1, s.Nm); i += PB_THREADS / 4) {
+        double v0 = 0.0, v1 = 0.0;
+        if (row4 < 3) {
+            rows((long)s.bead_off + i, row4, 6, 0, 1, v0, v1);
+            f(3 * i + row4, v0, v1);
+        }
+    }
+    const int l = threadIdx.x & 15, grp = l / 6, row6 = l % 6;
+    const unsigned team = 0xffffu << (threadIdx.x & 16);
+    for (int i = max(i0, s.Nm) + (threadIdx.x >> 4); i < i1; i += PB_THREADS / 16) {
+        const long b = (long)s.bead_off + i;
+        const int t0 = sptr[b], n = sptr[b + 1] - t0;
+        // leaf p of the tree: the pairs p, p + 32, ... of the list, in order
+        double v0 = 0.0, v1 = 0.0;
+        if (n <= 8) {
+            // leaves 0..7: ((0 + 4) + (2 + 6)) + ((1 + 5) + (3 + 7)); group 0 takes the even ones
+            double x0[4] = {0, 0, 0, 0}, x1[4] = {0, 0, 0, 0};
+            if (grp < 2)
+                for (int k = 0; k < 4; k++)
+                    if (2 * k + grp < n) rows(b, row6, 12, 2 * k + grp, 32, x0[k], x1[k]);
+            v0 = (x0[0] + x0[2]) + (x0[1] + x0[3]);
+            v1 = (x1[0] + x1[2]) + (x1[1] + x1[3]);
+        } else if (grp < 2) {
+            // the tree by levels, even leaves in group 0, odd ones in group 1
+            auto leaf = [&](int p, double &a0, double &a1) { a0 = 0.0; a1 = 0.0; if (p < n) rows(b, row6, 12, p, 32, a0, a1); };
+            for (int h = 0; h < 2; h++) {             // bit 1 of the leaf
+                double y0 = 0.0, y1 = 0.0;
+                for (int f = 0; f < 2; f++) {         // bit 2
+                    double z0 = 0.0, z1 = 0.0;
+                    for (int e = 0; e < 2; e++) {     // bit 3; bit 4 inside
+                        const int p = grp + 2 * h + 4 * f + 8 * e;
+                        double a0, a1, c0, c1;
+                        leaf(p, a0, a1);
+                        leaf(p + 16, c0, c1);
+                        a0 += c0; a1 += c1;
+                        if (e == 0) { z0 = a0; z1 = a1; } else { z0 += a0; z1 += a1; }
+                    }
+                    if (f == 0) { y0 = z0; y1 = z1; } else { y0 += z0; y1 += z1; }
+                }
+                if (h == 0) { v0 = y0; v1 = y1; } else { v0 += y0; v1 += y1; }
+            }
+        }
+        v0 += __shfl_sync(team, v0, l + 6, 16);
+        v1 += __shfl_sync(team, v1, l + 6, 16);
+        if (grp == 0) {
+            int tb, wb;
+            vel_dofs(s, i, tb, wb);
+            f((row6 < 3 ? tb : wb) + row6 % 3, v0, v1);
+        }
     }
 }
 
-// c = -b_bot (velocity layout), u_t = b_bot
-__global__ void k_ps_c(RedTable T, const Seg *__restrict__ segs, const double *__restrict__ b, double *__restrict__ c,
-                       double *__restrict__ u)
+// u_t = L y (+ add); optionally also into the force rows of a saddle vector
+__global__ void __launch_bounds__(PB_THREADS)
+k_ps_L(PairTab T, const int *__restrict__ sptr, const int *__restrict__ snbr, const int *__restrict__ cidx,
+       const double *__restrict__ S, const double *__restrict__ y, const double *__restrict__ add,
+       double *__restrict__ u, double *__restrict__ vel, double *__restrict__ x, const char *__restrict__ done,
+       int dstride)
+{
+    pdl_enter();
+    const PairBlk B = T.blk[blockIdx.x];
+    if (rep_done(done, dstride, B.rep)) return;
+    const Seg &s = T.segs[B.rep];
+    for_gather(B, s, sptr, snbr, cidx, S, y, nullptr, [&](int d, double v, double) {
+        if (add) v += add[s.vel_off + d];
+        if (u) u[s.top_off + d] = v;
+        if (vel) vel[s.vel_off + d] = v;
+        if (x) x[s.vec_off + d] = v;
+    });
+}
+
+// ---------------------------------------------------------------------------
+// pair-space CG.  The scalars of iteration k live in st[k & 1].
+struct PcgVec { double *y, *r, *z, *p, *Ap, *Lz, *Lp; };
+
+// r = L^T (g + M b_bot) (y, y2: the apply to b_bot), z = P r, y = 0; sums of r.z
+__global__ void __launch_bounds__(PB_THREADS)
+k_pc_init(PairTab T, const double *__restrict__ S, const double *__restrict__ P, const double *__restrict__ y,
+          const double *__restrict__ y2, const double *__restrict__ g, PcgVec V, double *__restrict__ prz)
+{
+    pdl_enter();
+    const PairBlk B = T.blk[blockIdx.x];
+    const Seg &s = T.segs[B.rep];
+    double dot = 0.0;
+    for_pairs(T, B, s, [&](long q, long lo, long hi, int nd, int a, unsigned team) {
+        const double ra = lt_row(s, lo, hi, a, nd, team, S + 144 * q, y, y2, g);
+        const double za = pm_matvec(P + 144 * q, a, nd, ra, team);
+        if (a < nd) {
+            const long e = 12 * q + a;
+            V.y[e] = 0.0; V.r[e] = ra; V.z[e] = za;
+            dot += ra * za;
+        }
+    });
+    dot = pb_sum(dot);
+    if (threadIdx.x == 0) prz[blockIdx.x] = dot;
+}
+
+// L z for the next direction, and the residual test ||D^{-1} L r||^2
+__global__ void __launch_bounds__(PB_THREADS)
+k_pc_gather(PairTab T, const int *__restrict__ sptr, const int *__restrict__ snbr, const int *__restrict__ cidx,
+            const double *__restrict__ S, PcgVec V, const double *__restrict__ D, const PcgScal *__restrict__ st,
+            double *__restrict__ perr)
+{
+    pdl_enter();
+    const PairBlk B = T.blk[blockIdx.x];
+    if (st[B.rep].done) return;
+    const Seg &s = T.segs[B.rep];
+    double err = 0.0;
+    for_gather(B, s, sptr, snbr, cidx, S, V.z, V.r, [&](int d, double lz, double lr) {
+        V.Lz[s.vel_off + d] = lz;
+        const double t = lr / D[s.vec_off + s.nm3nc11 + d];
+        err += t * t;
+    });
+    err = pb_sum(err);
+    if (threadIdx.x == 0) perr[blockIdx.x] = err;
+}
+
+// closes an iteration (k > 0) or the start (k = 0): the residual test, beta; then p = z + beta p,
+// u = L p = L z + beta L p
+__global__ void __launch_bounds__(PB_THREADS)
+k_pc_dir(PairTab T, const PcgScal *__restrict__ st0, PcgScal *__restrict__ st1, const double *__restrict__ prz,
+         const double *__restrict__ perr, PcgVec V, double *__restrict__ u, int k, int maxit, int *nactive)
+{
+    pdl_enter();
+    const PairBlk B = T.blk[blockIdx.x];
+    __shared__ PcgScal sm;
+    if (st0[B.rep].done) {
+        if (B.b == 0 && threadIdx.x == 0) st1[B.rep] = st0[B.rep];
+        return;
+    }
+    const double rz = rep_total(prz + B.first, B.G), err2 = rep_total(perr + B.first, B.G);
+    if (threadIdx.x == 0) {
+        PcgScal p = st0[B.rep];
+        p.err = sqrt(err2);
+        if (k > 0) p.it++;
+        if (p.err <= p.tol) { p.done = 1; p.reason = 2; }
+        else if (rz <= 0.0) { p.done = 1; p.reason = -8; }
+        else if (p.it >= maxit) { p.done = 1; p.reason = -3; }
+        else {
+            p.beta = k == 0 ? 0.0 : rz / p.rz;
+            p.rz = rz;
+        }
+        if (B.b == 0) {
+            if (p.done) atomicSub(nactive, 1);
+            st1[B.rep] = p;
+        }
+        sm = p;
+    }
+    __syncthreads();
+    if (sm.done) return;
+    const double beta = sm.beta;
+    const Seg &s = T.segs[B.rep];
+    for_pairs(T, B, s, [&](long q, long, long, int nd, int a, unsigned) {
+        const long e = 12 * q + a;
+        if (a < nd) V.p[e] = k == 0 ? V.z[e] : V.z[e] + beta * V.p[e];
+    });
+    auto dof = [&](int d) {
+        const long v = (long)s.vel_off + d;
+        const double t = k == 0 ? V.Lz[v] : V.Lz[v] + beta * V.Lp[v];
+        V.Lp[v] = t;
+        u[s.top_off + d] = t;
+    };
+    const int i0 = share(s.Np, B.b, B.G), i1 = share(s.Np, B.b + 1, B.G), c0 = max(i0 - s.Nm, 0), c1 = i1 - s.Nm;
+    for (int d = 3 * i0 + threadIdx.x; d < 3 * i1; d += PB_THREADS) dof(d);
+    for (int d = 3 * c0 + threadIdx.x; d < 3 * c1; d += PB_THREADS) dof(s.nm3nc3 + d);
+}
+
+// Ap = p + L^T (M L p); sums of p.Ap
+__global__ void __launch_bounds__(PB_THREADS)
+k_pc_apply(PairTab T, const double *__restrict__ S, const double *__restrict__ y, const double *__restrict__ y2, PcgVec V,
+           const PcgScal *__restrict__ st, double *__restrict__ pap)
+{
+    pdl_enter();
+    const PairBlk B = T.blk[blockIdx.x];
+    if (st[B.rep].done) return;
+    const Seg &s = T.segs[B.rep];
+    double dot = 0.0;
+    for_pairs(T, B, s, [&](long q, long lo, long hi, int nd, int a, unsigned team) {
+        const double v = lt_row(s, lo, hi, a, nd, team, S + 144 * q, y, y2, nullptr);
+        if (a < nd) {
+            const double pa = V.p[12 * q + a], w = v + pa;
+            V.Ap[12 * q + a] = w;
+            dot += pa * w;
+        }
+    });
+    dot = pb_sum(dot);
+    if (threadIdx.x == 0) pap[blockIdx.x] = dot;
+}
+
+// y += alpha p ; r -= alpha Ap ; z = P r ; sums of r.z.  A direction of non-positive curvature
+// stops the replica (its first block notes it; the others find the same sum).
+__global__ void __launch_bounds__(PB_THREADS)
+k_pc_update(PairTab T, const double *__restrict__ P, PcgVec V, PcgScal *__restrict__ st, const double *__restrict__ pap,
+            double *__restrict__ prz, int *nactive)
+{
+    pdl_enter();
+    const PairBlk B = T.blk[blockIdx.x];
+    if (st[B.rep].done) return;
+    const Seg &s = T.segs[B.rep];
+    struct In { double y, p, r, Ap; Row12 P; };
+    double dot = 0.0, alpha = 0.0;
+    bool stop = false;
+    for_pairs(T, B, s,
+        [&](long q, long, long, int nd, int a, unsigned) {
+            const long e = 12 * q + a;
+            In w{};
+            if (a < nd) { w.y = V.y[e]; w.p = V.p[e]; w.r = V.r[e]; w.Ap = V.Ap[e]; }
+            w.P = block_row(P + 144 * q, a, nd);
+            return w;
+        },
+        [&]() {
+            const double pAp = rep_total(pap + B.first, B.G);
+            stop = pAp <= 0.0;
+            if (stop && B.b == 0 && threadIdx.x == 0) { st[B.rep].reason = -8; st[B.rep].done = 1; atomicSub(nactive, 1); }
+            if (!stop) alpha = st[B.rep].rz / pAp;
+            return !stop;
+        },
+        [&](const In &w, long q, int nd, int a, unsigned team) {
+            const long e = 12 * q + a;
+            const double ra = w.r - alpha * w.Ap, za = row_dot(w.P, ra, team);
+            if (a < nd) {
+                V.y[e] = w.y + alpha * w.p;
+                V.r[e] = ra;
+                V.z[e] = za;
+                dot += ra * za;
+            }
+        });
+    if (stop) return;
+    dot = pb_sum(dot);
+    if (threadIdx.x == 0) prz[blockIdx.x] = dot;
+}
+
+// g = b_tt - (M [0 ; M_SS^{-1} b_S])_t, c = -b_bot (velocity layout), u_t = b_bot
+__global__ void k_ps_rhs(RedTable T, const Seg *__restrict__ segs, const double *__restrict__ b,
+                         const double *__restrict__ y2, double *__restrict__ g, double *__restrict__ c,
+                         double *__restrict__ u)
 {
     pdl_enter();
     const RBlk B = T.d_blk[blockIdx.x];
     const Seg &s = segs[B.rep];
     for (int e = threadIdx.x; e < B.len; e += RB_THREADS) {
-        long k = B.start + e;
-        int j = (int)(k - s.vel_off);
-        double v = b[s.vec_off + s.nm3nc11 + j];
+        const long k = (long)B.start + e;
+        const int j = (int)(k - s.vel_off);
+        const double v = b[s.vec_off + s.nm3nc11 + j];
+        g[k] = b[s.vec_off + j] - (s.ss_off >= 0 ? y2[s.top_off + j] : 0.0);
         c[k] = -v;
         u[s.top_off + j] = v;
     }
@@ -843,78 +939,20 @@ __global__ void k_ps_fin(RedTable T, const Seg *__restrict__ segs, const double 
     }
 }
 
-// copy F_t (velocity layout) into the force rows of the saddle solution
-__global__ void k_ps_ft(RedTable T, const Seg *__restrict__ segs, const double *__restrict__ ft, double *__restrict__ x)
+// F_S of the joint replicas (colloids beyond the dense stresslet limit) into u and the solution
+__global__ void k_ps_S(long ncoll, const int *__restrict__ coll_rep, const Seg *__restrict__ segs,
+                       const double *__restrict__ yS, double *__restrict__ u, double *__restrict__ x)
 {
     pdl_enter();
-    const RBlk B = T.d_blk[blockIdx.x];
-    const Seg &s = segs[B.rep];
-    for (int e = threadIdx.x; e < B.len; e += RB_THREADS) {
-        long k = B.start + e;
-        x[s.vec_off + (k - s.vel_off)] = ft[k];
-    }
-}
-
-// stresslet unknowns of the joint replicas (Nc > 0 without a dense M_SS
-// inverse), one thread per bead; vectors in mobility layout (S part), with
-// the inverse self block (1.8 I, 0.9 coupling of components 0 and 4) as the
-// preconditioner.  mode 0 init (r = b_S + y_S), 1 Ap = y_S, 2 update, 3 direction,
-// 4 finish (F_S into u and the solution).  Per-bead partials: a0 (r.z or p.Ap),
-// a1 (||D^{-1} r_S||^2); zero for every other bead.
-__global__ void k_ps_S(long ntot, const int *__restrict__ bead_offs, int R, const Seg *__restrict__ segs, int mode,
-                       const PcgScal *__restrict__ pc, const double *__restrict__ b, const double *__restrict__ y,
-                       const double *__restrict__ D, double *__restrict__ yS, double *__restrict__ rS,
-                       double *__restrict__ zS, double *__restrict__ pS, double *__restrict__ ApS,
-                       double *__restrict__ u, double *__restrict__ x, double *__restrict__ a0, double *__restrict__ a1)
-{
-    pdl_enter();
-    long bd = (long)blockIdx.x * blockDim.x + threadIdx.x;
-    if (bd >= ntot) return;
-    const int r = rep_of_b(bead_offs, R, bd);
-    const Seg &s = segs[r];
-    const int i = (int)(bd - s.bead_off);
-    const bool joint = s.Nc > 0 && s.ss_off < 0 && i >= s.Nm;
-    if (mode != 4 && pc[r].done) return;
-    if (!joint) {
-        if (mode <= 2) { if (a0) a0[bd] = 0.0; if (a1) a1[bd] = 0.0; }
-        return;
-    }
-    const int c = i - s.Nm;
-    const long t0 = (long)s.top_off + s.nm3nc6 + 5 * c;       // S entries in mobility layout
-    const long v0 = (long)s.vec_off + s.nm3nc6 + 5 * c;       // S rows of the saddle vector
-    const double det = 1.8 * 1.8 - 0.9 * 0.9;
-    double dot = 0.0, nrm = 0.0;
-    if (mode == 0 || mode == 2) {
-        double rv[5], zv[5];
-        for (int k = 0; k < 5; k++) {
-            if (mode == 0) { rv[k] = b[v0 + k] + y[t0 + k]; yS[t0 + k] = 0.0; }
-            else {
-                const double al = pc[r].alpha;
-                yS[t0 + k] += al * pS[t0 + k];
-                rv[k] = rS[t0 + k] - al * ApS[t0 + k];
-            }
-            rS[t0 + k] = rv[k];
-        }
-        zv[0] = (1.8 * rv[0] - 0.9 * rv[4]) / det;
-        zv[4] = (1.8 * rv[4] - 0.9 * rv[0]) / det;
-        for (int k = 1; k < 4; k++) zv[k] = rv[k] / 1.8;
-        for (int k = 0; k < 5; k++) {
-            zS[t0 + k] = zv[k];
-            dot += rv[k] * zv[k];
-            double t = rv[k] / D[v0 + k];
-            nrm += t * t;
-            if (mode == 0) { pS[t0 + k] = zv[k]; u[t0 + k] = zv[k]; }
-        }
-        a0[bd] = dot;
-        a1[bd] = nrm;
-    } else if (mode == 1) {
-        for (int k = 0; k < 5; k++) { double ap = y[t0 + k]; ApS[t0 + k] = ap; dot += pS[t0 + k] * ap; }
-        a0[bd] = dot;
-    } else if (mode == 3) {
-        const double be = pc[r].beta;
-        for (int k = 0; k < 5; k++) { double p = zS[t0 + k] + be * pS[t0 + k]; pS[t0 + k] = p; u[t0 + k] = p; }
-    } else {
-        for (int k = 0; k < 5; k++) { u[t0 + k] = yS[t0 + k]; x[v0 + k] = yS[t0 + k]; }
+    const long c = (long)blockIdx.x * blockDim.x + threadIdx.x;
+    if (c >= ncoll) return;
+    const Seg &s = segs[coll_rep[c]];
+    if (s.ss_off >= 0) return;
+    const long o = s.nm3nc6 + 5 * (c - s.coll_off);
+    for (int k = 0; k < 5; k++) {
+        const double v = yS[s.top_off + o + k];
+        u[s.top_off + o + k] = v;
+        x[s.vec_off + o + k] = v;
     }
 }
 
@@ -941,15 +979,60 @@ static void mr_apply(Engine &E, bool fp32, const void *dn, int ds, cudaStream_t 
 // the stresslet entries of the joint replicas' colloids (mobility layout).
 struct PMVec { double *pair; double *s; };
 struct PMArgs {
-    PMVec R[3], W[3], v, z, x;
+    PMVec R0, R1, R2;          // r_k, r_{k+1} (first Av), r_{k-1}
+    PMVec W0, W1, W2;          // w_{k-3}, w_{k-2}, w_{k-1} (formed by iteration k)
+    PMVec v, z, x;
+    const double *b, *g;       // right-hand side, g of the velocity rows
     const double *y;           // the apply's output (mobility layout; its S part is y_S)
     const double *y2;          // the dense stresslet block's share of the output (replicas with one)
     const double *S;           // pair square-root blocks (L = [B_q S_q])
     double *u;                 // the apply's input (mobility layout): its S part gets z_S
     const double *P;           // pair preconditioner blocks
-    double *part, *part2;      // per-pair partials
-    double *sA, *sB;           // per-bead partials
+    double *da, *db, *dn;      // v.Av, r.z, z.z (start): one number per pair, then one per bead
+    long npair;
 };
+
+// A replica's total of the dots d (per canonical pair, then per bead from d + npair on), the same
+// in every thread: thread t takes pairs t, t + 128, ... into eight sums joined in pairs, then the
+// beads likewise, then a shuffle tree and the warps in order.  Every block adds all of its
+// replica's numbers, 4500 for 1024 colloids, rather than one number per block, because this
+// order is part of the answer where the system is close to singular.
+__device__ __forceinline__ double strided_sum(const double *__restrict__ x, long lo, long hi)
+{
+    double acc[8] = {0, 0, 0, 0, 0, 0, 0, 0};
+    for (long q = lo + threadIdx.x; q < hi; q += 8 * PB_THREADS) {
+        double t[8];
+#pragma unroll
+        for (int u = 0; u < 8; u++) t[u] = q + u * PB_THREADS < hi ? x[q + u * PB_THREADS] : 0.0;
+#pragma unroll
+        for (int u = 0; u < 8; u++) acc[u] += t[u];
+    }
+    return ((acc[0] + acc[1]) + (acc[2] + acc[3])) + ((acc[4] + acc[5]) + (acc[6] + acc[7]));
+}
+
+__device__ __forceinline__ double pm_total(const PairTab &T, const Seg &s, const double *__restrict__ d, long npair)
+{
+    __shared__ double ws[PB_THREADS / 32];
+    const int q0 = T.cptr[s.bead_off], q1 = T.cptr[s.bead_off + s.Np];
+    // only a joint replica's colloids have numbers of their own
+    const double *db = d + npair;
+    double v = strided_sum(d, q0, q1) + (s.Nc > 0 && s.ss_off < 0 ? strided_sum(db, s.bead_off, (long)s.bead_off + s.Np) : 0.0);
+    for (int o = 16; o > 0; o >>= 1) v += __shfl_down_sync(0xffffffffu, v, o);
+    __syncthreads();
+    if ((threadIdx.x & 31) == 0) ws[threadIdx.x >> 5] = v;
+    __syncthreads();
+    double t = 0.0;
+    for (int w = 0; w < PB_THREADS / 32; w++) t += ws[w];
+    return t;
+}
+
+// a pair's dot over its team, stored by lane 0
+__device__ __forceinline__ void pair_dot(double v, unsigned team, int a, double *__restrict__ out)
+{
+#pragma unroll
+    for (int o = LT_LANES / 2; o > 0; o >>= 1) v += __shfl_xor_sync(team, v, o, LT_LANES);
+    if (a == 0) *out = v;
+}
 
 __device__ __forceinline__ void s_precond(const double r[5], double z[5])
 {
@@ -959,438 +1042,351 @@ __device__ __forceinline__ void s_precond(const double r[5], double z[5])
     for (int k = 1; k < 4; k++) z[k] = r[k] / 1.8;
 }
 
-// MINRES element work of pair t by a team of LT_LANES lanes, lane a owning entry a
-// of the pair vectors (a < 12); the partial dots join over the team by a fixed
-// butterfly.  mode as k_pm_elem.
-__device__ __forceinline__ int pm_pair_team(long t, int a, unsigned team, const int2 *__restrict__ pairs,
-                                             const int *__restrict__ bead_offs, int R, const Seg *__restrict__ segs,
-                                             const MinresScal *__restrict__ mr, int mode, int k, const PMArgs &A)
+// the loop over a block's share of a joint replica's colloids, one thread each: f(first entry of
+// the colloid's stresslet in mobility layout, in the saddle vector, its bead)
+template <class F>
+__device__ __forceinline__ void for_stresslets(const PairBlk &B, const Seg &s, F f)
 {
-    const long bead = pairs[t].x;
-    const int r = rep_of_b(bead_offs, R, bead);
-    const Seg &sp = segs[r];
-    const int nd = (bead - sp.bead_off) < sp.Nm ? 6 : 12;   // monomer pairs: 6 x 6 blocks
-    const MinresScal m = mr[r];
-    const long e = 12 * t + a;
-    const bool act = a < 12;
-    double dot0 = 0.0, dot1 = 0.0;
-    if (mode == 0) {
-        const double rv = act ? A.R[1].pair[e] : 0.0;
-        const double zv = pm_matvec(A.P + 144L * t, a, nd, rv, team);
-        if (act) {
-            A.z.pair[e] = zv; A.x.pair[e] = 0.0; A.v.pair[e] = 0.0;
-            A.W[0].pair[e] = 0.0; A.W[1].pair[e] = 0.0; A.W[2].pair[e] = 0.0;
-            dot0 = rv * zv;
-            dot1 = zv * zv;
-        }
-    } else if (mode == 1 || mode == 3) {
-        double *vv = A.v.pair;
-        if (act && m.pending) {
-            const double w = (vv[e] - m.up_oldeps * A.W[k % 3].pair[e] - m.up_delta * A.W[(k + 1) % 3].pair[e]) *
-                             m.up_ginv;
-            A.W[(k + 2) % 3].pair[e] = w;
-            A.x.pair[e] += m.up_phi * w;
-        }
-        if (mode == 1 && !m.done) {
-            // the pair rows of A z: z_q + S_q (y + y2) gathered at the pair's DOFs (the L^T of
-            // the apply; lane a gathers entry a and forms row a, columns in ascending order)
-            double ya = 0.0;
-            if (a < nd) {
-                const long bd = (a % 6) < 3 ? bead : (long)pairs[t].y;
-                int tb, wb;
-                vel_dofs(sp, (int)(bd - sp.bead_off), tb, wb);
-                const int d = (a < 6 ? tb : wb) + a % 3;
-                ya = A.y[sp.top_off + d] + (sp.ss_off >= 0 ? A.y2[sp.top_off + d] : 0.0);
-            }
-            const double *Sq = A.S + 144L * t + a * nd;
-            double sy = 0.0;
-#pragma unroll
-            for (int c = 0; c < 12; c++) {
-                const double yc = __shfl_sync(team, ya, c, LT_LANES);
-                if (a < nd && c < nd) sy += Sq[c] * yc;
-            }
-            if (act) {
-                const double az = sy + A.z.pair[e];
-                const double vq = A.z.pair[e] * m.sinv;
-                double x = m.sinv * az;
-                if (k >= 2) x -= (m.beta / m.oldb) * A.R[(k + 2) % 3].pair[e];
-                vv[e] = vq;
-                A.R[(k + 1) % 3].pair[e] = x;
-                dot0 = vq * x;
-            }
-        }
-    } else if (mode == 2 && !m.done) {
-        double rv = 0.0;
-        if (act) {
-            double *av = A.R[(k + 1) % 3].pair;
-            rv = av[e] - (m.alfa / m.beta) * A.R[k % 3].pair[e];
-            av[e] = rv;
-        }
-        const double zv = pm_matvec(A.P + 144L * t, a, nd, rv, team);
-        if (act) {
-            A.z.pair[e] = zv;
-            dot0 = rv * zv;
-        }
-    }
-    if (mode <= 2) {
-#pragma unroll
-        for (int o = LT_LANES / 2; o > 0; o >>= 1) {
-            dot0 += __shfl_xor_sync(team, dot0, o, LT_LANES);
-            dot1 += __shfl_xor_sync(team, dot1, o, LT_LANES);
-        }
-        if (a == 0) { A.part[t] = dot0; A.part2[t] = dot1; }
-    }
-    return r;
+    if (s.Nc == 0 || s.ss_off >= 0) return;
+    for (int c = share(s.Nc, B.b, B.G) + threadIdx.x; c < share(s.Nc, B.b + 1, B.G); c += PB_THREADS)
+        f((long)s.top_off + s.nm3nc6 + 5 * c, (long)s.vec_off + s.nm3nc6 + 5 * c, (long)s.bead_off + s.Nm + c);
 }
 
-// Per-replica MINRES scalar recurrences from the replica's totals t0, t1 (the
-// sums of the pair and bead partials of k_pm_elem); mode 0 init, 1 alpha, 2 beta.
-__device__ void pm_scalars(MinresScal *mr, int r, int mode, double t0, double t1, int maxit, double rtol,
-                           int *nactive)
-{
-    const MinresScal m0 = mr[r];
-    if (mode != 1 && m0.done) return;
-    if (mode == 1 && m0.done && !m0.pending) return;
-    MinresScal m = m0;
-    if (mode == 0) {
-        m = MinresScal{};
-        double np0 = sqrt(t1);
-        m.np = np0;
-        m.ttol = fmax(rtol * np0, 1e-50);
-        if (t0 < 0) { m.done = 1; m.reason = -8; }
-        else if (np0 <= m.ttol || t0 == 0.0) { m.done = 1; m.reason = 2; }
-        else {
-            m.beta = sqrt(t0); m.phibar = m.beta; m.cs = -1; m.sn = 0; m.sinv = 1.0 / m.beta;
-        }
-        if (m.done) atomicSub(nactive, 1);
-    } else if (mode == 1) {
-        if (m.pending) m.pending = 0;
-        if (!m.done) m.alfa = t0;
-    } else {
-        m.it += 1;
-        double bb = t0;
-        m.oldb = m.beta;
-        if (bb < 0) {
-            m.done = 1; m.reason = -8;
-        } else {
-            m.beta = sqrt(bb);
-            double oldeps = m.epsln;
-            double delta = m.cs * m.dbar + m.sn * m.alfa;
-            double gbar = m.sn * m.dbar - m.cs * m.alfa;
-            m.epsln = m.sn * m.beta;
-            m.dbar = -m.cs * m.beta;
-            double gamma = sqrt(gbar * gbar + m.beta * m.beta);
-            if (gamma < 2.2250738585072014e-308) gamma = 2.2250738585072014e-308;
-            m.cs = gbar / gamma;
-            m.sn = m.beta / gamma;
-            double phi = m.cs * m.phibar;
-            m.phibar = m.sn * m.phibar;
-            m.up_oldeps = oldeps; m.up_delta = delta; m.up_ginv = 1.0 / gamma; m.up_phi = phi;
-            m.pending = 1;
-            m.np = m.np * fabs(m.sn);
-            if (m.np <= m.ttol) { m.done = 1; m.reason = 2; }
-            else if (m.beta == 0.0) { m.done = 1; m.reason = 3; }
-            else if (m.it >= maxit) { m.done = 1; m.reason = -3; }
-            m.sinv = m.beta != 0.0 ? 1.0 / m.beta : 0.0;
-        }
-        if (m.done) atomicSub(nactive, 1);
-    }
-    mr[r] = m;
-}
-
-// Fixed-order sum of x[lo, hi) over the block: thread t takes lo + t, lo + t + B,
-// ... into eight independent accumulators (eight loads in flight), joined in order.
-__device__ __forceinline__ double block_strided_sum(const double *__restrict__ x, long lo, long hi)
-{
-    double acc[8] = {0, 0, 0, 0, 0, 0, 0, 0};
-    const long B = blockDim.x;
-    for (long q = lo + threadIdx.x; q < hi; q += 8 * B) {
-#pragma unroll
-        for (int u = 0; u < 8; u++)
-            if (q + u * B < hi) acc[u] += __ldcg(x + q + u * B);
-    }
-    return ((acc[0] + acc[1]) + (acc[2] + acc[3])) + ((acc[4] + acc[5]) + (acc[6] + acc[7]));
-}
-
-// In-kernel completion of the per-replica sums: every pair team and every bead
-// thread counts one item of its replica (warp-aggregated atomics after a
-// fence); the block whose count completes replica r sums r's pair partials (a
-// contiguous range, pairs being stored by lower bead) and bead partials in a
-// fixed order -- block_strided_sum, then a shuffle tree and the warps in
-// order, whichever block finishes -- and runs the scalar recurrence.
-struct PMRed {
-    int *cnt;                  // per replica, zero between launches
-    const int *cptr;           // canonical pair pointer by lower bead
-    int maxit;
-    double rtol;
-    int *nactive;
-};
-
-__device__ void pm_count_and_finish(int myrep, const Seg *__restrict__ segs, const PMArgs &A, const PMRed &red,
-                                    MinresScal *mr, int mode)
-{
-    __shared__ int s_n, s_list[1024];
-    __shared__ double s_sum[32][2];
-    if (threadIdx.x == 0) s_n = 0;
-    __threadfence();
-    __syncthreads();
-    const unsigned valid = __ballot_sync(0xffffffffu, myrep >= 0);
-    if (myrep >= 0) {
-        const unsigned grp = __match_any_sync(valid, myrep);
-        if ((int)(threadIdx.x & 31) == __ffs(grp) - 1) {
-            const Seg &s = segs[myrep];
-            const int total = red.cptr[s.bead_off + s.Np] - red.cptr[s.bead_off] + s.Np;
-            const int n = __popc(grp);
-            if (atomicAdd(&red.cnt[myrep], n) + n == total) s_list[atomicAdd(&s_n, 1)] = myrep;
-        }
-    }
-    __syncthreads();
-    const int nfin = s_n;
-    for (int i = 0; i < nfin; i++) {
-        const int r = s_list[i];
-        __threadfence();
-        const Seg &s = segs[r];
-        const long q0 = red.cptr[s.bead_off], q1 = red.cptr[s.bead_off + s.Np];
-        double v0 = block_strided_sum(A.part, q0, q1) + block_strided_sum(A.sA, s.bead_off, (long)s.bead_off + s.Np);
-        double v1 = block_strided_sum(A.part2, q0, q1) + block_strided_sum(A.sB, s.bead_off, (long)s.bead_off + s.Np);
-        for (int o = 16; o > 0; o >>= 1) {
-            v0 += __shfl_down_sync(0xffffffffu, v0, o);
-            v1 += __shfl_down_sync(0xffffffffu, v1, o);
-        }
-        if ((threadIdx.x & 31) == 0) { s_sum[threadIdx.x >> 5][0] = v0; s_sum[threadIdx.x >> 5][1] = v1; }
-        __syncthreads();
-        if (threadIdx.x == 0) {
-            double t0 = 0.0, t1 = 0.0;
-            for (int w = 0; w < (int)(blockDim.x >> 5); w++) { t0 += s_sum[w][0]; t1 += s_sum[w][1]; }
-            pm_scalars(mr, r, mode, t0, t1, red.maxit, red.rtol, red.nactive);
-            red.cnt[r] = 0;
-        }
-        __syncthreads();
-    }
-}
-
-// Teams of LT_LANES lanes per pair (global thread < npair * LT_LANES), then one
-// thread per bead (stresslet entries of joint-replica colloids, nothing for
-// other beads); modes 0..2 finish their replica sums in the same launch
-// (pm_count_and_finish).  No thread leaves early: every thread reaches the
-// block barriers of the finish.
-// mode 0 init, 1 alpha (pending w/x update, v = z/beta, Av), 2 beta (r_{k+1}, z = P r), 3 flush
-__global__ void k_pm_elem(long npair, long ntot, const int2 *__restrict__ pairs, const int *__restrict__ bead_offs,
-                          int R, const Seg *__restrict__ segs, MinresScal *mr, int mode, int k, PMArgs A, PMRed red)
+// rhs into r_1 (pairs L^T (g + Mr b_bot), stresslets b_S + (M b_bot)_S), z = P r, zeros; sums
+// of r.z and z.z
+__global__ void __launch_bounds__(PB_THREADS) k_pm_init(PairTab T, PMArgs A)
 {
     pdl_enter();
-    const long gt = (long)blockIdx.x * blockDim.x + threadIdx.x;
-    const long npt = npair * LT_LANES;
-    int myrep = -1;                                   // replica of the item this thread counts
-    if (gt < npt) {
-        const int a = threadIdx.x % LT_LANES;
-        const int r = pm_pair_team(gt / LT_LANES, a, 0xffffu << (threadIdx.x & 16), pairs, bead_offs, R, segs, mr,
-                                   mode, k, A);
-        if (a == 0) myrep = r;
-    } else if (gt - npt < ntot) {
-        const long bead = gt - npt;
-        const int r = rep_of_b(bead_offs, R, bead);
-        myrep = r;
-        const Seg &s0 = segs[r];
-        const int i = (int)(bead - s0.bead_off);
-        if (!(s0.Nc > 0 && s0.ss_off < 0 && i >= s0.Nm)) {
-            if (mode <= 2) { A.sA[bead] = 0.0; A.sB[bead] = 0.0; }
-        } else {
-            const long base = (long)s0.top_off + s0.nm3nc6 + 5 * (i - s0.Nm);
-            const int n = 5;
-            double *u_s = A.u + base;
-            const double *y_s = A.y + base;
-            const MinresScal m = mr[r];
-            auto V = [&](const PMVec &p) { return p.s + base; };
-            double dot0 = 0.0, dot1 = 0.0;
-            if (mode == 0) {
-                double rv[5], zv[5];
-                double *rr = V(A.R[1]);
-                for (int a = 0; a < n; a++) rv[a] = rr[a];
-                s_precond(rv, zv);
-                double *zz = V(A.z), *xx = V(A.x), *vv = V(A.v), *w0 = V(A.W[0]), *w1 = V(A.W[1]), *w2 = V(A.W[2]);
-                for (int a = 0; a < n; a++) {
-                    zz[a] = zv[a]; xx[a] = 0.0; vv[a] = 0.0; w0[a] = 0.0; w1[a] = 0.0; w2[a] = 0.0;
-                    dot0 += rv[a] * zv[a];
-                    dot1 += zv[a] * zv[a];
-                    u_s[a] = zv[a];
-                }
-            } else if (mode == 1 || mode == 3) {
-                double *vv = V(A.v);
-                if (m.pending) {
-                    double *wn = V(A.W[(k + 2) % 3]);
-                    const double *w1 = V(A.W[k % 3]), *w2 = V(A.W[(k + 1) % 3]);
-                    double *xx = V(A.x);
-                    for (int a = 0; a < n; a++) {
-                        double w = (vv[a] - m.up_oldeps * w1[a] - m.up_delta * w2[a]) * m.up_ginv;
-                        wn[a] = w;
-                        xx[a] += m.up_phi * w;
-                    }
-                }
-                if (mode == 1 && !m.done) {
-                    const double *zz = V(A.z);
-                    double *av = V(A.R[(k + 1) % 3]);
-                    const double *rm1 = V(A.R[(k + 2) % 3]);
-                    const double c1 = (k >= 2) ? m.beta / m.oldb : 0.0;
-                    for (int a = 0; a < n; a++) {
-                        double vq = zz[a] * m.sinv;
-                        double x = m.sinv * y_s[a];
-                        if (k >= 2) x -= c1 * rm1[a];
-                        vv[a] = vq;
-                        av[a] = x;
-                        dot0 += vq * x;
-                    }
-                }
-            } else if (mode == 2 && !m.done) {
-                double *av = V(A.R[(k + 1) % 3]);
-                const double *rk = V(A.R[k % 3]);
-                const double c2 = m.alfa / m.beta;
-                double rv[5], zv[5];
-                for (int a = 0; a < n; a++) { rv[a] = av[a] - c2 * rk[a]; av[a] = rv[a]; }
-                s_precond(rv, zv);
-                double *zz = V(A.z);
-                for (int a = 0; a < n; a++) {
-                    zz[a] = zv[a];
-                    dot0 += rv[a] * zv[a];
-                    u_s[a] = zv[a];
+    const PairBlk B = T.blk[blockIdx.x];
+    const Seg &s = T.segs[B.rep];
+    for_pairs(T, B, s, [&](long q, long lo, long hi, int nd, int a, unsigned team) {
+        const double ra = lt_row(s, lo, hi, a, nd, team, A.S + 144 * q, A.y, A.y2, A.g);
+        const double za = pm_matvec(A.P + 144 * q, a, nd, ra, team);
+        if (a < nd) {
+            const long e = 12 * q + a;
+            A.R1.pair[e] = ra; A.z.pair[e] = za;
+            A.x.pair[e] = 0.0; A.v.pair[e] = 0.0;
+            A.W0.pair[e] = 0.0; A.W1.pair[e] = 0.0; A.W2.pair[e] = 0.0;
+        }
+        pair_dot(ra * za, team, a, A.db + q);
+        pair_dot(za * za, team, a, A.dn + q);
+    });
+    for_stresslets(B, s, [&](long t, long v, long bead) {
+        double r[5], z[5], rz = 0.0, zz = 0.0;
+        for (int a = 0; a < 5; a++) r[a] = A.b[v + a] + A.y[t + a];
+        s_precond(r, z);
+        for (int a = 0; a < 5; a++) {
+            A.R1.s[t + a] = r[a]; A.z.s[t + a] = z[a];
+            A.x.s[t + a] = 0.0; A.v.s[t + a] = 0.0;
+            A.W0.s[t + a] = 0.0; A.W1.s[t + a] = 0.0; A.W2.s[t + a] = 0.0;
+            rz += r[a] * z[a];
+            zz += z[a] * z[a];
+            A.u[t + a] = z[a];
+        }
+        A.db[A.npair + bead] = rz;
+        A.dn[A.npair + bead] = zz;
+    });
+}
+
+// closes iteration k - 1 (or the start): scalars, pending w and x update; opens iteration k:
+// v = z / beta, Av = (z + L^T (y + y2)) / beta - (beta / oldb) r_{k-1} in pair rows, y_S / beta - ... in
+// stresslet rows; sums of v.Av
+__global__ void __launch_bounds__(PB_THREADS)
+k_pm_alpha(PairTab T, PMArgs A, const MinresScal *__restrict__ st0, MinresScal *__restrict__ st1, int k, int maxit,
+           double rtol, int *nactive)
+{
+    pdl_enter();
+    const PairBlk B = T.blk[blockIdx.x];
+    __shared__ MinresScal sm;
+    if (st0[B.rep].done) {
+        if (B.b == 0 && threadIdx.x == 0) st1[B.rep] = st0[B.rep];
+        return;
+    }
+    const Seg &s = T.segs[B.rep];
+    const MinresScal &m = sm;
+    double c1 = 0.0;
+    // entry t of one storage (pick), its inputs w: z, v, w_{k-3}, w_{k-2}, x, r_{k-1}; az: the row of A z;
+    // adds v Av to dot
+    struct In { double az, z, v, w0, w1, x, r; };
+    auto fetch = [&](auto pick, long t, double az) {
+        return In{az, pick(A.z)[t], pick(A.v)[t], pick(A.W0)[t], pick(A.W1)[t], pick(A.x)[t], k >= 2 ? pick(A.R2)[t] : 0.0};
+    };
+    auto entry = [&](auto pick, long t, const In &w, double &dot) {
+        if (m.pending) {
+            const double wn = (w.v - m.up_oldeps * w.w0 - m.up_delta * w.w1) * m.up_ginv;
+            pick(A.W2)[t] = wn;
+            pick(A.x)[t] = w.x + m.up_phi * wn;
+        }
+        if (!m.done) {
+            const double v = w.z * m.sinv;
+            double x = m.sinv * w.az;
+            if (k >= 2) x -= c1 * w.r;
+            pick(A.v)[t] = v;
+            pick(A.R1)[t] = x;
+            dot += v * x;
+        }
+    };
+    auto pair = [](const PMVec &p) { return p.pair; };
+    auto strs = [](const PMVec &p) { return p.s; };
+    for_pairs(T, B, s,
+        [&](long q, long lo, long hi, int nd, int a, unsigned team) {
+            const double sy = lt_row(s, lo, hi, a, nd, team, A.S + 144 * q, A.y, A.y2, nullptr);
+            In w{};
+            if (a < nd) { w = fetch(pair, 12 * q + a, 0.0); w.az = sy + w.z; }
+            return w;
+        },
+        [&]() {
+            const double bb = pm_total(T, s, A.db, A.npair), zz = k == 1 ? pm_total(T, s, A.dn, A.npair) : 0.0;
+            if (threadIdx.x == 0) {
+                MinresScal n = st0[B.rep];
+                if (k == 1) {
+                    n = MinresScal{};
+                    n.np = sqrt(zz);
+                    n.ttol = fmax(rtol * n.np, 1e-50);
+                    if (bb < 0) { n.done = 1; n.reason = -8; }
+                    else if (n.np <= n.ttol || bb == 0.0) { n.done = 1; n.reason = 2; }
+                    else { n.beta = sqrt(bb); n.phibar = n.beta; n.cs = -1; n.sn = 0; n.sinv = 1.0 / n.beta; }
+                } else
+                    minres_advance(n, bb, maxit);
+                sm = n;
+                if (B.b == 0) {
+                    if (n.done) atomicSub(nactive, 1);
+                    n.pending = 0;                         // applied below
+                    st1[B.rep] = n;
                 }
             }
-            if (mode <= 2) { A.sA[bead] = dot0; A.sB[bead] = dot1; }
+            __syncthreads();
+            c1 = k >= 2 && !m.done ? m.beta / m.oldb : 0.0;
+            return true;
+        },
+        [&](const In &w, long q, int nd, int a, unsigned team) {
+            double dot = 0.0;
+            if (a < nd) entry(pair, 12 * q + a, w, dot);
+            if (!m.done) pair_dot(dot, team, a, A.da + q);
+        });
+    for_stresslets(B, s, [&](long t, long, long bead) {
+        double dot = 0.0;
+        for (int a = 0; a < 5; a++) entry(strs, t + a, fetch(strs, t + a, A.y[t + a]), dot);
+        if (!m.done) A.da[A.npair + bead] = dot;
+    });
+}
+
+// r_{k+1} = Av - (alfa / beta) r_k, z = P r (z_S into the apply's input); sums of r.z
+__global__ void __launch_bounds__(PB_THREADS) k_pm_beta(PairTab T, PMArgs A, MinresScal *__restrict__ st)
+{
+    pdl_enter();
+    const PairBlk B = T.blk[blockIdx.x];
+    if (st[B.rep].done) return;
+    const Seg &s = T.segs[B.rep];
+    const PMVec Rn = A.R1, Rk = A.R0;
+    struct In { double r, k; Row12 P; };
+    double c2 = 0.0;
+    for_pairs(T, B, s,
+        [&](long q, long, long, int nd, int a, unsigned) {
+            In w{};
+            if (a < nd) { w.r = Rn.pair[12 * q + a]; w.k = Rk.pair[12 * q + a]; }
+            w.P = block_row(A.P + 144 * q, a, nd);
+            return w;
+        },
+        [&]() {
+            const double alfa = pm_total(T, s, A.da, A.npair);
+            if (B.b == 0 && threadIdx.x == 0) st[B.rep].alfa = alfa;
+            c2 = alfa / st[B.rep].beta;
+            return true;
+        },
+        [&](const In &w, long q, int nd, int a, unsigned team) {
+            const long e = 12 * q + a;
+            const double ra = a < nd ? w.r - c2 * w.k : 0.0, za = row_dot(w.P, ra, team);
+            if (a < nd) {
+                Rn.pair[e] = ra;
+                A.z.pair[e] = za;
+            }
+            pair_dot(ra * za, team, a, A.db + q);
+        });
+    for_stresslets(B, s, [&](long t, long, long bead) {
+        double r[5], z[5], dot = 0.0;
+        for (int a = 0; a < 5; a++) { r[a] = Rn.s[t + a] - c2 * Rk.s[t + a]; Rn.s[t + a] = r[a]; }
+        s_precond(r, z);
+        for (int a = 0; a < 5; a++) {
+            A.z.s[t + a] = z[a];
+            dot += r[a] * z[a];
+            A.u[t + a] = z[a];
         }
-    }
-    if (mode <= 2) pm_count_and_finish(myrep, segs, A, red, mr, mode);
+        A.db[A.npair + bead] = dot;
+    });
+}
+
+static int grow(double *&p, long n)
+{
+    cudaFree(p);
+    p = nullptr;
+    PS_CK(cudaMalloc(&p, sizeof(double) * n));
+    return PS_OK;
 }
 
 static int ensure_pair_space(Engine &E)
 {
-    long need = std::max<long>(E.lub_npairs, 1);
+    const long need = std::max<long>(E.lub_npairs, 1);
     if (need <= E.pair_cap) return PS_OK;
     E.ps_setup_valid = false;
-    cudaFree(E.d_pS); cudaFree(E.d_pP); cudaFree(E.d_ppart); cudaFree(E.d_ppart2);
-    for (auto &p : E.d_py_) cudaFree(p);
-    for (auto &p : E.d_pmp) cudaFree(p);
-    E.pair_cap = need * 3 / 2 + 256;
-    PS_CK(cudaMalloc(&E.d_pS, sizeof(double) * 144 * E.pair_cap));
-    PS_CK(cudaMalloc(&E.d_pP, sizeof(double) * 144 * E.pair_cap));
-    PS_CK(cudaMalloc(&E.d_ppart, sizeof(double) * E.pair_cap));
-    PS_CK(cudaMalloc(&E.d_ppart2, sizeof(double) * E.pair_cap));
-    for (auto &p : E.d_py_) PS_CK(cudaMalloc(&p, sizeof(double) * 12 * E.pair_cap));
-    for (auto &p : E.d_pmp) PS_CK(cudaMalloc(&p, sizeof(double) * 12 * E.pair_cap));
+    E.pair_cap = 0;
+    const long cap = need * 3 / 2 + 256;
+    int rc;
+    if ((rc = grow(E.d_pS, 144 * cap)) || (rc = grow(E.d_pP, 144 * cap))) return rc;
+    for (auto &p : E.d_py_)
+        if ((rc = grow(p, 12 * cap))) return rc;
+    E.pair_cap = cap;
     return PS_OK;
 }
+
+// the pair-space MINRES vectors, for the contexts that come to use them
+static int ensure_pm_space(Engine &E)
+{
+    if (E.pm_cap >= E.pair_cap) return PS_OK;
+    E.pm_cap = 0;
+    int rc;
+    for (auto &p : E.d_pmp)
+        if ((rc = grow(p, 12 * E.pair_cap))) return rc;
+    if ((rc = grow(E.d_pmd, 3 * (E.pair_cap + E.ntot)))) return rc;
+    // beads without stresslet unknowns never write theirs
+    PS_CK(cudaMemset(E.d_pmd, 0, sizeof(double) * 3 * (E.pair_cap + E.ntot)));
+    E.pm_cap = E.pair_cap;
+    return PS_OK;
+}
+
+static PairTab pair_tab(const Engine &E) { return {E.d_pblk, E.d_lub_pairs, E.d_lubc_ptr, E.d_segs}; }
+
+static void launch_ps_L(Engine &E, const double *y, const double *add, double *u, double *vel, double *x,
+                        const char *done, int dstride, cudaStream_t st)
+{
+    ps_launch(k_ps_L, (unsigned)E.n_pblk, PB_THREADS, 0, st, pair_tab(E), E.d_lub_ptr, E.d_lub_nbr, E.d_lub_cidx, E.d_pS, y,
+            add, u, vel, x, done, dstride);
+}
+
+// iterations of a pair-space solver are looked at by the host every check_every of them, long
+// solves less often (a missed stop costs launches of blocks that leave at once)
+static int next_check(int k, int check_every) { return k + std::max(check_every, std::min(k / 4, 4 * check_every)); }
 
 // MINRES iterations of the pair-space system; the setup (pair blocks, g, the
 // u_t = b_bot apply input) has run.  Returns the solution's pair and stresslet
 // storages in *ysol / *ssol.
-static int pair_minres(Engine &E, const double *b, const double *g, int maxit, double rtol, bool fp32,
-                       cudaStream_t st, double **ysol, double **ssol, int *iters)
+static int pair_minres(Engine &E, const double *b, const double *g, int maxit, double rtol, int check_every, bool fp32,
+                       cudaStream_t st, double **ysol, double **ssol, MinresScal **scal)
 {
-    const long npair = E.lub_npairs;
-    const int thr = 128;
-    const unsigned nbp = (unsigned)((std::max<long>(npair, 1) + PS_THREADS - 1) / PS_THREADS);
-    const unsigned nbp_lt = (unsigned)((std::max<long>(npair, 1) * LT_LANES + PS_THREADS - 1) / PS_THREADS);
-    const unsigned nbp_e = (unsigned)((std::max<long>(npair, 1) * 12 + PS_THREADS - 1) / PS_THREADS);
-    const unsigned nbb = (unsigned)((E.ntot + thr - 1) / thr);
-    const unsigned nbe = (unsigned)((npair * LT_LANES + E.ntot + thr - 1) / thr);
-    const char *dn = (const char *)&E.d_pmr[0].done;
     const int ds = (int)sizeof(MinresScal);
+    const unsigned nb = (unsigned)E.n_pblk;
+    const PairTab T = pair_tab(E);
+    int rc = ensure_pm_space(E);
+    if (rc) return rc;
     PMArgs A;
-    for (int k = 0; k < 3; k++) { A.R[k] = {E.d_pmp[k], E.d_pms[k]}; A.W[k] = {E.d_pmp[3 + k], E.d_pms[3 + k]}; }
+    // r_k lives in slot k % 3, w_k in slot 3 + k % 3
+    auto slots = [&](int k) {
+        PMVec *r[3] = {&A.R0, &A.R1, &A.R2}, *w[3] = {&A.W0, &A.W1, &A.W2};
+        for (int j = 0; j < 3; j++) {
+            const int i = (k + j) % 3;
+            *r[j] = {E.d_pmp[i], E.d_pms[i]};
+            *w[j] = {E.d_pmp[3 + i], E.d_pms[3 + i]};
+        }
+    };
+    slots(0);
     A.v = {E.d_pmp[6], E.d_pms[6]};
     A.z = {E.d_pmp[7], E.d_pms[7]};
     A.x = {E.d_pmp[8], E.d_pms[8]};
+    A.b = b;
+    A.g = g;
     A.y = E.d_py;
     A.y2 = E.d_py2;
     A.S = E.d_pS;
     A.u = E.d_pu;
     A.P = E.d_pP;
-    A.part = E.d_ppart; A.part2 = E.d_ppart2;
-    A.sA = E.d_sbead[0]; A.sB = E.d_sbead[1];
-    PS_CK(cudaMemsetAsync(E.d_pmr, 0, sizeof(MinresScal) * E.R, st));
-    if (!E.d_pm_cnt) {
-        PS_CK(cudaMalloc(&E.d_pm_cnt, sizeof(int) * E.R));
-        PS_CK(cudaMemsetAsync(E.d_pm_cnt, 0, sizeof(int) * E.R, st));
-    }
-    const PMRed red = {E.d_pm_cnt, E.d_lubc_ptr, maxit, rtol, E.d_nactive};
-    // rhs into R[1]: pairs L^T (g + Mr b_bot), stresslets b_S + (M b_bot)_S
-    mr_apply(E, fp32, dn, ds, st);
-    if (npair)
-        ps_launch(k_ps_LT, nbp_lt, PS_THREADS, 0, st, npair, E.d_lub_pairs, E.d_bead_offs, E.R, E.d_segs,
-                E.d_pS, E.d_py, E.d_py2, g, 1.0, nullptr, A.R[1].pair,
-                nullptr, dn, ds);
-    ps_launch(k_ps_S, nbb, thr, 0, st, E.ntot, E.d_bead_offs, E.R, E.d_segs, 0, E.d_pcg, b, E.d_py, E.d_D,
-            E.d_sv[0], A.R[1].s, E.d_sv[2], E.d_sv[3], E.d_sv[4], E.d_pu,
-            nullptr, A.sA, A.sB);
-    *E.h_nactive = E.R;
-    PS_CK(cudaMemcpyAsync(E.d_nactive, E.h_nactive, sizeof(int), cudaMemcpyHostToDevice, st));
-    ps_launch(k_pm_elem, nbe, thr, 0, st, npair, E.ntot, E.d_lub_pairs, E.d_bead_offs, E.R, E.d_segs,
-            E.d_pmr, 0, 0, A, red);
-    PS_CK(cudaMemcpyAsync(E.h_nactive, E.d_nactive, sizeof(int), cudaMemcpyDeviceToHost, st));
-    PS_CK(cudaStreamSynchronize(st));
-    int nact = *E.h_nactive, k = 0;
-    while (nact > 0 && k < maxit) {
-        for (int j = 0; j < 8 && k < maxit; j++) {
-            k++;
-            // Az = A z: u = [L z_y ; z_S] (z_S already in u), apply; mode 1 forms z_y + L^T (...)_t itself
-            launch_ps_L(E, A.z.pair, nullptr, nullptr, E.d_pu, nullptr, nullptr, dn, ds, st);
+    const long nd = E.pair_cap + E.ntot;
+    A.da = E.d_pmd; A.db = A.da + nd; A.dn = A.db + nd;
+    A.npair = E.pair_cap;
+    PS_CK(cudaMemsetAsync(E.d_pmr, 0, sizeof(MinresScal) * 2 * E.R, st));
+    mr_apply(E, fp32, nullptr, 0, st);
+    ps_launch(k_pm_init, nb, PB_THREADS, 0, st, T, A);
+    int nact = E.R;
+    MinresScal *last = E.d_pmr;
+    for (int k = 1, next = check_every + 1; nact > 0; k++) {
+        MinresScal *s0 = E.d_pmr + (long)E.R * ((k - 1) & 1), *s1 = E.d_pmr + (long)E.R * (k & 1);
+        const char *dn = (const char *)&s0[0].done;
+        slots(k);
+        // A z: u = [L z_y ; z_S] (z_S already in u), apply; k_pm_alpha forms z_y + L^T (...)_t itself
+        if (k <= maxit) {
+            launch_ps_L(E, A.z.pair, nullptr, E.d_pu, nullptr, nullptr, dn, ds, st);
             mr_apply(E, fp32, dn, ds, st);
-            ps_launch(k_pm_elem, nbe, thr, 0, st, npair, E.ntot, E.d_lub_pairs, E.d_bead_offs, E.R,
-                    E.d_segs, E.d_pmr, 1, k, A, red);
-            ps_launch(k_pm_elem, nbe, thr, 0, st, npair, E.ntot, E.d_lub_pairs, E.d_bead_offs, E.R,
-                    E.d_segs, E.d_pmr, 2, k, A, red);
         }
-        PS_CK(cudaMemcpyAsync(E.h_nactive, E.d_nactive, sizeof(int), cudaMemcpyDeviceToHost, st));
-        PS_CK(cudaStreamSynchronize(st));
-        nact = *E.h_nactive;
+        ps_launch(k_pm_alpha, nb, PB_THREADS, 0, st, T, A, s0, s1, k, maxit, rtol, E.d_nactive);
+        last = s1;
+        if (k == next || k > maxit) {
+            PS_CK(cudaMemcpyAsync(E.h_nactive, E.d_nactive, sizeof(int), cudaMemcpyDeviceToHost, st));
+            PS_CK(cudaStreamSynchronize(st));
+            nact = *E.h_nactive;
+            if (k > maxit) break;
+            next = next_check(k, check_every);
+        }
+        if (nact > 0) ps_launch(k_pm_beta, nb, PB_THREADS, 0, st, T, A, s1);
     }
-    // the last pending w/x update
-    ps_launch(k_pm_elem, nbe, thr, 0, st, npair, E.ntot, E.d_lub_pairs, E.d_bead_offs, E.R, E.d_segs,
-            E.d_pmr, 3, k + 1, A, red);
     PS_CK(cudaGetLastError());
     *ysol = A.x.pair;
     *ssol = A.x.s;
-    *iters = k;
+    *scal = last;
+    return PS_OK;
+}
+
+static int pair_cg(Engine &E, const double *g, int maxit, int check_every, bool fp32, cudaStream_t st, const PcgVec &V,
+                   PcgScal **scal)
+{
+    const int ds = (int)sizeof(PcgScal);
+    const unsigned nb = (unsigned)E.n_pblk;
+    const PairTab T = pair_tab(E);
+    double *pap = E.d_pbp, *prz = pap + E.n_pblk, *perr = prz + E.n_pblk;
+    // rhs = L^T (g + Mr b_bot)
+    mr_apply(E, fp32, nullptr, 0, st);
+    ps_launch(k_pc_init, nb, PB_THREADS, 0, st, T, E.d_pS, E.d_pP, E.d_py, E.d_py2, g, V, prz);
+    PcgScal *s1 = E.d_pcg;
+    int nact = E.R;
+    for (int k = 0, next = 0;; k++) {
+        // residual test of iteration k - 1 (or of the start), next direction
+        PcgScal *s0 = s1;
+        s1 = E.d_pcg + (long)E.R * ((k + 1) & 1);
+        ps_launch(k_pc_gather, nb, PB_THREADS, 0, st, T, E.d_lub_ptr, E.d_lub_nbr, E.d_lub_cidx, E.d_pS, V, E.d_D, s0, perr);
+        ps_launch(k_pc_dir, nb, PB_THREADS, 0, st, T, s0, s1, prz, perr, V, E.d_pu, k, maxit, E.d_nactive);
+        if (k == next || k >= maxit) {
+            PS_CK(cudaMemcpyAsync(E.h_nactive, E.d_nactive, sizeof(int), cudaMemcpyDeviceToHost, st));
+            PS_CK(cudaStreamSynchronize(st));
+            nact = *E.h_nactive;
+            if (nact <= 0 || k >= maxit) break;
+            next = next_check(k, check_every);
+        }
+        const char *dn = (const char *)&s1[0].done;
+        mr_apply(E, fp32, dn, ds, st);
+        ps_launch(k_pc_apply, nb, PB_THREADS, 0, st, T, E.d_pS, E.d_py, E.d_py2, V, s1, pap);
+        ps_launch(k_pc_update, nb, PB_THREADS, 0, st, T, E.d_pP, V, s1, pap, prz, E.d_nactive);
+    }
+    PS_CK(cudaGetLastError());
+    *scal = s1;
     return PS_OK;
 }
 
 static int pair_solve(Engine &E, const double *b, double *x, const ps_ksp_opts *o, ps_ksp_result *res,
                       cudaStream_t st, bool minres)
 {
-    RedTable &TV = E.red_vel, &TB = E.red_bead;
+    RedTable &TV = E.red_vel;
     const bool fp32 = E.precision == PS_PREC_MIXED;
     // CG converges in tens of iterations on positive definite far fields; a cap
     // hands the rare indefinite case to MINRES early
     const int maxit = minres ? (o->maxit > 0 ? o->maxit : 10000) : std::min(o->maxit > 0 ? o->maxit : 10000, 1000);
     const int check_every = o->check_every > 0 ? o->check_every : 8;
     const long npair = E.lub_npairs;
-    const int thr = 128;
-    const unsigned nbp = (unsigned)((std::max<long>(npair, 1) + PS_THREADS - 1) / PS_THREADS);
-    const unsigned nbp_lt = (unsigned)((std::max<long>(npair, 1) * LT_LANES + PS_THREADS - 1) / PS_THREADS);
-    const unsigned nbp_e = (unsigned)((std::max<long>(npair, 1) * 12 + PS_THREADS - 1) / PS_THREADS);
-    const unsigned nbb = (unsigned)((E.ntot + thr - 1) / thr);
     int rc = diag_saddle(E, E.d_D, st);
     if (rc) return rc;
     if ((rc = ensure_pair_space(E))) return rc;
-    double *yv = E.d_py_[0], *rv = E.d_py_[1], *zv = E.d_py_[2], *pv = E.d_py_[3], *Ap = E.d_py_[4];
-    double *yS = E.d_sv[0], *rS = E.d_sv[1], *zS = E.d_sv[2], *pS = E.d_sv[3], *ApS = E.d_sv[4];
-    double *sA = E.d_sbead[0], *sB = E.d_sbead[1];     // per-bead stresslet partials
-    // d_pr (nvel >= ntot doubles) holds the per-bead partials
-    double *cvel = E.d_pV, *g = E.d_pg, *tmp = E.d_tmp_vel, *bead_part = E.d_pr;
-    const void *dn = &E.d_pcg[0].done;
-    const int ds = (int)sizeof(PcgScal);
-    // stresslet unknowns join the CG only for replicas beyond the dense stresslet
-    // limit; without such replicas k_ps_S has nothing to do but keep the per-bead
-    // stresslet partials at zero, which one clear at the start does
-    const bool joint = E.n_ss_polish > 0;
-    if (!joint) {
-        PS_CK(cudaMemsetAsync(sA, 0, sizeof(double) * E.ntot, st));
-        PS_CK(cudaMemsetAsync(sB, 0, sizeof(double) * E.ntot, st));
-    }
-    PS_CK(cudaMemsetAsync(x, 0, sizeof(double) * E.nvec, st));
-    PS_CK(cudaMemsetAsync(E.d_pu, 0, sizeof(double) * E.ntop, st));
-    PS_CK(cudaMemsetAsync(E.d_pu2, 0, sizeof(double) * E.ntop, st));
-    PS_CK(cudaMemsetAsync(E.d_py2, 0, sizeof(double) * E.ntop, st));
-    ps_launch(k_pcg_start, E.red.nblk, RB_THREADS, 0, st, E.red, E.d_segs, b, E.d_D, E.d_pcg, o->rtol);
+    double *cvel = E.d_pV, *g = E.d_pg;
+    // replicas beyond the dense stresslet limit keep their stresslets as unknowns: their part of
+    // the apply's input starts at zero (elsewhere it is never written)
+    if (E.n_ss_polish) PS_CK(cudaMemsetAsync(E.d_pu, 0, sizeof(double) * E.ntop, st));
+    ps_launch(k_pcg_start, E.red.nblk, RB_THREADS, 0, st, E.red, b, E.d_D, E.d_pcg, o->rtol, E.R, E.d_nactive);
     // the pair blocks depend on the staged positions and the table only: solves
     // that share a staging (the deterministic and the noise solve) set them up once
     if (npair && !E.ps_setup_valid) {
@@ -1404,85 +1400,21 @@ static int pair_solve(Engine &E, const double *b, double *x, const ps_ksp_opts *
                 0, 0.0, E.d_pu2, 1, nullptr, 0);
         apply_operator(E, 1, E.d_pu2, E.d_py2, fp32, st, nullptr, 0, true);
     }
-    ps_launch(k_pcg_g, TV.nblk, RB_THREADS, 0, st, TV, E.d_segs, b, E.d_py2, g);
-    ps_launch(k_ps_c, TV.nblk, RB_THREADS, 0, st, TV, E.d_segs, b, cvel, E.d_pu);
+    ps_launch(k_ps_rhs, TV.nblk, RB_THREADS, 0, st, TV, E.d_segs, b, E.d_py2, g, cvel, E.d_pu);
     PS_CK(cudaGetLastError());
-    std::vector<PcgScal> hp(E.R);
-    PS_CK(cudaMemcpyAsync(hp.data(), E.d_pcg, sizeof(PcgScal) * E.R, cudaMemcpyDeviceToHost, st));
-    PS_CK(cudaStreamSynchronize(st));
-    int nact = 0;
-    for (auto &p : hp) nact += !p.done;
-    *E.h_nactive = nact;
-    PS_CK(cudaMemcpyAsync(E.d_nactive, E.h_nactive, sizeof(int), cudaMemcpyHostToDevice, st));
+    double *yv = E.d_py_[0], *yS = nullptr;
+    PcgScal *cs = nullptr;
+    MinresScal *ms = nullptr;
     if (minres) {
-        int nit = 0;
-        rc = pair_minres(E, b, g, maxit, o->rtol, fp32, st, &yv, &yS, &nit);
-        if (rc) return rc;
+        if ((rc = pair_minres(E, b, g, maxit, o->rtol, check_every, fp32, st, &yv, &yS, &ms))) return rc;
     } else {
-        if (nact) {
-            // rhs = L^T (g + Mr b_bot) (joint replicas: Mr -> M, and b_S + (M b_bot)_S) ; r = rhs ; z = P r ; p = z
-            mr_apply(E, fp32, dn, ds, st);
-            if (npair) {
-                ps_launch(k_ps_LT, nbp_lt, PS_THREADS, 0, st, npair, E.d_lub_pairs, E.d_bead_offs, E.R, E.d_segs,
-                        E.d_pS, E.d_py, E.d_py2, g, 1.0, nullptr, rv, nullptr,
-                        (const char *)dn, ds);
-                ps_launch(k_ps_init, nbp_lt, PS_THREADS, 0, st, npair, E.d_lub_pairs, E.d_bead_offs, E.R,
-                        E.d_segs, E.d_pP, yv, rv, zv, pv, E.d_ppart);
-            }
-        }
-        if (joint)
-            ps_launch(k_ps_S, nbb, thr, 0, st, E.ntot, E.d_bead_offs, E.R, E.d_segs, 0, E.d_pcg, b, E.d_py, E.d_D,
-                    yS, rS, zS, pS, ApS, E.d_pu, x, sA, sB);
-        // initial residual ||D^{-1} L r||^2 + ||D^{-1} r_S||^2
-        launch_ps_L(E, rv, nullptr, nullptr, nullptr, E.d_D, bead_part, (const char *)dn, ds, st);
-        ps_launch(k_ps_reduce, TB.nblk, RB_THREADS, 0, st, TB, E.d_lubc_ptr, E.d_ppart, bead_part, sA, sB,
-                E.d_pcg, 1, maxit, E.d_nactive);
-        PS_CK(cudaMemcpyAsync(E.h_nactive, E.d_nactive, sizeof(int), cudaMemcpyDeviceToHost, st));
-        PS_CK(cudaStreamSynchronize(st));
-        nact = *E.h_nactive;
-        int k = 0;
-        while (nact > 0 && k < maxit) {
-            for (int j = 0; j < check_every && k < maxit; j++, k++) {
-                // Ap = p + L^T Mr L p  (joint replicas: [p_y + L^T (M u)_t ; (M u)_S], u = [L p_y ; p_S])
-                launch_ps_L(E, pv, nullptr, nullptr, E.d_pu, nullptr, nullptr, (const char *)dn, ds, st);
-                mr_apply(E, fp32, dn, ds, st);
-                if (npair)
-                    ps_launch(k_ps_LT, nbp_lt, PS_THREADS, 0, st, npair, E.d_lub_pairs, E.d_bead_offs, E.R,
-                            E.d_segs, E.d_pS, E.d_py, E.d_py2, nullptr, 1.0,
-                            pv, Ap, E.d_ppart, (const char *)dn, ds);
-                if (joint)
-                    ps_launch(k_ps_S, nbb, thr, 0, st, E.ntot, E.d_bead_offs, E.R, E.d_segs, 1, E.d_pcg, b, E.d_py,
-                            E.d_D, yS, rS, zS, pS, ApS, E.d_pu, x, sA, nullptr);
-                ps_launch(k_ps_reduce, TB.nblk, RB_THREADS, 0, st, TB, E.d_lubc_ptr, E.d_ppart, nullptr, sA,
-                        nullptr, E.d_pcg, 0, maxit, E.d_nactive);
-                if (npair)
-                    ps_launch(k_ps_update, nbp_lt, PS_THREADS, 0, st, npair, E.d_lub_pairs, E.d_bead_offs, E.R,
-                            E.d_segs, E.d_pcg, E.d_pP, pv, Ap, yv, rv,
-                            zv, E.d_ppart);
-                if (joint)
-                    ps_launch(k_ps_S, nbb, thr, 0, st, E.ntot, E.d_bead_offs, E.R, E.d_segs, 2, E.d_pcg, b, E.d_py,
-                            E.d_D, yS, rS, zS, pS, ApS, E.d_pu, x, sA, sB);
-                launch_ps_L(E, rv, nullptr, nullptr, nullptr, E.d_D, bead_part, (const char *)dn, ds, st);
-                ps_launch(k_ps_reduce, TB.nblk, RB_THREADS, 0, st, TB, E.d_lubc_ptr, E.d_ppart, bead_part, sA,
-                        sB, E.d_pcg, 2, maxit, E.d_nactive);
-                if (npair)
-                    ps_launch(k_ps_dir, nbp_e, PS_THREADS, 0, st, npair, E.d_lub_pairs, E.d_bead_offs, E.R,
-                            E.d_pcg, zv, pv);
-                if (joint)
-                    ps_launch(k_ps_S, nbb, thr, 0, st, E.ntot, E.d_bead_offs, E.R, E.d_segs, 3, E.d_pcg, b, E.d_py,
-                            E.d_D, yS, rS, zS, pS, ApS, E.d_pu, x, nullptr, nullptr);
-            }
-            PS_CK(cudaMemcpyAsync(E.h_nactive, E.d_nactive, sizeof(int), cudaMemcpyDeviceToHost, st));
-            PS_CK(cudaStreamSynchronize(st));
-            nact = *E.h_nactive;
-        }
+        const PcgVec V = {E.d_py_[0], E.d_py_[1], E.d_py_[2], E.d_py_[3], E.d_py_[4], E.d_pz, E.d_pp};
+        if ((rc = pair_cg(E, g, maxit, check_every, fp32, st, V, &cs))) return rc;
     }
     // F_t = -b_bot + L y (into u_t and the force rows), then U = Mr F_t - g, F_S
-    launch_ps_L(E, yv, cvel, tmp, E.d_pu, nullptr, nullptr, nullptr, 0, st);
-    ps_launch(k_ps_ft, TV.nblk, RB_THREADS, 0, st, TV, E.d_segs, tmp, x);
-    if (joint)
-        ps_launch(k_ps_S, nbb, thr, 0, st, E.ntot, E.d_bead_offs, E.R, E.d_segs, 4, E.d_pcg, b, E.d_py, E.d_D,
-                yS, rS, zS, pS, ApS, E.d_pu, x, nullptr, nullptr);
+    launch_ps_L(E, yv, cvel, E.d_pu, nullptr, x, nullptr, 0, st);
+    if (E.n_ss_polish)
+        ps_launch(k_ps_S, (unsigned)((E.ncoll + 127) / 128), 128, 0, st, E.ncoll, E.d_coll_rep, E.d_segs, yS, E.d_pu, x);
     mr_apply(E, fp32, nullptr, 0, st);
     ps_launch(k_ps_fin, TV.nblk, RB_THREADS, 0, st, TV, E.d_segs, E.d_py, E.d_py2, g, x);
     if (E.n_ss_reps)
@@ -1492,27 +1424,22 @@ static int pair_solve(Engine &E, const double *b, double *x, const ps_ksp_opts *
     int worst = 1000, itmax = 0;
     long itsum = 0;
     double emax = 0;
+    auto add = [&](int done, int reason, int it, double err) {
+        worst = std::min(worst, done ? reason : -3);
+        itmax = std::max(itmax, it);
+        itsum += it;
+        emax = std::max(emax, err);
+    };
     if (minres) {
         std::vector<MinresScal> hm(E.R);
-        PS_CK(cudaMemcpyAsync(hm.data(), E.d_pmr, sizeof(MinresScal) * E.R, cudaMemcpyDeviceToHost, st));
+        PS_CK(cudaMemcpyAsync(hm.data(), ms, sizeof(MinresScal) * E.R, cudaMemcpyDeviceToHost, st));
         PS_CK(cudaStreamSynchronize(st));
-        for (auto &m : hm) {
-            int reason = m.done ? m.reason : -3;
-            worst = std::min(worst, reason);
-            itmax = std::max(itmax, m.it);
-            itsum += m.it;
-            emax = std::max(emax, m.np);
-        }
+        for (auto &m : hm) add(m.done, m.reason, m.it, m.np);
     } else {
-        PS_CK(cudaMemcpyAsync(hp.data(), E.d_pcg, sizeof(PcgScal) * E.R, cudaMemcpyDeviceToHost, st));
+        std::vector<PcgScal> hp(E.R);
+        PS_CK(cudaMemcpyAsync(hp.data(), cs, sizeof(PcgScal) * E.R, cudaMemcpyDeviceToHost, st));
         PS_CK(cudaStreamSynchronize(st));
-        for (auto &p : hp) {
-            int reason = p.done ? p.reason : -3;
-            worst = std::min(worst, reason);
-            itmax = std::max(itmax, p.it);
-            itsum += p.it;
-            emax = std::max(emax, p.err);
-        }
+        for (auto &p : hp) add(p.done, p.reason, p.it, p.err);
     }
     if (worst == 1000) worst = 2;
     if (res) { res->reason = worst; res->iters_max = itmax; res->iters_sum = itsum; res->rnorm_max = emax; }
@@ -1627,7 +1554,7 @@ int lub_noise(Engine &E, const double *z, double *rhs, cudaStream_t st)
                 E.d_lubc_ptr, E.d_rseed, E.d_rstep, E.d_zlub);
         z = E.d_zlub;
     }
-    launch_ps_L(E, z, nullptr, E.d_tmp_vel, nullptr, nullptr, nullptr, nullptr, 0, st);
+    launch_ps_L(E, z, nullptr, nullptr, E.d_tmp_vel, nullptr, nullptr, 0, st);
     const int thr = 256;
     ps_launch(k_lub_noise_add, (unsigned)((E.nvel + thr - 1) / thr), thr, 0, st,
             E.nvel, E.d_vel_offs, E.R, E.d_segs, E.d_tmp_vel, rhs);
