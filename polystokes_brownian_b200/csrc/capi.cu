@@ -55,7 +55,7 @@ static void free_engine(Engine &E)
     void *ptrs[] = {E.d_segs, E.d_vec_offs, E.d_top_offs, E.d_vel_offs, E.d_bead_offs, E.d_x, E.d_q, E.d_xpos0,
                     E.d_xn, E.d_pos64, E.d_pos32, E.d_pos32lo, E.d_aa_te2, E.d_chain, E.d_coll_rep, E.d_chs, E.d_time, E.d_ktrap, E.d_trapinfo,
                     E.d_aa_tiles, E.d_bb_tiles, E.d_partAA, E.d_partAB, E.d_partBB, E.d_partBA,
-                    E.d_tab, E.d_stale, E.d_aa_last, E.d_delta, E.d_schurQ, E.d_schurL, E.d_schur_reps, E.d_ss_reps,
+                    E.d_tab, E.d_stale, E.d_aa_last, E.d_delta, E.d_schurR, E.d_schur_reps, E.d_ss_reps,
                     E.d_bond_ptr, E.d_bond_nbr, E.d_bond_sgn, E.d_cell, E.d_cell_start, E.d_cell_sorted,
                     E.d_cell_count, E.d_cellgeo, E.d_cell_offs, E.d_nbr_ptr, E.d_nbr, E.d_nbr_count, E.d_lubtab,
                     E.d_luby, E.d_lub_diag, E.d_lub_ptr, E.d_lub_nbr, E.d_lub_cidx, E.d_tmp_vel, E.d_tmp_vel2, E.d_zlub, E.d_D, E.d_z, E.d_v, E.d_xw, E.d_Rr[0],
@@ -315,8 +315,7 @@ static int build(Engine &E, const ps_desc *descs, int R, int precision)
     TRY_ALLOC(E.d_partBB, sizeof(double) * top * E.nch_bb);
     TRY_ALLOC(E.d_partBA, sizeof(double) * 11 * std::max<long>(ba, 1));
     TRY_ALLOC(E.d_delta, sizeof(double) * std::max<long>(schur, 1));
-    TRY_ALLOC(E.d_schurQ, sizeof(double) * std::max<long>(schur, 1));
-    TRY_ALLOC(E.d_schurL, sizeof(double) * std::max<long>(schur, 1));
+    TRY_ALLOC(E.d_schurR, sizeof(double) * std::max<long>(schur, 1));
     // cells and pair lists
     TRY_ALLOC(E.d_cell, sizeof(int) * bead);
     TRY_ALLOC(E.d_cell_start, sizeof(int) * (cells + 1));

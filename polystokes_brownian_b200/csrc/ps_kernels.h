@@ -94,7 +94,7 @@ struct Engine {
 
     // arrowhead Schur floor (shell path)
     long nschur = 0;
-    double *d_delta = nullptr, *d_schurQ = nullptr, *d_schurL = nullptr;
+    double *d_delta = nullptr, *d_schurR = nullptr;
     int *d_schur_reps = nullptr; int n_schur_reps = 0;
     int *d_ss_reps = nullptr; int n_ss_reps = 0;   // replicas whose stresslet block is solved densely
     // Schur Lanczos noise of shell replicas above the dense Schur limit (slip_vel.cpp:283-288, 351-477)

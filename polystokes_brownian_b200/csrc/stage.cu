@@ -647,18 +647,25 @@ __global__ void k_assemble(int R, const Seg *__restrict__ segs, const double *__
 // ---------------------------------------------------------------------------
 // Arrowhead Schur floor (slip_vel.cpp:81-203), one block per shell replica:
 // S = Mcc_base - beta Mcm Mcm^T, eig, delta_j = max(0.1 - lambda_j, 0),
-// Delta = Q diag(delta) Q^T; Mcc_base holds the colloid self blocks plus the
-// colloid-colloid pair blocks (those the reference's shell cannot store).
-// Symmetric eigendecomposition by parallel-ordered Jacobi in shared memory.
+// Delta = Q diag(delta) Q^T, and the symmetric root of the floored S for the
+// noise; Mcc_base holds the colloid self blocks plus the colloid-colloid pair
+// blocks (those the reference's shell cannot store).
 //
-// Bound: latency (one block per replica, n <= 64).  The pair blocks of Mcm are
+// Bound: latency (one block per replica, n <= 55).  The pair blocks of Mcm are
 // evaluated once per (monomer, colloid), a chunk of monomers at a time in shared
-// memory, and every thread then adds the chunk to its Gram entries; a Jacobi
-// sweep is n - 1 rounds of n / 2 disjoint rotations.  220 monomers and 2
-// colloids (n = 22): 2090 us with the blocks re-evaluated for every Gram entry and
-// one rotation at a time, 147 us now.
+// memory, and summed into the Gram matrix by FP64 matrix instructions.  Where
+// S - 0.1 has positive pivots no eigenvalue is floored, Delta is zero and the
+// root comes from about seven Newton-Schulz iterations, three small products each;
+// otherwise from the eigenvectors, by parallel-ordered Jacobi, six sweeps of
+// n - 1 rounds with FP32 tangents.  220 monomers and 2 colloids (n = 22): 2000 us with
+// the blocks re-evaluated for every Gram entry and one rotation at a time, 147 us with
+// parallel rotations; now 22 us (Gram 8, pivots 4, root 8) with the floor inactive and
+// 104 us with it active; 5 colloids (n = 55) 72 and 719 us (1060 and 1020 by Jacobi with
+// FP64 tangents).
 constexpr int SCHUR_THREADS = 512;
-constexpr int SCHUR_BUF = 12288;      // doubles of the monomer chunk: 3 n per monomer
+constexpr int SCHUR_BUF = 20480;      // doubles of the monomer chunk: 3 n per monomer
+constexpr double SCHUR_FLOOR = 0.1;   // smallest eigenvalue kept
+constexpr double SCHUR_NORM = 100.0;  // row-sum norm up to which the root is iterated (a condition of 1000)
 
 // One sweep runs the round-robin schedule: with m = n rounded up to even, round t pairs
 // (m - 1, t) and ((t + k) mod (m - 1), (t - k) mod (m - 1)), k = 1 .. m/2 - 1; a pair that
@@ -676,21 +683,43 @@ __device__ __forceinline__ void jacobi_pair(int m, int t, int k, int &p, int &q)
     q = a < b ? b : a;
 }
 
+// The rotation that annihilates A[p][q]: its tangent in FP32, where a relative error of 1e-7 only
+// leaves 1e-7 of the entry for the next sweep, its cosine 1 / sqrt(1 + t^2) in FP64 (a
+// reciprocal-square-root estimate and one third-order step), so that c^2 + s^2 = 1 to rounding.
+// scale: one over the Frobenius norm; entries below 1e-18 of it are left (the sweeps end at 1e-15).
+__device__ __forceinline__ void jacobi_rot(const double *__restrict__ A, int n, int p, int q, double scale, double &c,
+                                           double &sn)
+{
+    c = 1.0; sn = 0.0;
+    if (q >= n) return;
+    // tan: 2 apq / (h +- sqrt(h^2 + 4 apq^2)), h = aqq - app
+    const float g = (float)(2.0 * A[p * n + q] * scale), h = (float)((A[q * n + q] - A[p * n + p]) * scale);
+    if (!(fabsf(g) > 2e-18f)) return;
+    const float x = fmaf(h, h, g * g);
+    const double t = __fdividef(h >= 0 ? g : -g, fabsf(h) + x * rsqrtf(x));
+    const double w = fma(t, t, 1.0), y = rsqrtf((float)w), e = fma(-(w * y), y, 1.0);
+    c = fma(y * e, fma(0.375, e, 0.5), y);
+    sn = t * c;
+}
+
+// A, Q: n x n row-major in shared memory, row j of Q the j-th vector; all threads of the block take
+// part.  Blocks of A go to the threads from the first one on, pairs of Q's rows from the last one
+// on, so that they share no warp at small n.
 __device__ void block_jacobi_eig(double *A, double *Q, int n, double *lam)
 {
-    // A, Q: n x n row-major in shared memory; all threads of the block participate
-    __shared__ double rc[PS_MAX_NC11_SCHUR / 2], rs[PS_MAX_NC11_SCHUR / 2];
-    __shared__ double wsum[2][SCHUR_THREADS / 32];
+    __shared__ double wsum[2][SCHUR_THREADS / 32], rc[PS_MAX_NC11_SCHUR / 2], rs[PS_MAX_NC11_SCHUR / 2];
     const int tid = threadIdx.x, lane = tid & 31, wid = tid >> 5;
-    const int m = (n + 1) & ~1, np = m / 2;
-    for (int k = tid; k < n * n; k += blockDim.x) Q[k] = (k / n == k % n) ? 1.0 : 0.0;
-    __syncthreads();
+    const int m = (n + 1) & ~1, np = m / 2, qid = SCHUR_THREADS - 1 - tid;
+    const int a_k1 = tid / np, a_k2 = tid % np, a_d1 = SCHUR_THREADS / np, a_d2 = SCHUR_THREADS % np;
+    const int q_k = qid / n, q_row = qid % n, q_dk = SCHUR_THREADS / n, q_dr = SCHUR_THREADS % n;
+    for (int k = tid; k < n * n; k += SCHUR_THREADS) Q[k] = k % (n + 1) == 0 ? 1.0 : 0.0;
     for (int sweep = 0; sweep < 60; sweep++) {
+        __syncthreads();
         double off = 0.0, tot = 0.0;
-        for (int k = tid; k < n * n; k += blockDim.x) {
+        for (int k = tid; k < n * n; k += SCHUR_THREADS) {
             const double v = A[k] * A[k];
             tot += v;
-            if (k / n != k % n) off += v;
+            if (k % (n + 1) != 0) off += v;
         }
         for (int o = 16; o > 0; o >>= 1) {
             off += __shfl_xor_sync(0xffffffffu, off, o);
@@ -699,59 +728,172 @@ __device__ void block_jacobi_eig(double *A, double *Q, int n, double *lam)
         if (lane == 0) { wsum[0][wid] = off; wsum[1][wid] = tot; }
         __syncthreads();
         off = 0.0; tot = 0.0;
-        for (int w = 0; w < (int)(blockDim.x >> 5); w++) { off += wsum[0][w]; tot += wsum[1][w]; }
+        for (int w = 0; w < SCHUR_THREADS / 32; w++) { off += wsum[0][w]; tot += wsum[1][w]; }
         if (off <= 1e-30 * tot || off == 0.0) break;      // the same sums in every thread
+        const double scale = rsqrt(tot);
         for (int t = 0; t < m - 1; t++) {
+            if (t) __syncthreads();
             if (tid < np) {
                 int p, q;
                 jacobi_pair(m, t, tid, p, q);
-                double c = 1.0, sn = 0.0;
+                jacobi_rot(A, n, p, q, scale, rc[tid], rs[tid]);
+            }
+            __syncthreads();
+            for (int k1 = a_k1, k2 = a_k2; k1 < np;) {
+                // block of row pair k1 and column pair k2: B <- J1^T B J2
+                int p1, q1, p2, q2;
+                jacobi_pair(m, t, k1, p1, q1);
+                jacobi_pair(m, t, k2, p2, q2);
+                const double c1 = rc[k1], s1 = rs[k1], c2 = rc[k2], s2 = rs[k2];
+                const bool h1 = q1 < n, h2 = q2 < n;
+                const double app = A[p1 * n + p2], apq = h2 ? A[p1 * n + q2] : 0.0;
+                const double aqp = h1 ? A[q1 * n + p2] : 0.0, aqq = h1 && h2 ? A[q1 * n + q2] : 0.0;
+                const double bpp = c2 * app - s2 * apq, bpq = s2 * app + c2 * apq;
+                const double bqp = c2 * aqp - s2 * aqq, bqq = s2 * aqp + c2 * aqq;
+                A[p1 * n + p2] = c1 * bpp - s1 * bqp;
+                if (h2) A[p1 * n + q2] = c1 * bpq - s1 * bqq;
+                if (h1) A[q1 * n + p2] = s1 * bpp + c1 * bqp;
+                if (h1 && h2) A[q1 * n + q2] = s1 * bpq + c1 * bqq;
+                k1 += a_d1; k2 += a_d2;
+                if (k2 >= np) { k2 -= np; k1++; }
+            }
+            for (int k = q_k, row = q_row; k < np;) {
+                int p, q;
+                jacobi_pair(m, t, k, p, q);
                 if (q < n) {
-                    const double apq = A[p * n + q];
-                    if (fabs(apq) >= 1e-300) {
-                        // tan of the rotation: 2 apq / (h +- sqrt(h^2 + 4 apq^2)), h = aqq - app
-                        const double h = A[q * n + q] - A[p * n + p], g = 2 * apq;
-                        const double tn = (h >= 0 ? g : -g) / (fabs(h) + sqrt(h * h + g * g));
-                        c = rsqrt(tn * tn + 1);
-                        sn = tn * c;
-                    }
+                    const double c = rc[k], sn = rs[k], qp = Q[p * n + row], qq = Q[q * n + row];
+                    Q[p * n + row] = c * qp - sn * qq;
+                    Q[q * n + row] = sn * qp + c * qq;
                 }
-                rc[tid] = c; rs[tid] = sn;
+                k += q_dk; row += q_dr;
+                if (row >= n) { row -= n; k++; }
             }
-            __syncthreads();
-            for (int w = tid; w < np * np + np * n; w += blockDim.x) {
-                if (w < np * np) {
-                    // block of row pair k1 and column pair k2: B <- J1^T B J2
-                    const int k1 = w / np, k2 = w % np;
-                    int p1, q1, p2, q2;
-                    jacobi_pair(m, t, k1, p1, q1);
-                    jacobi_pair(m, t, k2, p2, q2);
-                    const double c1 = rc[k1], s1 = rs[k1], c2 = rc[k2], s2 = rs[k2];
-                    const bool h1 = q1 < n, h2 = q2 < n;
-                    double app = A[p1 * n + p2], apq = h2 ? A[p1 * n + q2] : 0.0;
-                    double aqp = h1 ? A[q1 * n + p2] : 0.0, aqq = h1 && h2 ? A[q1 * n + q2] : 0.0;
-                    const double bpp = c2 * app - s2 * apq, bpq = s2 * app + c2 * apq;
-                    const double bqp = c2 * aqp - s2 * aqq, bqq = s2 * aqp + c2 * aqq;
-                    A[p1 * n + p2] = c1 * bpp - s1 * bqp;
-                    if (h2) A[p1 * n + q2] = c1 * bpq - s1 * bqq;
-                    if (h1) A[q1 * n + p2] = s1 * bpp + c1 * bqp;
-                    if (h1 && h2) A[q1 * n + q2] = s1 * bpq + c1 * bqq;
-                } else {
-                    const int v = w - np * np, k = v / n, row = v % n;
-                    int p, q;
-                    jacobi_pair(m, t, k, p, q);
-                    if (q < n) {
-                        const double c = rc[k], sn = rs[k], qp = Q[row * n + p], qq = Q[row * n + q];
-                        Q[row * n + p] = c * qp - sn * qq;
-                        Q[row * n + q] = sn * qp + c * qq;
-                    }
-                }
-            }
-            __syncthreads();
         }
     }
-    for (int i = tid; i < n; i += blockDim.x) lam[i] = A[i * n + i];
+    for (int i = tid; i < n; i += SCHUR_THREADS) lam[i] = A[i * n + i];
     __syncthreads();
+}
+
+// C += A B of 8 x 8 tiles over four of the inner index, FP64 matrix instruction: lane l holds
+// A[l / 4][l % 4], B[l % 4][l / 4] and C[l / 4][2 (l % 4) + 0, 1]
+__device__ __forceinline__ void dmma(double (&c)[2], double a, double b)
+{
+    asm volatile("mma.sync.aligned.m8n8k4.row.col.f64.f64.f64.f64 {%0, %1}, {%2}, {%3}, {%0, %1};"
+                 : "+d"(c[0]), "+d"(c[1]) : "d"(a), "d"(b));
+}
+
+// Matrices for dmma lie in shared memory with rows of ld, an odd multiple of 8: four rows of eight
+// doubles then meet every bank twice.  Tiles: the upper triangle of SCHUR_NT x SCHUR_NT at most.
+constexpr int SCHUR_NT = PS_MAX_NC11_SCHUR / 8, SCHUR_WARPS = SCHUR_THREADS / 32;
+constexpr int SCHUR_TILES = SCHUR_NT * (SCHUR_NT + 1) / 2;
+__host__ __device__ constexpr int schur_ld(int n) { return 8 * (((n + 7) / 8) | 1); }
+static_assert(schur_ld(PS_MAX_NC11_SCHUR / 11 * 11) <= PS_MAX_NC11_SCHUR, "orders are multiples of 11");
+
+// tile (I, J) of X^T Y over rows k0, k0 + kd, .. below k1, multiples of 4 (X = Y: the Gram matrix; X symmetric: the
+// product X Y), two sums in turn
+__device__ __forceinline__ void tile_mul(const double *X, const double *Y, int ld, int I, int J, int k0, int kd, int k1,
+                                         double (&c)[2])
+{
+    const int lane = threadIdx.x & 31;
+    const double *x = X + (lane & 3) * ld + 8 * I + (lane >> 2), *y = Y + (lane & 3) * ld + 8 * J + (lane >> 2);
+    double e[2] = {0.0, 0.0};
+    int k = k0;
+    for (; k + kd < k1; k += 2 * kd) {
+        dmma(c, x[k * ld], y[k * ld]);
+        dmma(e, x[(k + kd) * ld], y[(k + kd) * ld]);
+    }
+    if (k < k1) dmma(c, x[k * ld], y[k * ld]);
+    c[0] += e[0]; c[1] += e[1];
+}
+
+// S - floor 1 > 0, by its pivots, two columns at a time; W: n x n scratch.  All threads take part
+// and agree.
+__device__ bool block_above(const double *__restrict__ S, double *__restrict__ W, int n, double floor_)
+{
+    const int tid = threadIdx.x, i0 = tid / n, j0 = tid % n, di = SCHUR_THREADS / n, dj = SCHUR_THREADS % n;
+    for (int k = tid; k < n * n; k += SCHUR_THREADS) W[k] = S[k] - (k % (n + 1) == 0 ? floor_ : 0.0);
+    for (int k = 0; k < n; k += 2) {
+        __syncthreads();
+        const double a = W[k * n + k];
+        if (!(a > 0.0)) return false;
+        if (k + 1 == n) break;
+        const double b = W[(k + 1) * n + k], c = W[(k + 1) * n + k + 1], det = fma(a, c, -b * b);
+        if (!(det > 0.0)) return false;
+        const double inv = 1.0 / det;
+        for (int i = i0, j = j0; i < n;) {
+            if (j > k + 1 && i >= j) {
+                const double u0 = W[i * n + k], u1 = W[i * n + k + 1], v0 = W[j * n + k], v1 = W[j * n + k + 1];
+                W[i * n + j] -= (u0 * (c * v0 - b * v1) + u1 * (a * v1 - b * v0)) * inv;
+            }
+            i += di; j += dj;
+            if (j >= n) { j -= n; i++; }
+        }
+    }
+    return true;
+}
+
+// Upper tiles of the products of commuting symmetric matrices (offsets in shared memory), one warp
+// each, mirrored: one product (A0 B0) or, side by side, two.  POLY: C = (3 - A0 B0) / 2;
+// returns whether any entry of 1 - A0 B0 (of the n x n part) is above 1e-9.
+template <bool POLY>
+__device__ __forceinline__ bool sym_mul(int A0, int B0, int C0, int A1, int B1, int C1, const uchar2 *tiles, int ntile,
+                                        int n, int ld)
+{
+    extern __shared__ __align__(16) double sm[];
+    bool big = false;
+    const int lane = threadIdx.x & 31;
+    for (int t = threadIdx.x >> 5; t < (POLY ? 1 : 2) * ntile; t += SCHUR_WARPS) {
+        const bool second = !POLY && t >= ntile;
+        double *C = sm + (second ? C1 : C0);
+        const uchar2 tt = tiles[second ? t - ntile : t];
+        double v[2] = {0.0, 0.0};
+        tile_mul(sm + (second ? A1 : A0), sm + (second ? B1 : B0), ld, tt.x, tt.y, 0, 4, (n + 3) & ~3, v);
+        const int r = 8 * tt.x + (lane >> 2), c0 = 8 * tt.y + 2 * (lane & 3);
+#pragma unroll
+        for (int e = 0; e < 2; e++) {
+            const int c = c0 + e;
+            if (r > c) continue;
+            double o = v[e];
+            if (POLY) {
+                const double one = r == c;
+                if (c < n) big = big || !(fabs(one - o) <= 1e-9);
+                o = 0.5 * (3.0 * one - o);
+            }
+            C[r * ld + c] = o;
+            C[c * ld + r] = o;
+        }
+    }
+    return big;
+}
+
+// S^(1/2) of a symmetric S with eigenvalues in [floor, norm], floor > 0: the coupled Newton-Schulz iteration
+// (Higham, Functions of Matrices, section 6.3), Y <- Y T, Z <- T Z, T = (3 - Z Y) / 2, from Y = S / c,
+// Z = 1, every factor a polynomial of S and so symmetric.  c = norm / 1.9 keeps S / c below 2, where it
+// converges.  The step that leaves |1 - Z Y| at 1e-9 squares it.  S is the first of five buffers of
+// 64 x 64 in shared memory, all used up; returns the one that holds Y, rows of ld.
+__device__ const double *block_sqrt(const uchar2 *tiles, int ntile, int n, int ld, double norm, double &scale)
+{
+    extern __shared__ __align__(16) double sm[];
+    constexpr int MB = PS_MAX_NC11_SCHUR * PS_MAX_NC11_SCHUR;
+    const double c = norm * (1.0 / 1.9), ic = 1.0 / c;
+    scale = sqrt(c);
+    int Y = MB, Z = 2 * MB, Y2 = 3 * MB, Z2 = 0;
+    constexpr int P = 4 * MB;
+    for (int k = threadIdx.x; k < ld * ld; k += SCHUR_THREADS) {
+        const int i = k / ld, j = k % ld;
+        sm[Y + k] = i < n && j < n ? sm[i * n + j] * ic : 0.0;
+        sm[Z + k] = i == j && i < n ? 1.0 : 0.0;
+    }
+    __syncthreads();
+    for (int it = 0; it < 60; it++) {
+        const bool more = __syncthreads_or(sym_mul<true>(Z, Y, P, 0, 0, 0, tiles, ntile, n, ld));
+        sym_mul<false>(Y, P, Y2, P, Z, Z2, tiles, ntile, n, ld);
+        __syncthreads();
+        int o = Y; Y = Y2; Y2 = o;
+        o = Z; Z = Z2; Z2 = o;
+        if (!more) break;
+    }
+    return sm + Y;
 }
 
 // the 3 x 11 block of Mcm between monomer m and colloid c, columns by colloid component:
@@ -782,15 +924,16 @@ __device__ __forceinline__ void mcm_block(const Seg &s, const double *__restrict
 
 __global__ void __launch_bounds__(SCHUR_THREADS)
 k_schur(const Seg *__restrict__ segs, const int *__restrict__ reps, const double *__restrict__ x,
-        double *__restrict__ delta, double *__restrict__ schurQ, double *__restrict__ schurL,
-        const double *__restrict__ tab)
+        double *__restrict__ delta, double *__restrict__ schurR)
 {
     pdl_enter();
-    extern __shared__ double sm[];
+    extern __shared__ __align__(16) double sm[];
+    __shared__ uchar2 tiles[SCHUR_TILES];
     const int r = reps[blockIdx.x];
     const Seg &s = segs[r];
     const int n = s.nc11, Nm = s.Nm, Nc = s.Nc;
-    double *S = sm, *Q = sm + n * n, *lam = sm + 2 * n * n, *buf = sm + 2 * 64 * 64 + 64;
+    constexpr int MB = PS_MAX_NC11_SCHUR * PS_MAX_NC11_SCHUR;
+    double *S = sm, *Q = sm + MB, *buf = sm + 2 * MB, *lam = buf + SCHUR_BUF;
     // Mcc_base: self + BB pairs, built by applying the pair operator to unit vectors
     for (int k = threadIdx.x; k < n * n; k += blockDim.x) S[k] = 0.0;
     __syncthreads();
@@ -818,49 +961,73 @@ k_schur(const Seg *__restrict__ segs, const int *__restrict__ reps, const double
             S[rowi * n + colj] += out[k];
         }
     }
-    // Gram of Mcm over chunks of monomers; Q holds the upper triangle's sums meanwhile, each
-    // entry added to by one thread in monomer order
-    for (int w = threadIdx.x; w < n * n; w += blockDim.x) Q[w] = 0.0;
-    const int mch = SCHUR_BUF / (3 * n);
+    // Gram of Mcm over chunks of monomers, rows (monomer, axis): upper tiles, each by ng warps that take
+    // every ng-th group of four rows and keep their sums in Q's place (what the columns from n on
+    // hold goes to entries from n on alone, which nothing reads)
+    const int nt = (n + 7) / 8, ntile = nt * (nt + 1) / 2, ng = max(1, SCHUR_WARPS / ntile), ld = schur_ld(n);
+    const int lane = threadIdx.x & 31;
+    for (int w = threadIdx.x; w < 64 * ntile * ng; w += SCHUR_THREADS) Q[w] = 0.0;
+    if (threadIdx.x < nt)
+        for (int ta = threadIdx.x, tc = ta; tc < nt; tc++) tiles[ta * nt - ta * (ta - 1) / 2 + tc - ta] = make_uchar2(ta, tc);
+    const int mch = (SCHUR_BUF / ld - 3) / 3;
     for (int m0 = 0; m0 < Nm; m0 += mch) {
-        const int nm = min(mch, Nm - m0);
+        const int nm = min(mch, Nm - m0), rows = (3 * nm + 3) & ~3;
         __syncthreads();
-        for (int w = threadIdx.x; w < nm * Nc; w += blockDim.x) mcm_block(s, x, m0 + w / Nc, w % Nc, buf + 3 * n * (w / Nc), n);
+        for (int w = threadIdx.x; w < nm * Nc; w += SCHUR_THREADS) mcm_block(s, x, m0 + w / Nc, w % Nc, buf + 3 * ld * (w / Nc), ld);
+        for (int w = 3 * nm * ld + threadIdx.x; w < rows * ld; w += SCHUR_THREADS) buf[w] = 0.0;
         __syncthreads();
-        for (int w = threadIdx.x; w < n * n; w += blockDim.x) {
-            const int a = w / n, c = w % n;
-            if (c < a) continue;
-            double acc = Q[w];
-            for (int m = 0; m < nm; m++) {
-                const double *b = buf + 3 * n * m;
-                acc += b[a] * b[c] + b[n + a] * b[n + c] + b[2 * n + a] * b[2 * n + c];
-            }
-            Q[w] = acc;
+        for (int w = threadIdx.x >> 5; w < ntile * ng; w += SCHUR_WARPS) {
+            const uchar2 t = tiles[w % ntile];
+            double *q = Q + 64 * w + 2 * lane;
+            double v[2] = {q[0], q[1]};
+            tile_mul(buf, buf, ld, t.x, t.y, 4 * (w / ntile), 4 * ng, rows, v);
+            q[0] = v[0]; q[1] = v[1];
         }
     }
     __syncthreads();
-    for (int w = threadIdx.x; w < n * n; w += blockDim.x) {
-        const int a = w / n, c = w % n;
-        if (c < a) continue;
-        S[w] -= s.beta * Q[w];
-        if (c != a) S[c * n + a] -= s.beta * Q[w];
+    for (int w = threadIdx.x; w < 64 * ntile; w += SCHUR_THREADS) {
+        const uchar2 t = tiles[w >> 6];
+        const int a = 8 * t.x + ((w & 63) >> 3), c = 8 * t.y + (w & 7);
+        if (c < a || c >= n) continue;
+        double g = 0.0;
+        for (int k = 0; k < ng; k++) g += Q[64 * ntile * k + w];
+        S[a * n + c] -= s.beta * g;
+        if (c != a) S[c * n + a] -= s.beta * g;
     }
     __syncthreads();
+    // the floor's correction and the root of the floored complement
+    if (threadIdx.x < 64) {
+        double v = 0.0;
+        if (threadIdx.x < n)
+            for (int k = 0; k < n; k++) v += fabs(S[k * n + threadIdx.x]);
+        for (int o = 16; o > 0; o >>= 1) v = fmax(v, __shfl_xor_sync(0xffffffffu, v, o));
+        if (threadIdx.x % 32 == 0) lam[threadIdx.x / 32] = v;
+    }
+    double *D = delta + s.schur_off, *R = schurR + s.schur_off;
+    const bool above = block_above(S, buf, n, SCHUR_FLOOR);       // (its first barrier is lam's, too)
+    const double norm = fmax(lam[0], lam[1]);
+    __syncthreads();
+    if (above && norm <= SCHUR_NORM) {
+        double f;
+        const double *Y = block_sqrt(tiles, ntile, n, ld, norm, f);
+        for (int w = threadIdx.x; w < n * n; w += SCHUR_THREADS) {
+            D[w] = 0.0;
+            R[w] = f * Y[(w / n) * ld + w % n];
+        }
+        return;
+    }
     block_jacobi_eig(S, Q, n, lam);
-    double *D = delta + s.schur_off, *QQ = schurQ + s.schur_off, *LL = schurL + s.schur_off;
-    for (int w = threadIdx.x; w < n * n; w += blockDim.x) {
-        int a = w / n, bcol = w % n;
-        double corr = 0.0;
+    for (int w = threadIdx.x; w < n * n; w += SCHUR_THREADS) {
+        const int a = w / n, c = w % n;
+        double corr = 0.0, root = 0.0;
         for (int j = 0; j < n; j++) {
-            double d = lam[j] < 0.1 ? 0.1 - lam[j] : 0.0;
-            if (d == 0.0) continue;
-            corr += Q[a * n + j] * d * Q[bcol * n + j];
+            const double l = lam[j], q = Q[j * n + a] * Q[j * n + c];
+            if (l < SCHUR_FLOOR) corr += q * (SCHUR_FLOOR - l);
+            root += q * sqrt(l < SCHUR_FLOOR ? SCHUR_FLOOR : l);
         }
         D[w] = corr;
-        QQ[w] = Q[w];
+        R[w] = root;
     }
-    for (int j = threadIdx.x; j < n; j += blockDim.x) LL[j] = lam[j] < 0.1 ? 0.1 : lam[j];
-    (void)tab;
 }
 
 int stage_assemble(Engine &E, cudaStream_t st)
@@ -875,8 +1042,7 @@ int stage_schur(Engine &E, cudaStream_t st)
     if (!E.n_schur_reps) return PS_OK;
     size_t smem = sizeof(double) * (2 * 64 * 64 + 64 + SCHUR_BUF);
     PS_CK(cudaFuncSetAttribute(k_schur, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-    ps_launch(k_schur, E.n_schur_reps, SCHUR_THREADS, smem, st, E.d_segs, E.d_schur_reps, E.d_x, E.d_delta, E.d_schurQ, E.d_schurL,
-            E.d_tab);
+    ps_launch(k_schur, E.n_schur_reps, SCHUR_THREADS, smem, st, E.d_segs, E.d_schur_reps, E.d_x, E.d_delta, E.d_schurR);
     PS_CK(cudaGetLastError());
     return PS_OK;
 }

@@ -39,26 +39,19 @@ __global__ void k_zero_colloid_dofs(long ntop, const int *__restrict__ top_offs,
 }
 
 __global__ void k_shell_noise(const Seg *__restrict__ segs, const int *__restrict__ reps, const double *__restrict__ fb,
-                              const double *__restrict__ ymcm, const double *__restrict__ schurQ,
-                              const double *__restrict__ schurL, double *__restrict__ W)
+                              const double *__restrict__ ymcm, const double *__restrict__ schurR,
+                              double *__restrict__ W)
 {
     pdl_enter();
-    __shared__ double yv[PS_MAX_NC11_SCHUR];
     const int r = reps[blockIdx.x];
     const Seg &s = segs[r];
     const int n = s.nc11;
-    const double *Q = schurQ + s.schur_off, *L = schurL + s.schur_off;
+    const double *root = schurR + s.schur_off;
     const double *fc = fb + s.top_off + s.nm3;
     for (int i = threadIdx.x; i < s.nm3; i += blockDim.x) W[s.top_off + i] = sqrt(s.beta_inv) * fb[s.top_off + i];
-    for (int j = threadIdx.x; j < n; j += blockDim.x) {
-        double acc = 0.0;
-        for (int i = 0; i < n; i++) acc += Q[i * n + j] * fc[i];
-        yv[j] = sqrt(L[j]) * acc;
-    }
-    __syncthreads();
     for (int i = threadIdx.x; i < n; i += blockDim.x) {
         double acc = 0.0;
-        for (int j = 0; j < n; j++) acc += Q[i * n + j] * yv[j];
+        for (int j = 0; j < n; j++) acc += root[j * n + i] * fc[j];      // symmetric
         W[s.top_off + s.nm3 + i] = ymcm[s.top_off + s.nm3 + i] * sqrt(s.beta) + acc;
     }
 }
@@ -77,7 +70,7 @@ int slip_noise(Engine &E, const double *fb, double *W, const ps_sqrt_opts *o, ps
         apply_operator(E, 1, E.d_tmp_top, E.d_tmp_top2, false, st);
         if (E.n_schur_reps)
             ps_launch(k_shell_noise, E.n_schur_reps, 128, 0, st, E.d_segs, E.d_schur_reps, fb, E.d_tmp_top2,
-                    E.d_schurQ, E.d_schurL, W);
+                    E.d_schurR, W);
         if (E.n_sl_reps) {
             // above the dense Schur limit: Lanczos on the colloid Schur complement
             int nneg = 0;
