@@ -250,8 +250,8 @@ struct LzScal {
 // passes of classical Gram-Schmidt.  One thread owns one entry of the replica's
 // vector, in sub-blocks of 256 entries (a quarter of a reduction-table block).
 // The combine that forms q also forms the first pass's dots (k_combine), then
-// k_lz_sub_dots subtracts and forms the second pass's dots, k_lz_sub_norm
-// subtracts and forms the norm, k_lz_next tests for breakdown and scales.  Each
+// k_lz_sub_dots subtracts and forms the second pass's dots and the norm, and
+// k_lz_sub_scale subtracts, tests for breakdown and scales.  Each
 // kernel leaves its sub-blocks' sums in memory, and every block of the next one
 // adds its replica's sums itself, in a fixed order that depends on the vector's
 // length alone -- no counters and no fences, and a replica's noise does not depend
@@ -261,9 +261,10 @@ struct LzScal {
 // Bound: latency and L2 (the basis is read twice from L2 and once from L1 per
 // vector, k_lz_sub_dots reading its slices twice).  With 1024 entries per block of
 // 256 threads, or one cluster of eight blocks per replica, too few loads were in
-// flight: a vector with its apply took 42 us at 1024 beads (27 now), 72 us at the
-// 4097-bead brush (52 now), and the four sweeps of 64 replicas, 62000 beads, 100 us
-// (50 now).
+// flight: a vector with its apply took 42 us at 1024 beads (25 now), 72 us at the
+// 4097-bead brush (50 now), and the four sweeps of 64 replicas, 62000 beads, 100 us
+// (three, 37 us, now).  Taking the norm with the second dots instead of in a launch of its
+// own is 2 us of these.
 constexpr int LZ_SUB = RB_THREADS;                    // entries of a sub-block
 constexpr int LZC_CTAS = 8, LZC_HALVES = 2, LZC_THREADS = RB_THREADS * LZC_HALVES, LZC_SLOTS = 4;
 constexpr int LZC_VB = LZC_CTAS * LZC_HALVES;         // virtual RB-table blocks per cluster
@@ -278,21 +279,31 @@ __device__ __host__ __forceinline__ bool lz_fixed(const Seg &s)
 }
 static_assert(RB_SPAN == RB_EPT * LZ_SUB, "RB_EPT sub-blocks per table block");
 
-// the replica's total of the sub-block sums part[][i], i <= j, into h[] (shared)
+// the replica's total of the sub-block sums part[][i], i <= j, into h[] (shared); NORM: that of
+// npart[] into h[LZ_KMAX]
+template <bool NORM>
 __device__ __forceinline__ void lz_total(const RedTable &T, const RBlk &B, const Seg &s, const double *__restrict__ part,
-                                         int j, double *__restrict__ h)
+                                         const double *__restrict__ npart, int j, double *__restrict__ h)
 {
     __shared__ double sh4[RB_THREADS / LZ_KMAX][LZ_KMAX];
     constexpr int G = RB_THREADS / LZ_KMAX;
     const int i = threadIdx.x % LZ_KMAX, g = threadIdx.x / LZ_KMAX;
     const int nb = (s.nm3nc11 + LZ_SUB - 1) / LZ_SUB;
-    const double *p = part + (long)RB_EPT * T.d_first[B.rep] * LZ_KMAX + i;
-    double t = 0.0;
+    const long first = (long)RB_EPT * T.d_first[B.rep];
+    const double *p = part + first * LZ_KMAX + i;
+    double t = 0.0, n2 = 0.0;
+    const bool norm = NORM && threadIdx.x >= RB_THREADS - 32;      // the warp whose dots come last
+    if (norm)
+        for (int b = threadIdx.x & 31; b < nb; b += 32) n2 += npart[first + b];
     if (i <= j) {
 #pragma unroll 4
         for (int b = g; b < nb; b += G) t += p[(long)b * LZ_KMAX];
     }
     sh4[g][i] = t;
+    if (norm) {
+        for (int o = 16; o > 0; o >>= 1) n2 += __shfl_xor_sync(0xffffffffu, n2, o);
+        if (threadIdx.x == RB_THREADS - 1) h[LZ_KMAX] = n2;
+    }
     __syncthreads();
     if (threadIdx.x <= j) {
         double v = 0.0;
@@ -302,25 +313,30 @@ __device__ __forceinline__ void lz_total(const RedTable &T, const RBlk &B, const
     __syncthreads();
 }
 
-// q -= sum_i h_i V_i for this thread's entry, i = 0..j in order
+// q -= sum_i h_i V_i for this thread's entry, in four interleaved sums
 __device__ __forceinline__ double lz_subtract(const double *__restrict__ V, long ldv, long k, double q, int j,
                                               const double *__restrict__ h)
 {
-#pragma unroll 8
-    for (int i = 0; i <= j; i++) q -= h[i] * V[(long)i * ldv + k];
-    return q;
+    double t[4] = {0.0, 0.0, 0.0, 0.0};
+#pragma unroll 2
+    for (int i = 0; i <= j; i += 4)
+#pragma unroll
+        for (int c = 0; c < 4; c++)
+            if (i + c <= j) t[c] += h[i + c] * V[(long)(i + c) * ldv + k];
+    return q - ((t[0] + t[1]) + (t[2] + t[3]));
 }
 
 __global__ void k_lz_sub_dots(RedTable T, const Seg *__restrict__ segs, const double *__restrict__ V, long ldv,
                               double *__restrict__ q, int j, const LzScal *__restrict__ lz,
-                              const double *__restrict__ part1, double *__restrict__ alpha, double *__restrict__ part2)
+                              const double *__restrict__ part1, double *__restrict__ alpha, double *__restrict__ part2,
+                              double *__restrict__ npart)
 {
     pdl_enter();
     const RBlk B = T.d_blk[blockIdx.x];
     const int e = blockIdx.y * LZ_SUB + threadIdx.x;
     if (blockIdx.y * LZ_SUB >= B.len || lz[B.rep].done || lz_fixed(segs[B.rep])) return;
-    __shared__ double h[LZ_KMAX];
-    lz_total(T, B, segs[B.rep], part1, j, h);
+    __shared__ double h[LZ_KMAX], wn[RB_THREADS / 32];
+    lz_total<false>(T, B, segs[B.rep], part1, nullptr, j, h);
     const bool act = e < B.len;
     const long k = (long)B.start + e;
     double v = 0.0;
@@ -329,59 +345,47 @@ __global__ void k_lz_sub_dots(RedTable T, const Seg *__restrict__ segs, const do
         q[k] = v;
     }
     if (threadIdx.x == 0 && blockIdx.y == 0 && (int)blockIdx.x == T.d_first[B.rep]) alpha[(long)LZ_KMAX * B.rep + j] = h[j];
-    lz_block_dots(V, ldv, k, act, v, j, part2 + (long)LZ_KMAX * (RB_EPT * blockIdx.x + blockIdx.y));
+    double n2 = v * v;
+    for (int o = 16; o > 0; o >>= 1) n2 += __shfl_xor_sync(0xffffffffu, n2, o);
+    if ((threadIdx.x & 31) == 0) wn[threadIdx.x >> 5] = n2;
+    lz_block_dots(V, ldv, k, act, v, j, part2 + (long)LZ_KMAX * (RB_EPT * blockIdx.x + blockIdx.y));   // a barrier inside
+    if (threadIdx.x == RB_THREADS - 1) {
+        n2 = 0.0;
+        for (int w = 0; w < RB_THREADS / 32; w++) n2 += wn[w];
+        npart[RB_EPT * blockIdx.x + blockIdx.y] = n2;
+    }
 }
 
-__global__ void k_lz_sub_norm(RedTable T, const Seg *__restrict__ segs, const double *__restrict__ V, long ldv,
-                              double *__restrict__ q, int j, const LzScal *__restrict__ lz,
-                              const double *__restrict__ part2, double *__restrict__ alpha, double *__restrict__ npart)
+// Second subtraction, beta_j = ||q||, V_{j+1} = q / beta_j, m = j + 1; an invariant subspace stops
+// the replica.  The norm after the subtraction is that before it less the dots' squares (the
+// basis is orthonormal), so no further sum over the replica, and no further launch, is needed: the
+// dots of a second pass are rounding residues of the first, and only at a breakdown not far
+// smaller than q.  (done may be set by the replica's first block while others still read it: they
+// find the same breakdown themselves and write nothing either way.)
+__global__ void k_lz_sub_scale(RedTable T, const Seg *__restrict__ segs, double *__restrict__ V, long ldv,
+                               const double *__restrict__ q, int j, int kmax, LzScal *__restrict__ lz,
+                               const double *__restrict__ part2, const double *__restrict__ npart,
+                               double *__restrict__ alpha, double *__restrict__ betad)
 {
     pdl_enter();
     const RBlk B = T.d_blk[blockIdx.x];
     const int e = blockIdx.y * LZ_SUB + threadIdx.x;
     if (blockIdx.y * LZ_SUB >= B.len || lz[B.rep].done || lz_fixed(segs[B.rep])) return;
-    __shared__ double h[LZ_KMAX], sh[RB_THREADS / 32][1];
-    lz_total(T, B, segs[B.rep], part2, j, h);
-    double v[1] = {0.0};
-    if (e < B.len) {
-        const long k = (long)B.start + e;
-        const double t = lz_subtract(V, ldv, k, q[k], j, h);
-        q[k] = t;
-        v[0] = t * t;
-    }
-    if (threadIdx.x == 0 && blockIdx.y == 0 && (int)blockIdx.x == T.d_first[B.rep]) alpha[(long)LZ_KMAX * B.rep + j] += h[j];
-    block_sum<1>(v, sh);
-    if (threadIdx.x == 0) npart[RB_EPT * blockIdx.x + blockIdx.y] = v[0];
-}
-
-// beta_j = ||q||, V_{j+1} = q / beta_j, m = j + 1; an invariant subspace stops the replica.
-// (done may be set by the replica's first block while others still read it: they find the
-// same breakdown themselves and write nothing either way.)
-__global__ void k_lz_next(RedTable T, const Seg *__restrict__ segs, double *__restrict__ V, long ldv,
-                          const double *__restrict__ q, int j, int kmax, LzScal *__restrict__ lz,
-                          const double *__restrict__ npart, double *__restrict__ betad)
-{
-    pdl_enter();
-    const RBlk B = T.d_blk[blockIdx.x];
-    const int e = blockIdx.y * LZ_SUB + threadIdx.x;
-    if (blockIdx.y * LZ_SUB >= B.len || lz[B.rep].done || lz_fixed(segs[B.rep])) return;
-    __shared__ double tot;
-    const int first = T.d_first[B.rep];
-    if (threadIdx.x < 32) {
-        const int nb = (segs[B.rep].nm3nc11 + LZ_SUB - 1) / LZ_SUB;
-        double t = 0.0;
-        for (int b = threadIdx.x; b < nb; b += 32) t += npart[RB_EPT * first + b];
-        for (int o = 16; o > 0; o >>= 1) t += __shfl_xor_sync(0xffffffffu, t, o);
-        if (threadIdx.x == 0) tot = t;
-    }
-    __syncthreads();
-    const double bj = sqrt(tot);
+    __shared__ double h[LZ_KMAX + 1];
+    lz_total<true>(T, B, segs[B.rep], part2, npart, j, h);
+    double h2[4] = {0.0, 0.0, 0.0, 0.0};
+    for (int i = 0; i <= j; i += 4)
+#pragma unroll
+        for (int c = 0; c < 4; c++)
+            if (i + c <= j) h2[c] += h[i + c] * h[i + c];
+    const double bj = sqrt(fmax(h[LZ_KMAX] - ((h2[0] + h2[1]) + (h2[2] + h2[3])), 0.0));
     const bool broken = bj <= 1e-12 * lz[B.rep].b0;
     if (!broken && j + 1 < kmax && e < B.len) {
         const long k = (long)B.start + e;
-        V[(long)(j + 1) * ldv + k] = q[k] * (bj > 0 ? 1.0 / bj : 0.0);
+        V[(long)(j + 1) * ldv + k] = lz_subtract(V, ldv, k, q[k], j, h) * (bj > 0 ? 1.0 / bj : 0.0);
     }
-    if (threadIdx.x == 0 && blockIdx.y == 0 && (int)blockIdx.x == first) {
+    if (threadIdx.x == 0 && blockIdx.y == 0 && (int)blockIdx.x == T.d_first[B.rep]) {
+        alpha[(long)LZ_KMAX * B.rep + j] += h[j];
         lz[B.rep].m = j + 1;
         if (broken) lz[B.rep].done = 2;             // finalise with m = j + 1
         else if (j + 1 < kmax) betad[(long)LZ_KMAX * B.rep + j] = bj;
@@ -1034,9 +1038,9 @@ int lanczos_sqrt(Engine &E, const double *z, double *w, const ps_sqrt_opts *o, p
         if (any_fixed)
             ps_launch(k_lz_orth_cluster, E.R * LZC_CTAS, LZC_THREADS, 0, st, E.d_segs, V, ldv, q, j, kmax, lz, alpha, betad);
         if (any_free) {
-            ps_launch(k_lz_sub_dots, sub, RB_THREADS, 0, st, T, E.d_segs, V, ldv, q, j, lz, part1, alpha, part2);
-            ps_launch(k_lz_sub_norm, sub, RB_THREADS, 0, st, T, E.d_segs, V, ldv, q, j, lz, part2, alpha, npart);
-            ps_launch(k_lz_next, sub, RB_THREADS, 0, st, T, E.d_segs, V, ldv, q, j, kmax, lz, npart, betad);
+            ps_launch(k_lz_sub_dots, sub, RB_THREADS, 0, st, T, E.d_segs, V, ldv, q, j, lz, part1, alpha, part2, npart);
+            ps_launch(k_lz_sub_scale, sub, RB_THREADS, 0, st, T, E.d_segs, V, ldv, q, j, kmax, lz, part2, npart, alpha,
+                    betad);
         }
         if ((j + 1) % check == 0 && j + 1 < kmax) {
             if (pending) {
