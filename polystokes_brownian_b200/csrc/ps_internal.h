@@ -35,8 +35,10 @@ constexpr unsigned PDL_EARLY = 148;
 #ifdef __CUDACC__
 __device__ __forceinline__ void pdl_enter()
 {
-    asm volatile("griddepcontrol.wait;" ::: "memory");
-    if (gridDim.x * gridDim.y <= PDL_EARLY) asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+    if (gridDim.x * gridDim.y <= PDL_EARLY)
+        asm volatile("griddepcontrol.wait;\n\tgriddepcontrol.launch_dependents;" ::: "memory");
+    else
+        asm volatile("griddepcontrol.wait;" ::: "memory");
 }
 #endif
 
