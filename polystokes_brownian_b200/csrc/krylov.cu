@@ -137,7 +137,8 @@ __global__ void k_mr_init(RedTable T, const Seg *segs, const double *__restrict_
 //
 // Bound: latency (a dependent launch with an L2 round trip takes some 4 us).  516 beads, one
 // iteration: 21.5 us with a launch for each half and last-block sums, 16.5 us without
-// them, 14.2 us with the first half in the combine.
+// them, 14.9 us with the first half in the combine, 14.2 us with the vectors' loads ahead of
+// the totals.
 __global__ void k_mr_beta(RedTable T, const Seg *__restrict__ segs, double *__restrict__ Av, const double *__restrict__ rk,
                           const double *__restrict__ D, double *__restrict__ z, MinresScal *__restrict__ st,
                           const double *__restrict__ pa, double *__restrict__ pb)
@@ -148,13 +149,16 @@ __global__ void k_mr_beta(RedTable T, const Seg *__restrict__ segs, double *__re
     if (blockIdx.y * RB_THREADS >= B.len || st[B.rep].done) return;
     __shared__ double sh[RB_THREADS / 32][1];
     const int first = T.d_first[B.rep];
+    const bool act = e < B.len;
+    const long q = (long)B.start + e;
+    // asked for ahead of the total
+    const double av = act ? Av[q] : 0.0, r = act ? rk[q] : 0.0, d = act ? D[q] : 1.0, bt = st[B.rep].beta;
     const double alfa = rep_total(pa + RB_EPT * first, (segs[B.rep].n + RB_THREADS - 1) / RB_THREADS);
     if (blockIdx.y == 0 && (int)blockIdx.x == first && threadIdx.x == 0) st[B.rep].alfa = alfa;
     double s[1] = {0.0};
-    if (e < B.len) {
-        const long q = (long)B.start + e;
-        const double a = Av[q] - (alfa / st[B.rep].beta) * rk[q];
-        const double zq = a / D[q];
+    if (act) {
+        const double a = av - (alfa / bt) * r;
+        const double zq = a / d;
         Av[q] = a;
         z[q] = zq;
         s[0] = a * zq;

@@ -115,6 +115,12 @@ __device__ __forceinline__ void mr_alpha(const RedTable &T, const RBlk &B, int n
     __shared__ double sh[RB_THREADS / 32][1];
     const int first = T.d_first[B.rep];
     const bool lead = blockIdx.y == 0 && (int)blockIdx.x == first && threadIdx.x == 0;
+    // everything that does not wait for the scalars is asked for ahead of them
+    double z = 0.0, v = 0.0, w1 = 0.0, w2 = 0.0, xq = 0.0, rm = 0.0;
+    if (act) {
+        z = A.z[q];
+        if (A.k > 1) { v = A.v[q]; w1 = A.w1[q]; w2 = A.w2[q]; xq = A.x[q]; rm = A.rkm1[q]; }
+    }
     const double bb = A.k > 1 ? rep_total(A.pb + RB_EPT * first, (n + RB_THREADS - 1) / RB_THREADS) : 0.0;
     if (threadIdx.x == 0) {
         MinresScal m = A.st0[B.rep];
@@ -130,14 +136,14 @@ __device__ __forceinline__ void mr_alpha(const RedTable &T, const RBlk &B, int n
     double s[1] = {0.0};
     if (act) {
         if (sm.pending) {
-            const double wn = (A.v[q] - sm.up_oldeps * A.w1[q] - sm.up_delta * A.w2[q]) * sm.up_ginv;
+            const double wn = (v - sm.up_oldeps * w1 - sm.up_delta * w2) * sm.up_ginv;
             A.wnew[q] = wn;
-            A.x[q] += sm.up_phi * wn;
+            A.x[q] = xq + sm.up_phi * wn;
         }
         if (!sm.done) {
-            const double vq = A.z[q] * sm.sinv;
+            const double vq = z * sm.sinv;
             double a = Az * sm.sinv;
-            if (A.k >= 2) a -= (sm.beta / sm.oldb) * A.rkm1[q];
+            if (A.k >= 2) a -= (sm.beta / sm.oldb) * rm;
             A.v[q] = vq;
             Av[q] = a;
             s[0] = vq * a;
