@@ -45,9 +45,9 @@ METRIC = "bead-steps/s"
 FLOP_AA = 40      # algorithmic FLOP per directed monomer-monomer pair (F-F RPY)
 FLOP_BB = 250     # per directed colloid-colloid FTS pair (contracted block action, mul and add each counted)
 # DRAM bytes (read + write) of one launch of the roofline kernel, from one ncu
-# capture on the bench workload (profiles/k_rpy_aa_f2_ensemble256_lub.md:
-# dram__bytes_read.sum 16.47 MB + dram__bytes_write.sum 12.61 MB, chunk width 256)
-NCU_TRAFFIC = {("ensemble256_lub", "k_rpy_aa_f2"): {"bytes": 29.08e6, "chunk_cols": 256}}
+# capture on the bench workload (profiles/k_rpy_aa_f2_tile_pairs_ensemble256_lub.md:
+# dram__bytes_read.sum 16.88 MB + dram__bytes_write.sum 82.57 MB, widest tile edge 256)
+NCU_TRAFFIC = {("ensemble256_lub", "k_rpy_aa_f2"): {"bytes": 99.45e6, "tile_edge": 256}}
 
 
 def parse():
@@ -74,7 +74,7 @@ def parse():
                     help="profiler driver: build the workload and run S steps (no autotuning, no bench line)")
     ap.add_argument("--profile-kernel", type=int, default=0, metavar="K",
                     help="profiler driver: build the workload, stage it once, launch only the monomer pair kernel "
-                         "K times (default chunk width, no autotuning, no steps) and exit; prints no bench line")
+                         "K times (default tile edges, no autotuning, no steps) and exit; prints no bench line")
     return ap.parse_args()
 
 
@@ -106,7 +106,7 @@ def profile_kernel(args):
 
 def profile_steps(args):
     """A short, fixed step sequence for profiler captures of the step's kernels (launch
-    lists, the HBM-bound solver kernels): the workload at the default chunk width, S steps."""
+    lists, the HBM-bound solver kernels): the workload at the default tile edges, S steps."""
     import torch
     from polystokes_brownian_b200 import _capi
     from polystokes_brownian_b200.engine import Batch
@@ -675,7 +675,7 @@ def run_b200(args):
         torch.cuda.synchronize()
 
     b.stage()
-    aa_cols, aa_tune_ms = b.autotune(5)      # far-field chunk width for this GPU and workload
+    aa_cols, aa_tune_ms = b.autotune(5)      # far-field tile edge for this GPU and workload
     for _ in range(args.warmup):
         b.step(rtol=args.rtol, solver=solver)
     barrier()
@@ -741,8 +741,8 @@ def run_b200(args):
             "achieved": achieved, "peak": peak.value, "unit": "TFLOP/s",
             "frac": achieved / peak.value if peak.value else None,
             "traffic": NCU_TRAFFIC.get((name, kname), {}).get("bytes"),
-            "traffic_source": ("ncu dram__bytes_read.sum + dram__bytes_write.sum of one launch at chunk width "
-                               f"{NCU_TRAFFIC[(name, kname)]['chunk_cols']} (compute-bound: the FLOP roofline "
+            "traffic_source": ("ncu dram__bytes_read.sum + dram__bytes_write.sum of one launch at widest tile edge "
+                               f"{NCU_TRAFFIC[(name, kname)]['tile_edge']} (compute-bound: the FLOP roofline "
                                "applies)") if (name, kname) in NCU_TRAFFIC else None,
             "peak_source": "measured FMA throughput of this GPU in bench.py (ps_fma_peak); CUDA-core work, "
                            "no tensor-core or HBM denominator applies",

@@ -243,7 +243,7 @@ int structured_solve(Engine &E, const double *b, double *x, const ps_ksp_opts *o
                      cudaStream_t st);
 int schur_lanczos_noise(Engine &E, const double *fb, const double *ymcm, double *W, int *nneg, cudaStream_t st);
 int lanczos_sqrt(Engine &E, const double *z, double *w, const ps_sqrt_opts *o, ps_sqrt_result *res, cudaStream_t st);
-int build_red_table(Engine &E, RedTable &T, int layout);   // 0 saddle, 1 top, 2 velocity, 3 beads
+int build_red_table(Engine &E, RedTable &T, int layout);   // 0 saddle, 1 top, 2 velocity
 void free_red_table(RedTable &T);
 void seg_dot(Engine &E, RedTable &T, const double *a, const double *b, double *out_per_rep, cudaStream_t st);
 

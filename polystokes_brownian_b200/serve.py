@@ -163,7 +163,7 @@ class Server:
         b.set_aux(t, k, xp)
         b.set_replica_seeds([s.req.seed for s in slots], [s.rng_steps for s in slots])
         if not Server._tuned:
-            # one process-wide choice, so every later context chunks replicas the same way
+            # one process-wide choice, so every later context tiles replicas the same way
             b.stage()
             self.aa_chunk_cols, _ = b.autotune(3)
             Server._tuned = True
