@@ -265,10 +265,11 @@ struct LzScal {
 // Bound: latency and L2 (the basis is read twice from L2 and once from L1 per
 // vector, k_lz_sub_dots reading its slices twice).  With 1024 entries per block of
 // 256 threads, or one cluster of eight blocks per replica, too few loads were in
-// flight: a vector with its apply took 42 us at 1024 beads (25 now), 72 us at the
-// 4097-bead brush (50 now), and the four sweeps of 64 replicas, 62000 beads, 100 us
-// (three, 37 us, now).  Taking the norm with the second dots instead of in a launch of its
-// own is 2 us of these.
+// flight: a vector with its apply took 42 us at 1024 beads (23 now), 72 us at the
+// 4097-bead brush (49 now), and the four sweeps of 64 replicas, 62000 beads, 100 us
+// (three, 44 us, now).  Taking the norm with the second dots instead of in a launch of its
+// own is 2 us of these; holding the thread's entries of the first 32 vectors in registers, asked
+// for before the totals are added, 2 us more (k_lz_sub_dots 5.5 -> 4.4 us at 1024 beads).
 constexpr int LZ_SUB = RB_THREADS;                    // entries of a sub-block
 constexpr int LZC_CTAS = 8, LZC_HALVES = 2, LZC_THREADS = RB_THREADS * LZC_HALVES, LZC_SLOTS = 4;
 constexpr int LZC_VB = LZC_CTAS * LZC_HALVES;         // virtual RB-table blocks per cluster
@@ -283,17 +284,17 @@ __device__ __host__ __forceinline__ bool lz_fixed(const Seg &s)
 }
 static_assert(RB_SPAN == RB_EPT * LZ_SUB, "RB_EPT sub-blocks per table block");
 
-// the replica's total of the sub-block sums part[][i], i <= j, into h[] (shared); NORM: that of
-// npart[] into h[LZ_KMAX]
+// the replica's total of the sub-block sums part[][i], i <= j, into h[] (shared, zero beyond j); NORM: that
+// of npart[] into h[LZ_KMAX].  The replica's first table block and length come from the caller.
 template <bool NORM>
-__device__ __forceinline__ void lz_total(const RedTable &T, const RBlk &B, const Seg &s, const double *__restrict__ part,
+__device__ __forceinline__ void lz_total(int first_blk, int n, const double *__restrict__ part,
                                          const double *__restrict__ npart, int j, double *__restrict__ h)
 {
     __shared__ double sh4[RB_THREADS / LZ_KMAX][LZ_KMAX];
     constexpr int G = RB_THREADS / LZ_KMAX;
     const int i = threadIdx.x % LZ_KMAX, g = threadIdx.x / LZ_KMAX;
-    const int nb = (s.nm3nc11 + LZ_SUB - 1) / LZ_SUB;
-    const long first = (long)RB_EPT * T.d_first[B.rep];
+    const int nb = (n + LZ_SUB - 1) / LZ_SUB;
+    const long first = (long)RB_EPT * first_blk;
     const double *p = part + first * LZ_KMAX + i;
     double t = 0.0, n2 = 0.0;
     const bool norm = NORM && threadIdx.x >= RB_THREADS - 32;      // the warp whose dots come last
@@ -309,7 +310,7 @@ __device__ __forceinline__ void lz_total(const RedTable &T, const RBlk &B, const
         if (threadIdx.x == RB_THREADS - 1) h[LZ_KMAX] = n2;
     }
     __syncthreads();
-    if (threadIdx.x <= j) {
+    if (threadIdx.x < LZ_KMAX) {
         double v = 0.0;
         for (int c = 0; c < G; c++) v += sh4[c][threadIdx.x];
         h[threadIdx.x] = v;
@@ -317,16 +318,22 @@ __device__ __forceinline__ void lz_total(const RedTable &T, const RBlk &B, const
     __syncthreads();
 }
 
-// q -= sum_i h_i V_i for this thread's entry, in four interleaved sums
-__device__ __forceinline__ double lz_subtract(const double *__restrict__ V, long ldv, long k, double q, int j,
-                                              const double *__restrict__ h)
+// q -= sum_i h_i V_i for this thread's entry (v from lz_load), in four interleaved sums
+__device__ __forceinline__ double lz_subtract(const double (&v)[LZ_REG], const double *__restrict__ V, long ldv, long k,
+                                              bool act, double q, int j, const double *__restrict__ h)
 {
     double t[4] = {0.0, 0.0, 0.0, 0.0};
-#pragma unroll 2
-    for (int i = 0; i <= j; i += 4)
 #pragma unroll
-        for (int c = 0; c < 4; c++)
-            if (i + c <= j) t[c] += h[i + c] * V[(long)(i + c) * ldv + k];
+    for (int i = 0; i < LZ_REG; i += 8)
+        if (i <= j) {
+#pragma unroll
+            for (int c = 0; c < 8; c++) t[c & 3] += h[i + c] * v[i + c];
+        }
+    if (act)
+        for (int i = LZ_REG; i <= j; i += 8)
+#pragma unroll
+            for (int c = 0; c < 8; c++)
+                if (i + c <= j) t[c & 3] += h[i + c] * V[(long)(i + c) * ldv + k];
     return q - ((t[0] + t[1]) + (t[2] + t[3]));
 }
 
@@ -338,21 +345,22 @@ __global__ void k_lz_sub_dots(RedTable T, const Seg *__restrict__ segs, const do
     pdl_enter();
     const RBlk B = T.d_blk[blockIdx.x];
     const int e = blockIdx.y * LZ_SUB + threadIdx.x;
-    if (blockIdx.y * LZ_SUB >= B.len || lz[B.rep].done || lz_fixed(segs[B.rep])) return;
-    __shared__ double h[LZ_KMAX], wn[RB_THREADS / 32];
-    lz_total<false>(T, B, segs[B.rep], part1, nullptr, j, h);
+    if (blockIdx.y * LZ_SUB >= B.len) return;
+    const int first = T.d_first[B.rep];
     const bool act = e < B.len;
     const long k = (long)B.start + e;
-    double v = 0.0;
-    if (act) {
-        v = lz_subtract(V, ldv, k, q[k], j, h);
-        q[k] = v;
-    }
-    if (threadIdx.x == 0 && blockIdx.y == 0 && (int)blockIdx.x == T.d_first[B.rep]) alpha[(long)LZ_KMAX * B.rep + j] = h[j];
+    double vr[LZ_REG], v = act ? q[k] : 0.0;
+    lz_load(V, ldv, k, act, j, vr);
+    if (lz[B.rep].done || lz_fixed(segs[B.rep])) return;
+    __shared__ double h[LZ_KMAX], wn[RB_THREADS / 32];
+    lz_total<false>(first, segs[B.rep].nm3nc11, part1, nullptr, j, h);
+    v = lz_subtract(vr, V, ldv, k, act, v, j, h);
+    if (act) q[k] = v;
+    if (threadIdx.x == 0 && blockIdx.y == 0 && (int)blockIdx.x == first) alpha[(long)LZ_KMAX * B.rep + j] = h[j];
     double n2 = v * v;
     for (int o = 16; o > 0; o >>= 1) n2 += __shfl_xor_sync(0xffffffffu, n2, o);
     if ((threadIdx.x & 31) == 0) wn[threadIdx.x >> 5] = n2;
-    lz_block_dots(V, ldv, k, act, v, j, part2 + (long)LZ_KMAX * (RB_EPT * blockIdx.x + blockIdx.y));   // a barrier inside
+    lz_block_dots(vr, V, ldv, k, act, v, j, part2 + (long)LZ_KMAX * (RB_EPT * blockIdx.x + blockIdx.y));   // a barrier inside
     if (threadIdx.x == RB_THREADS - 1) {
         n2 = 0.0;
         for (int w = 0; w < RB_THREADS / 32; w++) n2 += wn[w];
@@ -374,21 +382,25 @@ __global__ void k_lz_sub_scale(RedTable T, const Seg *__restrict__ segs, double 
     pdl_enter();
     const RBlk B = T.d_blk[blockIdx.x];
     const int e = blockIdx.y * LZ_SUB + threadIdx.x;
-    if (blockIdx.y * LZ_SUB >= B.len || lz[B.rep].done || lz_fixed(segs[B.rep])) return;
+    if (blockIdx.y * LZ_SUB >= B.len) return;
+    const int first = T.d_first[B.rep];
+    const bool act = e < B.len;
+    const long k = (long)B.start + e;
+    double vr[LZ_REG];
+    const double qk = act ? q[k] : 0.0;
+    lz_load(V, ldv, k, act, j, vr);
+    if (lz[B.rep].done || lz_fixed(segs[B.rep])) return;
     __shared__ double h[LZ_KMAX + 1];
-    lz_total<true>(T, B, segs[B.rep], part2, npart, j, h);
+    lz_total<true>(first, segs[B.rep].nm3nc11, part2, npart, j, h);
     double h2[4] = {0.0, 0.0, 0.0, 0.0};
     for (int i = 0; i <= j; i += 4)
 #pragma unroll
-        for (int c = 0; c < 4; c++)
-            if (i + c <= j) h2[c] += h[i + c] * h[i + c];
+        for (int c = 0; c < 4; c++) h2[c] += h[i + c] * h[i + c];      // zero beyond j
     const double bj = sqrt(fmax(h[LZ_KMAX] - ((h2[0] + h2[1]) + (h2[2] + h2[3])), 0.0));
     const bool broken = bj <= 1e-12 * lz[B.rep].b0;
-    if (!broken && j + 1 < kmax && e < B.len) {
-        const long k = (long)B.start + e;
-        V[(long)(j + 1) * ldv + k] = lz_subtract(V, ldv, k, q[k], j, h) * (bj > 0 ? 1.0 / bj : 0.0);
-    }
-    if (threadIdx.x == 0 && blockIdx.y == 0 && (int)blockIdx.x == T.d_first[B.rep]) {
+    if (!broken && j + 1 < kmax && act)
+        V[(long)(j + 1) * ldv + k] = lz_subtract(vr, V, ldv, k, act, qk, j, h) * (bj > 0 ? 1.0 / bj : 0.0);
+    if (threadIdx.x == 0 && blockIdx.y == 0 && (int)blockIdx.x == first) {
         alpha[(long)LZ_KMAX * B.rep + j] += h[j];
         lz[B.rep].m = j + 1;
         if (broken) lz[B.rep].done = 2;             // finalise with m = j + 1

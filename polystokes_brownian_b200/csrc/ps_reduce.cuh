@@ -171,8 +171,70 @@ __device__ __forceinline__ double warp_sum16(double (&v)[16], int lane, int &idx
     return v[0] + __shfl_xor_sync(0xffffffffu, v[0], 1);
 }
 
-// A block's dots of its entries (one per thread: value q at index k, when act) with the
+// sums of 32 values over the warp; the lane ends with the total of value `lane`
+__device__ __forceinline__ double warp_sum32(double (&v)[32], int lane)
+{
+#pragma unroll
+    for (int h = 16; h >= 1; h >>= 1) {
+        const bool up = lane & h;
+#pragma unroll
+        for (int c = 0; c < h; c++) {
+            const double send = up ? v[c] : v[c + h], keep = up ? v[c + h] : v[c];
+            v[c] = keep + __shfl_xor_sync(0xffffffffu, send, h);
+        }
+    }
+    return v[0];
+}
+
+// Entry k (one per thread, when act) of the first LZ_REG of the vectors V_0..V_j, zero beyond: asked
+// for at a kernel's start, all at once, so that subtraction and dots find them in registers.
+constexpr int LZ_REG = 32;
+__device__ __forceinline__ void lz_load(const double *__restrict__ V, long ldv, long k, bool act, int j, double (&v)[LZ_REG])
+{
+#pragma unroll
+    for (int i = 0; i < LZ_REG; i++) v[i] = act && i <= j ? V[(long)i * ldv + k] : 0.0;
+}
+
+// A block's dots of its entries (one per thread: value q at index k, when act; v from lz_load) with the
 // Lanczos vectors V_0..V_j, into out[0..j]; RB_THREADS threads, every one of which takes part.
+__device__ __forceinline__ void lz_block_dots(const double (&v)[LZ_REG], const double *__restrict__ V, long ldv, long k,
+                                              bool act, double q, int j, double *__restrict__ out)
+{
+    __shared__ double sh[RB_THREADS / 32][LZ_KMAX];
+    const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
+    if (j < 16) {
+        double p[16];
+#pragma unroll
+        for (int c = 0; c < 16; c++) p[c] = v[c] * q;
+        int idx;
+        const double t = warp_sum16(p, lane, idx);
+        if (!(lane & 1)) sh[wid][idx] = t;
+    } else {
+        double p[LZ_REG];
+#pragma unroll
+        for (int c = 0; c < LZ_REG; c++) p[c] = v[c] * q;
+        sh[wid][lane] = warp_sum32(p, lane);
+    }
+    for (int i0 = LZ_REG; i0 <= j; i0 += 16) {
+        double p[16];
+#pragma unroll
+        for (int c = 0; c < 16; c++) p[c] = (act && i0 + c <= j) ? V[(long)(i0 + c) * ldv + k] * q : 0.0;
+        int idx;
+        const double t = warp_sum16(p, lane, idx);
+        if (!(lane & 1) && i0 + idx <= j) sh[wid][i0 + idx] = t;
+    }
+    __syncthreads();
+    if (threadIdx.x <= j) {
+        double t = 0.0;
+#pragma unroll
+        for (int w = 0; w < RB_THREADS / 32; w++) t += sh[w][threadIdx.x];
+        out[threadIdx.x] = t;
+    }
+}
+
+// The same from memory, sixteen vectors at a time: the combine of an apply forms q late and has many
+// blocks in flight, where 32 entries held since its start cost more blocks than they save waits (64
+// replicas 15.7 against 17.6 us a launch, 1024 beads 5.1 against 4.6).
 __device__ __forceinline__ void lz_block_dots(const double *__restrict__ V, long ldv, long k, bool act, double q, int j,
                                               double *__restrict__ out)
 {
