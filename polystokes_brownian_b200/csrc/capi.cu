@@ -730,7 +730,7 @@ int ps_autotune(ps_ctx *ctx, int32_t reps, int32_t *best_cols, double *ms, void 
     double t[4] = {0, 0, 0, 0};
     double *u = nullptr;
     PS_CK(cudaMalloc(&u, sizeof(double) * std::max<long>(E.ntop, 1)));
-    PS_CK(cudaMemset(u, 0, sizeof(double) * std::max<long>(E.ntop, 1)));
+    PS_CK(cudaMemsetAsync(u, 0, sizeof(double) * std::max<long>(E.ntop, 1), S(stream)));
     int best = ps::g_aa_chunk_cols, rc = PS_OK;
     double tbest = 1e300;
     for (int k = 0; k < 4 && rc == PS_OK; k++) {

@@ -130,6 +130,7 @@ int obs_reset(Engine &E, int nbins, double bond_max, double trap_max, int lags)
     PS_CK(cudaMemset(E.d_obs_ht, 0, sizeof(unsigned long long) * nbins * E.R));
     PS_CK(cudaMemset(E.d_obs_msd, 0, sizeof(double) * 6 * lags * nc));
     PS_CK(cudaMemset(E.d_obs_msdn, 0, sizeof(unsigned long long) * lags * nc));
+    PS_CK(cudaDeviceSynchronize());      // ps_observe adds on the caller's stream
     E.obs_nbins = nbins; E.obs_bmax = bond_max; E.obs_tmax = trap_max; E.obs_lags = lags; E.obs_n = 0;
     return PS_OK;
 }

@@ -1248,16 +1248,17 @@ static int ensure_pair_space(Engine &E)
 }
 
 // the pair-space MINRES vectors, for the contexts that come to use them
-static int ensure_pm_space(Engine &E)
+static int ensure_pm_space(Engine &E, cudaStream_t st)
 {
-    if (E.pm_cap >= E.pair_cap) return PS_OK;
+    if (E.pm_cap == E.pair_cap) return PS_OK;
     E.pm_cap = 0;
     int rc;
     for (auto &p : E.d_pmp)
         if ((rc = grow(p, 12 * E.pair_cap))) return rc;
     if ((rc = grow(E.d_pmd, 3 * (E.pair_cap + E.ntot)))) return rc;
-    // beads without stresslet unknowns never write theirs
-    PS_CK(cudaMemset(E.d_pmd, 0, sizeof(double) * 3 * (E.pair_cap + E.ntot)));
+    // beads without stresslet unknowns never write theirs; on the solve's stream, which alone orders it
+    // before the kernels that write the others'
+    PS_CK(cudaMemsetAsync(E.d_pmd, 0, sizeof(double) * 3 * (E.pair_cap + E.ntot), st));
     E.pm_cap = E.pair_cap;
     return PS_OK;
 }
@@ -1284,7 +1285,7 @@ static int pair_minres(Engine &E, const double *b, const double *g, int maxit, d
     const int ds = (int)sizeof(MinresScal);
     const unsigned nb = (unsigned)E.n_pblk;
     const PairTab T = pair_tab(E);
-    int rc = ensure_pm_space(E);
+    int rc = ensure_pm_space(E, st);
     if (rc) return rc;
     PMArgs A;
     // r_k lives in slot k % 3, w_k in slot 3 + k % 3
