@@ -396,7 +396,8 @@ __global__ void k_lz_sub_scale(RedTable T, const Seg *__restrict__ segs, double 
     for (int i = 0; i <= j; i += 4)
 #pragma unroll
         for (int c = 0; c < 4; c++) h2[c] += h[i + c] * h[i + c];      // zero beyond j
-    const double bj = sqrt(fmax(h[LZ_KMAX] - ((h2[0] + h2[1]) + (h2[2] + h2[3])), 0.0));
+    // a norm that is not a number stays one (fmax would make it 0, which reads as a breakdown)
+    const double n2 = h[LZ_KMAX] - ((h2[0] + h2[1]) + (h2[2] + h2[3])), bj = sqrt(n2 < 0.0 ? 0.0 : n2);
     const bool broken = bj <= 1e-12 * lz[B.rep].b0;
     if (!broken && j + 1 < kmax && act)
         V[(long)(j + 1) * ldv + k] = lz_subtract(vr, V, ldv, k, act, qk, j, h) * (bj > 0 ? 1.0 / bj : 0.0);
@@ -741,7 +742,7 @@ k_lz_check(int R, const Seg *__restrict__ segs, LzScal *__restrict__ lz, const L
     // f(T) e1 with U (U^T U)^(-1/2) in place of U, to first order in U^T U - I:
     // w = f (3 v - U^T U v) / 2, then U (3 w - U^T U w) / 2
     team_matvec(Z, ld, true, a, mr, 1.5, v, -0.5, b);
-    for (int j = tid; j < mr; j += LZE_THREADS) b[j] *= d[j] > 0 ? sqrt(d[j]) : 0.0;
+    for (int j = tid; j < mr; j += LZE_THREADS) b[j] *= d[j] < 0.0 ? 0.0 : sqrt(d[j]);   // a NaN stays one
     __syncthreads();
     team_matvec(Z, ld, false, b, mr, 0.0, b, 1.0, a);
     team_matvec(Z, ld, true, a, mr, 1.5, b, -0.5, b2);
@@ -818,7 +819,7 @@ __global__ void k_lz_check_ql(int R, const Seg *__restrict__ segs, LzScal *__res
         if (i < mr) {
             for (int j = 0; j < mr; j++) {
                 double th = d[j];
-                double sq = th > 0 ? sqrt(th) : 0.0;
+                double sq = th < 0.0 ? 0.0 : sqrt(th);      // a NaN stays one
                 gi += Z[i * mr + j] * sq * Z[0 * mr + j];
             }
             gi *= L.b0;
