@@ -245,9 +245,11 @@ int minres_solve(Engine &E, const double *b, double *x, const ps_ksp_opts *o, ps
 // two-pass Gram-Schmidt reorthogonalisation, projected spectrum floored at 0
 // (the policy of schur_sqrt_lanczos, slip_vel.cpp:351-477, applied to the full
 // grand mobility instead of SLEPc MFN/FNSQRT, slip_vel.cpp:27-49).
+// done after j vectors lives in done[j & 1]: the launches of vector j read it there and the
+// orthogonalisation's last one writes done[(j + 1) & 1], so that all threads of a launch see one value.
 struct LzScal {
     double b0;
-    int m, done, nneg;
+    int m, nneg, done[2];
 };
 
 // Reorthogonalisation of one Lanczos vector, q = M V_j against V_0..V_j: two
@@ -351,7 +353,7 @@ __global__ void k_lz_sub_dots(RedTable T, const Seg *__restrict__ segs, const do
     const long k = (long)B.start + e;
     double vr[LZ_REG], v = act ? q[k] : 0.0;
     lz_load(V, ldv, k, act, j, vr);
-    if (lz[B.rep].done || lz_fixed(segs[B.rep])) return;
+    if (lz[B.rep].done[j & 1] || lz_fixed(segs[B.rep])) return;
     __shared__ double h[LZ_KMAX], wn[RB_THREADS / 32];
     lz_total<false>(first, segs[B.rep].nm3nc11, part1, nullptr, j, h);
     v = lz_subtract(vr, V, ldv, k, act, v, j, h);
@@ -372,8 +374,7 @@ __global__ void k_lz_sub_dots(RedTable T, const Seg *__restrict__ segs, const do
 // the replica.  The norm after the subtraction is that before it less the dots' squares (the
 // basis is orthonormal), so no further sum over the replica, and no further launch, is needed: the
 // dots of a second pass are rounding residues of the first, and only at a breakdown not far
-// smaller than q.  (done may be set by the replica's first block while others still read it: they
-// find the same breakdown themselves and write nothing either way.)
+// smaller than q.
 __global__ void k_lz_sub_scale(RedTable T, const Seg *__restrict__ segs, double *__restrict__ V, long ldv,
                                const double *__restrict__ q, int j, int kmax, LzScal *__restrict__ lz,
                                const double *__restrict__ part2, const double *__restrict__ npart,
@@ -389,7 +390,13 @@ __global__ void k_lz_sub_scale(RedTable T, const Seg *__restrict__ segs, double 
     double vr[LZ_REG];
     const double qk = act ? q[k] : 0.0;
     lz_load(V, ldv, k, act, j, vr);
-    if (lz[B.rep].done || lz_fixed(segs[B.rep])) return;
+    if (lz_fixed(segs[B.rep])) return;
+    const bool lead = threadIdx.x == 0 && blockIdx.y == 0 && (int)blockIdx.x == first;
+    const int done = lz[B.rep].done[j & 1];
+    if (done) {
+        if (lead) lz[B.rep].done[(j + 1) & 1] = done;
+        return;
+    }
     __shared__ double h[LZ_KMAX + 1];
     lz_total<true>(first, segs[B.rep].nm3nc11, part2, npart, j, h);
     double h2[4] = {0.0, 0.0, 0.0, 0.0};
@@ -401,11 +408,11 @@ __global__ void k_lz_sub_scale(RedTable T, const Seg *__restrict__ segs, double 
     const bool broken = bj <= 1e-12 * lz[B.rep].b0;
     if (!broken && j + 1 < kmax && act)
         V[(long)(j + 1) * ldv + k] = lz_subtract(vr, V, ldv, k, act, qk, j, h) * (bj > 0 ? 1.0 / bj : 0.0);
-    if (threadIdx.x == 0 && blockIdx.y == 0 && (int)blockIdx.x == first) {
+    if (lead) {
         alpha[(long)LZ_KMAX * B.rep + j] += h[j];
         lz[B.rep].m = j + 1;
-        if (broken) lz[B.rep].done = 2;             // finalise with m = j + 1
-        else if (j + 1 < kmax) betad[(long)LZ_KMAX * B.rep + j] = bj;
+        lz[B.rep].done[(j + 1) & 1] = broken ? 2 : 0;      // 2: finalise with m = j + 1
+        if (!broken && j + 1 < kmax) betad[(long)LZ_KMAX * B.rep + j] = bj;
     }
 }
 
@@ -420,7 +427,7 @@ __global__ void k_lz_init(RedTable T, const Seg *__restrict__ segs, double *__re
     double inv = b0 > 0 ? 1.0 / b0 : 0.0;
     for (int e = threadIdx.x; e < B.len; e += RB_THREADS) V[B.start + e] = z[B.start + e] * inv;
     if (threadIdx.x == 0 && (B.start == T.d_blk[T.d_first[B.rep]].start)) {
-        lz[B.rep].b0 = skip ? 0.0 : b0; lz[B.rep].m = 0; lz[B.rep].done = (b0 == 0.0 || skip); lz[B.rep].nneg = 0;
+        lz[B.rep].b0 = skip ? 0.0 : b0; lz[B.rep].m = 0; lz[B.rep].done[0] = (b0 == 0.0 || skip); lz[B.rep].nneg = 0;
     }
 }
 
@@ -689,7 +696,7 @@ struct LzSpec {
 __global__ void __launch_bounds__(LZE_THREADS)
 k_lz_check(int R, const Seg *__restrict__ segs, LzScal *__restrict__ lz, const LzScal *__restrict__ snap, LzSpec *__restrict__ spec,
            const double *__restrict__ alpha, const double *__restrict__ betad, double *__restrict__ gbuf,
-           int m, double tol, int final_)
+           int m, int cur, double tol, int final_)
 {
     pdl_enter();
     extern __shared__ double sm[];
@@ -699,11 +706,12 @@ k_lz_check(int R, const Seg *__restrict__ segs, LzScal *__restrict__ lz, const L
     if (lz_fixed(segs[r])) return;
     const LzScal L = final_ ? lz[r] : snap[r];
     const int tid = threadIdx.x, lane = tid & 31, wid = tid >> 5;
-    if (!final_ && L.done) {
+    const int done = L.done[cur];
+    if (!final_ && done) {
         if (tid == 0) spec[r] = LzSpec{0, L.m, 1, 0};
         return;
     }
-    const int mr = L.done ? L.m : m;
+    const int mr = done ? L.m : m;
     if (mr <= 0) {
         if (!final_ && tid == 0) spec[r] = LzSpec{0, 0, 0, 0};
         return;
@@ -766,9 +774,9 @@ k_lz_check(int R, const Seg *__restrict__ segs, LzScal *__restrict__ lz, const L
         const int conv = sqrt(red[0][0] + red[1][0]) <= tol * sqrt(red[0][1] + red[1][1]);
         if (final_) {
             lz[r].nneg = rneg[0] + rneg[1];
-            if (!lz[r].done) {
+            if (!done) {
                 lz[r].m = mr;
-                lz[r].done = 1;
+                lz[r].done[cur] = 1;
             }
         } else {
             spec[r] = LzSpec{conv, mr, conv, 0};
@@ -786,7 +794,7 @@ k_lz_check(int R, const Seg *__restrict__ segs, LzScal *__restrict__ lz, const L
 // (k_lz_spec_apply).  g_prev is the previous check's g in both cases.
 __global__ void k_lz_check_ql(int R, const Seg *__restrict__ segs, LzScal *__restrict__ lz, const LzScal *__restrict__ snap, LzSpec *__restrict__ spec,
                            const double *__restrict__ alpha, const double *__restrict__ betad, double *__restrict__ gbuf,
-                           int m, double tol, int final_)
+                           int m, int cur, double tol, int final_)
 {
     pdl_enter();
     extern __shared__ double sm[];
@@ -794,11 +802,12 @@ __global__ void k_lz_check_ql(int R, const Seg *__restrict__ segs, LzScal *__res
     if (!lz_fixed(segs[r])) return;
     const LzScal L = final_ ? lz[r] : snap[r];
     const int lane = threadIdx.x;
-    if (!final_ && L.done) {
+    const int done = L.done[cur];
+    if (!final_ && done) {
         if (lane == 0) spec[r] = LzSpec{0, L.m, 1, 0};
         return;
     }
-    int mr = L.done ? L.m : m;
+    int mr = done ? L.m : m;
     if (mr <= 0) {
         if (!final_ && lane == 0) spec[r] = LzSpec{0, 0, 0, 0};
         return;
@@ -839,9 +848,9 @@ __global__ void k_lz_check_ql(int R, const Seg *__restrict__ segs, LzScal *__res
         const int conv = sqrt(diff2) <= tol * sqrt(nrm2);
         if (final_) {
             lz[r].nneg = nneg;
-            if (!lz[r].done) {
+            if (!done) {
                 lz[r].m = mr;
-                lz[r].done = 1;
+                lz[r].done[cur] = 1;
             }
         } else {
             spec[r] = LzSpec{conv, mr, conv, 0};
@@ -852,12 +861,12 @@ __global__ void k_lz_check_ql(int R, const Seg *__restrict__ segs, LzScal *__res
 // a speculative check's outcome, applied in stream order after the vectors that
 // ran beside it: a replica that had converged at m stops there (done, m), as if
 // the check had held the vectors back; the vectors it took meanwhile are unused
-__global__ void k_lz_spec_apply(int R, LzScal *__restrict__ lz, const LzSpec *__restrict__ spec)
+__global__ void k_lz_spec_apply(int R, LzScal *__restrict__ lz, const LzSpec *__restrict__ spec, int cur)
 {
     pdl_enter();
     const int r = blockIdx.x * blockDim.x + threadIdx.x;
     if (r >= R) return;
-    if (spec[r].conv) { lz[r].done = 1; lz[r].m = spec[r].m; }
+    if (spec[r].conv) { lz[r].done[cur] = 1; lz[r].m = spec[r].m; }
 }
 
 // w = V g (top layout)
@@ -882,8 +891,7 @@ __global__ void k_lz_combine(RedTable T, const double *__restrict__ V, long ldv,
 // phases and the cross-block sums read through distributed shared memory.  The
 // replica's vector is cut into the reduction table's RB_SPAN blocks, each half of a
 // block (RB_THREADS threads) forms an RB block's partials, and every sum over RB
-// blocks runs in block order.  A replica that is done leaves with its whole cluster
-// (the flag is read before any block writes it).
+// blocks runs in block order.  A replica that is done leaves with its whole cluster.
 namespace cgr = cooperative_groups;
 
 __global__ void __cluster_dims__(LZC_CTAS, 1, 1) __launch_bounds__(LZC_THREADS)
@@ -902,7 +910,12 @@ k_lz_orth_cluster(const Seg *__restrict__ segs, double *__restrict__ V, long ldv
     __shared__ double sh[LZC_THREADS / 32][8];
     __shared__ double hsh[LZ_KMAX + 1];
     const Seg &s = segs[r];
-    if (lz[r].done || !lz_fixed(s)) return;     // the whole cluster: no block has written lz yet
+    if (!lz_fixed(s)) return;                   // the whole cluster
+    const int done = lz[r].done[j & 1];
+    if (done) {
+        if (rank == 0 && threadIdx.x == 0) lz[r].done[(j + 1) & 1] = done;
+        return;
+    }
     const int n = s.nm3nc11;
     const long base = s.top_off;
     const int nb = (n + RB_SPAN - 1) / RB_SPAN, nslot = (nb + LZC_VB - 1) / LZC_VB;
@@ -1002,8 +1015,8 @@ k_lz_orth_cluster(const Seg *__restrict__ segs, double *__restrict__ V, long ldv
     if (rank == 0 && threadIdx.x == 0) {
         alpha[(long)LZ_KMAX * r + j] = alpha_j;
         lz[r].m = j + 1;
-        if (broken) lz[r].done = 2;             // invariant subspace: finalise with m = j + 1
-        else if (j + 1 < kmax) betad[(long)LZ_KMAX * r + j] = bj;
+        lz[r].done[(j + 1) & 1] = broken ? 2 : 0;   // 2, an invariant subspace: finalise with m = j + 1
+        if (!broken && j + 1 < kmax) betad[(long)LZ_KMAX * r + j] = bj;
     }
     if (!broken && j + 1 < kmax) {
         const double inv = bj > 0 ? 1.0 / bj : 0.0;
@@ -1046,10 +1059,11 @@ int lanczos_sqrt(Engine &E, const double *z, double *w, const ps_sqrt_opts *o, p
     LzSpec *spec = (LzSpec *)(snap + E.R);                   // the checks' outcomes
     LzSpec *hspec = (LzSpec *)E.h_spec;
     bool pending = false;
-    int j = 0;
+    int j = 0, cur = 0;                                      // cur: where done stands, the number of vectors & 1
     for (j = 0; j < kmax; j++) {
+        cur = (j + 1) & 1;
         const LzDots dots = {V, ldv, j, part1};
-        apply_operator(E, 1, V + (long)j * ldv, q, E.precision == PS_PREC_MIXED, st, &lz[0].done,
+        apply_operator(E, 1, V + (long)j * ldv, q, E.precision == PS_PREC_MIXED, st, &lz[0].done[j & 1],
                        (int)sizeof(LzScal), false, any_free ? &dots : nullptr);
         const dim3 sub((unsigned)T.nblk, RB_EPT);
         if (any_fixed)
@@ -1064,7 +1078,7 @@ int lanczos_sqrt(Engine &E, const double *z, double *w, const ps_sqrt_opts *o, p
                 // the previous check (normally finished long before): apply its outcomes
                 PS_CK(cudaEventSynchronize(E.ev_chk));
                 pending = false;
-                ps_launch(k_lz_spec_apply, (E.R + 127) / 128, 128, 0, st, E.R, lz, spec);
+                ps_launch(k_lz_spec_apply, (E.R + 127) / 128, 128, 0, st, E.R, lz, spec, cur);
                 bool all = true;
                 for (int r = 0; r < E.R; r++) all &= hspec[r].fin != 0;
                 if (all) break;
@@ -1075,10 +1089,10 @@ int lanczos_sqrt(Engine &E, const double *z, double *w, const ps_sqrt_opts *o, p
             PS_CK(cudaStreamWaitEvent(E.side2, E.ev_fork2, 0));
             if (any_free)
                 ps_launch(k_lz_check, E.R, LZE_THREADS, smem, E.side2, E.R, E.d_segs, lz, snap, spec, alpha, betad, gbuf,
-                        j + 1, tol, 0);
+                        j + 1, cur, tol, 0);
             if (any_fixed)
                 ps_launch(k_lz_check_ql, E.R, 32, smem_ql, E.side2, E.R, E.d_segs, lz, snap, spec, alpha, betad, gbuf, j + 1,
-                        tol, 0);
+                        cur, tol, 0);
             PS_CK(cudaMemcpyAsync(hspec, spec, sizeof(LzSpec) * E.R, cudaMemcpyDeviceToHost, E.side2));
             PS_CK(cudaEventRecord(E.ev_chk, E.side2));
             pending = true;
@@ -1087,15 +1101,15 @@ int lanczos_sqrt(Engine &E, const double *z, double *w, const ps_sqrt_opts *o, p
     if (pending) {
         // the last check's outcomes, and its g, ahead of the final estimate
         PS_CK(cudaStreamWaitEvent(st, E.ev_chk, 0));
-        ps_launch(k_lz_spec_apply, (E.R + 127) / 128, 128, 0, st, E.R, lz, spec);
+        ps_launch(k_lz_spec_apply, (E.R + 127) / 128, 128, 0, st, E.R, lz, spec, cur);
     }
     // final estimate: replicas at the cap, replicas stopped by breakdown, and the converged ones on their own m
     if (any_free)
         ps_launch(k_lz_check, E.R, LZE_THREADS, smem, st, E.R, E.d_segs, lz, snap, spec, alpha, betad, gbuf,
-                std::min(j + 1, kmax), tol, 1);
+                std::min(j + 1, kmax), cur, tol, 1);
     if (any_fixed)
         ps_launch(k_lz_check_ql, E.R, 32, smem_ql, st, E.R, E.d_segs, lz, snap, spec, alpha, betad, gbuf,
-                std::min(j + 1, kmax), tol, 1);
+                std::min(j + 1, kmax), cur, tol, 1);
     ps_launch(k_lz_combine, T.nblk, RB_THREADS, 0, st, T, V, ldv, lz, gbuf, w);
     PS_CK(cudaMemcpyAsync(hl.data(), lz, sizeof(LzScal) * E.R, cudaMemcpyDeviceToHost, st));
     PS_CK(cudaStreamSynchronize(st));

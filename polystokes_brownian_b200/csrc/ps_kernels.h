@@ -51,7 +51,7 @@ struct MrAlpha {
 // Per-replica scalars of the pair-space CG.
 struct PcgScal {
     double rz, beta, tol, err;
-    int it, done, reason, pad;
+    int it, done, reason, stop;      // stop: a direction of non-positive curvature, not yet counted as done
 };
 
 struct Engine {

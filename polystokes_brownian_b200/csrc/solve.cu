@@ -787,7 +787,7 @@ k_pc_gather(PairTab T, const int *__restrict__ sptr, const int *__restrict__ snb
 {
     pdl_enter();
     const PairBlk B = T.blk[blockIdx.x];
-    if (st[B.rep].done) return;
+    if (st[B.rep].done || st[B.rep].stop) return;
     const Seg &s = T.segs[B.rep];
     double err = 0.0;
     for_gather(B, s, sptr, snbr, cidx, S, V.z, V.r, [&](int d, double lz, double lr) {
@@ -810,6 +810,16 @@ k_pc_dir(PairTab T, const PcgScal *__restrict__ st0, PcgScal *__restrict__ st1, 
     __shared__ PcgScal sm;
     if (st0[B.rep].done) {
         if (B.b == 0 && threadIdx.x == 0) st1[B.rep] = st0[B.rep];
+        return;
+    }
+    if (st0[B.rep].stop) {                                 // the update before met non-positive curvature
+        if (B.b == 0 && threadIdx.x == 0) {
+            PcgScal p = st0[B.rep];
+            p.done = 1;
+            p.reason = -8;
+            st1[B.rep] = p;
+            atomicSub(nactive, 1);
+        }
         return;
     }
     const double rz = rep_total(prz + B.first, B.G), err2 = rep_total(perr + B.first, B.G);
@@ -871,11 +881,11 @@ k_pc_apply(PairTab T, const double *__restrict__ S, const double *__restrict__ y
     if (threadIdx.x == 0) pap[blockIdx.x] = dot;
 }
 
-// y += alpha p ; r -= alpha Ap ; z = P r ; sums of r.z.  A direction of non-positive curvature
-// stops the replica (its first block notes it; the others find the same sum).
+// y += alpha p ; r -= alpha Ap ; z = P r ; sums of r.z.  A direction of non-positive curvature stops the
+// replica: its first block notes it, which no block of this launch reads, and k_pc_dir makes it done.
 __global__ void __launch_bounds__(PB_THREADS)
 k_pc_update(PairTab T, const double *__restrict__ P, PcgVec V, PcgScal *__restrict__ st, const double *__restrict__ pap,
-            double *__restrict__ prz, int *nactive)
+            double *__restrict__ prz)
 {
     pdl_enter();
     const PairBlk B = T.blk[blockIdx.x];
@@ -895,7 +905,7 @@ k_pc_update(PairTab T, const double *__restrict__ P, PcgVec V, PcgScal *__restri
         [&]() {
             const double pAp = rep_total(pap + B.first, B.G);
             stop = pAp <= 0.0;
-            if (stop && B.b == 0 && threadIdx.x == 0) { st[B.rep].reason = -8; st[B.rep].done = 1; atomicSub(nactive, 1); }
+            if (stop && B.b == 0 && threadIdx.x == 0) st[B.rep].stop = 1;
             if (!stop) alpha = st[B.rep].rz / pAp;
             return !stop;
         },
@@ -1371,7 +1381,7 @@ static int pair_cg(Engine &E, const double *g, int maxit, int check_every, bool 
         const char *dn = (const char *)&s1[0].done;
         mr_apply(E, fp32, dn, ds, st);
         ps_launch(k_pc_apply, nb, PB_THREADS, 0, st, T, E.d_pS, E.d_py, E.d_py2, V, s1, pap);
-        ps_launch(k_pc_update, nb, PB_THREADS, 0, st, T, E.d_pP, V, s1, pap, prz, E.d_nactive);
+        ps_launch(k_pc_update, nb, PB_THREADS, 0, st, T, E.d_pP, V, s1, pap, prz);
     }
     PS_CK(cudaGetLastError());
     *scal = s1;
