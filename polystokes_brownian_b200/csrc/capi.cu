@@ -62,7 +62,7 @@ static void free_engine(Engine &E)
                     E.d_Rr[1], E.d_Rr[2], E.d_W[0], E.d_W[1], E.d_W[2], E.d_mr, E.d_mrp, E.d_nactive,
                     E.d_rhs, E.d_X, E.d_Xd, E.d_Xdet, E.d_Wn, E.d_vdn, E.d_vdc, E.d_vb, E.d_up, E.d_ud,
                     E.d_drift, E.d_sb, E.d_fext, E.d_fb, E.d_wr, E.d_tmp_top, E.d_tmp_top2, E.d_lzV, E.d_lzT,
-                    E.d_lzw, E.d_lzq, E.d_lzp, E.d_lzs, E.d_ssinv, E.d_pcg, E.d_pV, E.d_pz, E.d_pp,
+                    E.d_lzw, E.d_lzq, E.d_lzp, E.d_lzs, E.d_lz_ord, E.d_ssinv, E.d_pcg, E.d_pV, E.d_pz, E.d_pp,
                     E.d_pblk, E.d_pbp, E.d_pg, E.d_pu, E.d_py, E.d_pu2, E.d_py2, E.d_rseed, E.d_rstep,
                     E.d_lubc_ptr, E.d_lubc_nbr, E.d_lub_pairs, E.d_pS, E.d_pP, E.d_py_[0], E.d_py_[1], E.d_py_[2],
                     E.d_py_[3], E.d_py_[4], E.d_scan_sums, E.d_pmr,
@@ -162,7 +162,7 @@ static int build(Engine &E, const ps_desc *descs, int R, int precision)
             s.indef = 1;
             E.any_indef = true;
         }
-            s.n_mtiles = (d.Nm + TR - 1) / TR;
+        s.n_mtiles = (d.Nm + TR - 1) / TR;
         s.ba_off = (int)ba;
         if (d.Nc > 0) ba += (long)s.n_mtiles * d.Nc;
         if (d.Nm == 0 && d.Nc >= 2)
@@ -389,7 +389,10 @@ static int build(Engine &E, const ps_desc *descs, int R, int precision)
         const int KM = ps::LZ_KMAX;
         TRY_ALLOC(E.d_lzV, sizeof(double) * top * (KM + 1));
         TRY_ALLOC(E.d_lzq, sizeof(double) * top);
-        TRY_ALLOC(E.d_lzT, sizeof(double) * ((KM + 1) * R + KM * R * 2 + R));
+        TRY_ALLOC(E.d_lzT, sizeof(double) * ((KM + 1) * R + KM * R * 4 + R));
+        std::vector<int> ord;
+        ps::lz_ordered_list(E, ord);
+        if ((rc = upload(E.d_lz_ord, ord))) return rc;
         TRY_ALLOC(E.d_lzp, sizeof(double) * ps::RB_EPT * E.red_top.nblk * (2 * KM + 1));
         TRY_ALLOC(E.d_lzs, 96 * R);          // Lanczos scalars, their snapshot, the checks' speculative outcomes
     }

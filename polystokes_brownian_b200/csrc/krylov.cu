@@ -261,8 +261,8 @@ struct LzScal {
 // kernel leaves its sub-blocks' sums in memory, and every block of the next one
 // adds its replica's sums itself, in a fixed order that depends on the vector's
 // length alone -- no counters and no fences, and a replica's noise does not depend
-// on its batch.  Replicas whose far field may be indefinite take k_lz_orth_cluster and
-// the QL check instead (lz_fixed).
+// on its batch.  Replicas whose far field may be indefinite (Seg::indef) take
+// k_lz_orth_cluster or the k_lz_ord_* sweeps, and the QL check, instead.
 //
 // Bound: latency and L2 (the basis is read twice from L2 and once from L1 per
 // vector, k_lz_sub_dots reading its slices twice).  With 1024 entries per block of
@@ -273,17 +273,6 @@ struct LzScal {
 // own is 2 us of these; holding the thread's entries of the first 32 vectors in registers, asked
 // for before the totals are added, 2 us more (k_lz_sub_dots 5.5 -> 4.4 us at 1024 beads).
 constexpr int LZ_SUB = RB_THREADS;                    // entries of a sub-block
-constexpr int LZC_CTAS = 8, LZC_HALVES = 2, LZC_THREADS = RB_THREADS * LZC_HALVES, LZC_SLOTS = 4;
-constexpr int LZC_VB = LZC_CTAS * LZC_HALVES;         // virtual RB-table blocks per cluster
-// Replicas that keep the summation order of the reduction table's blocks, one cluster each, and the
-// QL iteration, up to LZC_VB * LZC_SLOTS blocks (5957 colloids).  Their far field may be
-// indefinite: about one in ten of the saddle solves that their noise drives is close to
-// singular, takes hundreds to thousands of iterations and returns, within rtol, whatever the
-// rounding before it selects, so another order of these sums moves positions by 1e-9 to 1e-6.
-__device__ __host__ __forceinline__ bool lz_fixed(const Seg &s)
-{
-    return s.indef && (s.nm3nc11 + RB_SPAN - 1) / RB_SPAN <= LZC_VB * LZC_SLOTS;
-}
 static_assert(RB_SPAN == RB_EPT * LZ_SUB, "RB_EPT sub-blocks per table block");
 
 // the replica's total of the sub-block sums part[][i], i <= j, into h[] (shared, zero beyond j); NORM: that
@@ -353,7 +342,7 @@ __global__ void k_lz_sub_dots(RedTable T, const Seg *__restrict__ segs, const do
     const long k = (long)B.start + e;
     double vr[LZ_REG], v = act ? q[k] : 0.0;
     lz_load(V, ldv, k, act, j, vr);
-    if (lz[B.rep].done[j & 1] || lz_fixed(segs[B.rep])) return;
+    if (lz[B.rep].done[j & 1] || segs[B.rep].indef) return;
     __shared__ double h[LZ_KMAX], wn[RB_THREADS / 32];
     lz_total<false>(first, segs[B.rep].nm3nc11, part1, nullptr, j, h);
     v = lz_subtract(vr, V, ldv, k, act, v, j, h);
@@ -390,7 +379,7 @@ __global__ void k_lz_sub_scale(RedTable T, const Seg *__restrict__ segs, double 
     double vr[LZ_REG];
     const double qk = act ? q[k] : 0.0;
     lz_load(V, ldv, k, act, j, vr);
-    if (lz_fixed(segs[B.rep])) return;
+    if (segs[B.rep].indef) return;
     const bool lead = threadIdx.x == 0 && blockIdx.y == 0 && (int)blockIdx.x == first;
     const int done = lz[B.rep].done[j & 1];
     if (done) {
@@ -703,7 +692,7 @@ k_lz_check(int R, const Seg *__restrict__ segs, LzScal *__restrict__ lz, const L
     __shared__ double red[2][2];
     __shared__ int rneg[2];
     const int r = blockIdx.x;
-    if (lz_fixed(segs[r])) return;
+    if (segs[r].indef) return;
     const LzScal L = final_ ? lz[r] : snap[r];
     const int tid = threadIdx.x, lane = tid & 31, wid = tid >> 5;
     const int done = L.done[cur];
@@ -784,7 +773,7 @@ k_lz_check(int R, const Seg *__restrict__ segs, LzScal *__restrict__ lz, const L
     }
 }
 
-// k_lz_check for the replicas that keep their order (lz_fixed), one warp per replica: QL, g summed
+// k_lz_check for the replicas reps[] that keep their order, one warp per replica: QL, g summed
 // eigenvalue by eigenvalue.  eig of T_m, g = b0 U sqrt(max(theta,0)) U^T e1,
 // convergence ||g - g_prev|| <= tol ||g|| (the Lanczos basis is orthonormal).
 // final_ = 1: the final estimate, on the replica's own m when it is done, into lz.
@@ -792,14 +781,13 @@ k_lz_check(int R, const Seg *__restrict__ segs, LzScal *__restrict__ lz, const L
 // snapshot `snap` of lz taken when it was launched (the vectors that follow
 // move lz on) and writes its outcome into spec; the host applies it later
 // (k_lz_spec_apply).  g_prev is the previous check's g in both cases.
-__global__ void k_lz_check_ql(int R, const Seg *__restrict__ segs, LzScal *__restrict__ lz, const LzScal *__restrict__ snap, LzSpec *__restrict__ spec,
+__global__ void k_lz_check_ql(const int *__restrict__ reps, LzScal *__restrict__ lz, const LzScal *__restrict__ snap, LzSpec *__restrict__ spec,
                            const double *__restrict__ alpha, const double *__restrict__ betad, double *__restrict__ gbuf,
                            int m, int cur, double tol, int final_)
 {
     pdl_enter();
     extern __shared__ double sm[];
-    const int r = blockIdx.x;
-    if (!lz_fixed(segs[r])) return;
+    const int r = reps[blockIdx.x];
     const LzScal L = final_ ? lz[r] : snap[r];
     const int lane = threadIdx.x;
     const int done = L.done[cur];
@@ -884,131 +872,305 @@ __global__ void k_lz_combine(RedTable T, const double *__restrict__ V, long ldv,
     }
 }
 
-// One Lanczos iteration's orthogonalisation of the replicas that keep their order (lz_fixed), in one
-// launch: one cluster of LZC_CTAS blocks per replica.  Both passes of the
-// reorthogonalisation (dots against V_0..V_j, then q -= V h), the norm, the
-// breakdown test and the next basis vector, with cluster barriers between the
-// phases and the cross-block sums read through distributed shared memory.  The
-// replica's vector is cut into the reduction table's RB_SPAN blocks, each half of a
-// block (RB_THREADS threads) forms an RB block's partials, and every sum over RB
-// blocks runs in block order.  A replica that is done leaves with its whole cluster.
+// Orthogonalisation of the replicas that keep the summation order of the reduction table's blocks
+// (Seg::indef).  Their far field may be indefinite: about one in ten of the saddle solves that
+// their noise drives is close to singular, takes hundreds to thousands of iterations and returns,
+// within rtol, whatever the rounding before it selects, so another order of these sums moves
+// positions by 1e-9 to 1e-6.  A replica's vector is cut into the table's RB_SPAN blocks, RB_THREADS
+// threads form a block's partials, and every sum over blocks runs in block order: both passes of the
+// reorthogonalisation (dots against V_0..V_j, then q -= V h), the norm, the breakdown test and the
+// next basis vector.  Two forms with the same bits:
+//   k_lz_orth_cluster   one launch, a cluster of LZC_CTAS blocks per replica, cluster barriers between the phases
+//                       and the cross-block sums read through distributed shared memory
+//   k_lz_ord_*          four launches over the table
+// The clusters are taken while all of a batch's are resident at once, and for replicas of one table block per
+// half-block.  Roots of 40 vectors by clusters and by the table, ms, reference pair scalars: 60 beads, 8
+// replicas 1.95 and 2.20, 28 replicas 2.35 and 2.38, 36 replicas 2.99 and 2.49, 256 replicas 9.65 and 3.00; 500
+// beads, 8 replicas 2.46 and 2.74, 28 replicas 3.26 and 3.24, 36 replicas 3.99 and 3.43, 128 replicas 9.66 and
+// 6.11; suspensions, one of 1024 colloids (11 table blocks) 2.62 and 2.92, 28 of 300 4.03 and 3.95; one of 2048
+// colloids (22 blocks, two one after the other in some clusters' blocks) 5.6 and 4.7.
+constexpr int LZC_CTAS = 8, LZC_HALVES = 2, LZC_THREADS = RB_THREADS * LZC_HALVES;
+constexpr int LZC_VB = LZC_CTAS * LZC_HALVES;         // table blocks of a cluster
+constexpr int LZC_MAX_REPS = 28;
+
+void lz_ordered_list(Engine &E, std::vector<int> &reps)
+{
+    bool fit = true;
+    for (int r = 0; r < E.R; r++)
+        if (E.segs[r].indef) {
+            reps.push_back(r);
+            fit = fit && E.segs[r].nm3nc11 <= LZC_VB * RB_SPAN;
+        }
+    E.n_lz_ord = (int)reps.size();
+    E.lz_cluster = fit && E.n_lz_ord <= LZC_MAX_REPS;
+}
+
+// Partial dots of q (held by the block's threads in qv) against V_0..V_j, one block of the
+// table; the last block of the replica sums the partials in block order into h[].
+__device__ __forceinline__ void lz_ord_block_dots(const RedTable &T, const RBlk &B, const double *__restrict__ V, long ldv,
+                                                  const double (&qv)[RB_EPT], int j, double *__restrict__ part,
+                                                  double *__restrict__ h)
+{
+    __shared__ double sh[RB_THREADS / 32][LZ_KMAX];
+    __shared__ bool last;
+    const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
+    // eight basis vectors per pass keep 8 x RB_EPT loads in flight.  Each dot is
+    // summed in element order and reduced by the same shuffle tree as one at a time.
+    for (int i0 = 0; i0 <= j; i0 += 8) {
+        double v[8];
+#pragma unroll
+        for (int c = 0; c < 8; c++) {
+            v[c] = 0.0;
+            if (i0 + c <= j) {
+                const double *Vi = V + (long)(i0 + c) * ldv + B.start;
+#pragma unroll
+                for (int k = 0; k < RB_EPT; k++) {
+                    const int e = threadIdx.x + k * RB_THREADS;
+                    if (e < B.len) v[c] += Vi[e] * qv[k];
+                }
+            }
+        }
+#pragma unroll
+        for (int c = 0; c < 8; c++) {
+            double t = v[c];
+            for (int o = 16; o > 0; o >>= 1) t += __shfl_down_sync(0xffffffffu, t, o);
+            if (lane == 0 && i0 + c <= j) sh[wid][i0 + c] = t;
+        }
+    }
+    __syncthreads();
+    if (threadIdx.x <= j) {
+        double t = 0;
+        for (int w = 0; w < RB_THREADS / 32; w++) t += sh[w][threadIdx.x];
+        part[(long)LZ_KMAX * RB_EPT * blockIdx.x + threadIdx.x] = t;
+    }
+    __threadfence();
+    __syncthreads();
+    if (threadIdx.x == 0) {
+        int t = atomicAdd(&T.d_counter[B.rep], 1);
+        last = (t == T.d_count[B.rep] - 1);
+    }
+    __syncthreads();
+    if (!last) return;
+    __threadfence();
+    int f = T.d_first[B.rep], c = T.d_count[B.rep];
+    if (threadIdx.x <= j) {
+        double t = 0;
+        for (int k = 0; k < c; k++) t += ((volatile double *)part)[(long)LZ_KMAX * RB_EPT * (f + k) + threadIdx.x];
+        h[(long)LZ_KMAX * B.rep + threadIdx.x] = t;
+    }
+    __syncthreads();
+    if (threadIdx.x == 0) T.d_counter[B.rep] = 0;
+}
+
+// a table block's entries (thread t of RB_THREADS holds t, t + RB_THREADS, ..) less sum_i h_i V_i, in the
+// order i = 0..j per entry; V: the block's part of V_0
+__device__ __forceinline__ void lz_ord_subtract(const double *__restrict__ V, long ldv, int len, int t, int j,
+                                                const double *__restrict__ h, double (&acc)[RB_EPT])
+{
+#pragma unroll 4
+    for (int i = 0; i <= j; i++) {
+        const double hi = h[i];
+        const double *Vi = V + (long)i * ldv;
+#pragma unroll
+        for (int k = 0; k < RB_EPT; k++) {
+            const int e = t + k * RB_THREADS;
+            if (e < len) acc[k] -= hi * Vi[e];
+        }
+    }
+}
+
+// the thread's part of q.q, entry by entry onto zero (a sum of the four squares alone may be contracted otherwise)
+__device__ __forceinline__ double lz_ord_square(int len, int t, const double (&v)[RB_EPT])
+{
+    double x = 0.0;
+#pragma unroll
+    for (int k = 0; k < RB_EPT; k++)
+        if (t + k * RB_THREADS < len) x += v[k] * v[k];
+    return x;
+}
+
+// a table block's entries into registers, zero beyond its length, and back
+__device__ __forceinline__ void lz_ord_load(const double *__restrict__ q, int len, int t, double (&v)[RB_EPT])
+{
+#pragma unroll
+    for (int k = 0; k < RB_EPT; k++) {
+        const int e = t + k * RB_THREADS;
+        v[k] = e < len ? q[e] : 0.0;
+    }
+}
+__device__ __forceinline__ void lz_ord_store(double *__restrict__ q, int len, int t, const double (&v)[RB_EPT], double f)
+{
+#pragma unroll
+    for (int k = 0; k < RB_EPT; k++) {
+        const int e = t + k * RB_THREADS;
+        if (e < len) q[e] = v[k] * f;
+    }
+}
+
+// h = V_0..V_j dotted with q (first pass of the Gram-Schmidt step)
+__global__ void k_lz_ord_dots(RedTable T, const Seg *__restrict__ segs, const double *__restrict__ V, long ldv,
+                              const double *__restrict__ q, int j, const LzScal *__restrict__ lz, double *__restrict__ part,
+                              double *__restrict__ h)
+{
+    pdl_enter();
+    const RBlk B = T.d_blk[blockIdx.x];
+    if (lz[B.rep].done[j & 1] || !segs[B.rep].indef) return;
+    double qv[RB_EPT];
+    lz_ord_load(q + B.start, B.len, threadIdx.x, qv);
+    lz_ord_block_dots(T, B, V, ldv, qv, j, part, h);
+}
+
+// the first pass's subtraction and the second pass's dots in one sweep: alpha_j = h_j, h2 = V_0..V_j
+// dotted with the new q, which the block still holds in registers
+__global__ void k_lz_ord_sub_dots(RedTable T, const Seg *__restrict__ segs, const double *__restrict__ V, long ldv,
+                                  double *__restrict__ q, int j, const LzScal *__restrict__ lz,
+                                  const double *__restrict__ h, double *__restrict__ alpha, double *__restrict__ part,
+                                  double *__restrict__ h2)
+{
+    pdl_enter();
+    const RBlk B = T.d_blk[blockIdx.x];
+    if (lz[B.rep].done[j & 1] || !segs[B.rep].indef) return;
+    const double *hr = h + (long)LZ_KMAX * B.rep;
+    double acc[RB_EPT];
+    lz_ord_load(q + B.start, B.len, threadIdx.x, acc);
+    lz_ord_subtract(V + B.start, ldv, B.len, threadIdx.x, j, hr, acc);
+    lz_ord_store(q + B.start, B.len, threadIdx.x, acc, 1.0);
+    if (threadIdx.x == 0 && (int)blockIdx.x == T.d_first[B.rep]) alpha[(long)LZ_KMAX * B.rep + j] = 0.0 + hr[j];
+    lz_ord_block_dots(T, B, V, ldv, acc, j, part, h2);
+}
+
+// the second pass's subtraction, the norm and the breakdown test in one sweep: alpha_j += h2_j, nrm2 = q.q
+// summed as the segmented dot sums it; the replica's last block records m = j + 1 and stops the
+// replica on an invariant subspace
+__global__ void k_lz_ord_sub_norm(RedTable T, const Seg *__restrict__ segs, const double *__restrict__ V, long ldv,
+                                  double *__restrict__ q, int j, LzScal *__restrict__ lz, const double *__restrict__ h2,
+                                  double *__restrict__ alpha, double *__restrict__ nrm2)
+{
+    pdl_enter();
+    __shared__ double sh[RB_THREADS / 32][1];
+    const RBlk B = T.d_blk[blockIdx.x];
+    if (!segs[B.rep].indef) return;
+    const bool lead = threadIdx.x == 0 && (int)blockIdx.x == T.d_first[B.rep];
+    const int done = lz[B.rep].done[j & 1];
+    if (done) {
+        if (lead) lz[B.rep].done[(j + 1) & 1] = done;
+        return;
+    }
+    const double *hr = h2 + (long)LZ_KMAX * B.rep;
+    double acc[RB_EPT];
+    lz_ord_load(q + B.start, B.len, threadIdx.x, acc);
+    lz_ord_subtract(V + B.start, ldv, B.len, threadIdx.x, j, hr, acc);
+    lz_ord_store(q + B.start, B.len, threadIdx.x, acc, 1.0);
+    if (lead) alpha[(long)LZ_KMAX * B.rep + j] = alpha[(long)LZ_KMAX * B.rep + j] + hr[j];
+    double v[1] = {lz_ord_square(B.len, threadIdx.x, acc)};
+    block_sum<1>(v, sh);
+    double tot[1];
+    if (finish_block<1>(T, B, blockIdx.x, v, tot)) {
+        nrm2[B.rep] = tot[0];
+        lz[B.rep].m = j + 1;
+        lz[B.rep].done[(j + 1) & 1] = sqrt(tot[0]) <= 1e-12 * lz[B.rep].b0 ? 2 : 0;   // 2: finalise with m = j + 1
+    }
+}
+
+// V_{j+1} = q / ||q||; beta_j = ||q||  (norm from nrm2[rep])
+__global__ void k_lz_ord_next(RedTable T, const Seg *__restrict__ segs, double *__restrict__ V, long ldv,
+                              const double *__restrict__ q, int j, const LzScal *__restrict__ lz,
+                              const double *__restrict__ nrm2, double *__restrict__ betad)
+{
+    pdl_enter();
+    const RBlk B = T.d_blk[blockIdx.x];
+    if (lz[B.rep].done[(j + 1) & 1] || !segs[B.rep].indef) return;
+    const double bj = sqrt(nrm2[B.rep]);
+    const double inv = bj > 0 ? 1.0 / bj : 0.0;
+    for (int e = threadIdx.x; e < B.len; e += RB_THREADS) V[(long)(j + 1) * ldv + B.start + e] = q[B.start + e] * inv;
+    if (threadIdx.x == 0 && (int)blockIdx.x == T.d_first[B.rep]) betad[(long)LZ_KMAX * B.rep + j] = bj;
+}
+
 namespace cgr = cooperative_groups;
 
 __global__ void __cluster_dims__(LZC_CTAS, 1, 1) __launch_bounds__(LZC_THREADS)
-k_lz_orth_cluster(const Seg *__restrict__ segs, double *__restrict__ V, long ldv, double *__restrict__ q, int j,
-                  int kmax, LzScal *__restrict__ lz, double *__restrict__ alpha, double *__restrict__ betad)
+k_lz_orth_cluster(const Seg *__restrict__ segs, const int *__restrict__ reps, double *__restrict__ V, long ldv,
+                  const double *__restrict__ q, int j, int kmax, LzScal *__restrict__ lz, double *__restrict__ alpha,
+                  double *__restrict__ betad)
 {
     pdl_enter();
     cgr::cluster_group cl = cgr::this_cluster();
     const int rank = (int)cl.block_rank();
-    const int r = blockIdx.x / LZC_CTAS;
+    const int r = reps[blockIdx.x / LZC_CTAS];
     const int half = threadIdx.x / RB_THREADS, t = threadIdx.x % RB_THREADS;
     const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
     constexpr int HW = RB_THREADS / 32;                   // warps per half
-    __shared__ double part[2][LZC_HALVES][LZC_SLOTS][LZ_KMAX + 1];   // per pass: RB-block partial dots
-    __shared__ double npart[LZC_HALVES][LZC_SLOTS];       // RB-block partial norms
+    __shared__ double part[2][LZC_HALVES][LZ_KMAX];       // per pass: the table block's partial dots
+    __shared__ double npart[LZC_HALVES];                  // ... and partial norms
     __shared__ double sh[LZC_THREADS / 32][8];
-    __shared__ double hsh[LZ_KMAX + 1];
+    __shared__ double hsh[LZ_KMAX];
     const Seg &s = segs[r];
-    if (!lz_fixed(s)) return;                   // the whole cluster
     const int done = lz[r].done[j & 1];
-    if (done) {
+    if (done) {                                 // the whole cluster
         if (rank == 0 && threadIdx.x == 0) lz[r].done[(j + 1) & 1] = done;
         return;
     }
-    const int n = s.nm3nc11;
-    const long base = s.top_off;
-    const int nb = (n + RB_SPAN - 1) / RB_SPAN, nslot = (nb + LZC_VB - 1) / LZC_VB;
-    const int vb = rank * LZC_HALVES + half;
-    double alpha_j = 0.0;
+    const int n = s.nm3nc11, nb = (n + RB_SPAN - 1) / RB_SPAN;
+    const int rb = rank * LZC_HALVES + half;              // this half's table block
+    const int len = rb < nb ? min(RB_SPAN, n - rb * RB_SPAN) : 0;
+    const long st = (long)s.top_off + (long)rb * RB_SPAN;
+    double alpha_j = 0.0, qv[RB_EPT];
+    lz_ord_load(q + st, len, t, qv);
     for (int pass = 0; pass < 2; pass++) {
-        for (int sl = 0; sl < nslot; sl++) {
-            const int rb = vb + LZC_VB * sl;
-            const long st = (long)rb * RB_SPAN;
-            const int len = rb < nb ? min(RB_SPAN, n - rb * RB_SPAN) : 0;
-            double qv[RB_EPT];
+        for (int i0 = 0; i0 <= j; i0 += 8) {
+            double v[8];
 #pragma unroll
-            for (int k = 0; k < RB_EPT; k++) {
-                const int e = t + k * RB_THREADS;
-                qv[k] = e < len ? q[base + st + e] : 0.0;
-            }
-            for (int i0 = 0; i0 <= j; i0 += 8) {
-                double v[8];
+            for (int c = 0; c < 8; c++) {
+                v[c] = 0.0;
+                if (i0 + c <= j) {
+                    const double *Vi = V + (long)(i0 + c) * ldv + st;
 #pragma unroll
-                for (int c = 0; c < 8; c++) {
-                    v[c] = 0.0;
-                    if (i0 + c <= j) {
-                        const double *Vi = V + (long)(i0 + c) * ldv + base + st;
-#pragma unroll
-                        for (int k = 0; k < RB_EPT; k++) {
-                            const int e = t + k * RB_THREADS;
-                            if (e < len) v[c] += Vi[e] * qv[k];
-                        }
+                    for (int k = 0; k < RB_EPT; k++) {
+                        const int e = t + k * RB_THREADS;
+                        if (e < len) v[c] += Vi[e] * qv[k];
                     }
                 }
-#pragma unroll
-                for (int c = 0; c < 8; c++) {
-                    double x = v[c];
-                    for (int o = 16; o > 0; o >>= 1) x += __shfl_down_sync(0xffffffffu, x, o);
-                    if (lane == 0) sh[wid][c] = x;
-                }
-                __syncthreads();
-                if (t < 8 && i0 + t <= j) {
-                    double x = 0.0;
-                    for (int w = 0; w < HW; w++) x += sh[half * HW + w][t];
-                    part[pass][half][sl][i0 + t] = x;
-                }
-                __syncthreads();
             }
+#pragma unroll
+            for (int c = 0; c < 8; c++) {
+                double x = v[c];
+                for (int o = 16; o > 0; o >>= 1) x += __shfl_down_sync(0xffffffffu, x, o);
+                if (lane == 0) sh[wid][c] = x;
+            }
+            __syncthreads();
+            if (t < 8 && i0 + t <= j) {
+                double x = 0.0;
+                for (int w = 0; w < HW; w++) x += sh[half * HW + w][t];
+                part[pass][half][i0 + t] = x;
+            }
+            __syncthreads();
         }
         cl.sync();
-        for (int i = threadIdx.x; i <= j; i += LZC_THREADS) {   // h_i over the RB blocks in block order
+        for (int i = threadIdx.x; i <= j; i += LZC_THREADS) {   // h_i over the table blocks in block order
             double h = 0.0;
-            for (int rb = 0; rb < nb; rb++) {
-                const int v2 = rb % LZC_VB;
-                h += cl.map_shared_rank(&part[pass][v2 % LZC_HALVES][rb / LZC_VB][0], v2 / LZC_HALVES)[i];
-            }
+            for (int b = 0; b < nb; b++)
+                h += cl.map_shared_rank(&part[pass][b % LZC_HALVES][0], b / LZC_HALVES)[i];
             hsh[i] = h;
         }
         __syncthreads();
-        for (int sl = 0; sl < nslot; sl++) {                   // q -= sum_i h_i V_i, i = 0..j per element
-            const int rb = vb + LZC_VB * sl;
-            if (rb >= nb) break;
-            const long st = (long)rb * RB_SPAN;
-            const int len = min(RB_SPAN, n - rb * RB_SPAN);
-            for (int k = 0; k < RB_EPT; k++) {
-                const int e = t + k * RB_THREADS;
-                if (e >= len) break;
-                double acc = q[base + st + e];
-                for (int i = 0; i <= j; i++) acc -= hsh[i] * V[(long)i * ldv + base + st + e];
-                q[base + st + e] = acc;
-            }
-        }
+        lz_ord_subtract(V + st, ldv, len, t, j, hsh, qv);
         alpha_j += hsh[j];
         __syncthreads();
     }
-    for (int sl = 0; sl < nslot; sl++) {                       // RB-block norms, as seg_dot
-        const int rb = vb + LZC_VB * sl;
-        const long st = (long)rb * RB_SPAN;
-        const int len = rb < nb ? min(RB_SPAN, n - rb * RB_SPAN) : 0;
-        double x = 0.0;
-        for (int e = t; e < len; e += RB_THREADS) x += q[base + st + e] * q[base + st + e];
+    {                                                          // the block's norm, as seg_dot sums it
+        double x = lz_ord_square(len, t, qv);
         for (int o = 16; o > 0; o >>= 1) x += __shfl_down_sync(0xffffffffu, x, o);
         if (lane == 0) sh[wid][0] = x;
         __syncthreads();
         if (t == 0) {
             double y = 0.0;
             for (int w = 0; w < HW; w++) y += sh[half * HW + w][0];
-            npart[half][sl] = y;
+            npart[half] = y;
         }
-        __syncthreads();
     }
     cl.sync();
     double nrm2 = 0.0;
-    for (int rb = 0; rb < nb; rb++) {
-        const int v2 = rb % LZC_VB;
-        nrm2 += cl.map_shared_rank(&npart[v2 % LZC_HALVES][rb / LZC_VB], v2 / LZC_HALVES)[0];
-    }
+    for (int b = 0; b < nb; b++) nrm2 += cl.map_shared_rank(&npart[b % LZC_HALVES], b / LZC_HALVES)[0];
     cl.sync();                                  // no block leaves while others read its shared memory
     const double bj = sqrt(nrm2);
     const bool broken = bj <= 1e-12 * lz[r].b0;
@@ -1018,16 +1180,7 @@ k_lz_orth_cluster(const Seg *__restrict__ segs, double *__restrict__ V, long ldv
         lz[r].done[(j + 1) & 1] = broken ? 2 : 0;   // 2, an invariant subspace: finalise with m = j + 1
         if (!broken && j + 1 < kmax) betad[(long)LZ_KMAX * r + j] = bj;
     }
-    if (!broken && j + 1 < kmax) {
-        const double inv = bj > 0 ? 1.0 / bj : 0.0;
-        for (int sl = 0; sl < nslot; sl++) {
-            const int rb = vb + LZC_VB * sl;
-            if (rb >= nb) break;
-            const long st = (long)rb * RB_SPAN;
-            const int len = min(RB_SPAN, n - rb * RB_SPAN);
-            for (int e = t; e < len; e += RB_THREADS) V[(long)(j + 1) * ldv + base + st + e] = q[base + st + e] * inv;
-        }
-    }
+    if (!broken && j + 1 < kmax) lz_ord_store(V + (long)(j + 1) * ldv + st, len, t, qv, bj > 0 ? 1.0 / bj : 0.0);
 }
 
 int lanczos_sqrt(Engine &E, const double *z, double *w, const ps_sqrt_opts *o, ps_sqrt_result *res, cudaStream_t st)
@@ -1050,8 +1203,8 @@ int lanczos_sqrt(Engine &E, const double *z, double *w, const ps_sqrt_opts *o, p
     ps_launch(k_lz_init, T.nblk, RB_THREADS, 0, st, T, E.d_segs, V, z, lz, nrm2);
     PS_CK(cudaMemsetAsync(gbuf, 0, sizeof(double) * (LZ_KMAX + 1) * E.R, st));
     const int check = 8;   // convergence test every 8 vectors; the cap is handled after the loop
-    bool any_fixed = false, any_free = false;
-    for (const Seg &sg : E.segs) (lz_fixed(sg) ? any_fixed : any_free) = true;
+    const bool any_free = E.n_lz_ord < E.R;
+    double *h = nrm2 + E.R, *h2 = h + (long)LZ_KMAX * E.R;  // [R][LZ_KMAX]: both passes' dots of the ordered replicas
     const size_t smem = sizeof(double) * LZE_SMEM, smem_ql = sizeof(double) * (4 * LZ_KMAX + LZ_KMAX * LZ_KMAX);
     PS_CK(cudaFuncSetAttribute(k_lz_check, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
     std::vector<LzScal> hl(E.R);
@@ -1066,8 +1219,17 @@ int lanczos_sqrt(Engine &E, const double *z, double *w, const ps_sqrt_opts *o, p
         apply_operator(E, 1, V + (long)j * ldv, q, E.precision == PS_PREC_MIXED, st, &lz[0].done[j & 1],
                        (int)sizeof(LzScal), false, any_free ? &dots : nullptr);
         const dim3 sub((unsigned)T.nblk, RB_EPT);
-        if (any_fixed)
-            ps_launch(k_lz_orth_cluster, E.R * LZC_CTAS, LZC_THREADS, 0, st, E.d_segs, V, ldv, q, j, kmax, lz, alpha, betad);
+        if (E.n_lz_ord && E.lz_cluster)
+            ps_launch(k_lz_orth_cluster, E.n_lz_ord * LZC_CTAS, LZC_THREADS, 0, st, E.d_segs, E.d_lz_ord, V, ldv, q, j, kmax,
+                    lz, alpha, betad);
+        else if (E.n_lz_ord) {
+            // the ordered replicas' blocks leave their part of part2 to these sums
+            ps_launch(k_lz_ord_dots, T.nblk, RB_THREADS, 0, st, T, E.d_segs, V, ldv, q, j, lz, part2, h);
+            ps_launch(k_lz_ord_sub_dots, T.nblk, RB_THREADS, 0, st, T, E.d_segs, V, ldv, q, j, lz, h, alpha, part2, h2);
+            ps_launch(k_lz_ord_sub_norm, T.nblk, RB_THREADS, 0, st, T, E.d_segs, V, ldv, q, j, lz, h2, alpha, nrm2);
+            if (j + 1 < kmax)
+                ps_launch(k_lz_ord_next, T.nblk, RB_THREADS, 0, st, T, E.d_segs, V, ldv, q, j, lz, nrm2, betad);
+        }
         if (any_free) {
             ps_launch(k_lz_sub_dots, sub, RB_THREADS, 0, st, T, E.d_segs, V, ldv, q, j, lz, part1, alpha, part2, npart);
             ps_launch(k_lz_sub_scale, sub, RB_THREADS, 0, st, T, E.d_segs, V, ldv, q, j, kmax, lz, part2, npart, alpha,
@@ -1090,8 +1252,8 @@ int lanczos_sqrt(Engine &E, const double *z, double *w, const ps_sqrt_opts *o, p
             if (any_free)
                 ps_launch(k_lz_check, E.R, LZE_THREADS, smem, E.side2, E.R, E.d_segs, lz, snap, spec, alpha, betad, gbuf,
                         j + 1, cur, tol, 0);
-            if (any_fixed)
-                ps_launch(k_lz_check_ql, E.R, 32, smem_ql, E.side2, E.R, E.d_segs, lz, snap, spec, alpha, betad, gbuf, j + 1,
+            if (E.n_lz_ord)
+                ps_launch(k_lz_check_ql, E.n_lz_ord, 32, smem_ql, E.side2, E.d_lz_ord, lz, snap, spec, alpha, betad, gbuf, j + 1,
                         cur, tol, 0);
             PS_CK(cudaMemcpyAsync(hspec, spec, sizeof(LzSpec) * E.R, cudaMemcpyDeviceToHost, E.side2));
             PS_CK(cudaEventRecord(E.ev_chk, E.side2));
@@ -1107,8 +1269,8 @@ int lanczos_sqrt(Engine &E, const double *z, double *w, const ps_sqrt_opts *o, p
     if (any_free)
         ps_launch(k_lz_check, E.R, LZE_THREADS, smem, st, E.R, E.d_segs, lz, snap, spec, alpha, betad, gbuf,
                 std::min(j + 1, kmax), cur, tol, 1);
-    if (any_fixed)
-        ps_launch(k_lz_check_ql, E.R, 32, smem_ql, st, E.R, E.d_segs, lz, snap, spec, alpha, betad, gbuf,
+    if (E.n_lz_ord)
+        ps_launch(k_lz_check_ql, E.n_lz_ord, 32, smem_ql, st, E.d_lz_ord, lz, snap, spec, alpha, betad, gbuf,
                 std::min(j + 1, kmax), cur, tol, 1);
     ps_launch(k_lz_combine, T.nblk, RB_THREADS, 0, st, T, V, ldv, lz, gbuf, w);
     PS_CK(cudaMemcpyAsync(hl.data(), lz, sizeof(LzScal) * E.R, cudaMemcpyDeviceToHost, st));

@@ -99,7 +99,7 @@ struct Seg {
     int nper;          // monomers per chain
     int ss_off;        // offset of the inverse stresslet block (nc5^2 doubles), -1 if none
     int nch_bb;        // column chunks of the colloid far field (a function of Nc alone)
-    int indef;         // the replica's far field may be indefinite (krylov.cu lz_fixed)
+    int indef;         // the replica's far field may be indefinite (krylov.cu, k_lz_orth_cluster)
     int aa_nt;         // tiles of the monomer far field (0: no monomer pairs), and as many partial slots per row
     long paa_off;      // this replica's monomer far-field partials: aa_nt slots of nm3 doubles
     // monomer-monomer scalars as x = c0/r + c1/r^3, y = c2/r + c3/r^3 (r > 2 beta)

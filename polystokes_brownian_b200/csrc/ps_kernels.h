@@ -182,6 +182,8 @@ struct Engine {
     int lz_kmax = 0;
     double *d_lzV = nullptr, *d_lzT = nullptr, *d_lzp = nullptr, *d_lzw = nullptr, *d_lzq = nullptr;
     double *d_lzs = nullptr;
+    int *d_lz_ord = nullptr, n_lz_ord = 0;         // replicas that keep the order of their Lanczos sums (Seg::indef)
+    bool lz_cluster = false;                       // ... in one cluster launch per vector
 
     cudaStream_t side2 = nullptr;                  // Lanczos convergence checks beside the next basis vectors
     cudaEvent_t ev_fork2 = nullptr, ev_chk = nullptr;
@@ -243,6 +245,7 @@ int structured_solve(Engine &E, const double *b, double *x, const ps_ksp_opts *o
                      cudaStream_t st);
 int schur_lanczos_noise(Engine &E, const double *fb, const double *ymcm, double *W, int *nneg, cudaStream_t st);
 int lanczos_sqrt(Engine &E, const double *z, double *w, const ps_sqrt_opts *o, ps_sqrt_result *res, cudaStream_t st);
+void lz_ordered_list(Engine &E, std::vector<int> &reps);       // fills n_lz_ord and lz_cluster
 int build_red_table(Engine &E, RedTable &T, int layout);   // 0 saddle, 1 top, 2 velocity
 void free_red_table(RedTable &T);
 void seg_dot(Engine &E, RedTable &T, const double *a, const double *b, double *out_per_rep, cudaStream_t st);
