@@ -93,7 +93,7 @@ static int build(Engine &E, const ps_desc *descs, int R, int precision)
     long bead = 0, coll = 0, vec = 0, top = 0, vel = 0, schur = 0, ba = 0, cells = 0, ssinv = 0;
     std::vector<int> bead_offs(R + 1), vec_offs(R + 1), top_offs(R + 1), vel_offs(R + 1);
     std::vector<long> cell_offs(R + 1);
-    std::vector<Tile> bb, bbw;
+    std::vector<Tile> bb;
     std::vector<int> schur_reps, ss_reps, sl_reps;
     long slv = 0;
     int ss_polish = 0;
@@ -165,12 +165,6 @@ static int build(Engine &E, const ps_desc *descs, int R, int precision)
         s.n_mtiles = (d.Nm + TR - 1) / TR;
         s.ba_off = (int)ba;
         if (d.Nc > 0) ba += (long)s.n_mtiles * d.Nc;
-        if (d.Nm == 0 && d.Nc >= 2)
-        {
-            const bool wide = bb_wide(d.Nc, s.nch_bb);
-            const int tr = wide ? BB_WIDE : BB_TILE;
-            for (int t = 0; t * tr < d.Nc; t++) (wide ? bbw : bb).push_back({r, t * tr, std::min(tr, d.Nc - t * tr), t});
-        }
         bead_offs[r] = (int)bead; vec_offs[r] = (int)vec; top_offs[r] = (int)top; vel_offs[r] = (int)vel;
         cell_offs[r] = cells;
         cells += CELL_CAP_PER_MONO * d.Nm + CELL_CAP_BASE;
@@ -198,9 +192,20 @@ static int build(Engine &E, const ps_desc *descs, int R, int precision)
     auto by_cost = [&](const Tile &a, const Tile &b) {
         return E.segs[a.rep].Np > E.segs[b.rep].Np || (E.segs[a.rep].Np == E.segs[b.rep].Np && a.rep < b.rep);
     };
+    long nb[2] = {0, 0};               // blocks of the colloid far field's own kernel, narrow and wide tiles
+    for (const Seg &s : E.segs)
+        if (s.Nm == 0 && s.Nc >= 2) {
+            nb[0] += (s.Nc + BB_TILE - 1) / BB_TILE * (long)s.nch_bb;
+            nb[1] += (s.Nc + BB_WIDE - 1) / BB_WIDE * (long)s.nch_bb;
+        }
+    E.bb_wide = bb_wide(nb[0], nb[1]);
+    const int tr = E.bb_wide ? BB_WIDE : BB_TILE;
+    for (int r = 0; r < R; r++) {
+        const int Nc = E.segs[r].Nc;
+        if (E.segs[r].Nm == 0 && Nc >= 2)
+            for (int t = 0; t * tr < Nc; t++) bb.push_back({r, t * tr, std::min(tr, Nc - t * tr), t});
+    }
     std::stable_sort(bb.begin(), bb.end(), by_cost);
-    E.n_bb_wide = (int)bbw.size();
-    bb.insert(bb.begin(), bbw.begin(), bbw.end());
     E.n_bb_tiles = (int)bb.size();
     // grid extent in chunks: the largest per-replica chunk count
     E.nch_bb = 1;

@@ -122,12 +122,15 @@ constexpr int aa_tile_edge(int Nm) { return Nm <= 1536 ? 64 : (Nm <= 12288 ? 128
 struct AaTile { int rep, I, J, S; };
 constexpr int FAR_AB = 0, FAR_BB = -1;
 
-// Column chunk width of the colloid far field, for up to BB_MAX_CHUNKS chunks, and its row tiles:
-// BB_TILE rows (four blocks per SM), BB_WIDE rows (one block per SM) where those are one wave that
-// nearly fills the chip.  Both add in the same order.  One launch with 32 and with 128 rows:
-// 512 colloids 9.6 and 17.8 us, 1024 colloids (128 wide blocks) 19.8 and 18.1, 1600 (325) 37.9 and 51.1.
+// Column chunk width of the colloid far field, for up to BB_MAX_CHUNKS chunks, and the row tiles of its own
+// kernel (replicas without monomers): BB_TILE rows, or BB_WIDE rows for the whole context.  Both add in
+// the same order, so the choice may look at the launch: wide where the wide blocks find an SM each and the
+// narrow ones would put four on some SM, which then works through as many rows a column, in four blocks
+// that each load the columns.  One launch with 32 and with 128 rows, us: 928 colloids (435 narrow blocks, three
+// an SM) 15.9 and 17.5; 960 (450) 19.8 and 17.9; 1024 (512) 19.8 and 17.9; two replicas of 768 (576) 19.8 and
+// 17.8; 1025 (153 wide blocks) 19.0 and 32.1; two of 1024 31.0 and 34.4; 1600 38.1 and 50.2.
 constexpr int BB_TILE = 32, BB_WIDE = 128, BB_CHUNK_COLS = 64, BB_MAX_CHUNKS = 64;
-constexpr bool bb_wide(int Nc, int nch) { return (Nc + BB_WIDE - 1) / BB_WIDE * nch <= 148 && Nc > 896; }
+constexpr bool bb_wide(long narrow_blocks, long wide_blocks) { return wide_blocks <= 148 && narrow_blocks > 3 * 148; }
 
 // Row tile of the far-field pair kernels.
 struct Tile { int rep; int row0; int nrow; int mtile; };

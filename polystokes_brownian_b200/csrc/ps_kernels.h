@@ -82,8 +82,9 @@ struct Engine {
 
     // far-field pair work lists
     AaTile *d_aa_tiles = nullptr;    // n_far_pre monomer-colloid and colloid blocks, then n_aa_tiles monomer tile pairs
-    Tile *d_bb_tiles = nullptr;      // colloid row tiles of the replicas without monomers, the n_bb_wide wide ones first
-    int n_far_pre = 0, n_aa_tiles = 0, n_bb_tiles = 0, n_bb_wide = 0, nch_bb = 1;
+    Tile *d_bb_tiles = nullptr;      // colloid row tiles of the replicas without monomers, BB_WIDE rows each or BB_TILE
+    int n_far_pre = 0, n_aa_tiles = 0, n_bb_tiles = 0, nch_bb = 1;
+    bool bb_wide = false;
     long part_stride = 0;
     double *d_partAA = nullptr, *d_partAB = nullptr, *d_partBB = nullptr, *d_partBA = nullptr;
     long nba = 0;

@@ -902,12 +902,14 @@ static void launch_far(Engine &E, const double *u, int in_top, bool fp32, int fi
 
 static void launch_bb(Engine &E, const double *u, int in_top, cudaStream_t st, const char *done, int dstride)
 {
-    if (E.n_bb_wide)
-        ps_launch(k_rpy_bb<BB_WIDE>, dim3(E.n_bb_wide, E.nch_bb), BB_WIDE * BB_SPLIT, 0, st, E.d_segs, E.d_bb_tiles,
-                E.d_pos64, u, in_top, E.d_partBB, E.part_stride, done, dstride);
-    if (E.n_bb_tiles > E.n_bb_wide)
-        ps_launch(k_rpy_bb<BB_ROWS>, dim3(E.n_bb_tiles - E.n_bb_wide, E.nch_bb), BB_ROWS * BB_SPLIT, 0, st, E.d_segs,
-                E.d_bb_tiles + E.n_bb_wide, E.d_pos64, u, in_top, E.d_partBB, E.part_stride, done, dstride);
+    if (!E.n_bb_tiles) return;
+    const dim3 grid(E.n_bb_tiles, E.nch_bb);
+    if (E.bb_wide)
+        ps_launch(k_rpy_bb<BB_WIDE>, grid, BB_WIDE * BB_SPLIT, 0, st, E.d_segs, E.d_bb_tiles, E.d_pos64, u, in_top, E.d_partBB,
+                E.part_stride, done, dstride);
+    else
+        ps_launch(k_rpy_bb<BB_ROWS>, grid, BB_ROWS * BB_SPLIT, 0, st, E.d_segs, E.d_bb_tiles, E.d_pos64, u, in_top, E.d_partBB,
+                E.part_stride, done, dstride);
 }
 
 void apply_operator(Engine &E, int mode, const double *x, double *y, bool fp32, cudaStream_t st,
