@@ -277,8 +277,10 @@ uint64_t ps_kernel_launches(void);
  * edge in {128, 256, 512, 1024} (reps applies each, CUDA events; tiles are at
  * most 256 wide, so 512 and 1024 stand for no lower limit than 256) and keeps
  * the fastest for this context and for every context created afterwards in the
- * process.  The edge is process-wide so that a replica's arithmetic stays
- * independent of its batch.
+ * process.  Edges that cut every replica of the context alike are timed once and
+ * reported alike (replicas of up to 12288 monomers have tiles of at most 128 in
+ * any case), and where all four do, the edge in force stays.  The edge is
+ * process-wide so that a replica's arithmetic stays independent of its batch.
  * best_cols / ms (4 timings, candidate order) may be NULL. */
 int ps_autotune(ps_ctx *ctx, int32_t reps, int32_t *best_cols, double *ms, void *stream);
 

@@ -729,7 +729,6 @@ int ps_time_kernel(ps_ctx *ctx, int32_t which, int32_t reps, const double *u, do
 
 uint64_t ps_kernel_launches(void) { return (uint64_t)ps_launch_count; }
 
-
 int ps_autotune(ps_ctx *ctx, int32_t reps, int32_t *best_cols, double *ms, void *stream)
 {
     if (!ctx) return PS_ERR_ARG;
@@ -739,17 +738,22 @@ int ps_autotune(ps_ctx *ctx, int32_t reps, int32_t *best_cols, double *ms, void 
     double *u = nullptr;
     PS_CK(cudaMalloc(&u, sizeof(double) * std::max<long>(E.ntop, 1)));
     PS_CK(cudaMemsetAsync(u, 0, sizeof(double) * std::max<long>(E.ntop, 1), S(stream)));
-    int best = ps::g_aa_chunk_cols, rc = PS_OK;
-    double tbest = 1e300;
+    // candidates that cut this context alike are one measurement; a context that they all cut alike leaves
+    // the edge in force as it is, for the sake of the contexts to come
+    const int now = ps::g_aa_chunk_cols;
+    int rc = PS_OK;
     for (int k = 0; k < 4 && rc == PS_OK; k++) {
-        if ((rc = ps::set_aa_chunking(E, cand[k]))) break;
-        rc = ps::time_pairs(E, 3, reps > 0 ? reps : 5, u, &t[k], S(stream));   // apply incl. combine
-        if (rc == PS_OK && t[k] < tbest) { tbest = t[k]; best = cand[k]; }
+        if (k > 0 && ps::same_aa_chunking(E, cand[k], cand[k - 1])) t[k] = t[k - 1];
+        else if (!(rc = ps::set_aa_chunking(E, cand[k])))
+            rc = ps::time_pairs(E, 3, reps > 0 ? reps : 5, u, &t[k], S(stream));   // apply incl. combine
     }
     cudaFree(u);
-    if (rc) return rc;
+    const int first = (int)(std::min_element(t, t + 4) - t);
+    const int best = std::any_of(cand, cand + 4, [&](const int &c) { return c == now && t[&c - cand] == t[first]; }) ? now : cand[first];
+    // a failure (memory) leaves the context with the edge it had
+    const int back = ps::set_aa_chunking(E, rc ? now : best);
+    if (rc || back) return rc ? rc : back;
     ps::g_aa_chunk_cols = best;
-    if ((rc = ps::set_aa_chunking(E, best))) return rc;
     if (best_cols) *best_cols = best;
     if (ms) for (int k = 0; k < 4; k++) ms[k] = t[k];
     return PS_OK;

@@ -196,6 +196,7 @@ struct Engine {
 // independent of its batch); set by ps_autotune
 extern int g_aa_chunk_cols;
 int set_aa_chunking(Engine &E, int cols);
+bool same_aa_chunking(const Engine &E, int a, int b);      // whether both widest edges cut the context's replicas alike
 
 // true when p is host memory (pageable or pinned): the C-ABI accepts host
 // pointers for state and noise arguments and copies them itself

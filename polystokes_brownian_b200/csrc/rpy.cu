@@ -940,6 +940,15 @@ void apply_operator(Engine &E, int mode, const double *x, double *y, bool fp32, 
 
 int g_aa_chunk_cols = AA_TILE_MAX;
 
+static int capped_edge(const Seg &s, int cols) { return std::min(aa_tile_edge(s.Nm), std::max(cols, AA_TILE_MIN)); }
+
+bool same_aa_chunking(const Engine &E, int a, int b)
+{
+    return std::all_of(E.segs.begin(), E.segs.end(), [&](const Seg &s) {
+        return !s.mm_HI || s.Nm < 2 || capped_edge(s, a) == capped_edge(s, b);
+    });
+}
+
 // tiles of the monomer far field for a widest edge of `cols`: per-replica edges and
 // partial slots, the list of tile pairs (large tiles first) and the partial buffer
 int set_aa_chunking(Engine &E, int cols)
@@ -949,7 +958,7 @@ int set_aa_chunking(Engine &E, int cols)
     for (int r = 0; r < E.R; r++) {
         Seg &s = E.segs[r];
         const bool on = s.mm_HI && s.Nm >= 2;
-        const int S = std::min(aa_tile_edge(s.Nm), std::max(cols, AA_TILE_MIN));
+        const int S = capped_edge(s, cols);
         s.aa_nt = on ? (s.Nm + S - 1) / S : 0;
         s.paa_off = off;
         off += (long)s.aa_nt * s.nm3;
@@ -980,6 +989,7 @@ int set_aa_chunking(Engine &E, int cols)
     if (!tiles.empty())
         PS_CK(cudaMemcpy(E.d_aa_tiles, tiles.data(), sizeof(AaTile) * tiles.size(), cudaMemcpyHostToDevice));
     PS_CK(cudaMemcpy(E.d_segs, E.segs.data(), sizeof(Seg) * E.segs.size(), cudaMemcpyHostToDevice));
+    PS_CK(cudaDeviceSynchronize());      // a copy from pageable memory may return ahead of its transfer
     return PS_OK;
 }
 
