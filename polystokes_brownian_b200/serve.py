@@ -73,6 +73,7 @@ class _Slot:
     done_steps: int = 0
     rng_steps: int = 0
     admitted: float = 0.0
+    footprint: int = 0
     result: Result | None = None
 
 
@@ -80,15 +81,17 @@ class _Slot:
 AA_TILE_EDGES = ((1536, 64), (12288, 128), (math.inf, 256))
 
 
-def footprint_bytes(sysm: System, precision: int = _capi.PS_PREC_MIXED, lanczos_kmax: int = 64) -> int:
+def footprint_bytes(sysm: System, precision: int = _capi.PS_PREC_MIXED, lanczos_kmax: int = 64,
+                    widest_edge: int = 256) -> int:
     """Device bytes one replica holds in a context: saddle vectors (13), mobility
     vectors incl. the Lanczos basis (kmax + 6), far-field partials (one slot per
-    monomer tile, AA_TILE_EDGES as aa_tile_edge in csrc/ps_internal.h),
-    velocity vectors (27), positions, lists."""
+    monomer tile, AA_TILE_EDGES as aa_tile_edge in csrc/ps_internal.h, at most the
+    widest edge that the autotuner left in force), velocity vectors (27), positions,
+    lists."""
     p = sysm.params
     Nm, Nc = p["Nm"], p["Nc"]
     n, top, vel, Np = 6 * Nm + 17 * Nc, 3 * Nm + 11 * Nc, 3 * Nm + 6 * Nc, Nm + Nc
-    nch = max(1, math.ceil(Nm / next(e for n_max, e in AA_TILE_EDGES if Nm <= n_max)))
+    nch = max(1, math.ceil(Nm / min(widest_edge, next(e for n_max, e in AA_TILE_EDGES if Nm <= n_max))))
     b = 8 * (13 * n + (lanczos_kmax + 6 + nch) * top + 27 * vel) + 160 * Np + 4 * 16 * Np
     if Nc and 5 * Nc <= 64:
         b += 8 * (5 * Nc) ** 2
@@ -113,6 +116,7 @@ def make_trace(n_req: int, rate: float, seed: int = 0, nmin: int = 64, nmax: int
 
 class Server:
     _tuned = False
+    aa_chunk_cols = 256                     # the process's widest tile edge
 
     def __init__(self, precision: int = _capi.PS_PREC_MIXED, budget_bytes: float = 150e9, max_slots: int = 256,
                  rtol: float = 1e-6, solver: int = _capi.PS_SOLVE_STRUCTURED, rebuild_every: int = 1,
@@ -165,7 +169,7 @@ class Server:
         if not Server._tuned:
             # one process-wide choice, so every later context tiles replicas the same way
             b.stage()
-            self.aa_chunk_cols, _ = b.autotune(3)
+            Server.aa_chunk_cols, _ = b.autotune(3)
             Server._tuned = True
         self.rebuilds += 1
         return b
@@ -209,10 +213,10 @@ class Server:
                     b.close()
                 groups = []
                 for s in finished:
-                    used -= footprint_bytes(s.req.system, self.precision)
+                    used -= s.footprint
                 active = live
                 while pending and pending[0].arrival <= now() and len(active) < self.max_slots:
-                    fb = footprint_bytes(pending[0].system, self.precision)
+                    fb = footprint_bytes(pending[0].system, self.precision, widest_edge=Server.aa_chunk_cols)
                     if fb > self.budget:
                         req = pending.popleft()
                         results.append(Result(req.rid, np.zeros(0), np.zeros(0), 0, req.arrival, now(), now(),
@@ -223,6 +227,7 @@ class Server:
                     req = pending.popleft()
                     used += fb
                     active.append(self._admit(req, now()))
+                    active[-1].footprint = fb
                 if not active:
                     if pending:
                         wait = pending[0].arrival - now()
