@@ -58,11 +58,11 @@ static void free_engine(Engine &E)
                     E.d_tab, E.d_stale, E.d_aa_last, E.d_delta, E.d_schurR, E.d_schur_reps, E.d_ss_reps,
                     E.d_bond_ptr, E.d_bond_nbr, E.d_bond_sgn, E.d_cell, E.d_cell_start, E.d_cell_sorted,
                     E.d_cell_count, E.d_cellgeo, E.d_cell_offs, E.d_nbr_ptr, E.d_nbr, E.d_nbr_count, E.d_lubtab,
-                    E.d_luby, E.d_lub_diag, E.d_lub_ptr, E.d_lub_nbr, E.d_lub_cidx, E.d_tmp_vel, E.d_tmp_vel2, E.d_zlub, E.d_D, E.d_z, E.d_v, E.d_xw, E.d_Rr[0],
+                    E.d_luby, E.d_lub_diag, E.d_lub_ptr, E.d_lub_nbr, E.d_lub_cidx, E.d_tmp_vel, E.d_tmp_vel2, E.d_zlub, E.d_D, E.d_z, E.d_v, E.d_Rr[0],
                     E.d_Rr[1], E.d_Rr[2], E.d_W[0], E.d_W[1], E.d_W[2], E.d_mr, E.d_mrp, E.d_nactive,
                     E.d_rhs, E.d_X, E.d_Xd, E.d_Xdet, E.d_Wn, E.d_vdn, E.d_vdc, E.d_vb, E.d_up, E.d_ud,
                     E.d_drift, E.d_sb, E.d_fext, E.d_fb, E.d_wr, E.d_tmp_top, E.d_tmp_top2, E.d_lzV, E.d_lzT,
-                    E.d_lzw, E.d_lzq, E.d_lzp, E.d_lzs, E.d_lz_ord, E.d_ssinv, E.d_pcg, E.d_pV, E.d_pz, E.d_pp,
+                    E.d_lzq, E.d_lzp, E.d_lzs, E.d_lz_ord, E.d_ssinv, E.d_pcg, E.d_pV, E.d_pz, E.d_pp,
                     E.d_pblk, E.d_pbp, E.d_pg, E.d_pu, E.d_py, E.d_pu2, E.d_py2, E.d_rseed, E.d_rstep,
                     E.d_lubc_ptr, E.d_lubc_nbr, E.d_lub_pairs, E.d_pS, E.d_pP, E.d_py_[0], E.d_py_[1], E.d_py_[2],
                     E.d_py_[3], E.d_py_[4], E.d_scan_sums, E.d_pmr,
@@ -187,7 +187,6 @@ static int build(Engine &E, const ps_desc *descs, int R, int precision)
     E.ncells = cells;
     E.need_cells = true;
     E.n_schur_reps = (int)schur_reps.size();
-    E.any_shell_schur = E.n_schur_reps > 0;
     // heavy tiles first (columns per tile ~ N of the replica)
     auto by_cost = [&](const Tile &a, const Tile &b) {
         return E.segs[a.rep].Np > E.segs[b.rep].Np || (E.segs[a.rep].Np == E.segs[b.rep].Np && a.rep < b.rep);
@@ -368,7 +367,6 @@ static int build(Engine &E, const ps_desc *descs, int R, int precision)
     for (double **p : velbufs) TRY_ALLOC(*p, sizeof(double) * vel);
     // lubricated structured solve
     if (E.any_lub || ss_polish) {
-        E.n_ssinv = ssinv;
         TRY_ALLOC(E.d_ssinv, sizeof(double) * std::max<long>(ssinv, 1));
         TRY_ALLOC(E.d_pcg, sizeof(ps::PcgScal) * 2 * R);
         double **pv[] = {&E.d_pV, &E.d_pz, &E.d_pp, &E.d_pg};

@@ -119,14 +119,6 @@ __device__ __forceinline__ void lub_pair_coeffs(const double f[10], double a, do
     for (int k = 6; k < 10; k++) g[k] = sc * f[k];
 }
 
-__device__ __forceinline__ void lub_pair_entries(const double d[3], const double f[10], double a, bool mono, int p,
-                                                 int qq, double *Rm)
-{
-    double g[10];
-    lub_pair_coeffs(f, a, g);
-    pair_block_entries(d, g, mono, p, qq, Rm);
-}
-
 // square root (eigenvalues floored at 0) of the symmetric 2 x 2 [[a, b], [b, c]]
 // by one Jacobi rotation: returns its entries tt, tr, rr
 __device__ __forceinline__ void sqrt_sym2(double a, double b, double c, double &tt, double &tr, double &rr)
@@ -164,18 +156,6 @@ __device__ inline void colloid_pair_sqrt_coeffs(const double k[10], double g[10]
     g[4] = 0.5 * (trI + trII); g[5] = 0.5 * (trI - trII);
     g[6] = 0.5 * (sq(cIIp) + sq(cIp)); g[7] = 0.5 * (sq(cIIp) - sq(cIp));
     g[8] = 0.5 * (rrII + rrI); g[9] = 0.5 * (rrII - rrI);
-}
-
-__device__ inline void lub_pair_block(const Seg &s, const double *__restrict__ x, const double *__restrict__ tab, int nrow,
-                               long lo, long hi, bool mono, double *Rm)
-{
-    const double a = mono ? s.beta : 1.0;
-    double d[3], f[10];
-    lub_pair_geom(s, x, tab, nrow, lo, hi, a, d, f);
-    const int nd = mono ? 6 : 12;
-    for (int k = 0; k < nd * nd; k++) Rm[k] = 0.0;
-    for (int p = 0; p < 3; p++)
-        for (int qq = 0; qq < 3; qq++) lub_pair_entries(d, f, a, mono, p, qq, Rm);
 }
 
 // Monomer pair block in closed form.  K = [[A11, A12], [A12, A11]] with

@@ -219,28 +219,6 @@ __device__ __forceinline__ void gt_flat(const T e[3], T xg, T yg, T G[15])
     }
 }
 
-// ht[k][i][j] = yh (e_i w_jk + e_j w_ik), w_ab = eps_abl e_l (mob.cpp:258-276)
-template <class T>
-__device__ __forceinline__ void ht_flat(const T e[3], T yh, T H[15])
-{
-    // w = eps . e (antisymmetric)
-    T w[3][3];
-    w[0][0] = 0; w[1][1] = 0; w[2][2] = 0;
-    w[0][1] = e[2]; w[1][0] = -e[2];
-    w[0][2] = -e[1]; w[2][0] = e[1];
-    w[1][2] = e[0]; w[2][1] = -e[0];
-#pragma unroll
-    for (int k = 0; k < 3; k++) {
-        auto h = [&](int i, int j) -> T { return yh * (e[i] * w[j][k] + e[j] * w[i][k]); };
-        T h22 = h(2, 2);
-        H[k * 5 + 0] = h(0, 0) - h22;
-        H[k * 5 + 1] = T(2) * h(0, 1);
-        H[k * 5 + 2] = T(2) * h(0, 2);
-        H[k * 5 + 3] = T(2) * h(1, 2);
-        H[k * 5 + 4] = h(1, 1) - h22;
-    }
-}
-
 // stress-strain rank-4 tensor entry (mob.cpp:279-298)
 template <class T>
 __device__ __forceinline__ T m4(const T e[3], int i, int j, int k, int l, T xm, T ym, T zm)

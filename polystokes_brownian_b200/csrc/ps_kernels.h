@@ -61,7 +61,7 @@ struct Engine {
     std::vector<Seg> segs;
     long ntot = 0, ncoll = 0, nvec = 0, ntop = 0, nvel = 0;
     int maxNp = 0;
-    bool any_lub = false, any_shell_schur = false, any_kT = false, any_mmhi = false;
+    bool any_lub = false, any_kT = false, any_mmhi = false;
     bool any_aa_ref = false, any_aa_rpy = false;   // replicas with monomers in the reference's / RPY pair scalars
 
     Seg *d_segs = nullptr;
@@ -115,7 +115,6 @@ struct Engine {
     // cell list / pair lists
     int *d_cell = nullptr, *d_cell_start = nullptr, *d_cell_sorted = nullptr, *d_cell_count = nullptr;
     int *d_cell_big = nullptr, *d_cell_nbig = nullptr, *d_cell_tmp = nullptr;   // cells of more than 64 members
-    long ncell_cap = 0;
     double *d_cellgeo = nullptr;     // per replica: org[3], size[3], nc[3] (as double), periodic
     long *d_cell_offs = nullptr;     // per replica: first cell
     long ncells = 0;
@@ -159,11 +158,11 @@ struct Engine {
     RedTable red_top;                // over mobility vectors
     RedTable red_vel;                // over velocity vectors (lubricated PCG)
     // lubricated structured solve: inverse stresslet blocks, PCG state (velocity layout)
-    double *d_ssinv = nullptr; long n_ssinv = 0;
+    double *d_ssinv = nullptr;
     PcgScal *d_pcg = nullptr;
     double *d_pV = nullptr, *d_pz = nullptr, *d_pp = nullptr, *d_pg = nullptr;   // -b_bot, L z, L p, g
     double *d_pu = nullptr, *d_py = nullptr, *d_pu2 = nullptr, *d_py2 = nullptr;   // mobility layout
-    double *d_D = nullptr, *d_z = nullptr, *d_v = nullptr, *d_xw = nullptr;
+    double *d_D = nullptr, *d_z = nullptr, *d_v = nullptr;
     double *d_Rr[3] = {nullptr, nullptr, nullptr}, *d_W[3] = {nullptr, nullptr, nullptr};
     MinresScal *d_mr = nullptr;
     double *d_mrp = nullptr;         // MINRES sub-block sums of both dots
@@ -181,7 +180,7 @@ struct Engine {
 
     // Lanczos workspace
     int lz_kmax = 0;
-    double *d_lzV = nullptr, *d_lzT = nullptr, *d_lzp = nullptr, *d_lzw = nullptr, *d_lzq = nullptr;
+    double *d_lzV = nullptr, *d_lzT = nullptr, *d_lzp = nullptr, *d_lzq = nullptr;
     double *d_lzs = nullptr;
     int *d_lz_ord = nullptr, n_lz_ord = 0;         // replicas that keep the order of their Lanczos sums (Seg::indef)
     bool lz_cluster = false;                       // ... in one cluster launch per vector
@@ -224,7 +223,6 @@ int fma_peak(int fp64, double *tflops, cudaStream_t st);
 int rsqrt_check(const double *a, long n, unsigned long long *max_ulp, cudaStream_t st);
 // lub.cu
 void lub_apply(Engine &E, const double *x_saddle, double *y_vel, cudaStream_t st);
-void lub_apply_vel(Engine &E, const double *u_vel, double *y_vel, cudaStream_t st);
 int lub_build(Engine &E, cudaStream_t st);
 int lub_diag(Engine &E, cudaStream_t st);
 int lub_noise(Engine &E, const double *z, double *rhs, cudaStream_t st);

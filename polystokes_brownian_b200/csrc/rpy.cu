@@ -757,22 +757,7 @@ __global__ void k_rsqrt_check(long n, const double *__restrict__ a, unsigned lon
 // Combine: self terms + pair partials (fixed order) + constraint blocks.
 // mode 0: saddle   y = [[M, B], [B^T, -R_lub]] x   (vectors in saddle layout)
 // mode 1: mobility y_top = M u                      (vectors in top layout)
-__device__ __forceinline__ int find_rep(const int *__restrict__ offs, int R, long k)
-{
-    int lo = 0, hi = R;   // offs[R] = total
-    while (hi - lo > 1) {
-        int mid = (lo + hi) >> 1;
-        if (offs[mid] <= k) lo = mid; else hi = mid;
-    }
-    return lo;
-}
 
-// One block column per entry of the replica-aligned block table of the output
-// layout (saddle vectors for mode 0, mobility vectors for mode 1), so the
-// replica is known without a search and a converged replica's blocks leave at
-// once; blockIdx.y splits an entry's span so that each thread sums one output
-// (a single large replica otherwise leaves most SMs idle while every thread
-// walks its chunk partials four times over).
 // v + the n partial sums p[0], p[stride], ... in order, eight loads in flight
 __device__ __forceinline__ double add_slots(double v, const double *__restrict__ p, int n, long stride)
 {
@@ -840,10 +825,14 @@ __device__ __forceinline__ double combine_entry(const Seg &sg, int mode, int i, 
     return v;
 }
 
+// A block of the grid per entry of the replica-aligned block table of the output layout (saddle vectors for
+// mode 0, mobility vectors for mode 1) and sub-block of it (blockIdx.y), an output per thread: the
+// replica is known without a search, a converged replica's blocks leave at once, and a single
+// replica's partial sums are read by as many threads as it has outputs.
 template <int TAIL, class X>
 __global__ void k_combine(const Seg *__restrict__ segs, RedTable T, int mode, const double *__restrict__ x,
                           const double *__restrict__ partAA, int with_aa,
-                          const double *__restrict__ partAB, const double *__restrict__ partBB, int nchBB,
+                          const double *__restrict__ partAB, const double *__restrict__ partBB,
                           const double *__restrict__ partBA, const double *__restrict__ delta,
                           const double *__restrict__ lub_y, long part_stride, double *__restrict__ y,
                           const char *__restrict__ done, int done_stride, X tail)
@@ -929,13 +918,13 @@ void apply_operator(Engine &E, int mode, const double *x, double *y, bool fp32, 
     const int with_aa = skip_aa ? 0 : 1;
     if (dots)
         ps_launch(k_combine<CB_DOTS, LzDots>, grid, RB_THREADS, 0, st, E.d_segs, T, mode, x, E.d_partAA, with_aa, E.d_partAB, E.d_partBB,
-                E.nch_bb, E.d_partBA, E.d_delta, lub_y, E.part_stride, y, dn, done_stride, *dots);
+                E.d_partBA, E.d_delta, lub_y, E.part_stride, y, dn, done_stride, *dots);
     else if (mr)
         ps_launch(k_combine<CB_MINRES, MrAlpha>, grid, RB_THREADS, 0, st, E.d_segs, T, mode, x, E.d_partAA, with_aa, E.d_partAB, E.d_partBB,
-                E.nch_bb, E.d_partBA, E.d_delta, lub_y, E.part_stride, y, dn, done_stride, *mr);
+                E.d_partBA, E.d_delta, lub_y, E.part_stride, y, dn, done_stride, *mr);
     else
         ps_launch(k_combine<CB_PLAIN, NoTail>, grid, RB_THREADS, 0, st, E.d_segs, T, mode, x, E.d_partAA, with_aa, E.d_partAB, E.d_partBB,
-                E.nch_bb, E.d_partBA, E.d_delta, lub_y, E.part_stride, y, dn, done_stride, NoTail{});
+                E.d_partBA, E.d_delta, lub_y, E.part_stride, y, dn, done_stride, NoTail{});
 }
 
 int g_aa_chunk_cols = AA_TILE_MAX;

@@ -288,71 +288,6 @@ __device__ __forceinline__ bool rep_done(const char *done, int stride, int r)
     return done && *(const int *)(done + (long)r * stride);
 }
 
-// velocity DOFs of the pair in pair-DOF order: U_lo, U_hi, W_lo, W_hi
-__device__ __forceinline__ void pair_dofs(const Seg &s, long lo, long hi, bool mono, int dof[12], int &nd)
-{
-    int il = (int)(lo - s.bead_off), ih = (int)(hi - s.bead_off);
-    int tl, wl, th, wh;
-    vel_dofs(s, il, tl, wl);
-    vel_dofs(s, ih, th, wh);
-    nd = mono ? 6 : 12;
-    for (int k = 0; k < 3; k++) {
-        dof[k] = tl + k; dof[3 + k] = th + k;
-        if (!mono) { dof[6 + k] = wl + k; dof[9 + k] = wh + k; }
-    }
-}
-
-// two-body FT far-field mobility of the pair in pair-DOF order, symmetrised
-__device__ void pair_mobility(const Seg &s, const double *__restrict__ x, const double *__restrict__ chain, long lo,
-                              long hi, bool mono, double *M)
-{
-    const int nd = mono ? 6 : 12;
-    for (int k = 0; k < nd * nd; k++) M[k] = 0.0;
-    double dx = x[3 * lo] - x[3 * hi], dy = x[3 * lo + 1] - x[3 * hi + 1], dz = x[3 * lo + 2] - x[3 * hi + 2];
-    double r2 = dx * dx + dy * dy + dz * dz, rinv = 1.0 / sqrt(r2), r = r2 * rinv;
-    double e[3] = {dx * rinv, dy * rinv, dz * rinv};
-    if (mono) {
-        r = ref_pair_dist(dx, dy, dz);   // the reference's distance decides the near/far branch
-        rinv = 1.0 / r;
-        for (int k = 0; k < 6; k++) M[k * 6 + k] = s.beta_inv;
-        bool coupled = s.mm_HI && !(s.chain_HI && chain[lo] == chain[hi]);
-        if (coupled) {
-            double xs, ys;
-            if (s.aa_mode == PS_AA_RPY) aa_scalars_rpy<double>(r, rinv, 2.0 * s.beta, xs, ys);
-            else aa_scalars<double>(r, rinv, 2.0 * s.beta, xs, ys);
-            for (int a = 0; a < 3; a++)
-                for (int c = 0; c < 3; c++) {
-                    double v = (xs - ys) * e[a] * e[c] + (a == c ? ys : 0.0);
-                    M[a * 6 + 3 + c] = v;
-                    M[(3 + a) * 6 + c] = v;
-                }
-        }
-        return;
-    }
-    for (int k = 0; k < 3; k++) {
-        M[k * 12 + k] = 1.0; M[(3 + k) * 12 + 3 + k] = 1.0;
-        M[(6 + k) * 12 + 6 + k] = 0.75; M[(9 + k) * 12 + 9 + k] = 0.75;
-    }
-    // the partner's (F, T) column -> this bead's (U, W) rows, e = (x_lo - x_hi)/r as in the BB kernel
-    for (int side = 0; side < 2; side++) {
-        const bool is_lo = side == 0;
-        const int rowU = is_lo ? 0 : 3, rowW = is_lo ? 6 : 9, colF = is_lo ? 3 : 0, colT = is_lo ? 9 : 6;
-        for (int c = 0; c < 6; c++) {
-            double in[11], out[11];
-            for (int k = 0; k < 11; k++) { in[k] = 0.0; out[k] = 0.0; }
-            in[c] = 1.0;
-            bb_apply<double>(e, r, rinv, is_lo, in, out);
-            int col = c < 3 ? colF + c : colT + (c - 3);
-            for (int a = 0; a < 3; a++) { M[(rowU + a) * 12 + col] = out[a]; M[(rowW + a) * 12 + col] = out[3 + a]; }
-        }
-    }
-    for (int a = 0; a < 12; a++)
-        for (int c = a + 1; c < 12; c++) {
-            double v = 0.5 * (M[a * 12 + c] + M[c * 12 + a]);
-            M[a * 12 + c] = v; M[c * 12 + a] = v;
-        }
-}
-
 // shared-memory scratch of one warp for one colloid pair
 struct PsWarpSmem {
     double K[144], Q[144], S[144], M[144];
@@ -1508,16 +1443,8 @@ int structured_solve(Engine &E, const double *b, double *x, const ps_ksp_opts *o
     apply_operator(E, 0, x, y, fp32, st);       // y_top = M F
     ps_launch(k_struct_u, nb, thr, 0, st, E.nvec, E.d_vec_offs, E.R, E.d_segs, b, y, x);
     PS_CK(cudaGetLastError());
-    ps_ksp_result r0 = {2, 0, 0, 0.0};
-    if (E.n_ss_polish) {
-        ps_ksp_opts po = *o;
-        po.warm = 1;
-        po.method = PS_SOLVE_MINRES;
-        int rc = minres_solve(E, b, x, &po, &r0, st);
-        if (rc == PS_ERR_CUDA) return rc;
-    }
-    if (res) *res = r0;
-    return r0.reason;
+    if (res) *res = {2, 0, 0, 0.0};
+    return 2;
 }
 
 // ---------------------------------------------------------------------------
