@@ -392,10 +392,10 @@ static int build(Engine &E, const ps_desc *descs, int R, int precision)
         const int KM = ps::LZ_KMAX;
         TRY_ALLOC(E.d_lzV, sizeof(double) * top * (KM + 1));
         TRY_ALLOC(E.d_lzq, sizeof(double) * top);
-        TRY_ALLOC(E.d_lzT, sizeof(double) * ((KM + 1) * R + KM * R * 4 + R));
         std::vector<int> ord;
         ps::lz_ordered_list(E, ord);
-        if ((rc = upload(E.d_lz_ord, ord))) return rc;
+        if (!ord.empty() && (rc = upload(E.d_lz_ord, ord))) return rc;
+        TRY_ALLOC(E.d_lzT, sizeof(double) * ((KM + 1) * R + KM * R * (ord.empty() ? 2 : 4) + R));
         TRY_ALLOC(E.d_lzp, sizeof(double) * ps::RB_EPT * E.red_top.nblk * (2 * KM + 1));
         TRY_ALLOC(E.d_lzs, 96 * R);          // Lanczos scalars, their snapshot, the checks' speculative outcomes
     }

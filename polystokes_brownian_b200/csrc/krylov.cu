@@ -379,11 +379,10 @@ __global__ void k_lz_sub_scale(RedTable T, const Seg *__restrict__ segs, double 
     double vr[LZ_REG];
     const double qk = act ? q[k] : 0.0;
     lz_load(V, ldv, k, act, j, vr);
-    if (segs[B.rep].indef) return;
     const bool lead = threadIdx.x == 0 && blockIdx.y == 0 && (int)blockIdx.x == first;
-    const int done = lz[B.rep].done[j & 1];
-    if (done) {
-        if (lead) lz[B.rep].done[(j + 1) & 1] = done;
+    const int done = lz[B.rep].done[j & 1], indef = segs[B.rep].indef;
+    if (done || indef) {
+        if (lead && !indef) lz[B.rep].done[(j + 1) & 1] = done;
         return;
     }
     __shared__ double h[LZ_KMAX + 1];
