@@ -42,6 +42,12 @@ int build_red_table(Engine &E, RedTable &T, int layout)
         cnt[r] = nb;
     }
     T.nblk = (int)blk.size();
+    // where blocks are many, none beyond the longest one's length (4000 replicas of 3 beads: an apply 22 us for 30)
+    T.nsub = RB_EPT;
+    if (T.nblk > 4 * 148) {
+        T.nsub = 1;
+        for (const RBlk &b : blk) T.nsub = std::max(T.nsub, (b.len + RB_THREADS - 1) / RB_THREADS);
+    }
     PS_CK(cudaMalloc(&T.d_blk, sizeof(RBlk) * T.nblk));
     PS_CK(cudaMalloc(&T.d_first, sizeof(int) * E.R));
     PS_CK(cudaMalloc(&T.d_count, sizeof(int) * E.R));
@@ -194,7 +200,7 @@ int minres_solve(Engine &E, const double *b, double *x, const ps_ksp_opts *o, ps
     *E.h_nactive = nact;
     PS_CK(cudaMemcpyAsync(E.d_nactive, E.h_nactive, sizeof(int), cudaMemcpyHostToDevice, st));
     double *pa = E.d_mrp, *pb = pa + (long)RB_EPT * T.nblk;
-    const dim3 sub((unsigned)T.nblk, RB_EPT);
+    const dim3 sub((unsigned)T.nblk, (unsigned)T.nsub);
     MinresScal *last = E.d_mr;
     // the apply of iteration k closes iteration k - 1, so the check stands between the apply and
     // k_mr_beta, and a solve that converged at k - 1 has spent one apply of iteration k
@@ -1217,7 +1223,7 @@ int lanczos_sqrt(Engine &E, const double *z, double *w, const ps_sqrt_opts *o, p
         const LzDots dots = {V, ldv, j, part1};
         apply_operator(E, 1, V + (long)j * ldv, q, E.precision == PS_PREC_MIXED, st, &lz[0].done[j & 1],
                        (int)sizeof(LzScal), false, any_free ? &dots : nullptr);
-        const dim3 sub((unsigned)T.nblk, RB_EPT);
+        const dim3 sub((unsigned)T.nblk, (unsigned)T.nsub);
         if (E.n_lz_ord && E.lz_cluster)
             ps_launch(k_lz_orth_cluster, E.n_lz_ord * LZC_CTAS, LZC_THREADS, 0, st, E.d_segs, E.d_lz_ord, V, ldv, q, j, kmax,
                     lz, alpha, betad);

@@ -26,6 +26,7 @@ struct PairBlk { int rep, b, G, first; };
 
 struct RedTable {
     int nblk = 0;
+    int nsub = 1;                // second extent of the grids with a thread per entry: sub-blocks of an entry of the table
     RBlk *d_blk = nullptr;       // per block
     int *d_first = nullptr;      // per replica: first block
     int *d_count = nullptr;      // per replica: number of blocks
@@ -84,6 +85,7 @@ struct Engine {
     AaTile *d_aa_tiles = nullptr;    // n_far_pre monomer-colloid and colloid blocks, then n_aa_tiles monomer tile pairs
     Tile *d_bb_tiles = nullptr;      // colloid row tiles of the replicas without monomers, BB_WIDE rows each or BB_TILE
     int n_far_pre = 0, n_aa_tiles = 0, n_bb_tiles = 0, nch_bb = 1;
+    bool aa_narrow[2] = {false, false};   // FP64, FP32: two warps per monomer tile pair, in a launch of their own
     bool bb_wide = false;
     long part_stride = 0;
     double *d_partAA = nullptr, *d_partAB = nullptr, *d_partBB = nullptr, *d_partBA = nullptr;

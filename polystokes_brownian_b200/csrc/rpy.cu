@@ -416,6 +416,54 @@ __device__ __forceinline__ void aa_f2_cell(const float4 *__restrict__ sXY, const
     }
 }
 
+// columns [j0, j0 + S) of a tile as aa_f2_cell reads them, padding beyond the replica, by nt threads
+template <int P>
+__device__ __forceinline__ void aa_load_columns_f(const Seg &sg, int Nm, const float4 *__restrict__ pos,
+                                                  const float4 *__restrict__ plo, const double *__restrict__ u, int uoff,
+                                                  int j0, int S, int tid, int nt, float4 (&cols)[5][P])
+{
+    for (int p = tid; p < S / 2; p += nt) {
+        float4 A[2], B[2];
+        float v[2][3];
+#pragma unroll
+        for (int h = 0; h < 2; h++) {
+            const int j = j0 + 2 * p + h;
+            if (j < Nm) {
+                A[h] = pos[sg.bead_off + j]; B[h] = plo[sg.bead_off + j];
+                for (int a = 0; a < 3; a++) v[h][a] = (float)u[uoff + 3 * j + a];
+            } else {
+                A[h] = make_float4(AAC_PAD, AAC_PAD, AAC_PAD, __int_as_float(0x7fc00000));
+                B[h] = make_float4(0.f, 0.f, 0.f, 0.f);
+                v[h][0] = v[h][1] = v[h][2] = 0.f;
+            }
+        }
+        cols[0][p] = make_float4(-A[0].x, -A[1].x, -A[0].y, -A[1].y);
+        cols[1][p] = make_float4(-A[0].z, -A[1].z, v[0][0], v[1][0]);
+        cols[2][p] = make_float4(v[0][1], v[1][1], v[0][2], v[1][2]);
+        cols[3][p] = make_float4(B[0].x, B[1].x, B[0].y, B[1].y);
+        cols[4][p] = make_float4(B[0].z, B[1].z, A[0].w, A[1].w);
+    }
+}
+
+// rows R.iA and R.iB (padding beyond the replica; i0: a bead of the replica)
+__device__ __forceinline__ void aa_load_rows_f(const Seg &sg, int Nm, const float4 *__restrict__ pos, const double *__restrict__ u,
+                                               int uoff, int i0, AaRowsF &R)
+{
+    const bool actA = R.iA < Nm, actB = R.iB < Nm;
+    R.gA = sg.bead_off + (actA ? R.iA : i0); R.gB = sg.bead_off + (actB ? R.iB : i0);
+    {
+        const float nan = __int_as_float(0x7fc00000);
+        const float4 pad = make_float4(-AAC_PAD, -AAC_PAD, -AAC_PAD, nan);
+        const float4 PA = actA ? pos[R.gA] : pad, PB = actB ? pos[R.gB] : pad;
+        R.ax = f2(PA.x); R.ay = f2(PA.y); R.az = f2(PA.z); R.bx = f2(PB.x); R.by = f2(PB.y); R.bz = f2(PB.z);
+        R.wA = PA.w; R.wB = PB.w;
+        for (int a = 0; a < 3; a++) {
+            R.au[a] = f2(actA ? (float)u[uoff + 3 * R.iA + a] : 0.f);
+            R.bu[a] = f2(actB ? (float)u[uoff + 3 * R.iB + a] : 0.f);
+        }
+    }
+}
+
 constexpr int AAF_THREADS = 128;
 
 template <bool REF>
@@ -454,27 +502,7 @@ k_rpy_aa_f2(const Seg *__restrict__ segs, const AaTile *__restrict__ tiles, cons
     const int Nm = sg.Nm, S = tl.S, tid = threadIdx.x, lane = tid & 31, w = tid >> 5;
     const int i0 = tl.I * S, j0 = tl.J * S;
     const int uoff = in_top ? sg.top_off : sg.vec_off;
-    for (int p = tid; p < S / 2; p += AAF_THREADS) {
-        float4 A[2], B[2];
-        float v[2][3];
-#pragma unroll
-        for (int h = 0; h < 2; h++) {
-            const int j = j0 + 2 * p + h;
-            if (j < Nm) {
-                A[h] = pos[sg.bead_off + j]; B[h] = plo[sg.bead_off + j];
-                for (int a = 0; a < 3; a++) v[h][a] = (float)u[uoff + 3 * j + a];
-            } else {
-                A[h] = make_float4(AAC_PAD, AAC_PAD, AAC_PAD, __int_as_float(0x7fc00000));
-                B[h] = make_float4(0.f, 0.f, 0.f, 0.f);
-                v[h][0] = v[h][1] = v[h][2] = 0.f;
-            }
-        }
-        sCols[0][p] = make_float4(-A[0].x, -A[1].x, -A[0].y, -A[1].y);
-        sCols[1][p] = make_float4(-A[0].z, -A[1].z, v[0][0], v[1][0]);
-        sCols[2][p] = make_float4(v[0][1], v[1][1], v[0][2], v[1][2]);
-        sCols[3][p] = make_float4(B[0].x, B[1].x, B[0].y, B[1].y);
-        sCols[4][p] = make_float4(B[0].z, B[1].z, A[0].w, A[1].w);
-    }
+    aa_load_columns_f(sg, Nm, pos, plo, u, uoff, j0, S, tid, AAF_THREADS, sCols);
     // the warp's share: edge 64, one cell in four bands of 8 steps; 128, 2 x 2 cells; 256, one
     // row group of four cells each
     const int rg = S == 64 ? 0 : (S == 128 ? w >> 1 : w);
@@ -484,19 +512,7 @@ k_rpy_aa_f2(const Seg *__restrict__ segs, const AaTile *__restrict__ tiles, cons
     const int cslot = S == 64 ? w : rg, ncslot = S == 128 ? 2 : 4;
     AaRowsF R;
     R.iA = i0 + 64 * rg + lane; R.iB = R.iA + 32;
-    const bool actA = R.iA < Nm, actB = R.iB < Nm;
-    R.gA = sg.bead_off + (actA ? R.iA : i0); R.gB = sg.bead_off + (actB ? R.iB : i0);
-    {
-        const float nan = __int_as_float(0x7fc00000);
-        const float4 pad = make_float4(-AAC_PAD, -AAC_PAD, -AAC_PAD, nan);
-        const float4 PA = actA ? pos[R.gA] : pad, PB = actB ? pos[R.gB] : pad;
-        R.ax = f2(PA.x); R.ay = f2(PA.y); R.az = f2(PA.z); R.bx = f2(PB.x); R.by = f2(PB.y); R.bz = f2(PB.z);
-        R.wA = PA.w; R.wB = PB.w;
-        for (int a = 0; a < 3; a++) {
-            R.au[a] = f2(actA ? (float)u[uoff + 3 * R.iA + a] : 0.f);
-            R.bu[a] = f2(actB ? (float)u[uoff + 3 * R.iB + a] : 0.f);
-        }
-    }
+    aa_load_rows_f(sg, Nm, pos, u, uoff, i0, R);
     const bool chain_hi = sg.chain_HI != 0, diag = tl.I == tl.J;
     const float2 fa = f2(sg.aa_c[0] - sg.aa_c[2]), fb = f2(sg.aa_c[1] - sg.aa_c[3]);
     const float2 fc = f2(sg.aa_c[2]), fd = f2(sg.aa_c[3]);
@@ -619,6 +635,61 @@ __device__ __forceinline__ void aa_d2_cell(const double2 *__restrict__ sXY, cons
     }
 }
 
+__device__ __forceinline__ AaScalD aa_scal_d(const Seg &sg)
+{
+    AaScalD K;
+    double c0, c1, c2, c3;
+    if (sg.aa_mode == PS_AA_RPY) {
+        const double b = sg.beta, b2 = b * b;
+        c0 = 1.5; c1 = -b2; c2 = 0.75; c3 = 0.5 * b2;
+        K.n0 = 1.0 / b; K.n1 = -0.1875 / b2; K.n2 = 1.0 / b; K.n3 = -0.28125 / b2;
+    } else {
+        c0 = 0.375; c1 = -2.0; c2 = 0.75; c3 = -0.5;
+        K.n0 = -1.0; K.n1 = 0.375; K.n2 = 1.0; K.n3 = -0.28125;
+    }
+    K.tb = 2.0 * sg.beta; K.ca = c0 - c2; K.cb = c1 - c3; K.cc = c2; K.cd = c3;
+    K.tb2f = (float)(K.tb * K.tb * (1.0 + 1e-6));
+    return K;
+}
+
+// columns [j0, j0 + S) of a tile as aa_d2_cell reads them, padding beyond the replica, by nt threads
+template <int P>
+__device__ __forceinline__ void aa_load_columns_d(const Seg &sg, int Nm, const double4 *__restrict__ pos,
+                                                  const double *__restrict__ u, int uoff, int j0, int S, int tid, int nt,
+                                                  double2 (&cols)[3][P], double *__restrict__ w)
+{
+    for (int p = tid; p < S; p += nt) {
+        const int j = j0 + p;
+        if (j < Nm) {
+            const double4 P = pos[sg.bead_off + j];
+            const double *v = u + uoff + 3 * j;
+            cols[0][p] = make_double2(P.x, P.y);
+            cols[1][p] = make_double2(P.z, v[0]);
+            cols[2][p] = make_double2(v[1], v[2]);
+            w[p] = P.w;
+        } else {
+            cols[0][p] = make_double2(AAC_PAD, AAC_PAD);
+            cols[1][p] = make_double2(AAC_PAD, 0.0);
+            cols[2][p] = make_double2(0.0, 0.0);
+            w[p] = __longlong_as_double(0x7ff8000000000000ll);
+        }
+    }
+}
+
+// rows iA and iB (padding beyond the replica)
+__device__ __forceinline__ void aa_load_rows_d(const Seg &sg, int Nm, const double4 *__restrict__ pos, const double *__restrict__ u,
+                                               int uoff, int iA, int iB, double4 &PA, double4 &PB, double (&uA)[3],
+                                               double (&uB)[3])
+{
+    const bool actA = iA < Nm, actB = iB < Nm;
+    const double4 pad = make_double4(-AAC_PAD, -AAC_PAD, -AAC_PAD, __longlong_as_double(0x7ff8000000000000ll));
+    PA = actA ? pos[sg.bead_off + iA] : pad; PB = actB ? pos[sg.bead_off + iB] : pad;
+    for (int a = 0; a < 3; a++) {
+        uA[a] = actA ? u[uoff + 3 * iA + a] : 0.0;
+        uB[a] = actB ? u[uoff + 3 * iB + a] : 0.0;
+    }
+}
+
 constexpr int AAD_THREADS = 256;
 
 __global__ void __launch_bounds__(AAD_THREADS, 2)
@@ -653,22 +724,7 @@ k_rpy_aa_d2(const Seg *__restrict__ segs, const AaTile *__restrict__ tiles, cons
     const int Nm = sg.Nm, S = tl.S, tid = threadIdx.x, lane = tid & 31, w = tid >> 5;
     const int i0 = tl.I * S, j0 = tl.J * S;
     const int uoff = in_top ? sg.top_off : sg.vec_off;
-    for (int p = tid; p < S; p += AAD_THREADS) {
-        const int j = j0 + p;
-        if (j < Nm) {
-            const double4 P = pos[sg.bead_off + j];
-            const double *v = u + uoff + 3 * j;
-            sCols[0][p] = make_double2(P.x, P.y);
-            sCols[1][p] = make_double2(P.z, v[0]);
-            sCols[2][p] = make_double2(v[1], v[2]);
-            sW[p] = P.w;
-        } else {
-            sCols[0][p] = make_double2(AAC_PAD, AAC_PAD);
-            sCols[1][p] = make_double2(AAC_PAD, 0.0);
-            sCols[2][p] = make_double2(0.0, 0.0);
-            sW[p] = __longlong_as_double(0x7ff8000000000000ll);
-        }
-    }
+    aa_load_columns_d(sg, Nm, pos, u, uoff, j0, S, tid, AAD_THREADS, sCols, sW);
     // the warp's share: edge 64, one 64 x 32 cell per column group in four bands of 8 steps;
     // 128, 2 x 4 cells; 256, a row group's four cells of one half of the columns
     const int rg = S == 64 ? 0 : (S == 128 ? w >> 2 : w >> 1);
@@ -677,29 +733,11 @@ k_rpy_aa_d2(const Seg *__restrict__ segs, const AaTile *__restrict__ tiles, cons
     const int rslot = S == 64 ? w : (S == 128 ? w & 3 : w & 1), nrslot = S == 64 ? 8 : (S == 128 ? 4 : 2);
     const int cslot = S == 64 ? w >> 1 : rg, ncslot = S == 128 ? 2 : 4;
     const int iA = i0 + 64 * rg + lane, iB = iA + 32;
-    const bool actA = iA < Nm, actB = iB < Nm;
-    const double4 pad = make_double4(-AAC_PAD, -AAC_PAD, -AAC_PAD, __longlong_as_double(0x7ff8000000000000ll));
-    const double4 PA = actA ? pos[sg.bead_off + iA] : pad, PB = actB ? pos[sg.bead_off + iB] : pad;
+    double4 PA, PB;
     double uA[3], uB[3];
-    for (int a = 0; a < 3; a++) {
-        uA[a] = actA ? u[uoff + 3 * iA + a] : 0.0;
-        uB[a] = actB ? u[uoff + 3 * iB + a] : 0.0;
-    }
+    aa_load_rows_d(sg, Nm, pos, u, uoff, iA, iB, PA, PB, uA, uB);
     const bool chain_hi = sg.chain_HI != 0, diag = tl.I == tl.J;
-    AaScalD K;
-    {
-        double c0, c1, c2, c3;
-        if (sg.aa_mode == PS_AA_RPY) {
-            const double b = sg.beta, b2 = b * b;
-            c0 = 1.5; c1 = -b2; c2 = 0.75; c3 = 0.5 * b2;
-            K.n0 = 1.0 / b; K.n1 = -0.1875 / b2; K.n2 = 1.0 / b; K.n3 = -0.28125 / b2;
-        } else {
-            c0 = 0.375; c1 = -2.0; c2 = 0.75; c3 = -0.5;
-            K.n0 = -1.0; K.n1 = 0.375; K.n2 = 1.0; K.n3 = -0.28125;
-        }
-        K.tb = 2.0 * sg.beta; K.ca = c0 - c2; K.cb = c1 - c3; K.cc = c2; K.cd = c3;
-        K.tb2f = (float)(K.tb * K.tb * (1.0 + 1e-6));
-    }
+    const AaScalD K = aa_scal_d(sg);
     __syncthreads();
     double racc[6] = {0, 0, 0, 0, 0, 0};
     for (int cg = cg0; cg < cg0 + ncg; cg++) {
@@ -737,6 +775,148 @@ k_rpy_aa_d2(const Seg *__restrict__ segs, const AaTile *__restrict__ tiles, cons
         if (!diag && 3 * j0 + e < sg.nm3) {
             double v = 0.0;
             for (int q = 0; q < ncslot; q++) v += sCol[3 * S * q + e];
+            oJ[e] = v;
+        }
+    }
+}
+
+// ---------------------------------------------------------------------------
+// Tile pairs of edge 64 by two warps each, for launches of many: the bands that the block kernels give to a
+// warp each are taken one after the other, and the same sums are joined in the same order, so the
+// slots hold the same bits.  A block of all bands spreads a lone replica; where the tile pairs fill the
+// chip many times over, its barriers, its idle warps and the steps that meet padding only are what a
+// launch takes.  Padding adds exact zeros, so cells of padding columns and, in a diagonal cell, steps
+// without a pair are left out.
+//
+// Taken for contexts whose tile pairs are all of edge 64 and more than AAN_MIN_TILES (two and one waves of the
+// block kernels in FP64 and FP32), or, where monomer-colloid and colloid blocks then need a launch of
+// their own, than AAN_MIN_WITH_PRE (four waves) unless every replica has a few beads only.  One apply, block
+// -> two warps, us, FP64 / FP32: 1000 replicas of 3 beads 22.7 -> 8.1 / 14.5 -> 8.0, of 65 beads 57.3 ->
+// 30.7 / 33.7 -> 27.5, 100 of 1000 beads 240 -> 185 / 124 -> 104; 30 of 200 beads (300 tile pairs) 12.1 ->
+// 16.3 / 10.0 -> 12.2; with probes, 128 replicas of 64 to 700 beads (2000 tile pairs) 46.4 -> 42.4 / 28.0 ->
+// 29.2, 48 of them 22.4 -> 26.9 / 15.8 -> 19.4.
+constexpr int AAN_THREADS = 64, AAN_BLOCKS = 8;
+constexpr int AAN_MIN_TILES = 4 * 148, AAN_MIN_WITH_PRE[2] = {8 * 148, 16 * 148};      // FP64, FP32
+
+// [s0, s1) and [s2, s0 + 8): the steps of a diagonal band that meet a pair, where rows sit in lanes below nr and
+// lane l holds column (l + s) mod 32, one of nc
+__device__ __forceinline__ void aa_band_steps(int s0, int nr, int nc, int &s1, int &s2)
+{
+    s1 = min(s0 + 8, max(s0, nc));
+    s2 = min(s0 + 8, max(s1, 33 - nr));
+}
+
+__global__ void __launch_bounds__(AAN_THREADS, AAN_BLOCKS)
+k_rpy_aa_dn(const Seg *__restrict__ segs, const AaTile *__restrict__ tiles, const double4 *__restrict__ pos,
+            const double *__restrict__ u, int in_top, double *__restrict__ paa, const char *__restrict__ done, int done_stride)
+{
+    pdl_enter();
+    __shared__ double2 sCols[3][64];
+    __shared__ double sW[64], sRow[8 * 192], sCol[4 * 192];
+    const AaTile tl = tiles[blockIdx.x];
+    if (done && *(const int *)(done + (long)tl.rep * done_stride)) return;
+    const Seg &sg = segs[tl.rep];
+    const int Nm = sg.Nm, tid = threadIdx.x, lane = tid & 31, w = tid >> 5;
+    const int i0 = 64 * tl.I, j0 = 64 * tl.J, uoff = in_top ? sg.top_off : sg.vec_off;
+    aa_load_columns_d(sg, Nm, pos, u, uoff, j0, 64, tid, AAN_THREADS, sCols, sW);
+    const int iA = i0 + lane, iB = iA + 32;
+    double4 PA, PB;
+    double uA[3], uB[3];
+    aa_load_rows_d(sg, Nm, pos, u, uoff, iA, iB, PA, PB, uA, uB);
+    const bool chain_hi = sg.chain_HI != 0, diag = tl.I == tl.J;
+    const AaScalD K = aa_scal_d(sg);
+    __syncthreads();
+    for (int q = 4 * w; q < 4 * w + 4; q++) {              // band q / 2 of column group q mod 2
+        const int b = q >> 1, s0 = 8 * b, o = 32 * (q & 1), jc = j0 + o;
+        double t[6] = {0, 0, 0, 0, 0, 0}, c[3] = {0, 0, 0};
+        if (jc >= Nm) ;
+        else if (diag) {
+            int s1, s2;
+            aa_band_steps(s0, Nm - i0, Nm - jc, s1, s2);
+            for (int h = 0; h < 2; h++)
+                aa_d2_cell<false, true>(sCols[0] + o, sCols[1] + o, sCols[2] + o, sW + o, jc, h ? s2 : s0,
+                                        h ? s0 + 8 - s2 : s1 - s0, iA, iB, chain_hi, PA, PB, uA, uB, K, t, c);
+        } else if (chain_hi)
+            aa_d2_cell<true, true>(sCols[0] + o, sCols[1] + o, sCols[2] + o, sW + o, jc, s0, 8, iA, iB, true, PA, PB, uA, uB,
+                                   K, t, c);
+        else
+            aa_d2_cell<true, false>(sCols[0] + o, sCols[1] + o, sCols[2] + o, sW + o, jc, s0, 8, iA, iB, false, PA, PB, uA, uB,
+                                    K, t, c);
+        double *r = sRow + 192 * q + 3 * lane, *o3 = sCol + 192 * b + 3 * (o + ((lane + s0 + 8) & 31));
+        for (int a = 0; a < 3; a++) { r[a] = t[a]; r[96 + a] = t[3 + a]; o3[a] = c[a]; }
+    }
+    __syncthreads();
+    double *oI = paa + sg.paa_off + (long)tl.J * sg.nm3 + 3 * i0, *oJ = paa + sg.paa_off + (long)tl.I * sg.nm3 + 3 * j0;
+    for (int e = tid; e < 192; e += AAN_THREADS) {
+        if (3 * i0 + e < sg.nm3) {
+            double v = 0.0;
+            for (int q = 0; q < 8; q++) v += sRow[192 * q + e];
+            oI[e] = v;
+        }
+        if (!diag && 3 * j0 + e < sg.nm3) {
+            double v = 0.0;
+            for (int q = 0; q < 4; q++) v += sCol[192 * q + e];
+            oJ[e] = v;
+        }
+    }
+}
+
+template <bool REF>
+__global__ void __launch_bounds__(AAN_THREADS, AAN_BLOCKS)
+k_rpy_aa_fn(const Seg *__restrict__ segs, const AaTile *__restrict__ tiles, const float4 *__restrict__ pos,
+            const float4 *__restrict__ plo, const float *__restrict__ aa_te2, const double4 *__restrict__ p64,
+            const double *__restrict__ u, int in_top, double *__restrict__ paa, const char *__restrict__ done, int done_stride)
+{
+    pdl_enter();
+    __shared__ float4 sCols[5][32];
+    __shared__ double sRow[4 * 192];
+    __shared__ float sCol[4 * 192];
+    const AaTile tl = tiles[blockIdx.x];
+    if (done && *(const int *)(done + (long)tl.rep * done_stride)) return;
+    const Seg &sg = segs[tl.rep];
+    if ((sg.aa_mode == PS_AA_REFERENCE) != REF) return;
+    const int Nm = sg.Nm, tid = threadIdx.x, lane = tid & 31, w = tid >> 5;
+    const int i0 = 64 * tl.I, j0 = 64 * tl.J, uoff = in_top ? sg.top_off : sg.vec_off;
+    aa_load_columns_f(sg, Nm, pos, plo, u, uoff, j0, 64, tid, AAN_THREADS, sCols);
+    AaRowsF R;
+    R.iA = i0 + lane; R.iB = R.iA + 32;
+    aa_load_rows_f(sg, Nm, pos, u, uoff, i0, R);
+    const bool chain_hi = sg.chain_HI != 0, diag = tl.I == tl.J;
+    const float2 fa = f2(sg.aa_c[0] - sg.aa_c[2]), fb = f2(sg.aa_c[1] - sg.aa_c[3]);
+    const float2 fc = f2(sg.aa_c[2]), fd = f2(sg.aa_c[3]);
+    const float te2 = aa_te2[tl.rep];
+    __syncthreads();
+    for (int b = 2 * w; b < 2 * w + 2; b++) {
+        const int s0 = 8 * b;
+        float2 t[6] = {f2(0.f), f2(0.f), f2(0.f), f2(0.f), f2(0.f), f2(0.f)}, c[3] = {f2(0.f), f2(0.f), f2(0.f)};
+        if (diag) {
+            int s1, s2;
+            aa_band_steps(s0, Nm - i0, (Nm - j0 + 1) / 2, s1, s2);
+            for (int h = 0; h < 2; h++)
+                aa_f2_cell<false, true, REF>(sCols[0], sCols[1], sCols[2], sCols[3], sCols[4], j0, h ? s2 : s0,
+                                             h ? s0 + 8 - s2 : s1 - s0, chain_hi, R, plo, fa, fb, fc, fd, sg, te2, p64, t, c);
+        } else if (chain_hi)
+            aa_f2_cell<true, true, REF>(sCols[0], sCols[1], sCols[2], sCols[3], sCols[4], j0, s0, 8, true, R, plo, fa, fb, fc,
+                                        fd, sg, te2, p64, t, c);
+        else
+            aa_f2_cell<true, false, REF>(sCols[0], sCols[1], sCols[2], sCols[3], sCols[4], j0, s0, 8, false, R, plo, fa, fb, fc,
+                                         fd, sg, te2, p64, t, c);
+        double *r = sRow + 192 * b + 3 * lane;
+        for (int a = 0; a < 3; a++) { r[a] = (double)(t[a].x + t[a].y); r[96 + a] = (double)(t[3 + a].x + t[3 + a].y); }
+        float *o3 = sCol + 192 * b + 6 * ((lane + s0 + 8) & 31);
+        for (int a = 0; a < 3; a++) { o3[a] = c[a].x; o3[3 + a] = c[a].y; }
+    }
+    __syncthreads();
+    double *oI = paa + sg.paa_off + (long)tl.J * sg.nm3 + 3 * i0, *oJ = paa + sg.paa_off + (long)tl.I * sg.nm3 + 3 * j0;
+    for (int e = tid; e < 192; e += AAN_THREADS) {
+        if (3 * i0 + e < sg.nm3) {
+            double v = 0.0;
+            for (int q = 0; q < 4; q++) v += sRow[192 * q + e];
+            oI[e] = v;
+        }
+        if (!diag && 3 * j0 + e < sg.nm3) {
+            double v = 0.0;
+            for (int q = 0; q < 4; q++) v += (double)sCol[192 * q + e];
             oJ[e] = v;
         }
     }
@@ -847,7 +1027,7 @@ __global__ void k_combine(const Seg *__restrict__ segs, RedTable T, int mode, co
     }
     const Seg &sg = segs[r];
     const int xo = mode == 0 ? sg.vec_off : sg.top_off;
-    // grid.y = RB_EPT: one entry per thread
+    // one entry per thread
     const int e = blockIdx.y * RB_THREADS + threadIdx.x;
     const long k = (long)B.start + e;
     double out = 0.0;
@@ -889,6 +1069,24 @@ static void launch_far(Engine &E, const double *u, int in_top, bool fp32, int fi
                 u, in_top, O, done, dstride);
 }
 
+// the monomer tile pairs where k_rpy_aa_dn and k_rpy_aa_fn take them all (set_aa_chunking)
+static void launch_far_narrow(Engine &E, const double *u, int in_top, bool fp32, cudaStream_t st, const char *done, int dstride)
+{
+    const int n = E.n_aa_tiles;
+    if (!n || !E.aa_narrow[fp32]) return;
+    const AaTile *tiles = E.d_aa_tiles + E.n_far_pre;
+    if (!fp32) {
+        ps_launch(k_rpy_aa_dn, n, AAN_THREADS, 0, st, E.d_segs, tiles, E.d_pos64, u, in_top, E.d_partAA, done, dstride);
+        return;
+    }
+    if (E.any_aa_rpy)
+        ps_launch(k_rpy_aa_fn<false>, n, AAN_THREADS, 0, st, E.d_segs, tiles, E.d_pos32, E.d_pos32lo, E.d_aa_te2, E.d_pos64, u,
+                in_top, E.d_partAA, done, dstride);
+    if (E.any_aa_ref)
+        ps_launch(k_rpy_aa_fn<true>, n, AAN_THREADS, 0, st, E.d_segs, tiles, E.d_pos32, E.d_pos32lo, E.d_aa_te2, E.d_pos64, u,
+                in_top, E.d_partAA, done, dstride);
+}
+
 static void launch_bb(Engine &E, const double *u, int in_top, cudaStream_t st, const char *done, int dstride)
 {
     if (!E.n_bb_tiles) return;
@@ -906,7 +1104,8 @@ void apply_operator(Engine &E, int mode, const double *x, double *y, bool fp32, 
 {
     int in_top = mode == 1;
     const char *dn = (const char *)done;
-    launch_far(E, x, in_top, fp32, 0, E.n_far_pre + (skip_aa ? 0 : E.n_aa_tiles), st, dn, done_stride);
+    launch_far(E, x, in_top, fp32, 0, E.n_far_pre + (skip_aa || E.aa_narrow[fp32] ? 0 : E.n_aa_tiles), st, dn, done_stride);
+    if (!skip_aa) launch_far_narrow(E, x, in_top, fp32, st, dn, done_stride);
     launch_bb(E, x, in_top, st, dn, done_stride);
     const double *lub_y = nullptr;
     if (mode == 0 && E.any_lub) {
@@ -914,7 +1113,7 @@ void apply_operator(Engine &E, int mode, const double *x, double *y, bool fp32, 
         lub_y = E.d_luby;
     }
     const RedTable &T = mode == 0 ? E.red : E.red_top;
-    const dim3 grid((unsigned)T.nblk, RB_EPT);
+    const dim3 grid((unsigned)T.nblk, (unsigned)T.nsub);
     const int with_aa = skip_aa ? 0 : 1;
     if (dots)
         ps_launch(k_combine<CB_DOTS, LzDots>, grid, RB_THREADS, 0, st, E.d_segs, T, mode, x, E.d_partAA, with_aa, E.d_partAB, E.d_partBB,
@@ -964,6 +1163,10 @@ int set_aa_chunking(Engine &E, int cols)
     std::stable_sort(tiles.begin(), tiles.end(), [](const AaTile &a, const AaTile &b) { return a.S > b.S; });
     E.n_aa_tiles = (int)tiles.size();
     E.n_far_pre = (int)pre.size();
+    const bool narrow = std::all_of(tiles.begin(), tiles.end(), [](const AaTile &t) { return t.S == AA_TILE_MIN; });
+    const bool tiny = std::all_of(E.segs.begin(), E.segs.end(), [](const Seg &s) { return s.Nm <= 32; });
+    for (int f = 0; f < 2; f++)
+        E.aa_narrow[f] = narrow && E.n_aa_tiles > (pre.empty() || tiny ? AAN_MIN_TILES : AAN_MIN_WITH_PRE[f]);
     tiles.insert(tiles.begin(), pre.begin(), pre.end());
     PS_CK(cudaDeviceSynchronize());
     cudaFree(E.d_partAA);
@@ -994,7 +1197,8 @@ int time_pairs(Engine &E, int which, int reps, const double *u, double *ms, cuda
     cudaEventCreate(&b);
     auto launch = [&]() {
         if (which == 0) {
-            launch_far(E, u, 1, fp32, E.n_far_pre, E.n_aa_tiles, st, nullptr, 0);
+            if (!E.aa_narrow[fp32]) launch_far(E, u, 1, fp32, E.n_far_pre, E.n_aa_tiles, st, nullptr, 0);
+            launch_far_narrow(E, u, 1, fp32, st, nullptr, 0);
         } else if (which == 1) {
             launch_far(E, u, 1, fp32, 0, E.n_far_pre, st, nullptr, 0);
         } else if (which == 2) {
