@@ -8,10 +8,12 @@
 // src/init.cpp:217-241): convergence when ||B r0||_2 * prod|s_k| <= rtol * ref,
 // ref = ||B r0|| for a zero guess and ||B b|| for a nonzero guess.
 //
-// Reductions are segmented per replica: each block covers a contiguous range of
-// one replica; the last block of a replica to arrive (atomic counter) sums the
-// partials in fixed order and runs that replica's scalar update, so the result
-// never depends on other replicas or on block scheduling.
+// Reductions are segmented per replica: each block covers a contiguous range of one
+// replica and leaves its sum in memory, and every block of the next kernel adds its
+// replica's sums itself in fixed order (rep_total, lz_total), so the result never depends
+// on other replicas or on block scheduling.  A solve's start, single dots and the ordered
+// sweeps of the square root (k_lz_ord_*) instead leave the totals to the replica's last
+// block to arrive (finish_block).
 #include <cmath>
 #include <cstdio>
 #include <vector>
@@ -273,9 +275,9 @@ struct LzScal {
 // Bound: latency and L2 (the basis is read twice from L2 and once from L1 per
 // vector, k_lz_sub_dots reading its slices twice).  With 1024 entries per block of
 // 256 threads, or one cluster of eight blocks per replica, too few loads were in
-// flight: a vector with its apply took 42 us at 1024 beads (23 now), 72 us at the
-// 4097-bead brush (49 now), and the four sweeps of 64 replicas, 62000 beads, 100 us
-// (three, 44 us, now).  Taking the norm with the second dots instead of in a launch of its
+// flight: a vector with its apply took 42 us at 1024 beads (23 this way), 72 us at the
+// 4097-bead brush (49 this way), and the sweeps of 64 replicas, 62000 beads, 100 us
+// (44 this way).  Taking the norm with the second dots instead of in a launch of its
 // own is 2 us of these; holding the thread's entries of the first 32 vectors in registers, asked
 // for before the totals are added, 2 us more (k_lz_sub_dots 5.5 -> 4.4 us at 1024 beads).
 constexpr int LZ_SUB = RB_THREADS;                    // entries of a sub-block
@@ -885,8 +887,9 @@ __global__ void k_lz_combine(RedTable T, const double *__restrict__ V, long ldv,
 // threads form a block's partials, and every sum over blocks runs in block order: both passes of the
 // reorthogonalisation (dots against V_0..V_j, then q -= V h), the norm, the breakdown test and the
 // next basis vector.  Two forms with the same bits:
-//   k_lz_orth_cluster   one launch, a cluster of LZC_CTAS blocks per replica, cluster barriers between the phases
-//                       and the cross-block sums read through distributed shared memory
+//   k_lz_orth_cluster   one launch, a cluster of LZC_CTAS blocks per replica, cluster barriers between the phases,
+//                       the cross-block sums read through distributed shared memory and the entries of q held in
+//                       registers throughout (1024 colloids 27 us a launch, 30 with q read and written per pass)
 //   k_lz_ord_*          four launches over the table
 // The clusters are taken while all of a batch's are resident at once, and for replicas of one table block per
 // half-block.  Roots of 40 vectors by clusters and by the table, ms, reference pair scalars: 60 beads, 8

@@ -1,7 +1,9 @@
 // ps_reduce.cuh -- segmented per-replica reductions shared by the Krylov
-// solvers: a block covers a contiguous range of one replica's vector; the last
-// block of a replica to arrive (atomic counter) sums the partials in fixed
-// order, so results never depend on block scheduling or on other replicas.
+// solvers: a block covers a contiguous range of one replica's vector, and the
+// blocks' sums are added in fixed order, so results never depend on block
+// scheduling or on other replicas.  Two ways to the total: every block of the next
+// kernel adds them (rep_total), or the replica's last block to arrive does, by an
+// atomic counter (finish_block).
 #pragma once
 #include "ps_kernels.h"
 

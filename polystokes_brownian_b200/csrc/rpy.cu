@@ -172,10 +172,10 @@ __device__ __forceinline__ void ab_block(const Seg &sg, int rep, int mt, const t
 // Bound: the chain of a pair's dependent FP64 operations; small blocks spread a suspension
 // over all SMs.  Against blocks of 128 rows, one launch: 300
 // colloids 17.0 -> 9.2 us, 512 17.8 -> 9.6, 1600 51.1 -> 37.9.
-// The order of the sums and the arithmetic of a pair are what they were: the solves of a
-// suspension whose far field is close to singular return, within rtol, whatever their rounding
-// selects.  (A pair action of 140 operations for 190 and chunks of 32 columns gave 14.9 us at
-// 1024 colloids, and positions off by 1e-6 in one step of ten.)
+// The order of the sums (columns in a chunk by group, groups, chunks) and the arithmetic of a pair are
+// part of the answer: the solves of a suspension whose far field is close to singular return, within
+// rtol, whatever their rounding selects.  (A pair action of 140 operations for 190 and chunks of 32
+// columns gave 14.9 us at 1024 colloids, and positions off by 1e-6 in one step of ten.)
 constexpr int BB_ROWS = BB_TILE, BB_CT = 64;
 struct BbSmem { double4 sp[BB_CT]; double su[BB_CT * 11]; };
 
@@ -1046,7 +1046,7 @@ __global__ void k_combine(const Seg *__restrict__ segs, RedTable T, int mode, co
 // host launchers
 // Far-field blocks of the replicas with monomers: monomer-colloid and colloid-colloid
 // blocks first (E.n_far_pre of them), then the monomer tile pairs, in one launch per
-// pair-scalar family (they were three launches, two of them on a side stream: 6 us of
+// pair-scalar family (in launches of their own on a side stream, the first two kinds cost 6 us of
 // fork and join on an apply of 12 us).  Colloid-colloid FTS blocks stay FP64 in the mixed
 // form: near contact the far-field FTS mobility is ill-conditioned and FP32 blocks leave a
 // 1.2e-6 velocity error on a suspension at gap 0.01 (FP64: tracks rtol); they are cheap

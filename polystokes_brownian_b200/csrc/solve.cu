@@ -467,7 +467,7 @@ static void launch_ps_setup(Engine &E, cudaStream_t st)
 // depends on the replica alone.
 //
 // Bound: latency (a dependent launch with an L2 round trip, 3 to 4 us each).  A CG
-// iteration of a lubricated replica took 7 launches beside the applies, now 4: the
+// iteration of a lubricated replica took 7 launches beside the applies; 4 this way: the
 // direction, L^T, the update, and one gather for L z and for the residual test's L r
 // (u = L p is kept by its own recurrence L p = L z + beta L p).  Lubricated steps: 980
 // beads 5.50 -> 5.25 ms, 64 replicas of 62000 beads 22.8 -> 19.8 ms.
